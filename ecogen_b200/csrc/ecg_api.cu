@@ -58,14 +58,14 @@ __global__ void k_derived(const double* __restrict__ S, int64_t n, int np, int d
   for (int k = 0; k < np; k++) {
     a[k] = S[(int64_t)k * n + i];
     r[k] = S[(int64_t)(np + k) * n + i];
-    EosParams q{eos[k].type, eos[k].gamma, eos[k].pinf, eos[k].b, eos[k].cv, eos[k].eref, eos[k].sref};
+    const EosParams q = make_eos_params(eos[k]);
     pk[k] = eos_fix_p(q, p);
     rho += a[k] * r[k];
     pm += a[k] * pk[k];
   }
   if (pmix) pmix[i] = pm;
   for (int k = 0; k < np; k++) {
-    EosParams q{eos[k].type, eos[k].gamma, eos[k].pinf, eos[k].b, eos[k].cv, eos[k].eref, eos[k].sref};
+    const EosParams q = make_eos_params(eos[k]);
     if (T) T[(int64_t)k * n + i] = eos_T(q, eps, r[k], pk[k]);
     if (Y) Y[(int64_t)k * n + i] = a[k] * r[k] / dmax(rho, eps);
   }
@@ -95,7 +95,7 @@ __global__ void k_ptueq_derived(const double* __restrict__ S, int64_t n, ecg_eos
 __global__ void k_euler_derived(const double* __restrict__ S, int64_t n, ecg_eos e0, double eps, double* T) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  EosParams q{e0.type, e0.gamma, e0.pinf, e0.b, e0.cv, e0.eref, e0.sref};
+  const EosParams q = make_eos_params(e0);
   T[i] = eos_T(q, eps, S[i], S[n + i]);
 }
 

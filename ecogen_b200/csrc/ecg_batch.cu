@@ -130,16 +130,16 @@ __global__ void ECG_BATCH_BOUNDS(TB) k_batch(BatchParams B, Model<NP> M0) {
         double d = dsqrt(x * x);
 #pragma unroll
         for (int k = 0; k < NP; k++) {
-          ssl[k * SS + e] = ddiv(sq[(FL::A + k) * RS + rr] - sq[(FL::A + k) * RS + rl], d);
-          ssl[(NP + k) * SS + e] = ddiv(sq[(FL::R + k) * RS + rr] - sq[(FL::R + k) * RS + rl], d);
+          ssl[k * SS + e] = ndiv(sq[(FL::A + k) * RS + rr] - sq[(FL::A + k) * RS + rl], d);
+          ssl[(NP + k) * SS + e] = ndiv(sq[(FL::R + k) * RS + rr] - sq[(FL::R + k) * RS + rl], d);
           double pR = eos_fix_p(M.eos[k], sq[FL::P * RS + rr]), pL = eos_fix_p(M.eos[k], sq[FL::P * RS + rl]);
-          ssl[(2 * NP + k) * SS + e] = ddiv(pR - pL, d);
+          ssl[(2 * NP + k) * SS + e] = ndiv(pR - pL, d);
         }
-        ssl[(3 * NP) * SS + e] = ddiv(sq[FL::U * RS + rr] - sq[FL::U * RS + rl], d);
+        ssl[(3 * NP) * SS + e] = ndiv(sq[FL::U * RS + rr] - sq[FL::U * RS + rl], d);
       }
       __syncthreads();
     }
-    double dtmax = 1.e10;
+    double wmax = wave_none(false);
     for (int j = tid; j <= TC; j += TB) {
       int gl = org + j - 1;
       if (gl < 0 || gl + 1 >= n) continue;
@@ -167,7 +167,7 @@ __global__ void ECG_BATCH_BOUNDS(TB) k_batch(BatchParams B, Model<NP> M0) {
       }
       double Fn[3];
       Flux<NP> F;
-      hllc<NP>(M, tl, ug, tr, vg, C.lcfl, C.lcfl, dtmax, Fn, F);
+      hllc<NP>(M, tl, ug, tr, vg, false, C.lcfl, C.lcfl, wmax, Fn, F);
       F.mom[0] = Fn[0];
 #pragma unroll
       for (int k = 0; k < NP; k++) {
@@ -213,9 +213,9 @@ __global__ void ECG_BATCH_BOUNDS(TB) k_batch(BatchParams B, Model<NP> M0) {
         F.uStar = sfl[(3 * NP + 3) * FS + j];
         acc_face<NP, 1>(C.coefA, side == 0, F, an, pn, aa, am, ae, amom, aE);
       }
-      if (g == 0) boundary_face<NP, 1>(M, P.q, nn, cell, 0, true, C.lcfl, C.coefA, dtmax, an, pn, aa, am, ae, amom, aE);
+      if (g == 0) boundary_face<NP, 1>(M, P.q, nn, cell, 0, true, false, C.lcfl, C.coefA, wmax, an, pn, aa, am, ae, amom, aE);
       if (g == n - 1)
-        boundary_face<NP, 1>(M, P.q, nn, cell, 0, false, C.lcfl, C.coefA, dtmax, an, pn, aa, am, ae, amom, aE);
+        boundary_face<NP, 1>(M, P.q, nn, cell, 0, false, false, C.lcfl, C.coefA, wmax, an, pn, aa, am, ae, amom, aE);
       kapila_rebuild<NP, 1, PASS>(P, M, nn, cell, B.scal[c].dt, an, rn, pn, aa, am, ae, amom, aE, cp);
     }
     SeedGate<NP> sg;
@@ -236,17 +236,17 @@ __global__ void ECG_BATCH_BOUNDS(TB) k_batch(BatchParams B, Model<NP> M0) {
       total.nonfinite += cc.nonfinite;
       max_iters = max_iters > cc.iters ? max_iters : cc.iters;
     }
-    // ---- segmented min: this item's faces belong to case c only
-    double v = dtmax;
+    // ---- segmented reduction: this item's faces belong to case c only
+    double v = wmax;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
     if ((tid & 31) == 0) red[tid >> 5] = v;
     __syncthreads();
     if (tid < 32) {
-      v = (tid < TB / 32) ? red[tid] : 1.e10;
+      v = (tid < TB / 32) ? red[tid] : wave_none(false);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-      if (tid == 0) atomic_min_pos_double(&B.scal[c].dtmax_bits, v);
+      for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+      if (tid == 0) atomic_min_pos_double(&B.scal[c].dtmax_bits, wave_dtmax(v, false, C.lcfl));
     }
     __syncthreads();
   }

@@ -5,7 +5,7 @@
 // to the last bits except where a math function's result differs from glibc's by
 // an ulp (epow, ecg_pow.cuh: in about 0.1 % of the calls, where glibc's pow is
 // not correctly rounded; exp of the THINC reconstruction).  Divisions and square
-// roots go through ddiv / dsqrt (ecg_ieee.cuh), which return the IEEE quotient and
+// roots go through ndiv / dsqrt (ecg_ieee.cuh), which return the IEEE quotient and
 // root bit for bit without a branch.  Kernels are built with --fmad=false so that
 // no multiply-add is contracted, as in the reference's x86-64 SSE2 build.
 //
@@ -43,27 +43,27 @@ __device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b 
 // src/Eos/EosIG.cpp:64-257, src/Eos/EosSG.cpp:66-257, src/Eos/EosNASG.cpp:68-280
 
 __device__ __forceinline__ double eos_T(const EosParams& q, double eps, double rho, double p) {
-  if (q.type == ECG_EOS_IG) return ddiv(ddiv(ddiv(p, q.gamma - 1.), dmax(rho, eps)), q.cv);
-  if (q.type == ECG_EOS_SG) return ddiv(ddiv(ddiv(p + q.pinf, q.gamma - 1.), dmax(rho, eps)), q.cv);
-  return ddiv(ddiv(ddiv((p + q.pinf) * dmax(1. - rho * q.b, eps), q.gamma - 1.), q.cv), dmax(rho, eps));
+  if (q.type == ECG_EOS_IG) return ndiv(ndiv(cdiv(p, q.gm1, q.ig), dmax(rho, eps)), q.cv);
+  if (q.type == ECG_EOS_SG) return ndiv(ndiv(cdiv(p + q.pinf, q.gm1, q.ig), dmax(rho, eps)), q.cv);
+  return ndiv(ndiv(cdiv((p + q.pinf) * dmax(1. - rho * q.b, eps), q.gm1, q.ig), q.cv), dmax(rho, eps));
 }
 
 __device__ __forceinline__ double eos_e(const EosParams& q, double eps, double rho, double p) {
-  if (q.type == ECG_EOS_IG) return ddiv(ddiv(p, q.gamma - 1.), dmax(rho, eps)) + q.eref;
-  if (q.type == ECG_EOS_SG) return ddiv(ddiv(p + q.gamma * q.pinf, q.gamma - 1.), dmax(rho, eps)) + q.eref;
-  return ddiv(ddiv((p + q.gamma * q.pinf) * dmax(1. - rho * q.b, eps), q.gamma - 1.), dmax(rho, eps)) + q.eref;
+  if (q.type == ECG_EOS_IG) return ndiv(cdiv(p, q.gm1, q.ig), dmax(rho, eps)) + q.eref;
+  if (q.type == ECG_EOS_SG) return ndiv(cdiv(p + q.gpinf, q.gm1, q.ig), dmax(rho, eps)) + q.eref;
+  return ndiv(cdiv((p + q.gpinf) * dmax(1. - rho * q.b, eps), q.gm1, q.ig), dmax(rho, eps)) + q.eref;
 }
 
 __device__ __forceinline__ double eos_p(const EosParams& q, double eps, double rho, double e) {
-  if (q.type == ECG_EOS_IG) return (q.gamma - 1.) * rho * (e - q.eref);
-  if (q.type == ECG_EOS_SG) return (q.gamma - 1.) * rho * (e - q.eref) - q.gamma * q.pinf;
-  return (ddiv(rho * (q.gamma - 1.) * (e - q.eref), dmax(1. - rho * q.b, eps)) - q.gamma * q.pinf);
+  if (q.type == ECG_EOS_IG) return q.gm1 * rho * (e - q.eref);
+  if (q.type == ECG_EOS_SG) return q.gm1 * rho * (e - q.eref) - q.gpinf;
+  return (ndiv(rho * q.gm1 * (e - q.eref), dmax(1. - rho * q.b, eps)) - q.gpinf);
 }
 
 __device__ __forceinline__ double eos_c(const EosParams& q, double eps, double rho, double p) {
-  if (q.type == ECG_EOS_IG) return dsqrt(ddiv(q.gamma * p, dmax(rho, eps)));
-  if (q.type == ECG_EOS_SG) return dsqrt(ddiv(q.gamma * (p + q.pinf), dmax(rho, eps)));
-  return dsqrt(ddiv(q.gamma * (p + q.pinf), dmax(rho * (1. - rho * q.b), eps)));
+  if (q.type == ECG_EOS_IG) return dsqrt(ndiv(q.gamma * p, dmax(rho, eps)));
+  if (q.type == ECG_EOS_SG) return dsqrt(ndiv(q.gamma * (p + q.pinf), dmax(rho, eps)));
+  return dsqrt(ndiv(q.gamma * (p + q.pinf), dmax(rho * (1. - rho * q.b), eps)));
 }
 
 __device__ __forceinline__ double nonzero(double a, double eps) {  // Tools::returnNonZeroValue src/Tools.cpp:134
@@ -74,9 +74,9 @@ __device__ __forceinline__ double nonzero(double a, double eps) {  // Tools::ret
 
 __device__ __forceinline__ double eos_p_isentropic(const EosParams& q, double eps, double p0, double rho0,
                                                    double rho1) {
-  if (q.type == ECG_EOS_IG) return p0 * epow(ddiv(rho1, dmax(rho0, eps)), q.gamma);
-  if (q.type == ECG_EOS_SG) return (p0 + q.pinf) * epow(ddiv(rho1, dmax(rho0, eps)), q.gamma) - q.pinf;
-  return (p0 + q.pinf) * epow(ddiv(rho1, dmax(rho0, eps)), q.gamma) * epow(ddiv(1. - rho0 * q.b, 1. - rho1 * q.b), q.gamma) -
+  if (q.type == ECG_EOS_IG) return p0 * epow(ndiv(rho1, dmax(rho0, eps)), q.gamma);
+  if (q.type == ECG_EOS_SG) return (p0 + q.pinf) * epow(ndiv(rho1, dmax(rho0, eps)), q.gamma) - q.pinf;
+  return (p0 + q.pinf) * epow(ndiv(rho1, dmax(rho0, eps)), q.gamma) * epow(ndiv(1. - rho0 * q.b, 1. - rho1 * q.b), q.gamma) -
          q.pinf;
 }
 
@@ -86,33 +86,29 @@ __device__ __forceinline__ double eos_rho_pfinal(const EosParams& q, double eps,
   if (q.type == ECG_EOS_IG) {
     num = q.gamma * p1;
     denom = num + p0 - p1;
-    rho1 = ddiv(rho0 * num, dmax(denom, eps));
-    *drhodp = ddiv(rho0 * q.gamma * p0, dmax(denom * denom, eps));
+    rho1 = ndiv(rho0 * num, dmax(denom, eps));
+    *drhodp = ndiv(rho0 * q.gamma * p0, dmax(denom * denom, eps));
     return rho1;
   }
   if (q.type == ECG_EOS_SG) {
     num = q.gamma * (p1 + q.pinf);
     denom = num + p0 - p1;
-    rho1 = ddiv(rho0 * num, nonzero(denom, eps));
-    *drhodp = ddiv(rho0 * q.gamma * (p0 + q.pinf), dmax(denom * denom, eps));
+    rho1 = ndiv(rho0 * num, nonzero(denom, eps));
+    *drhodp = ndiv(rho0 * q.gamma * (p0 + q.pinf), dmax(denom * denom, eps));
     return rho1;
   }
   num = q.gamma * (p1 + q.pinf);
   denom = num + p0 - p1 + q.b * rho0 * (p1 - p0);
-  rho1 = ddiv(rho0 * num, nonzero(denom, eps));
-  *drhodp = ddiv(rho0 * q.gamma * (p0 + q.pinf - q.b * rho0 * (p0 + q.pinf)), nonzero(denom * denom, eps));
+  rho1 = ndiv(rho0 * num, nonzero(denom, eps));
+  *drhodp = ndiv(rho0 * q.gamma * (p0 + q.pinf - q.b * rho0 * (p0 + q.pinf)), nonzero(denom * denom, eps));
   return rho1;
 }
 
 // verifyAndModifyPressure (EosIG.cpp:250, EosSG.cpp:252, EosNASG.cpp:268)
-__device__ __forceinline__ double eos_fix_p(const EosParams& q, double p) {
-  if (q.type == ECG_EOS_IG) return (p < 1.e-8) ? 1.e-8 : p;
-  double floor = -(1. - 1.e-15) * q.pinf + 1.e-15;
-  return (p <= floor) ? floor : p;
-}
+__device__ __forceinline__ double eos_fix_p(const EosParams& q, double p) { return (p < q.pfloor) ? q.pfloor : p; }
 
 __device__ __forceinline__ void eos_rho_max(const EosParams& q, double& rho) {  // verifyAndCorrectDensityMax(density)
-  if (q.type == ECG_EOS_NASG && rho > ddiv(1., q.b) - 1.) rho = ddiv(1., q.b) - 1.;
+  if (q.type == ECG_EOS_NASG && rho > ndiv(1., q.b) - 1.) rho = ndiv(1., q.b) - 1.;
 }
 
 // ------------------------------------------------------------------------------ model parameters
@@ -185,7 +181,7 @@ __device__ __forceinline__ void fulfill(const Model<NP>& M, Thermo<NP>& t) {
   double cF = 0.;
 #pragma unroll
   for (int k = 0; k < NP; k++) {
-    t.Y[k] = ddiv(t.a[k] * t.r[k], dmax(t.rho, M.eps));
+    t.Y[k] = ndiv(t.a[k] * t.r[k], dmax(t.rho, M.eps));
     cF += t.Y[k] * c[k] * c[k];
   }
   t.cF = dsqrt(cF);
@@ -230,6 +226,21 @@ __device__ __forceinline__ void to_global(int axis, bool neg, const double f[3],
   }
 }
 
+// The time-step restriction of the faces a thread solves, min lCFL / |s| over the waves faster than 1e-3,
+// carried as a value to be maximised: the fastest |s| itself on a uniform mesh, where every cell has the
+// same lCFL and a correctly rounded quotient falls monotonically with its divisor, so that the minimum of
+// the quotients is the quotient by the maximum (one division per block in place of two per face); minus
+// the smallest lCFL / |s| on a stretched mesh.  A NaN speed is ignored, as in the minimum.
+__device__ __forceinline__ double wave_none(bool stretched) { return stretched ? -1.e10 : 0.; }
+__device__ __forceinline__ void wave_add(double& w, bool stretched, double s, double lcfl) {
+  if (!stretched) w = dmax(w, fabs(s));
+  else if (fabs(s) > 1.e-3) w = dmax(w, -ndiv(1. * lcfl, fabs(s)));
+}
+__device__ __forceinline__ double wave_dtmax(double w, bool stretched, double lcfl) {
+  if (stretched) return -w;
+  return (w > 1.e-3) ? dmin(1.e10, ndiv(1. * lcfl, w)) : 1.e10;
+}
+
 // Face flux of the Kapila / UEq system, in the absolute frame.
 template <int NP>
 struct Flux {
@@ -240,19 +251,19 @@ struct Flux {
 };
 
 // HLLC: ModUEq::solveRiemannIntern src/Models/UEq/ModUEq.cpp:113-267.  L and R carry local-frame
-// velocities ul/ur (normal first).  dtmax is min-updated with lCFL/|s|.
+// velocities ul/ur (normal first).  wmax collects the wave speeds (wave_add).
 template <int NP>
 __device__ ECG_HLLC_INLINE void hllc(const Model<NP>& M, const Thermo<NP>& L, const double ul[3],
-                                     const Thermo<NP>& R, const double ur[3], double dxL, double dxR,
-                                     double& dtmax, double Fn[3], Flux<NP>& F) {
+                                     const Thermo<NP>& R, const double ur[3], bool stretched, double dxL,
+                                     double dxR, double& wmax, double Fn[3], Flux<NP>& F) {
   double uL = ul[0], cL = L.cF, pL = L.pm, rhoL = L.rho;
   double uR = ur[0], cR = R.cF, pR = R.pm, rhoR = R.rho;
   double sL = dmin(uL - cL, uR - cR);
   double sR = dmax(uR + cR, uL + cL);
-  if (fabs(sL) > 1.e-3) dtmax = dmin(dtmax, ddiv(1. * dxL, fabs(sL)));
-  if (fabs(sR) > 1.e-3) dtmax = dmin(dtmax, ddiv(1. * dxR, fabs(sR)));
+  wave_add(wmax, stretched, sL, dxL);
+  wave_add(wmax, stretched, sR, dxR);
   double mL = rhoL * (sL - uL), mR = rhoR * (sR - uR);
-  double sM = ddiv(pR - pL + mL * uL - mR * uR, mL - mR);
+  double sM = ndiv(pR - pL + mL * uL - mR * uR, mL - mR);
   if (fabs(sM) < 1.e-8) sM = 0.;
   F.sM = sM;
   if (sL >= 0. || sR <= 0.) {
@@ -284,13 +295,13 @@ __device__ ECG_HLLC_INLINE void hllc(const Model<NP>& M, const Thermo<NP>& L, co
     double e[NP];
     const double em = side_energy<NP>(M, S, e);
     double Et = em + 0.5 * (us[0] * us[0] + us[1] * us[1] + us[2] * us[2]);
-    double rhoStar = ddiv(mK, sK - sM);
-    double EStar = Et + (sM - uK) * (sM + ddiv(pK, mK));
+    double rhoStar = ndiv(mK, sK - sM);
+    double EStar = Et + (sM - uK) * (sM + ndiv(pK, mK));
     double pStar = mK * (sM - uK) + pK;
 #pragma unroll
     for (int k = 0; k < NP; k++) {
       double mk = S.r[k] * (sK - uK);
-      double rks = ddiv(mk, sK - sM);
+      double rks = ndiv(mk, sK - sM);
       eos_rho_max(M.eos[k], rks);
       double pks = eos_p_isentropic(M.eos[k], M.eps, S.p[k], S.r[k], rks);
       double eks = eos_e(M.eos[k], M.eps, rks, pks);
@@ -319,13 +330,13 @@ __device__ __forceinline__ double limiter(int kind, double s1, double s2) {
       return slope;
     case ECG_LIM_VANLEER: {
       double sum = s1 + s2;
-      if ((fabs(sum) > 1e-6) && (prod > 1e-6)) slope = ddiv(2. * prod, sum);
+      if ((fabs(sum) > 1e-6) && (prod > 1e-6)) slope = ndiv(2. * prod, sum);
       return slope;
     }
     case ECG_LIM_VANALBADA: {
       double sum = s1 + s2;
       if ((fabs(s1) > 1e-6) && (fabs(s2) > 1e-6) && (fabs(sum) > 1e-6) && (prod > 1e-6))
-        slope = ddiv(prod * sum, s1 * s1 + s2 * s2);
+        slope = ndiv(prod * sum, s1 * s1 + s2 * s2);
       return slope;
     }
     case ECG_LIM_SUPERBEE:
@@ -391,7 +402,7 @@ __device__ __forceinline__ bool relax_pinf(const Model<NP>& M, double a[NP], dou
   int iteration = 0;
   do {
     iteration++;
-    ps -= ddiv(f, df);
+    ps -= ndiv(f, df);
 #pragma unroll
     for (int k = 0; k < NP; k++) ps = eos_fix_p(M.eos[k], ps);
     f = -1.;
@@ -399,8 +410,8 @@ __device__ __forceinline__ bool relax_pinf(const Model<NP>& M, double a[NP], dou
 #pragma unroll
     for (int k = 0; k < NP; k++) {
       rS[k] = eos_rho_pfinal(M.eos[k], M.eps, p[k], r[k], ps, &drhodp);
-      aS[k] = ddiv(a[k] * r[k], rS[k]);
-      double dalpha = ddiv(a[k] * r[k] * drhodp, rS[k] * rS[k]);
+      aS[k] = ndiv(a[k] * r[k], rS[k]);
+      double dalpha = ndiv(a[k] * r[k] * drhodp, rS[k] * rS[k]);
       f += aS[k];
       df -= dalpha;
     }
@@ -425,13 +436,13 @@ __device__ __forceinline__ bool relax_pinf(const Model<NP>& M, double a[NP], dou
       if (j != k) sumZj += zk[j];
     pI += sumZj * (p[k] - 0.);
   }
-  pI = ddiv(pI, sumZk * (NP - 1));
+  pI = ndiv(pI, sumZk * (NP - 1));
 #pragma unroll
   for (int k = 0; k < NP; k++) pI = eos_fix_p(M.eos[k], pI);
 #pragma unroll
   for (int k = 0; k < NP; k++) {
     double rr = eos_rho_pfinal(M.eos[k], M.eps, p[k], r[k], pI, &drhodp);
-    a[k] = ddiv(a[k] * r[k], rr);
+    a[k] = ndiv(a[k] * r[k], rr);
     r[k] = rr;
   }
   pstar = pI;
@@ -480,8 +491,8 @@ __device__ __forceinline__ void pinf_eval(const Model<NP>& M, const double a[NP]
 #pragma unroll
   for (int k = 0; k < NP; k++) {
     rS[k] = eos_rho_pfinal(M.eos[k], M.eps, p[k], r[k], s.ps, &drhodp);
-    aS[k] = ddiv(a[k] * r[k], rS[k]);
-    double dalpha = ddiv(a[k] * r[k] * drhodp, rS[k] * rS[k]);
+    aS[k] = ndiv(a[k] * r[k], rS[k]);
+    double dalpha = ndiv(a[k] * r[k] * drhodp, rS[k] * rS[k]);
     s.f += aS[k];
     s.df -= dalpha;
   }
@@ -506,7 +517,7 @@ __device__ __forceinline__ void pinf_finish(const Model<NP>& M, double a[NP], do
                                             int max_iter, bool accept = false) {
   while (fabs(s.f) > 1e-10 && s.it < max_iter) {
     s.it++;
-    s.ps -= ddiv(s.f, s.df);
+    s.ps -= ndiv(s.f, s.df);
     pinf_eval<NP>(M, a, r, s, p, aS, rS);
   }
   st.iters = s.it;
@@ -530,13 +541,13 @@ __device__ __forceinline__ void pinf_finish(const Model<NP>& M, double a[NP], do
       if (j != k) sumZj += zk[j];
     pI += sumZj * (p[k] - 0.);
   }
-  pI = ddiv(pI, sumZk * (NP - 1));
+  pI = ndiv(pI, sumZk * (NP - 1));
 #pragma unroll
   for (int k = 0; k < NP; k++) pI = eos_fix_p(M.eos[k], pI);
 #pragma unroll
   for (int k = 0; k < NP; k++) {
     double rr = eos_rho_pfinal(M.eos[k], M.eps, p[k], r[k], pI, &drhodp);
-    a[k] = ddiv(a[k] * r[k], rr);
+    a[k] = ndiv(a[k] * r[k], rr);
     r[k] = rr;
   }
   pstar = pI;
@@ -565,37 +576,37 @@ __device__ __forceinline__ double compute_tsat(const EosParams& L, const EosPara
                                                bool& err, PtmuCount* pc = nullptr, double T0 = -1.) {
   double gL = L.gamma, piL = (L.type == ECG_EOS_IG) ? 0. : L.pinf, cvL = L.cv, e0L = L.eref, s0L = L.sref;
   double gV = V.gamma, piV = (V.type == ECG_EOS_IG) ? 0. : V.pinf, cvV = V.cv, e0V = V.eref, s0V = V.sref;
-  double A = ddiv(gL * cvL - gV * cvV + s0V - s0L, gV * cvV - cvV);
-  double B = ddiv(e0L - e0V, gV * cvV - cvV);
-  double C = ddiv(gV * cvV - gL * cvL, gV * cvV - cvV);
-  double D = ddiv(gL * cvL - cvL, gV * cvV - cvV);
+  double A = ndiv(gL * cvL - gV * cvV + s0V - s0L, gV * cvV - cvV);
+  double B = ndiv(e0L - e0V, gV * cvV - cvV);
+  double C = ndiv(gV * cvV - gL * cvL, gV * cvV - cvV);
+  double D = ndiv(gL * cvL - cvL, gV * cvV - cvV);
   int iteration = 0;
-  bool seeded = T0 > 0. && T0 < ddiv(0.5 * B, C);
-  double Tsat = seeded ? T0 : ddiv(0.1 * B, C), f = 0., df = 1.;
+  bool seeded = T0 > 0. && T0 < ndiv(0.5 * B, C);
+  double Tsat = seeded ? T0 : ndiv(0.1 * B, C), f = 0., df = 1.;
   // ln(p + pInf) of both phases do not depend on the iterate: evaluated once per solve (the same
   // values enter the same sum, so f has the bits of the reference's per-iteration evaluation)
   const double lnV = elog(p + piV), lnL = elog(p + piL);
   do {
-    Tsat -= ddiv(f, df);
-    if (seeded && !(Tsat > 0. && Tsat < ddiv(B, C))) {  // a seeded iterate left the root's branch
+    Tsat -= ndiv(f, df);
+    if (seeded && !(Tsat > 0. && Tsat < ndiv(B, C))) {  // a seeded iterate left the root's branch
       seeded = false;
-      Tsat = ddiv(0.1 * B, C);
+      Tsat = ndiv(0.1 * B, C);
     }
     iteration++;
     if (iteration > 50) {
       err = true;
       break;
     }
-    f = A + ddiv(B, Tsat) + C * elog(Tsat) - lnV + D * lnL;
-    df = ddiv(C, Tsat) - ddiv(B, Tsat * Tsat);
+    f = A + ndiv(B, Tsat) + C * elog(Tsat) - lnV + D * lnL;
+    df = ndiv(C, Tsat) - ndiv(B, Tsat * Tsat);
   } while (fabs(f) > 1e-10);
   if (pc) {
     pc->tsat_calls++;
     pc->tsat_iters += (unsigned int)iteration;
     pc->tsat_max = max(pc->tsat_max, (unsigned int)iteration);
   }
-  double dfdp = ddiv(-1., p + piV) + ddiv(D, p + piL);
-  *dTsat = ddiv(-dfdp, df);
+  double dfdp = ndiv(-1., p + piV) + ndiv(D, p + piL);
+  *dTsat = ndiv(-dfdp, df);
   return Tsat;
 }
 
@@ -603,26 +614,26 @@ __device__ __forceinline__ double compute_tsat(const EosParams& L, const EosPara
 __device__ __forceinline__ double eos_rho_sat(const EosParams& q, double eps, double p, double Tsat, double dTsat,
                                               double* drhodp) {
   double pp = (q.type == ECG_EOS_IG) ? p : p + q.pinf;
-  double g1cvT = (q.gamma - 1.) * q.cv * Tsat;
+  double g1cvT = q.gm1 * q.cv * Tsat;
   double den = (q.type == ECG_EOS_NASG) ? g1cvT + q.b * (p + q.pinf) : g1cvT;
-  double d = (q.gamma - 1.) * q.cv * Tsat - pp * (q.gamma - 1.) * q.cv * dTsat;
-  *drhodp = ddiv(d, dmax(den * den, eps));
-  return ddiv(pp, dmax(den, eps));
+  double d = q.gm1 * q.cv * Tsat - pp * q.gm1 * q.cv * dTsat;
+  *drhodp = ndiv(d, dmax(den * den, eps));
+  return ndiv(pp, dmax(den, eps));
 }
 
 // computeDensityEnergySaturation (EosIG.cpp:184, EosSG.cpp:186, EosNASG.cpp:203)
 __device__ __forceinline__ double eos_rhoe_sat(const EosParams& q, double p, double rho, double drhodp,
                                                double* drhoedp) {
   if (q.type == ECG_EOS_IG) {
-    *drhoedp = ddiv(1., q.gamma - 1.) + drhodp * q.eref;
-    return ddiv(p, q.gamma - 1.) + rho * q.eref;
+    *drhoedp = q.ig + drhodp * q.eref;
+    return cdiv(p, q.gm1, q.ig) + rho * q.eref;
   }
   if (q.type == ECG_EOS_SG) {
-    *drhoedp = ddiv(1., q.gamma - 1.) + drhodp * q.eref;
-    return ddiv(p + q.gamma * q.pinf, q.gamma - 1.) + rho * q.eref;
+    *drhoedp = q.ig + drhodp * q.eref;
+    return cdiv(p + q.gpinf, q.gm1, q.ig) + rho * q.eref;
   }
-  *drhoedp = ddiv(1. - rho * q.b, q.gamma - 1.) + drhodp * (q.eref - ddiv(q.b * (p + q.gamma * q.pinf), q.gamma - 1.));
-  return ddiv((p + q.gamma * q.pinf) * (1. - rho * q.b), q.gamma - 1.) + rho * q.eref;
+  *drhoedp = cdiv(1. - rho * q.b, q.gm1, q.ig) + drhodp * (q.eref - cdiv(q.b * (p + q.gpinf), q.gm1, q.ig));
+  return cdiv((p + q.gpinf) * (1. - rho * q.b), q.gm1, q.ig) + rho * q.eref;
 }
 
 // RelaxationPTMu::relaxation src/Relaxations/RelaxationPTMu.cpp:73-200.  rhomix / emix are the
@@ -677,7 +688,7 @@ __device__ __forceinline__ bool relax_ptmu(const Model<NP>& M, int liq, int vap,
   double Tstart = T_seed;  // start of the next T_sat solve (seeded form)
   if (p_seed > 0.) pStar = p_seed;
   do {
-    pStar -= ddiv(f, df);
+    pStar -= ndiv(f, df);
     iteration++;
     if (iteration > 50) {
       err = true;
@@ -689,8 +700,8 @@ __device__ __forceinline__ bool relax_ptmu(const Model<NP>& M, int liq, int vap,
     if (T_seed > 0.) Tstart = Tsat;
     rhoLSat = eos_rho_sat(EL, M.eps, pStar, Tsat, dTsat, &drhoLSat);
     rhoVSat = eos_rho_sat(EV, M.eps, pStar, Tsat, dTsat, &drhoVSat);
-    aLSat = ddiv(rho - rhoVSat, rhoLSat - rhoVSat);
-    daLSat = ddiv(-drhoVSat * (rhoLSat - rhoVSat) - (rho - rhoVSat) * (drhoLSat - drhoVSat),
+    aLSat = ndiv(rho - rhoVSat, rhoLSat - rhoVSat);
+    daLSat = ndiv(-drhoVSat * (rhoLSat - rhoVSat) - (rho - rhoVSat) * (drhoLSat - drhoVSat),
                   (rhoLSat - rhoVSat) * (rhoLSat - rhoVSat));
     aVSat = 1. - aLSat;
     daVSat = -daLSat;
@@ -700,8 +711,8 @@ __device__ __forceinline__ bool relax_ptmu(const Model<NP>& M, int liq, int vap,
     rhoeVSat = eos_rhoe_sat(EV, pStar, rhoVSat, drhoVSat, &drhoeVSat);
     f -= (aLSat * rhoeLSat + aVSat * rhoeVSat);
     df -= (daLSat * rhoeLSat + aLSat * drhoeLSat + daVSat * rhoeVSat + aVSat * drhoeVSat);
-    f = ddiv(f, rhoe);
-    df = ddiv(df, rhoe);
+    f = ndiv(f, rhoe);
+    df = ndiv(df, rhoe);
   } while (fabs(f) > 1e-10);
   if (pc) {
     pc->solve = 1;
@@ -736,7 +747,7 @@ __device__ __forceinline__ double correction_pressure(const Model<NP>& M, const 
     pp -= a[k] * (gpi * (1. - r[k] * cov) + r[k] * q.eref);
     denom += a[k] * ig * (1. - r[k] * cov);
   }
-  return ddiv(pp, denom);
+  return ndiv(pp, denom);
 }
 
 }  // namespace ecg

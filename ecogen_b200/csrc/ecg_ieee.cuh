@@ -69,6 +69,40 @@ __device__ __forceinline__ double ddiv(double a, double b) {
   return (q1 == q1) ? q1 : q0;  // NaN only when an operand is zero, infinite or NaN
 }
 
+// a / b of the step kernels: ddiv with the Newton steps a quotient needs.  Two steps leave y at RN(1/b)
+// for all but one divisor in 1e8 (the second step's result before rounding is 1/b (1 - 2^-79), so y can
+// only fall one ulp short, and does when 1/b lies within 2^-26 ulp above a midpoint); the correction
+// RN(q + r y) multiplies an error of at most one ulp of y into a term of one ulp of q, so the quotient is
+// RN(a / b) unless a / b lies within 2^-51 ulp of a midpoint between doubles.  The residual is taken as
+// b q - a, which gives a zero quotient its sign for b > 0 without the copysign.
+// Why: the face kernels are bound by instruction issue and the FP64 pipe, and half their FP64 work is
+// division.  Measured with the EOS constants' divisions by cdiv and the wave speeds' divisions once per block
+// (wave_add), same bits in every field (one B200, step of mid-run states, CUDA events): 3D three-phase
+// 256^3 18.75 -> 16.41 ms (X faces 2.35 -> 2.00, Y faces 2.11 -> 1.78, cells 2.65 -> 2.47), 2D two-phase
+// 2048^2 2.47 -> 2.18 ms, p-T-mu 1024^2 1.64 -> 1.34, PTUEq 2048^2 2.31 -> 1.94, Euler 2048^2 1.30 -> 1.11,
+// 4096 tubes 4.35 -> 3.56.  Without the NaN select as well the same steps would take 8-12 % less; it stays:
+// an infinite state must give the reference's quotient.
+__device__ __forceinline__ double ndiv(double a, double b) {
+  const double y0 = rcp_approx(b);
+  double e = fma(-b, y0, 1.0);
+  double y = fma(y0, e, y0);
+  e = fma(-b, y, 1.0);
+  y = fma(y, e, y);
+  const double q = a * y;
+  const double r = fma(b, q, -a);
+  const double q1 = fma(-r, y, q);
+  return (q1 == q1) ? q1 : a * y0;  // NaN only when an operand is zero, infinite or NaN
+}
+
+// a / b for a divisor whose correctly rounded reciprocal y = RN(1/b) is at hand (EOS constants, computed on
+// the host): Markstein's correction alone.
+__device__ __forceinline__ double cdiv(double a, double b, double y) {
+  const double q = a * y;
+  const double r = fma(b, q, -a);
+  const double q1 = fma(-r, y, q);
+  return (q1 == q1) ? q1 : q;
+}
+
 // sqrt(x), correctly rounded (see above)
 __device__ __forceinline__ double dsqrt(double x) {
   const double y0 = rsqrt_approx(x);
@@ -81,8 +115,8 @@ __device__ __forceinline__ double dsqrt(double x) {
   h = fma(h, r, h);
   const double d = fma(-g, g, x);
   const double s = fma(d, h, g);
-  const bool normal = (x > 0.) && (x < __longlong_as_double(0x7ff0000000000000ll));
-  return normal ? s : ((x < 0.) ? __longlong_as_double(0x7ff8000000000000ll) : x);
+  // s is NaN exactly for zero, negative, infinite and NaN operands; of these +-0 and +inf are their own roots
+  return (s == s || x < 0.) ? s : x;
 }
 
 }  // namespace ecg

@@ -71,11 +71,11 @@ __device__ ECG_RECON_INLINE void reconstruct_side(const Model<NP>& M, const Step
     const double sg = (hi - lo > 0.) ? 1. : -1.;
     const double qmin = dmin(hi, lo);
     const double qmax = dmax(hi, lo) - qmin;
-    const double C = ddiv(alphaCell - qmin + 1.e-20, qmax + 1.e-20);
+    const double C = ndiv(alphaCell - qmin + 1.e-20, qmax + 1.e-20);
     const double B = exp(sg * beta * (2. * C - 1.));
-    const double A = ddiv(ddiv(B, P.thinc_cosh) - 1., P.thinc_tanh);
+    const double A = ndiv(ndiv(B, P.thinc_cosh) - 1., P.thinc_tanh);
     double na = right ? qmin + 0.5 * qmax * (1. + sg * A)
-                      : qmin + 0.5 * qmax * (1. + ddiv(sg * (P.thinc_tanh + A), 1. + A * P.thinc_tanh));
+                      : qmin + 0.5 * qmax * (1. + ndiv(sg * (P.thinc_tanh + A), 1. + A * P.thinc_tanh));
     if (na < eps) na = eps;
     if (na > 1. - eps) na = 1. - eps;
     t.a[0] = na;
@@ -145,7 +145,8 @@ __device__ __forceinline__ void acc_face(double cA, bool add, const Flux<NP>& F,
 // BoundCond::computeFlux src/BoundConds/BoundCond.cpp:61; the buffer cell is fulfilled first, :84).
 template <int NP, int DIM>
 __device__ __forceinline__ void boundary_face(const Model<NP>& M, const double* q, int64_t nn, int64_t cell, int ax,
-                                              bool neg, double lcfl, double coefA, double& dtmax, const double an[NP],
+                                              bool neg, bool stretched, double lcfl, double coefA, double& wmax,
+                                              const double an[NP],
                                               const double pn[NP], double aa[NP], double am[NP], double ae[NP],
                                               double amom[DIM], double& aE, double* sM_out = nullptr) {
   using FL = Fields<NP, DIM>;
@@ -163,7 +164,7 @@ __device__ __forceinline__ void boundary_face(const Model<NP>& M, const double* 
   fulfill<NP>(M, t);
   to_local(ax, neg, ug, ul);
   Flux<NP> F;
-  hllc<NP>(M, t, ul, t, ul, lcfl, lcfl, dtmax, Fn, F);
+  hllc<NP>(M, t, ul, t, ul, stretched, lcfl, lcfl, wmax, Fn, F);
   to_global(ax, neg, Fn, F.mom);
   acc_face<NP, DIM>(coefA, false, F, an, pn, aa, am, ae, amom, aE);
   if (sM_out) *sM_out = F.sM;
@@ -204,10 +205,11 @@ __device__ __forceinline__ void wall_side(const Model<NP>& M, const int lim[4], 
 // fulfilled buffer cell t with face-frame velocity ul.  Returns the normal momentum flux pStar; every other
 // flux component, sM and uStar are zero.
 template <int NP>
-__device__ __forceinline__ double wall_pstar(const Thermo<NP>& t, const double ul[3], double lcfl, double& dtmax) {
+__device__ __forceinline__ double wall_pstar(const Thermo<NP>& t, const double ul[3], bool stretched, double lcfl,
+                                             double& wmax) {
   const double uL = ul[0], cL = t.cF, pL = t.pm, rhoL = t.rho;
   const double sL = dmin(uL - cL, -uL - cL);
-  if (fabs(sL) > 1.e-3) dtmax = dmin(dtmax, ddiv(1. * lcfl, fabs(sL)));
+  wave_add(wmax, stretched, sL, lcfl);
   return rhoL * (uL - sL) * uL + pL;
 }
 
@@ -292,15 +294,15 @@ __device__ __forceinline__ void kapila_rebuild(const StepParams& P, const Model<
   double rhoMel = 0.;
 #pragma unroll
   for (int k = 0; k < NP; k++) {
-    aa[k] = ddiv(aa[k], un_sum);
+    aa[k] = ndiv(aa[k], un_sum);
     rhoMel += am[k];
     a[k] = aa[k];
-    r[k] = ddiv(am[k], dmax(aa[k], M.eps));
-    if (M.eos[k].type == ECG_EOS_NASG && r[k] > ddiv(1., M.eos[k].b) - 1.) {  // verifyAndCorrectDensityMax(mass)
-      r[k] = ddiv(1., M.eos[k].b) - 1.;
-      a[k] = ddiv(am[k], r[k]);
+    r[k] = ndiv(am[k], dmax(aa[k], M.eps));
+    if (M.eos[k].type == ECG_EOS_NASG && r[k] > ndiv(1., M.eos[k].b) - 1.) {  // verifyAndCorrectDensityMax(mass)
+      r[k] = ndiv(1., M.eos[k].b) - 1.;
+      a[k] = ndiv(am[k], r[k]);
     }
-    double ek = ddiv(ae[k], dmax(am[k], M.eps));
+    double ek = ndiv(ae[k], dmax(am[k], M.eps));
     pk[k] = eos_p(M.eos[k], M.eps, r[k], ek);
     phase_fix_ar(M.eps, a[k], r[k]);
     pk[k] = eos_fix_p(M.eos[k], pk[k]);
@@ -309,12 +311,12 @@ __device__ __forceinline__ void kapila_rebuild(const StepParams& P, const Model<
   double usq = 0.;
 #pragma unroll
   for (int d = 0; d < DIM; d++) {
-    u[d] = ddiv(amom[d], rhoMel);
+    u[d] = ndiv(amom[d], rhoMel);
     if (fabs(u[d]) < 1.e-8) u[d] = 0.;
     usq += u[d] * u[d];
   }
   cp.usq = usq;
-  cp.E = ddiv(aE, rhoMel);
+  cp.E = ndiv(aE, rhoMel);
   // mixture density (and internal energy for p-T-mu) of the rebuilt state
   double rhomix = 0.;
 #pragma unroll
@@ -345,7 +347,7 @@ __device__ __forceinline__ double rebuilt_emix(const Model<NP>& M, const double 
   double emix = 0.;
 #pragma unroll
   for (int k = 0; k < NP; k++) {
-    double Y = ddiv(a[k] * r[k], dmax(rhomix, M.eps));
+    double Y = ndiv(a[k] * r[k], dmax(rhomix, M.eps));
     emix += Y * eos_e(M.eos[k], M.eps, r[k], p[k]);
   }
   return emix;
@@ -411,21 +413,21 @@ __device__ __forceinline__ void relax_pt(const Model<NP>& M, double a[NP], doubl
   const double pInf1 = (E1.type == ECG_EOS_IG) ? 0. : E1.pinf, pInf2 = (E2.type == ECG_EOS_IG) ? 0. : E2.pinf;
   const double q = Y[0] * E1.eref + Y[1] * E2.eref;
   const double cvMel = Y[0] * E1.cv + Y[1] * E2.cv;
-  const double A1 = ddiv(Y[0] * (E1.gamma - 1.) * E1.cv, cvMel) * (rho0 * (emix - q) - pInf1);
-  const double A2 = ddiv(Y[1] * (E2.gamma - 1.) * E2.cv, cvMel) * (rho0 * (emix - q) - pInf2);
+  const double A1 = ndiv(Y[0] * (E1.gamma - 1.) * E1.cv, cvMel) * (rho0 * (emix - q) - pInf1);
+  const double A2 = ndiv(Y[1] * (E2.gamma - 1.) * E2.cv, cvMel) * (rho0 * (emix - q) - pInf2);
   const double pressure = 0.5 * (A1 + A2 - (pInf1 + pInf2)) +
                           dsqrt(0.25 * (A2 - A1 - (pInf2 - pInf1)) * (A2 - A1 - (pInf2 - pInf1)) + A1 * A2);
   double temperature = 0.;
-  temperature += ddiv(Y[0] * (E1.gamma - 1.) * E1.cv, pressure + pInf1);
-  temperature += ddiv(Y[1] * (E2.gamma - 1.) * E2.cv, pressure + pInf2);
-  temperature = ddiv(1., temperature * rho0);
+  temperature += ndiv(Y[0] * (E1.gamma - 1.) * E1.cv, pressure + pInf1);
+  temperature += ndiv(Y[1] * (E2.gamma - 1.) * E2.cv, pressure + pInf2);
+  temperature = ndiv(1., temperature * rho0);
   double rS[2], aS[2];
 #pragma unroll
   for (int k = 0; k < 2; k++) {
     const EosParams& E = M.eos[k];
     const double den = dmax((E.gamma - 1.) * E.cv * temperature, M.eps);
-    rS[k] = (E.type == ECG_EOS_IG) ? ddiv(pressure, den) : ddiv(pressure + E.pinf, den);
-    aS[k] = ddiv(a[k] * r[k], rS[k]);
+    rS[k] = (E.type == ECG_EOS_IG) ? ndiv(pressure, den) : ndiv(pressure + E.pinf, den);
+    aS[k] = ndiv(a[k] * r[k], rS[k]);
   }
 #pragma unroll
   for (int k = 0; k < 2; k++) {
@@ -521,7 +523,7 @@ __device__ __forceinline__ void kapila_finish(const StepParams& P, const Model<N
     double Y[NP], emix = 0.;
 #pragma unroll
     for (int k = 0; k < NP; k++) {
-      Y[k] = ddiv(a0[k] * r0[k], dmax(rhomix, M.eps));
+      Y[k] = ndiv(a0[k] * r0[k], dmax(rhomix, M.eps));
       emix += Y[k] * eos_e(M.eos[k], M.eps, r0[k], p0[k]);
     }
     relax_pt<NP>(M, a, r, pk, Y, emix, rhomix);

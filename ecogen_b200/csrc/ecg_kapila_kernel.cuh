@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(KapilaStep<NP, DIM, PASS, NTM>::NTH,
     for (int j = 0; j < NTM; j++)
       if (j < P.ntr) tn[j] = P.sn[(int64_t)(FL::NS + j) * nn + cell];
   }
-  double dtmax = 1.e10;
+  double wmax = wave_none(G.stretched);
   double wallp[DIM];  // normal momentum flux of the cell's symmetry sides, per axis
 #pragma unroll
   for (int d = 0; d < DIM; d++) wallp[d] = 0.;
@@ -150,23 +150,23 @@ __global__ void __launch_bounds__(KapilaStep<NP, DIM, PASS, NTM>::NTH,
 #pragma unroll
           for (int f = 0; f < FL::NSL + NTM; f++) ssl[f * SS + e] = 0.;
           const double wd = G.wslope[2 * ax + sd];
-          if (fabs(wd) > 1.e-8) ssl[(3 * NP + ax) * SS + e] = ddiv(sq[(FL::U + ax) * RS + (sd ? rl : rr)], wd);
+          if (fabs(wd) > 1.e-8) ssl[(3 * NP + ax) * SS + e] = ndiv(sq[(FL::U + ax) * RS + (sd ? rl : rr)], wd);
           continue;
         }
         double d = G.dcc[ax][gl];
 #pragma unroll
         for (int k = 0; k < NP; k++) {
-          ssl[k * SS + e] = ddiv(sq[(FL::A + k) * RS + rr] - sq[(FL::A + k) * RS + rl], d);
-          ssl[(NP + k) * SS + e] = ddiv(sq[(FL::R + k) * RS + rr] - sq[(FL::R + k) * RS + rl], d);
+          ssl[k * SS + e] = ndiv(sq[(FL::A + k) * RS + rr] - sq[(FL::A + k) * RS + rl], d);
+          ssl[(NP + k) * SS + e] = ndiv(sq[(FL::R + k) * RS + rr] - sq[(FL::R + k) * RS + rl], d);
           double pr = eos_fix_p(M.eos[k], sq[FL::P * RS + rr]), pl = eos_fix_p(M.eos[k], sq[FL::P * RS + rl]);
-          ssl[(2 * NP + k) * SS + e] = ddiv(pr - pl, d);
+          ssl[(2 * NP + k) * SS + e] = ndiv(pr - pl, d);
         }
 #pragma unroll
         for (int dd = 0; dd < DIM; dd++)
-          ssl[(3 * NP + dd) * SS + e] = ddiv(sq[(FL::U + dd) * RS + rr] - sq[(FL::U + dd) * RS + rl], d);
+          ssl[(3 * NP + dd) * SS + e] = ndiv(sq[(FL::U + dd) * RS + rr] - sq[(FL::U + dd) * RS + rl], d);
 #pragma unroll
         for (int j = 0; j < NTM; j++)  // Transport::computeSlopeTransport
-          if (j < P.ntr) ssl[(FL::NSL + j) * SS + e] = ddiv(str[j * RS + rr] - str[j * RS + rl], d);
+          if (j < P.ntr) ssl[(FL::NSL + j) * SS + e] = ndiv(str[j * RS + rr] - str[j * RS + rl], d);
       }
       __syncthreads();
     }
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(KapilaStep<NP, DIM, PASS, NTM>::NTH,
       gf[ax] = gl + 1;
       const double lR = cell_lcfl(G, gf[0], gf[1], gf[2]);
       Flux<NP> F;
-      hllc<NP>(M, tl, ul, tr, ur, lL, lR, dtmax, Fn, F);
+      hllc<NP>(M, tl, ul, tr, ur, G.stretched, lL, lR, wmax, Fn, F);
       to_global(ax, false, Fn, F.mom);
 #pragma unroll
       for (int k = 0; k < NP; k++) {
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(KapilaStep<NP, DIM, PASS, NTM>::NTH,
           cell_thermo<NP, DIM>(M, sq, RS, rc, t, ug);
         }
         to_local(ax, sd == 0, ug, ul);
-        wallp[ax] = wall_pstar<NP>(t, ul, cell_lcfl(G, gc[0], gc[1], gc[2]), dtmax);
+        wallp[ax] = wall_pstar<NP>(t, ul, G.stretched, cell_lcfl(G, gc[0], gc[1], gc[2]), wmax);
       }
     }
     __syncthreads();
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(KapilaStep<NP, DIM, PASS, NTM>::NTH,
       if (G.bc[bf] == ECG_BC_SYMMETRY)
         wall_acc<NP, DIM>(ax, neg, wallp[ax], cAb, an, pn, aa, am, ae, amom, aE);
       else
-        boundary_face<NP, DIM>(M, P.q, nn, cell, ax, neg, cell_lcfl(G, gc[0], gc[1], gc[2]), cAb, dtmax, an, pn, aa,
+        boundary_face<NP, DIM>(M, P.q, nn, cell, ax, neg, G.stretched, cell_lcfl(G, gc[0], gc[1], gc[2]), cAb, wmax, an, pn, aa,
                                am, ae, amom, aE, &sMb);
 #pragma unroll
       for (int t = 0; t < NTM; t++) {  // transports: T sM on a non-reflecting side, nothing on a symmetry side
@@ -358,16 +358,16 @@ __global__ void __launch_bounds__(KapilaStep<NP, DIM, PASS, NTM>::NTH,
 
   // ---- dtMax: block min, one atomic per block
   __shared__ double red[32];
-  double v = dtmax;
+  double v = wmax;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+  for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   if ((tid & 31) == 0) red[tid >> 5] = v;
   __syncthreads();
   if (tid < 32) {
-    v = (tid < K::NTH / 32) ? red[tid] : 1.e10;
+    v = (tid < K::NTH / 32) ? red[tid] : wave_none(G.stretched);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (tid == 0) atomic_min_pos_double(P.dtmax_bits, v);
+    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (tid == 0) atomic_min_pos_double(P.dtmax_bits, wave_dtmax(v, G.stretched, G.lcfl));
   }
 }
 

@@ -172,26 +172,26 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
 #pragma unroll
         for (int f = 0; f < FL::NSL; f++) ssl[f * SS + e] = 0.;
         const double wd = G.wslope[2 * AX + sd];
-        if (fabs(wd) > 1.e-8) ssl[(3 * NP + AX) * SS + e] = ddiv(sq[(FL::U + AX) * RS + (sd ? rl : rr)], wd);
+        if (fabs(wd) > 1.e-8) ssl[(3 * NP + AX) * SS + e] = ndiv(sq[(FL::U + AX) * RS + (sd ? rl : rr)], wd);
         continue;
       }
       const double d = G.dcc[AX][gl];
 #pragma unroll
       for (int k = 0; k < NP; k++) {
-        ssl[k * SS + e] = ddiv(sq[(FL::A + k) * RS + rr] - sq[(FL::A + k) * RS + rl], d);
-        ssl[(NP + k) * SS + e] = ddiv(sq[(FL::R + k) * RS + rr] - sq[(FL::R + k) * RS + rl], d);
+        ssl[k * SS + e] = ndiv(sq[(FL::A + k) * RS + rr] - sq[(FL::A + k) * RS + rl], d);
+        ssl[(NP + k) * SS + e] = ndiv(sq[(FL::R + k) * RS + rr] - sq[(FL::R + k) * RS + rl], d);
         double pr = eos_fix_p(M.eos[k], sq[FL::P * RS + rr]), pl = eos_fix_p(M.eos[k], sq[FL::P * RS + rl]);
-        ssl[(2 * NP + k) * SS + e] = ddiv(pr - pl, d);
+        ssl[(2 * NP + k) * SS + e] = ndiv(pr - pl, d);
       }
 #pragma unroll
       for (int dd = 0; dd < DIM; dd++)
-        ssl[(3 * NP + dd) * SS + e] = ddiv(sq[(FL::U + dd) * RS + rr] - sq[(FL::U + dd) * RS + rl], d);
+        ssl[(3 * NP + dd) * SS + e] = ndiv(sq[(FL::U + dd) * RS + rr] - sq[(FL::U + dd) * RS + rl], d);
     }
     __syncthreads();
   }
 
   // ---- one face per thread
-  double dtmax = 1.e10;
+  double wmax = wave_none(G.stretched);
   {
     const int line = AX == 0 ? tid / FT::TF : tid % FT::W, fl = AX == 0 ? tid % FT::TF : tid / FT::W;
     const int f = f0 + fl;
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
             cell_thermo<NP, DIM>(M, sq, RS, rc, t, ug);
           }
           to_local(AX, neg, ug, ul);
-          const double pstar = wall_pstar<NP>(t, ul, lc, dtmax);
+          const double pstar = wall_pstar<NP>(t, ul, G.stretched, lc, wmax);
 #pragma unroll
           for (int k = 0; k < NP; k++) F.a[k] = F.m[k] = F.en[k] = 0.;
           F.E = 0.;
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
         } else {
           cell_thermo<NP, DIM>(M, sq, RS, rc, t, ug);
           to_local(AX, neg, ug, ul);
-          hllc<NP>(M, t, ul, t, ul, lc, lc, dtmax, Fn, F);
+          hllc<NP>(M, t, ul, t, ul, G.stretched, lc, lc, wmax, Fn, F);
         }
         to_global(AX, neg, Fn, F.mom);
       } else {
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
         const double lL = cell_lcfl(G, gf[0], gf[1], gf[2]);
         gf[AX] = gl + 1;
         const double lR = cell_lcfl(G, gf[0], gf[1], gf[2]);
-        hllc<NP>(M, tl, ul, tr, ur, lL, lR, dtmax, Fn, F);
+        hllc<NP>(M, tl, ul, tr, ur, G.stretched, lL, lR, wmax, Fn, F);
         to_global(AX, false, Fn, F.mom);
       }
       const int64_t nfa = split_nfaces(G.n, AX);
@@ -297,18 +297,18 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
     }
   }
 
-  // ---- dtMax: block min, one atomic per block
+  // ---- dtMax: block reduction of the wave speeds, one atomic per block
   __shared__ double red[32];
-  double v = dtmax;
+  double v = wmax;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+  for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   if ((tid & 31) == 0) red[tid >> 5] = v;
   __syncthreads();
   if (tid < 32) {
-    v = (tid < FT::NTH / 32) ? red[tid] : 1.e10;
+    v = (tid < FT::NTH / 32) ? red[tid] : wave_none(G.stretched);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (tid == 0) atomic_min_pos_double(P.dtmax_bits, v);
+    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (tid == 0) atomic_min_pos_double(P.dtmax_bits, wave_dtmax(v, G.stretched, G.lcfl));
   }
 }
 

@@ -55,16 +55,16 @@ __device__ __forceinline__ void euler_complete(const EosParams& q, double eps, E
 
 // ModEuler::solveRiemannIntern src/Models/Euler/ModEuler.cpp:105-225 (strict sL > 0 / sR < 0).
 __device__ __forceinline__ void hllc_euler(const EulerSide& L, const double ul[3], const EulerSide& R,
-                                           const double ur[3], double dxL, double dxR, double& dtmax, double& Fm,
+                                           const double ur[3], bool stretched, double dxL, double dxR, double& wmax, double& Fm,
                                            double Fn[3], double& FE, double* sM_out = nullptr) {
   double uL = ul[0], vL = ul[1], wL = ul[2], pL = L.p, rhoL = L.rho, cL = L.c, EL = L.E;
   double uR = ur[0], vR = ur[1], wR = ur[2], pR = R.p, rhoR = R.rho, cR = R.c, ER = R.E;
   double sL = dmin(uL - cL, uR - cR);
   double sR = dmax(uR + cR, uL + cL);
-  if (fabs(sL) > 1.e-3) dtmax = dmin(dtmax, ddiv(1. * dxL, fabs(sL)));
-  if (fabs(sR) > 1.e-3) dtmax = dmin(dtmax, ddiv(1. * dxR, fabs(sR)));
+  wave_add(wmax, stretched, sL, dxL);
+  wave_add(wmax, stretched, sR, dxR);
   double mL = rhoL * (sL - uL), mR = rhoR * (sR - uR);
-  double sM = ddiv(pR - pL + mL * uL - mR * uR, mL - mR);
+  double sM = ndiv(pR - pL + mL * uL - mR * uR, mL - mR);
   if (fabs(sM) < 1.e-8) sM = 0.;
   if (sM_out) *sM_out = sM;
   if (sL > 0.) {
@@ -81,8 +81,8 @@ __device__ __forceinline__ void hllc_euler(const EulerSide& L, const double ul[3
     FE = (rhoR * ER + pR) * uR;
   } else if (sM >= 0.) {
     double pStar = mL * (sM - uL) + pL;
-    double rhoStar = ddiv(mL, sL - sM);
-    double Estar = EL + (sM - uL) * (sM + ddiv(pL, mL));
+    double rhoStar = ndiv(mL, sL - sM);
+    double Estar = EL + (sM - uL) * (sM + ndiv(pL, mL));
     Fm = rhoStar * sM;
     Fn[0] = rhoStar * sM * sM + pStar;
     Fn[1] = rhoStar * sM * vL;
@@ -90,8 +90,8 @@ __device__ __forceinline__ void hllc_euler(const EulerSide& L, const double ul[3
     FE = (rhoStar * Estar + pStar) * sM;
   } else {
     double pStar = mR * (sM - uR) + pR;
-    double rhoStar = ddiv(mR, sR - sM);
-    double Estar = ER + (sM - uR) * (sM + ddiv(pR, mR));
+    double rhoStar = ndiv(mR, sR - sM);
+    double Estar = ER + (sM - uR) * (sM + ndiv(pR, mR));
     Fm = rhoStar * sM;
     Fn[0] = rhoStar * sM * sM + pStar;
     Fn[1] = rhoStar * sM * vR;
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(EulerStep<DIM, PASS, NTM>::NTH,
     for (int t = 0; t < NTM; t++)
       if (t < P.ntr) tn[t] = P.sn[(int64_t)(NS + t) * nn + cell];
   }
-  double dtmax = 1.e10;
+  double wmax = wave_none(G.stretched);
   double wallp[DIM];  // normal momentum flux of the cell's symmetry sides, per axis
 #pragma unroll
   for (int d = 0; d < DIM; d++) wallp[d] = 0.;
@@ -185,15 +185,15 @@ __global__ void __launch_bounds__(EulerStep<DIM, PASS, NTM>::NTH,
 #pragma unroll
           for (int f = 0; f < K::NSL + NTM; f++) ssl[f * SS + e] = 0.;
           const double wd = G.wslope[2 * ax + sd];
-          if (fabs(wd) > 1.e-8) ssl[(2 + ax) * SS + e] = ddiv(sq[(2 + ax) * RS + (sd ? rl : rr)], wd);
+          if (fabs(wd) > 1.e-8) ssl[(2 + ax) * SS + e] = ndiv(sq[(2 + ax) * RS + (sd ? rl : rr)], wd);
           continue;
         }
         double d = G.dcc[ax][gl];
 #pragma unroll
-        for (int f = 0; f < K::NSL; f++) ssl[f * SS + e] = ddiv(sq[f * RS + rr] - sq[f * RS + rl], d);
+        for (int f = 0; f < K::NSL; f++) ssl[f * SS + e] = ndiv(sq[f * RS + rr] - sq[f * RS + rl], d);
 #pragma unroll
         for (int t = 0; t < NTM; t++)  // Transport::computeSlopeTransport
-          if (t < P.ntr) ssl[(K::NSL + t) * SS + e] = ddiv(str[t * RS + rr] - str[t * RS + rl], d);
+          if (t < P.ntr) ssl[(K::NSL + t) * SS + e] = ndiv(str[t * RS + rr] - str[t * RS + rl], d);
       }
       __syncthreads();
     }
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(EulerStep<DIM, PASS, NTM>::NTH,
       const double lL = cell_lcfl(G, gf[0], gf[1], gf[2]);
       gf[ax] = gl + 1;
       const double lR = cell_lcfl(G, gf[0], gf[1], gf[2]);
-      hllc_euler(L, ul, R, ur, lL, lR, dtmax, Fm, Fn, FE, &sM);
+      hllc_euler(L, ul, R, ur, G.stretched, lL, lR, wmax, Fm, Fn, FE, &sM);
       to_global(ax, false, Fn, Fg);
       sfl[0 * FS + e] = Fm;
 #pragma unroll
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(EulerStep<DIM, PASS, NTM>::NTH,
         // ModEuler::solveRiemannWall src/Models/Euler/ModEuler.cpp:368-409
         const double uL = ul[0], cL = S.c, pL = S.p, rhoL = S.rho;
         const double sL = dmin(uL - cL, -uL - cL);
-        if (fabs(sL) > 1.e-3) dtmax = dmin(dtmax, ddiv(1. * cell_lcfl(G, gc[0], gc[1], gc[2]), fabs(sL)));
+        wave_add(wmax, G.stretched, sL, cell_lcfl(G, gc[0], gc[1], gc[2]));
         wallp[ax] = rhoL * uL * (uL - sL) + pL;
       }
     }
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(EulerStep<DIM, PASS, NTM>::NTH,
       to_local(ax, neg, S.u, ul);
       double sMb = 0.;
       const double lc = cell_lcfl(G, gc[0], gc[1], gc[2]);
-      hllc_euler(S, ul, S, ul, lc, lc, dtmax, Fm, Fn, FE, &sMb);
+      hllc_euler(S, ul, S, ul, G.stretched, lc, lc, wmax, Fm, Fn, FE, &sMb);
       to_global(ax, neg, Fn, Fg);
       const double cA = cell_coefA(G, ax, gc[0], gc[1], gc[2]);
       am -= cA * Fm;
@@ -406,11 +406,11 @@ __global__ void __launch_bounds__(EulerStep<DIM, PASS, NTM>::NTH,
     aE = aE * scale + 1. * (rn * En);
 #pragma unroll
     for (int d = 0; d < DIM; d++) {
-      u[d] = ddiv(amom[d], am);
+      u[d] = ndiv(amom[d], am);
       if (fabs(u[d]) < 1.e-8) u[d] = 0.;
       usq += u[d] * u[d];
     }
-    double E = ddiv(aE, am);
+    double E = ndiv(aE, am);
     double e = E - 0.5 * usq;
     double p = eos_p(q, eps, am, e);
     P.out[cell] = am;
@@ -423,16 +423,16 @@ __global__ void __launch_bounds__(EulerStep<DIM, PASS, NTM>::NTH,
       if (t < P.ntr) P.out[(int64_t)(NS + t) * nn + cell] = tn[t] + at[t] * scale;
   }
   __shared__ double red[32];
-  double v = dtmax;
+  double v = wmax;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+  for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   if ((tid & 31) == 0) red[tid >> 5] = v;
   __syncthreads();
   if (tid < 32) {
-    v = (tid < K::NTH / 32) ? red[tid] : 1.e10;
+    v = (tid < K::NTH / 32) ? red[tid] : wave_none(G.stretched);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (tid == 0) atomic_min_pos_double(P.dtmax_bits, v);
+    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (tid == 0) atomic_min_pos_double(P.dtmax_bits, wave_dtmax(v, G.stretched, G.lcfl));
   }
 }
 
@@ -444,7 +444,7 @@ static cudaError_t euler_one(const StepParams& P, const Geometry& G, const ecg_e
   auto kern = k_euler_step<DIM, PASS, NTM>;
   const size_t sm = K::smem_bytes();
   if (prepare) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  EosParams q{eos[0].type, eos[0].gamma, eos[0].pinf, eos[0].b, eos[0].cv, eos[0].eref, eos[0].sref};
+  const EosParams q = make_eos_params(eos[0]);
   dim3 grid((G.n[0] + TS::X - 1) / TS::X, (G.n[1] + TS::Y - 1) / TS::Y, (G.n[2] + TS::Z - 1) / TS::Z);
   kern<<<grid, K::NTH, sm, s>>>(P, G, q, eps);
   return cudaGetLastError();

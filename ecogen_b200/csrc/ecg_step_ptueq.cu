@@ -55,8 +55,8 @@ __device__ __forceinline__ double pt_pinf(const EosParams& q) { return q.type ==
 
 // computeDensity(p, T) of an IG or SG phase (EosIG.cpp:85, EosSG.cpp:87).
 __device__ __forceinline__ double pt_rho(const EosParams& q, double p, double T) {
-  const double den = dmax(((q.gamma - 1.) * q.cv * T), 0.);
-  return q.type == ECG_EOS_IG ? ddiv(p, den) : ddiv(p + q.pinf, den);
+  const double den = dmax((q.gm1 * q.cv * T), 0.);
+  return q.type == ECG_EOS_IG ? ndiv(p, den) : ndiv(p + q.pinf, den);
 }
 
 // One side of a face (or a cell) with its derived quantities.
@@ -80,7 +80,7 @@ __device__ __forceinline__ void pt_complete(const PtEos& M, PtSide& s) {
   for (int k = 0; k < 2; k++) s.rho += s.a[k] * s.r[k];
   double Y[2];
 #pragma unroll
-  for (int k = 0; k < 2; k++) Y[k] = ddiv(s.a[k] * s.r[k], s.rho);
+  for (int k = 0; k < 2; k++) Y[k] = ndiv(s.a[k] * s.r[k], s.rho);
   s.e = 0.;
   s.c = 0.;
 #pragma unroll
@@ -94,16 +94,16 @@ __device__ __forceinline__ void pt_complete(const PtEos& M, PtSide& s) {
 // ModPTUEq::solveRiemannIntern src/Models/PTUEq/ModPTUEq.cpp:113-227 on face-frame velocities;
 // the total energy uses the face-frame squared norm, as the reference's projected buffer cells do.
 __device__ __forceinline__ void hllc_pt(const PtSide& L, const double ul[3], const PtSide& R, const double ur[3],
-                                        double dxL, double dxR, double& dtmax, double Fm[2], double Fn[3],
+                                        bool stretched, double dxL, double dxR, double& wmax, double Fm[2], double Fn[3],
                                         double& FE) {
   const double uL = ul[0], cL = L.c, pL = L.p, rhoL = L.rho;
   const double uR = ur[0], cR = R.c, pR = R.p, rhoR = R.rho;
   const double sL = dmin(uL - cL, uR - cR);
   const double sR = dmax(uR + cR, uL + cL);
-  if (fabs(sL) > 1.e-3) dtmax = dmin(dtmax, ddiv(dxL, fabs(sL)));
-  if (fabs(sR) > 1.e-3) dtmax = dmin(dtmax, ddiv(dxR, fabs(sR)));
+  wave_add(wmax, stretched, sL, dxL);
+  wave_add(wmax, stretched, sR, dxR);
   const double mL = rhoL * (sL - uL), mR = rhoR * (sR - uR);
-  double sM = ddiv(pR - pL + mL * uL - mR * uR, mL - mR);
+  double sM = ndiv(pR - pL + mL * uL - mR * uR, mL - mR);
   if (fabs(sM) < 1.e-8) sM = 0.;
   if (sL >= 0.) {
 #pragma unroll
@@ -123,22 +123,22 @@ __device__ __forceinline__ void hllc_pt(const PtSide& L, const double ul[3], con
     FE = (rhoR * Et + pR) * uR;
   } else if (sM >= 0.) {
     const double Et = L.e + 0.5 * (ul[0] * ul[0] + ul[1] * ul[1] + ul[2] * ul[2]);
-    const double rhoStar = ddiv(mL, sL - sM);
-    const double EStar = Et + (sM - uL) * (sM + ddiv(pL, mL));
+    const double rhoStar = ndiv(mL, sL - sM);
+    const double EStar = Et + (sM - uL) * (sM + ndiv(pL, mL));
     const double pStar = mL * (sM - uL) + pL;
 #pragma unroll
-    for (int k = 0; k < 2; k++) Fm[k] = ddiv(L.a[k] * L.r[k] * (sL - uL), sL - sM) * sM;
+    for (int k = 0; k < 2; k++) Fm[k] = ndiv(L.a[k] * L.r[k] * (sL - uL), sL - sM) * sM;
     Fn[0] = rhoStar * sM * sM + pStar;
     Fn[1] = rhoStar * ul[1] * sM;
     Fn[2] = rhoStar * ul[2] * sM;
     FE = (rhoStar * EStar + pStar) * sM;
   } else {
     const double Et = R.e + 0.5 * (ur[0] * ur[0] + ur[1] * ur[1] + ur[2] * ur[2]);
-    const double rhoStar = ddiv(mR, sR - sM);
-    const double EStar = Et + (sM - uR) * (sM + ddiv(pR, mR));
+    const double rhoStar = ndiv(mR, sR - sM);
+    const double EStar = Et + (sM - uR) * (sM + ndiv(pR, mR));
     const double pStar = mR * (sM - uR) + pR;
 #pragma unroll
-    for (int k = 0; k < 2; k++) Fm[k] = ddiv(R.a[k] * R.r[k] * (sR - uR), sR - sM) * sM;
+    for (int k = 0; k < 2; k++) Fm[k] = ndiv(R.a[k] * R.r[k] * (sR - uR), sR - sM) * sM;
     Fn[0] = rhoStar * sM * sM + pStar;
     Fn[1] = rhoStar * ur[1] * sM;
     Fn[2] = rhoStar * ur[2] * sM;
@@ -186,7 +186,7 @@ __global__ void ECG_PTUEQ_BOUNDS(DIM, PASS) k_ptueq_step(StepParams P, Geometry 
   double am[2] = {0., 0.}, amom[DIM], aE = 0.;
 #pragma unroll
   for (int d = 0; d < DIM; d++) amom[d] = 0.;
-  double dtmax = 1.e10;
+  double wmax = wave_none(G.stretched);
 
 #pragma unroll
   for (int ax = 0; ax < DIM; ax++) {
@@ -219,7 +219,7 @@ __global__ void ECG_PTUEQ_BOUNDS(DIM, PASS) k_ptueq_step(StepParams P, Geometry 
         int rl = line * RL + (j - 1 + K::H), rr = rl + 1;
         double d = G.dcc[ax][gl];
 #pragma unroll
-        for (int f = 0; f < K::NSL; f++) ssl[f * SS + e] = ddiv(sq[f * RS + rr] - sq[f * RS + rl], d);
+        for (int f = 0; f < K::NSL; f++) ssl[f * SS + e] = ndiv(sq[f * RS + rr] - sq[f * RS + rl], d);
       }
       __syncthreads();
     }
@@ -282,11 +282,11 @@ __global__ void ECG_PTUEQ_BOUNDS(DIM, PASS) k_ptueq_step(StepParams P, Geometry 
             const double sg = (hi - lo > 0.) ? 1. : -1.;
             const double qmin = dmin(hi, lo);
             const double qmax = dmax(hi, lo) - qmin;
-            const double C = ddiv(aCell - qmin + 1.e-20, qmax + 1.e-20);
+            const double C = ndiv(aCell - qmin + 1.e-20, qmax + 1.e-20);
             const double B = exp(sg * beta * (2. * C - 1.));
-            const double A = ddiv(ddiv(B, P.thinc_cosh) - 1., P.thinc_tanh);
+            const double A = ndiv(ndiv(B, P.thinc_cosh) - 1., P.thinc_tanh);
             double na = right ? qmin + 0.5 * qmax * (1. + sg * A)
-                              : qmin + 0.5 * qmax * (1. + ddiv(sg * (P.thinc_tanh + A), 1. + A * P.thinc_tanh));
+                              : qmin + 0.5 * qmax * (1. + ndiv(sg * (P.thinc_tanh + A), 1. + A * P.thinc_tanh));
             if (na < eps) na = eps;
             if (na > 1. - eps) na = 1. - eps;
             s.a[0] = na;
@@ -306,7 +306,7 @@ __global__ void ECG_PTUEQ_BOUNDS(DIM, PASS) k_ptueq_step(StepParams P, Geometry 
       const double lL = cell_lcfl(G, gf[0], gf[1], gf[2]);
       gf[ax] = gl + 1;
       const double lR = cell_lcfl(G, gf[0], gf[1], gf[2]);
-      hllc_pt(S[0], ul, S[1], ur, lL, lR, dtmax, Fm, Fn, FE);
+      hllc_pt(S[0], ul, S[1], ur, G.stretched, lL, lR, wmax, Fm, Fn, FE);
       to_global(ax, false, Fn, Fg);
       sfl[0 * FS + e] = Fm[0];
       sfl[1 * FS + e] = Fm[1];
@@ -370,7 +370,7 @@ __global__ void ECG_PTUEQ_BOUNDS(DIM, PASS) k_ptueq_step(StepParams P, Geometry 
         // ModPTUEq::solveRiemannWall src/Models/PTUEq/ModPTUEq.cpp:233-265 (first order only)
         const double uL = ul[0];
         const double sL = dmin(uL - s.c, -uL - s.c);
-        if (fabs(sL) > 1.e-3) dtmax = dmin(dtmax, ddiv(lc, fabs(sL)));
+        wave_add(wmax, G.stretched, sL, lc);
         Fn[0] = s.rho * (uL - sL) * uL + s.p;
         Fn[1] = Fn[2] = 0.;
         to_global(ax, neg, Fn, Fg);
@@ -379,7 +379,7 @@ __global__ void ECG_PTUEQ_BOUNDS(DIM, PASS) k_ptueq_step(StepParams P, Geometry 
         continue;
       }
       double Fm[2], FE;
-      hllc_pt(s, ul, s, ul, lc, lc, dtmax, Fm, Fn, FE);
+      hllc_pt(s, ul, s, ul, G.stretched, lc, lc, wmax, Fm, Fn, FE);
       to_global(ax, neg, Fn, Fg);
       am[0] -= cA * Fm[0];
       am[1] -= cA * Fm[1];
@@ -415,43 +415,43 @@ __global__ void ECG_PTUEQ_BOUNDS(DIM, PASS) k_ptueq_step(StepParams P, Geometry 
     double u[3] = {0., 0., 0.};
 #pragma unroll
     for (int d = 0; d < DIM; d++) {
-      u[d] = ddiv(mom[d], rhoMel);
+      u[d] = ndiv(mom[d], rhoMel);
       if (fabs(u[d]) < 1.e-8) u[d] = 0.;
     }
-    const double ie = ddiv(rE, rhoMel) - 0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+    const double ie = ndiv(rE, rhoMel) - 0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
     const EosParams& E1 = M.e[0];
     const EosParams& E2 = M.e[1];
     const double pInf1 = pt_pinf(E1), pInf2 = pt_pinf(E2);
-    const double Y1 = ddiv(m[0], rhoMel), Y2 = ddiv(m[1], rhoMel);
+    const double Y1 = ndiv(m[0], rhoMel), Y2 = ndiv(m[1], rhoMel);
     const double q = Y1 * E1.eref + Y2 * E2.eref;
     const double cvMel = Y1 * E1.cv + Y2 * E2.cv;
-    const double A1 = ddiv(Y1 * (E1.gamma - 1.) * E1.cv, cvMel) * (rhoMel * (ie - q) - pInf1);
-    const double A2 = ddiv(Y2 * (E2.gamma - 1.) * E2.cv, cvMel) * (rhoMel * (ie - q) - pInf2);
+    const double A1 = ndiv(Y1 * (E1.gamma - 1.) * E1.cv, cvMel) * (rhoMel * (ie - q) - pInf1);
+    const double A2 = ndiv(Y2 * (E2.gamma - 1.) * E2.cv, cvMel) * (rhoMel * (ie - q) - pInf2);
     const double p = 0.5 * (A1 + A2 - (pInf1 + pInf2)) +
                      dsqrt(0.25 * (A2 - A1 - (pInf2 - pInf1)) * (A2 - A1 - (pInf2 - pInf1)) + A1 * A2);
     double Tm = 0.;
-    Tm += ddiv(ddiv(m[0], rhoMel) * (E1.gamma - 1.) * E1.cv, p + pInf1);
-    Tm += ddiv(ddiv(m[1], rhoMel) * (E2.gamma - 1.) * E2.cv, p + pInf2);
-    Tm = ddiv(1., Tm * rhoMel);
-    P.out[cell] = ddiv(m[0], pt_rho(E1, p, Tm));
-    P.out[nn + cell] = ddiv(m[1], pt_rho(E2, p, Tm));
+    Tm += ndiv(ndiv(m[0], rhoMel) * (E1.gamma - 1.) * E1.cv, p + pInf1);
+    Tm += ndiv(ndiv(m[1], rhoMel) * (E2.gamma - 1.) * E2.cv, p + pInf2);
+    Tm = ndiv(1., Tm * rhoMel);
+    P.out[cell] = ndiv(m[0], pt_rho(E1, p, Tm));
+    P.out[nn + cell] = ndiv(m[1], pt_rho(E2, p, Tm));
     P.out[(int64_t)FP * nn + cell] = p;
     P.out[(int64_t)FT * nn + cell] = Tm;
 #pragma unroll
     for (int d = 0; d < DIM; d++) P.out[(int64_t)(FU + d) * nn + cell] = u[d];
-    if (PASS != PASS_PRED) P.out[(int64_t)(FU + DIM) * nn + cell] = ddiv(rE, rhoMel);
+    if (PASS != PASS_PRED) P.out[(int64_t)(FU + DIM) * nn + cell] = ndiv(rE, rhoMel);
   }
   __shared__ double red[32];
-  double v = dtmax;
+  double v = wmax;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+  for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   if ((tid & 31) == 0) red[tid >> 5] = v;
   __syncthreads();
   if (tid < 32) {
-    v = (tid < K::NTH / 32) ? red[tid] : 1.e10;
+    v = (tid < K::NTH / 32) ? red[tid] : wave_none(G.stretched);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (tid == 0) atomic_min_pos_double(P.dtmax_bits, v);
+    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (tid == 0) atomic_min_pos_double(P.dtmax_bits, wave_dtmax(v, G.stretched, G.lcfl));
   }
 }
 
@@ -465,7 +465,7 @@ static cudaError_t ptueq_one(const StepParams& P, const Geometry& G, const ecg_e
   if (prepare) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   PtEos M;
   for (int k = 0; k < 2; k++)
-    M.e[k] = EosParams{eos[k].type, eos[k].gamma, eos[k].pinf, eos[k].b, eos[k].cv, eos[k].eref, eos[k].sref};
+    M.e[k] = make_eos_params(eos[k]);
   dim3 grid((G.n[0] + TS::X - 1) / TS::X, (G.n[1] + TS::Y - 1) / TS::Y, (G.n[2] + TS::Z - 1) / TS::Z);
   kern<<<grid, K::NTH, sm, s>>>(P, G, M);
   return cudaGetLastError();

@@ -15,12 +15,22 @@ struct EosParams {
   // sendSpecialMixtureEos constants (src/Eos/EosSG.cpp:196): gamma*pInf/(gamma-1) (0 for IG) and
   // 1/(gamma-1), evaluated once on the host (IEEE division, the same value as in the kernels).
   double gpi, ig;
+  // gamma - 1, gamma*pInf and the floor verifyAndModifyPressure puts under a pressure (EosIG.cpp:250,
+  // EosSG.cpp:252): the values the expressions would have in a kernel, which then reads them as constant
+  // operands.  ig is RN(1 / gm1), so a division by gm1 needs only its correction (cdiv).
+  double gm1, gpinf, pfloor;
 };
 
+#ifdef __CUDACC__
+__host__ __device__
+#endif
 inline EosParams make_eos_params(const ecg_eos& e) {
-  EosParams q{e.type, e.gamma, e.pinf, e.b, e.cv, e.eref, e.sref, 0., 0.};
+  EosParams q{e.type, e.gamma, e.pinf, e.b, e.cv, e.eref, e.sref, 0., 0., 0., 0., 0.};
   q.gpi = (e.type == ECG_EOS_IG) ? 0. : e.gamma * e.pinf / (e.gamma - 1.);
   q.ig = 1. / (e.gamma - 1.);
+  q.gm1 = e.gamma - 1.;
+  q.gpinf = e.gamma * e.pinf;
+  q.pfloor = (e.type == ECG_EOS_IG) ? 1.e-8 : -(1. - 1.e-15) * e.pinf + 1.e-15;
   return q;
 }
 
