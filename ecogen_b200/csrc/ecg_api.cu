@@ -232,17 +232,18 @@ namespace {
 // Distances of the MUSCL reconstruction per axis, with the reference's arithmetic: cell centres
 // (i + 0.5) * d, face position centre + 0.5 * d, lengths as Coord::norm of a difference
 // (src/Meshes/Element.cpp:77-113, src/Maths/Coord.cpp:82).
-// Then, per axis, the cell sizes (stretched meshes).
+// Then, per axis, the cell sizes (stretched meshes), and the reciprocals of the centre distances.
 void distance_tables(const ecg_case& c, const std::vector<double>* sz, const std::vector<double>* ctr,
                      std::vector<double>& h) {
   int nmax = std::max({c.ncells[0], c.ncells[1], c.ncells[2]});
-  h.assign(12 * (size_t)nmax, 0.);
+  h.assign(15 * (size_t)nmax, 0.);
   for (int a = 0; a < 3; a++) {
     for (int i = 0; i < c.ncells[a]; i++) h[(size_t)(9 + a) * nmax + i] = sz[a][i];
     for (int i = 0; i + 1 < c.ncells[a]; i++) {
       double pl = ctr[a][i], pr = ctr[a][i + 1], pf = pl + 0.5 * sz[a][i];
       double x = pl - pr, y = pf - pl, z = pf - pr;
       h[(size_t)(3 * a + 0) * nmax + i] = std::sqrt(x * x + 0. * 0. + 0. * 0.);
+      h[(size_t)(12 + a) * nmax + i] = 1. / h[(size_t)(3 * a + 0) * nmax + i];
       h[(size_t)(3 * a + 1) * nmax + i] = std::sqrt(y * y + 0. * 0. + 0. * 0.);
       h[(size_t)(3 * a + 2) * nmax + i] = std::sqrt(z * z + 0. * 0. + 0. * 0.);
     }
@@ -580,6 +581,7 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
     x->geo.dfl[a] = x->dist + (size_t)(3 * a + 1) * nmax;
     x->geo.dfr[a] = x->dist + (size_t)(3 * a + 2) * nmax;
     x->geo.dsz[a] = x->dist + (size_t)(9 + a) * nmax;
+    x->geo.rdcc[a] = x->dist + (size_t)(12 + a) * nmax;
   }
   x->geo.dim = x->dim;
   x->geo.stretched = case_stretched(*c) ? 1 : 0;

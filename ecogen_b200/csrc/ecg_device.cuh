@@ -60,10 +60,24 @@ __device__ __forceinline__ double eos_p(const EosParams& q, double eps, double r
   return (ndiv(rho * q.gm1 * (e - q.eref), dmax(1. - rho * q.b, eps)) - q.gpinf);
 }
 
+// eos_e and eos_c of a density that phase_fix_ar has clamped: rho >= 1e-15 >= eps (or NaN), so the floor
+// dmax(rho, eps) of the ideal and stiffened gas is the density itself.
+__device__ __forceinline__ double eos_e_clamped(const EosParams& q, double eps, double rho, double p) {
+  if (q.type == ECG_EOS_IG) return ndiv(cdiv(p, q.gm1, q.ig), rho) + q.eref;
+  if (q.type == ECG_EOS_SG) return ndiv(cdiv(p + q.gpinf, q.gm1, q.ig), rho) + q.eref;
+  return eos_e(q, eps, rho, p);
+}
+
 __device__ __forceinline__ double eos_c(const EosParams& q, double eps, double rho, double p) {
   if (q.type == ECG_EOS_IG) return dsqrt(ndiv(q.gamma * p, dmax(rho, eps)));
   if (q.type == ECG_EOS_SG) return dsqrt(ndiv(q.gamma * (p + q.pinf), dmax(rho, eps)));
   return dsqrt(ndiv(q.gamma * (p + q.pinf), dmax(rho * (1. - rho * q.b), eps)));
+}
+
+__device__ __forceinline__ double eos_c_clamped(const EosParams& q, double eps, double rho, double p) {
+  if (q.type == ECG_EOS_IG) return dsqrt(ndiv(q.gamma * p, rho));
+  if (q.type == ECG_EOS_SG) return dsqrt(ndiv(q.gamma * (p + q.pinf), rho));
+  return eos_c(q, eps, rho, p);
 }
 
 __device__ __forceinline__ double nonzero(double a, double eps) {  // Tools::returnNonZeroValue src/Tools.cpp:134
@@ -72,11 +86,13 @@ __device__ __forceinline__ double nonzero(double a, double eps) {  // Tools::ret
   return sg * eps;
 }
 
+template <bool CLAMPED>
 __device__ __forceinline__ double eos_p_isentropic(const EosParams& q, double eps, double p0, double rho0,
                                                    double rho1) {
-  if (q.type == ECG_EOS_IG) return p0 * epow(ndiv(rho1, dmax(rho0, eps)), q.gamma);
-  if (q.type == ECG_EOS_SG) return (p0 + q.pinf) * epow(ndiv(rho1, dmax(rho0, eps)), q.gamma) - q.pinf;
-  return (p0 + q.pinf) * epow(ndiv(rho1, dmax(rho0, eps)), q.gamma) * epow(ndiv(1. - rho0 * q.b, 1. - rho1 * q.b), q.gamma) -
+  const double ratio = ndiv(rho1, CLAMPED ? rho0 : dmax(rho0, eps));
+  if (q.type == ECG_EOS_IG) return p0 * epow(ratio, q.gamma);
+  if (q.type == ECG_EOS_SG) return (p0 + q.pinf) * epow(ratio, q.gamma) - q.pinf;
+  return (p0 + q.pinf) * epow(ratio, q.gamma) * epow(ndiv(1. - rho0 * q.b, 1. - rho1 * q.b), q.gamma) -
          q.pinf;
 }
 
@@ -166,11 +182,13 @@ struct Thermo {
   double rho, pm, cF;
 };
 
-template <int NP>
+// CLAMPED: the densities have been through phase_fix_ar (a reconstructed side).
+template <int NP, bool CLAMPED = false>
 __device__ __forceinline__ void fulfill(const Model<NP>& M, Thermo<NP>& t) {
   double c[NP];
 #pragma unroll
-  for (int k = 0; k < NP; k++) c[k] = eos_c(M.eos[k], M.eps, t.r[k], t.p[k]);
+  for (int k = 0; k < NP; k++)
+    c[k] = CLAMPED ? eos_c_clamped(M.eos[k], M.eps, t.r[k], t.p[k]) : eos_c(M.eos[k], M.eps, t.r[k], t.p[k]);
   t.rho = 0.;
   t.pm = 0.;
 #pragma unroll
@@ -188,12 +206,12 @@ __device__ __forceinline__ void fulfill(const Model<NP>& M, Thermo<NP>& t) {
 }
 
 // PhaseUEq::extendedCalculusPhase energies and MixUEq::computeMixtureVariables' e = sum_k Y_k e_k.
-template <int NP>
+template <int NP, bool CLAMPED = false>
 __device__ __forceinline__ double side_energy(const Model<NP>& M, const Thermo<NP>& t, double e[NP]) {
   double em = 0.;
 #pragma unroll
   for (int k = 0; k < NP; k++) {
-    e[k] = eos_e(M.eos[k], M.eps, t.r[k], t.p[k]);
+    e[k] = CLAMPED ? eos_e_clamped(M.eos[k], M.eps, t.r[k], t.p[k]) : eos_e(M.eos[k], M.eps, t.r[k], t.p[k]);
     em += t.Y[k] * e[k];
   }
   return em;
@@ -251,8 +269,8 @@ struct Flux {
 };
 
 // HLLC: ModUEq::solveRiemannIntern src/Models/UEq/ModUEq.cpp:113-267.  L and R carry local-frame
-// velocities ul/ur (normal first).  wmax collects the wave speeds (wave_add).
-template <int NP>
+// velocities ul/ur (normal first).  wmax collects the wave speeds (wave_add).  CLAMPED: see fulfill.
+template <int NP, bool CLAMPED = false>
 __device__ ECG_HLLC_INLINE void hllc(const Model<NP>& M, const Thermo<NP>& L, const double ul[3],
                                      const Thermo<NP>& R, const double ur[3], bool stretched, double dxL,
                                      double dxR, double& wmax, double Fn[3], Flux<NP>& F) {
@@ -272,7 +290,7 @@ __device__ ECG_HLLC_INLINE void hllc(const Model<NP>& M, const Thermo<NP>& L, co
     const double* us = left ? ul : ur;
     double un = us[0], rhoS = S.rho, pS = S.pm;
     double e[NP];
-    const double em = side_energy<NP>(M, S, e);
+    const double em = side_energy<NP, CLAMPED>(M, S, e);
 #pragma unroll
     for (int k = 0; k < NP; k++) {
       F.a[k] = S.a[k] * sM;
@@ -293,7 +311,7 @@ __device__ ECG_HLLC_INLINE void hllc(const Model<NP>& M, const Thermo<NP>& L, co
     double mK = left ? mL : mR;
     double uK = us[0], pK = S.pm;
     double e[NP];
-    const double em = side_energy<NP>(M, S, e);
+    const double em = side_energy<NP, CLAMPED>(M, S, e);
     double Et = em + 0.5 * (us[0] * us[0] + us[1] * us[1] + us[2] * us[2]);
     double rhoStar = ndiv(mK, sK - sM);
     double EStar = Et + (sM - uK) * (sM + ndiv(pK, mK));
@@ -303,7 +321,7 @@ __device__ ECG_HLLC_INLINE void hllc(const Model<NP>& M, const Thermo<NP>& L, co
       double mk = S.r[k] * (sK - uK);
       double rks = ndiv(mk, sK - sM);
       eos_rho_max(M.eos[k], rks);
-      double pks = eos_p_isentropic(M.eos[k], M.eps, S.p[k], S.r[k], rks);
+      double pks = eos_p_isentropic<CLAMPED>(M.eos[k], M.eps, S.p[k], S.r[k], rks);
       double eks = eos_e(M.eos[k], M.eps, rks, pks);
       F.a[k] = S.a[k] * sM;
       F.m[k] = S.a[k] * rks * sM;

@@ -81,6 +81,95 @@ __device__ ECG_RECON_INLINE void reconstruct_side(const Model<NP>& M, const Step
     t.a[0] = na;
     t.a[1] = 1. - na;
   }
+  fulfill<NP, true>(M, t);
+}
+
+// ---- limited slopes per cell (one limiter in all four slots)
+//
+// With one limiter the interface detector decides nothing, and every limiter is symmetric in its two
+// slopes, bit for bit (a product, a sum, a minimum of absolute values; same-signed arguments where the sign
+// is taken from one of them).  So the limited slope the left side of a cell's upper face uses is the one the
+// right side of its lower face uses: each is computed once per cell instead of twice, from the staged cells
+// themselves (no plane of face slopes to fill first).  The corrector stages no time-n alpha_0 plane either.
+// Measured on one B200 (mid-run states, CUDA events, face kernel of a pass): 3D three-phase 256^3 with minmod
+// 2.02 -> 1.89 ms (X), 1.80 -> 1.68 (Y), 1.82 -> 1.68 (Z), the step 16.34 -> 15.57 ms; 2D two-phase 2048^2
+// with van Leer 0.332 -> 0.309 and 0.312 -> 0.296 ms, the step 2.17 -> 2.10 ms.
+// prev / next: the cell's neighbours along the axis; dm, rm / dp, rp: centre distances of its two faces and
+// their reciprocals.  pone: the pressures of the three cells lie above every phase's floor, so the phase
+// pressures are all the cell's one pressure and have one slope.
+template <int NP, int DIM, int LIMC>
+__device__ __forceinline__ void cell_slopes(const Model<NP>& M, const double* sq, int RS, int prev, int rc, int next,
+                                            double dm, double rm, double dp, double rp, bool pone, double* lsl,
+                                            int LS, int e) {
+  using FL = Fields<NP, DIM>;
+  auto lim = [&](double a, double b, double c) { return limiter(LIMC, cdiv(b - a, dm, rm), cdiv(c - b, dp, rp)); };
+#pragma unroll
+  for (int k = 0; k < 2 * NP; k++)  // alpha_k, rho_k
+    lsl[k * LS + e] = lim(sq[k * RS + prev], sq[k * RS + rc], sq[k * RS + next]);
+  const double a = sq[FL::P * RS + prev], b = sq[FL::P * RS + rc], c = sq[FL::P * RS + next];
+  if (pone) {
+    const double l = lim(a, b, c);
+#pragma unroll
+    for (int k = 0; k < NP; k++) lsl[(2 * NP + k) * LS + e] = l;
+  } else {
+#pragma unroll
+    for (int k = 0; k < NP; k++)
+      lsl[(2 * NP + k) * LS + e] = lim(eos_fix_p(M.eos[k], a), eos_fix_p(M.eos[k], b), eos_fix_p(M.eos[k], c));
+  }
+#pragma unroll
+  for (int d = 0; d < DIM; d++)
+    lsl[(3 * NP + d) * LS + e] =
+        lim(sq[(FL::U + d) * RS + prev], sq[(FL::U + d) * RS + rc], sq[(FL::U + d) * RS + next]);
+}
+
+// One side of an internal face from the cell's limited slopes: reconstruct_side's extrapolation and clamps.
+// pone: no pressure of the block's cells is below a floor (one slope and one extrapolation for all phases).
+template <int NP, int DIM>
+__device__ __forceinline__ void extrapolate_side(const Model<NP>& M, const double* sq, int RS, int rc, const double* lsl,
+                                                 int LS, int ec, double dist, double sign, bool pone, Thermo<NP>& t,
+                                                 double u[3]) {
+  using FL = Fields<NP, DIM>;
+  const double pc = sq[FL::P * RS + rc];
+#pragma unroll
+  for (int k = 0; k < NP; k++) {
+    double a = sq[(FL::A + k) * RS + rc], r = sq[(FL::R + k) * RS + rc];
+    a += (sign * lsl[k * LS + ec]) * dist;
+    r += (sign * lsl[(NP + k) * LS + ec]) * dist;
+    phase_fix_ar(M.eps, a, r);
+    eos_rho_max(M.eos[k], r);
+    t.a[k] = a;
+    t.r[k] = r;
+  }
+  if (pone) {
+    const double p = pc + (sign * lsl[2 * NP * LS + ec]) * dist;
+#pragma unroll
+    for (int k = 0; k < NP; k++) t.p[k] = eos_fix_p(M.eos[k], p);
+  } else {
+#pragma unroll
+    for (int k = 0; k < NP; k++)
+      t.p[k] = eos_fix_p(M.eos[k], eos_fix_p(M.eos[k], pc) + (sign * lsl[(2 * NP + k) * LS + ec]) * dist);
+  }
+  u[0] = u[1] = u[2] = 0.;
+#pragma unroll
+  for (int d = 0; d < DIM; d++) u[d] = sq[(FL::U + d) * RS + rc] + (sign * lsl[(3 * NP + d) * LS + ec]) * dist;
+  fulfill<NP, true>(M, t);
+}
+
+// The buffer cell of a symmetry side (wall_side) from the cell's limited slopes.
+template <int NP, int DIM>
+__device__ __forceinline__ void wall_side_limited(const Model<NP>& M, const double* sq, int RS, int rc,
+                                                  const double* lsl, int LS, int ec, double dist, Thermo<NP>& t,
+                                                  double u[3]) {
+  using FL = Fields<NP, DIM>;
+#pragma unroll
+  for (int k = 0; k < NP; k++) {
+    t.a[k] = sq[(FL::A + k) * RS + rc] + lsl[k * LS + ec] * dist;
+    t.r[k] = sq[(FL::R + k) * RS + rc] + lsl[(NP + k) * LS + ec] * dist;
+    t.p[k] = eos_fix_p(M.eos[k], sq[FL::P * RS + rc]) + lsl[(2 * NP + k) * LS + ec] * dist;
+  }
+  u[0] = u[1] = u[2] = 0.;
+#pragma unroll
+  for (int d = 0; d < DIM; d++) u[d] = sq[(FL::U + d) * RS + rc] + lsl[(3 * NP + d) * LS + ec] * dist;
   fulfill<NP>(M, t);
 }
 

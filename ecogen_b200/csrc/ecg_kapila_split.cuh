@@ -37,16 +37,19 @@ __device__ __forceinline__ int64_t split_fid(const int n[3], int ax, int f, int 
   return (int64_t)i + (int64_t)n[0] * ((int64_t)j + (int64_t)n[1] * f);
 }
 
-template <int NP, int DIM, int AX, int PASS>
+template <int NP, int DIM, int AX, int PASS, int TYPES>
 struct FaceKernelShape {
   using FL = Fields<NP, DIM>;
   using FT = FaceTile<AX>;
   static constexpr bool O2 = (PASS != PASS_O1);
-  static constexpr int NA0 = (PASS == PASS_CORR) ? 1 : 0;  // separate time-n alpha_0 plane
+  // one limiter compiled in: limited slopes per cell (cell_slopes), no interface detector
+  static constexpr bool LSL = O2 && code_limiter(TYPES) >= 0;
+  static constexpr int NA0 = (PASS == PASS_CORR && !LSL) ? 1 : 0;  // separate time-n alpha_0 plane
+  static constexpr int SS = LSL ? FT::LS : FT::SS;                 // one slope plane
   static constexpr size_t staged_bytes() { return sizeof(double) * (size_t)FT::RS * (FL::NQ + NA0); }
   // staged planes, slope planes, the staging mbarrier, and room to align the base to 128 bytes
   static constexpr size_t smem_bytes() {
-    return staged_bytes() + (O2 ? sizeof(double) * (size_t)FT::SS * FL::NSL : 0) + sizeof(uint64_t) + 128;
+    return staged_bytes() + (O2 ? sizeof(double) * (size_t)SS * FL::NSL : 0) + sizeof(uint64_t) + 128;
   }
 };
 
@@ -92,10 +95,10 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
                    const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap ma0, int tma) {
   const Model<NP> M = specialize_eos<NP, TYPES>(M0);
   using FT = FaceTile<AX>;
-  using KS = FaceKernelShape<NP, DIM, AX, PASS>;
+  using KS = FaceKernelShape<NP, DIM, AX, PASS, TYPES>;
   using FL = Fields<NP, DIM>;
-  constexpr bool O2 = KS::O2;
-  constexpr int RS = FT::RS, SS = FT::SS, CP = FT::CP;
+  constexpr bool O2 = KS::O2, LSL = KS::LSL;
+  constexpr int RS = FT::RS, SS = KS::SS, CP = FT::CP;
   extern __shared__ unsigned char smem_raw[];
   double* smem = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
   double* sq = smem;                                // [NQ][RS]
@@ -123,7 +126,7 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
     // one tensor copy of the box (x, y[, z], field) for all primitive fields, one for the time-n
     // alpha_0 plane; cells outside the mesh arrive as zeros
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + KS::staged_bytes() / sizeof(double) +
-                                                (O2 ? (size_t)FT::SS * FL::NSL : 0));
+                                                (O2 ? (size_t)SS * FL::NSL : 0));
     if (tid == 0) mbar_init(bar, 1);
     __syncthreads();
     if (tid == 0) {
@@ -157,8 +160,44 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
     }
   }
   __syncthreads();
+  // ---- limited slopes (MUSCL, one limiter): cell f0 - 1 + s of every line, s in [0, TF]
+  bool pone = true;  // no pressure read by this block's faces is below a phase's floor
+  if (LSL) {
+    double pf = M.eos[0].pfloor;
+#pragma unroll
+    for (int k = 1; k < NP; k++) pf = dmax(pf, M.eos[k].pfloor);
+    for (int e = tid; e < SS; e += FT::NTH) {
+      const int line = AX == 0 ? e / FT::LP : e % FT::W, s = AX == 0 ? e % FT::LP : e / FT::W;
+      const int c = f0 - 1 + s;
+      if (c < 0 || c >= nax || l0 + line >= G.n[ob]) continue;
+      const int rc = FT::cidx(line, s + 1);
+      if (c == 0 || c == nax - 1) {
+        // no face beyond: the missing slope is zero, and so is every limited one, except the velocity
+        // along the axis at a symmetry side, whose slope there is u over the centre-to-face coordinate
+        // (BoundCondWallO2Cartesian::computeSlopes :84-108)
+#pragma unroll
+        for (int f = 0; f < FL::NSL; f++) ssl[f * SS + e] = 0.;
+        const int sd = c == 0 ? 0 : 1;
+        const double wd = G.wslope[2 * AX + sd];
+        if (G.bc[2 * AX + sd] == ECG_BC_SYMMETRY && fabs(wd) > 1.e-8) {
+          const double* su = sq + (FL::U + AX) * RS;
+          const double so = sd ? ndiv(su[rc] - su[FT::cidx(line, s)], G.dcc[AX][c - 1])
+                               : ndiv(su[FT::cidx(line, s + 2)] - su[rc], G.dcc[AX][c]);
+          ssl[(3 * NP + AX) * SS + e] = limiter(code_limiter(TYPES), ndiv(su[rc], wd), so);
+        }
+        pone = pone && sq[FL::P * RS + rc] >= pf;
+        continue;
+      }
+      const int prev = FT::cidx(line, s), next = FT::cidx(line, s + 2);
+      const bool one = sq[FL::P * RS + prev] >= pf && sq[FL::P * RS + rc] >= pf && sq[FL::P * RS + next] >= pf;
+      pone = pone && one;
+      cell_slopes<NP, DIM, code_limiter(TYPES)>(M, sq, RS, prev, rc, next, G.dcc[AX][c - 1], G.rdcc[AX][c - 1],
+                                                G.dcc[AX][c], G.rdcc[AX][c], one, ssl, SS, e);
+    }
+    pone = __syncthreads_and(pone);
+  }
   // ---- face slopes (MUSCL): slope s at face g = f0 - 1 + s, between cells g-1 and g
-  if (O2) {
+  if (O2 && !LSL) {
     for (int e = tid; e < SS; e += FT::NTH) {
       const int line = AX == 0 ? e / FT::SP : e % FT::W, s = AX == 0 ? e % FT::SP : e / FT::W;
       const int gl = f0 - 2 + s;  // left cell of the face
@@ -217,7 +256,10 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
         Thermo<NP> t;
         double ug[3], ul[3];
         if (G.bc[2 * AX + sd] == ECG_BC_SYMMETRY) {
-          if (O2) {
+          if (LSL) {
+            wall_side_limited<NP, DIM>(M, sq, RS, rc, ssl, SS, FT::lidx(line, sd == 0 ? fl + 1 : fl),
+                                       G.wdist[2 * AX + sd], t, ug);
+          } else if (O2) {
             const int fw = FT::sidx(line, fl + 1), fo = FT::sidx(line, sd == 0 ? fl + 2 : fl);
             wall_side<NP, DIM>(M, P.lim, sq, RS, rc, ssl, SS, fw, fo, a0[rc], G.wdist[2 * AX + sd], t, ug);
           } else {
@@ -247,6 +289,9 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
         if (!O2) {
           cell_thermo<NP, DIM>(M, sq, RS, rl, tl, ug);
           cell_thermo<NP, DIM>(M, sq, RS, rr, tr, vg);
+        } else if (LSL) {
+          extrapolate_side<NP, DIM>(M, sq, RS, rl, ssl, SS, FT::lidx(line, fl), G.dfl[AX][gl], 1., pone, tl, ug);
+          extrapolate_side<NP, DIM>(M, sq, RS, rr, ssl, SS, FT::lidx(line, fl + 1), G.dfr[AX][gl], -1., pone, tr, vg);
         } else {
           const int f1 = FT::sidx(line, fl + 1);  // this face
           const bool hasL = (gl - 1 >= 0), hasR = (gl + 2 < nax);
@@ -275,7 +320,7 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
         const double lL = cell_lcfl(G, gf[0], gf[1], gf[2]);
         gf[AX] = gl + 1;
         const double lR = cell_lcfl(G, gf[0], gf[1], gf[2]);
-        hllc<NP>(M, tl, ul, tr, ur, G.stretched, lL, lR, wmax, Fn, F);
+        hllc<NP, O2>(M, tl, ul, tr, ur, G.stretched, lL, lR, wmax, Fn, F);
         to_global(AX, false, Fn, F.mom);
       }
       const int64_t nfa = split_nfaces(G.n, AX);
@@ -410,7 +455,7 @@ template <int NP, int DIM, int AX, int PASS, int TYPES>
 cudaError_t launch_faces(const StepParams& P, const Geometry& G, const Model<NP>& M, cudaStream_t s, bool prepare) {
   using FT = FaceTile<AX>;
   auto kern = k_kapila_faces<NP, DIM, AX, PASS, TYPES>;
-  const size_t sm = FaceKernelShape<NP, DIM, AX, PASS>::smem_bytes();
+  const size_t sm = FaceKernelShape<NP, DIM, AX, PASS, TYPES>::smem_bytes();
   if (prepare) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   // tensor maps of the buffers this pass reads (TMA staging), when the context built them
   CUtensorMap mq{}, ma0{};
@@ -421,7 +466,7 @@ cudaError_t launch_faces(const StepParams& P, const Geometry& G, const Model<NP>
       if (P.fmaps->buf[b] && P.fmaps->buf[b] == P.q) q = &P.fmaps->q[b][AX];
       if (P.fmaps->buf[b] && P.fmaps->buf[b] == P.sn) a = &P.fmaps->a0[b][AX];
     }
-    if (q && (PASS != PASS_CORR || a)) {
+    if (q && (!FaceKernelShape<NP, DIM, AX, PASS, TYPES>::NA0 || a)) {
       mq = *q;
       if (a) ma0 = *a;
       tma = 1;

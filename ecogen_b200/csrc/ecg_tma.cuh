@@ -45,8 +45,11 @@ struct FaceTile {
   static constexpr int SP = TF + 2;  // slopes per line: faces f0-1 .. f0+TF
   static constexpr int RS = W * CP;  // one staged plane
   static constexpr int SS = W * SP;  // one slope plane
+  static constexpr int LP = TF + 1;  // limited slopes per line: cells f0-1 .. f0+TF-1
+  static constexpr int LS = W * LP;  // one plane of them
   __host__ __device__ static constexpr int cidx(int line, int pos) { return AX == 0 ? line * CP + pos : pos * W + line; }
   __host__ __device__ static constexpr int sidx(int line, int s) { return AX == 0 ? line * SP + s : s * W + line; }
+  __host__ __device__ static constexpr int lidx(int line, int s) { return AX == 0 ? line * LP + s : s * W + line; }
   // extent of the staged box along x, y, z (the tensor's first three dimensions)
   static constexpr int box(int d) {
     return AX == 0 ? (d == 0 ? CP : (d == 1 ? W : 1)) : (d == 0 ? W : (d == AX ? CP : 1));

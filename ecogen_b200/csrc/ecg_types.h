@@ -45,6 +45,7 @@ struct Geometry {
   // Distances used by the MUSCL reconstruction, per axis and face position (indexed by the
   // left cell i of face (i, i+1)): centre-to-centre, face-to-left-centre, face-to-right-centre.
   const double* dcc[3];
+  const double* rdcc[3];  // RN(1 / dcc)
   const double* dfl[3];
   const double* dfr[3];
   // Sides Xm, Xp, Ym, Yp, Zm, Zp (index 2*axis + plus): boundary condition, centre-minus-face
