@@ -1,14 +1,20 @@
-// Batched independent 1D cases: one persistent kernel per pass pulls (case, tile) work items from
-// a device queue.
+// Batched independent 1D cases: every pass is one face-flux kernel and one cell kernel over all cases.
 //
 // The reference runs independent cases one after the other (src/main.cpp:82-133), each with its
 // own time loop.  Here all cases live in one concatenated structure-of-arrays state (case c owns
-// cells [off_c, off_c + n_c)), every pass (first order, or MUSCL predictor then corrector) is one
-// launch of #SM x occupancy blocks that loop over the work items, and each case keeps its own dt:
-// the min of lCFL/|s| over a case's faces is reduced per work item and merged into the case's slot
-// with one atomicMin (a segmented min-reduction), then a per-case update sets dt_c = cfl_c dtMax_c.
-// The step sequence is captured once as a CUDA graph.  Tile size and block size are picked by a
-// small autotuner that times each candidate on a copy of the state.
+// cells [off_c, off_c + n_c) and faces [off_c + c, off_c + c + n_c]), every pass (first order, or MUSCL
+// predictor then corrector) is two launches over lists of (case, first face) and (case, first cell) items,
+// one block per item, and each case keeps its own dt: the fastest wave of an item's faces merges into the
+// case's slot with one atomicMin (a segmented min-reduction), then a per-case update sets
+// dt_c = cfl_c dtMax_c.  The step sequence is captured once as a CUDA graph.  The faces of an item (the
+// tile) are picked by a small autotuner that times each candidate on a copy of the state.
+//
+// Why two kernels: one kernel per pass (persistent blocks over a queue of tiles) held the face work, the
+// cell update and the seeded update at once, spilled 1.1 KB a thread at 80 registers and met four barriers
+// per tile, at which warps waited for the slowest cell's Newton iteration.  The face fluxes cost
+// 160 bytes of HBM traffic per cell and pass, which the passes have to spare.  Measured on one B200
+// (4096 two-phase tubes, 8.6 M cells, MUSCL + van Leer, mid-run states, host copies of a 40-step pass
+// included): 3.54 -> 3.30 ms per step; 64 tubes (0.13 M cells) 131 -> 111 us.  Same bits.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -16,34 +22,19 @@
 #include <vector>
 
 #include "ecg_internal.h"
-#include "ecg_kapila_cell.cuh"
+#include "ecg_kapila_split.cuh"
 
-// Register budget of the batched kernels: ECG_BATCH_SM_THREADS > 0 asks the compiler to fit
-// ECG_BATCH_SM_THREADS / TB blocks of TB threads on an SM (more resident warps, fewer registers a
-// thread); 0 leaves the register count to the compiler.  Measured on 4096 batched two-phase tubes
-// (cell-updates/s, tile chosen by the autotuner): no budget (168 registers, 12 warps per SM) 1168 M;
-// 512 threads 1448 M; 640: 1464 M; 896 (85 registers at 256-cell tiles, 24 warps) 1628-1658 M;
-// 1024: 1599 M; 1152: 1602 M.
+// Resident threads per SM asked of the face kernel (registers 65536 / threads; 896: 72 registers, as the 2D
+// face kernels, whose code it shares).
 #ifndef ECG_BATCH_SM_THREADS
 #define ECG_BATCH_SM_THREADS 896
-#endif
-// Cells of one work item for TB threads: TB - ECG_BATCH_ITEM_TRIM.  With a trim of 1 the item's
-// TB faces take one round of the block; with 0 the item has TB + 1 faces and one warp computes two
-// while the block waits at the next barrier.  Measured on 4096 batched tubes: trim 0 1657 M, trim 1
-// 2066 M cell-updates/s.
-#ifndef ECG_BATCH_ITEM_TRIM
-#define ECG_BATCH_ITEM_TRIM 1
-#endif
-#if ECG_BATCH_SM_THREADS > 0
-#define ECG_BATCH_BOUNDS(TB) __launch_bounds__(TB, (ECG_BATCH_SM_THREADS / (TB) > 0 ? ECG_BATCH_SM_THREADS / (TB) : 1))
-#else
-#define ECG_BATCH_BOUNDS(TB) __launch_bounds__(TB)
 #endif
 
 namespace ecg {
 
 struct BatchCase {
   int64_t off;
+  int64_t fbase;  // first face
   int n;
   double dx, coefA, lcfl, cfl;
 };
@@ -58,208 +49,211 @@ struct BatchParams {
   StepParams P;              // q / sn / out point at the concatenated state (stride = total cells)
   const BatchCase* cases;
   BatchScalars* scal;
-  const int2* items;         // (case, first cell)
-  int nitems;
-  unsigned int* queue;       // work counter of this pass
+  const int2* items;         // (case, first face) of the face kernel, (case, first cell) of the cell kernel
+  double* flux;              // face fluxes, stride nfaces
+  int64_t nfaces;
 };
 
-template <int NP, int TB, int PASS>
+// A face item: TB - 1 faces of one case for TB threads, so that the TB cells whose limited slopes they read
+// take one round of the block.
+template <int NP, int TB, int PASS, int TYPES>
 struct BatchTile {
-  static constexpr int TC = TB - ECG_BATCH_ITEM_TRIM;  // cells of one work item
-  static constexpr int H = (PASS == PASS_O1) ? 1 : 2;
-  static constexpr int RL = TC + 2 * H;
-  static constexpr int NQ = Fields<NP, 1>::NQ + ((PASS == PASS_CORR) ? 1 : 0);
-  static constexpr int NS = (PASS == PASS_O1) ? 0 : TC + 3;
+  static constexpr bool O2 = (PASS != PASS_O1);
+  static constexpr bool LSL = O2 && code_limiter(TYPES) >= 0;
+  static constexpr int TF = TB - 1;
+  static constexpr int H = O2 ? 2 : 1;               // cells staged before the first face
+  static constexpr int RL = TF + (O2 ? 3 : 1);
+  static constexpr int NA0 = (PASS == PASS_CORR && !LSL) ? 1 : 0;
+  static constexpr int SS = O2 ? (LSL ? TF + 1 : TF + 2) : 1;
   static constexpr size_t smem_bytes() {
-    return sizeof(double) * ((size_t)RL * NQ + (size_t)NS * Fields<NP, 1>::NSL + (size_t)(TC + 1) * Fields<NP, 1>::NFL);
+    return sizeof(double) * ((size_t)RL * (Fields<NP, 1>::NQ + NA0) + (O2 ? (size_t)SS * Fields<NP, 1>::NSL : 0));
   }
 };
 
 template <int NP, int TB, int PASS, int TYPES>
-__global__ void ECG_BATCH_BOUNDS(TB) k_batch(BatchParams B, Model<NP> M0) {
+__global__ void __launch_bounds__(TB, ECG_BATCH_SM_THREADS / TB) k_batch_faces(BatchParams B, Model<NP> M0) {
   const Model<NP> M = specialize_eos<NP, TYPES>(M0);  // EOS types compiled in for the shipped workload
   using FL = Fields<NP, 1>;
-  using K = BatchTile<NP, TB, PASS>;
-  constexpr bool O2 = (PASS != PASS_O1);
-  constexpr int TC = K::TC;
-  constexpr int RS = K::RL;
-  constexpr int SS = O2 ? K::NS : 1;
-  constexpr int FS = TC + 1;
+  using K = BatchTile<NP, TB, PASS, TYPES>;
+  constexpr bool O2 = K::O2, LSL = K::LSL;
+  constexpr int TF = K::TF, RS = K::RL, SS = K::SS;
   extern __shared__ double smem[];
   double* sq = smem;
   double* sa0 = sq + (size_t)FL::NQ * RS;
-  double* ssl = sq + (size_t)K::NQ * RS;
-  double* sfl = ssl + (O2 ? (size_t)FL::NSL * SS : 0);
-  __shared__ int s_item;
-  __shared__ double red[32];
+  double* ssl = sa0 + (size_t)K::NA0 * RS;
   const StepParams& P = B.P;
   const int64_t nn = P.n;
   const int tid = threadIdx.x;
-  CellCounters total;
-  unsigned int max_iters = 0;
-
-  for (;;) {
-    if (tid == 0) s_item = (int)atomicAdd(B.queue, 1u);
-    __syncthreads();
-    const int item = s_item;
-    __syncthreads();
-    if (item >= B.nitems) break;
-    const int c = B.items[item].x;
-    const int org = B.items[item].y;
-    const BatchCase C = B.cases[c];
-    const int n = C.n;
-    // ---- stage the tile and its halo of this case
-    for (int e = tid; e < RS; e += TB) {
-      int g = org + e - K::H;
-      if (g >= 0 && g < n) {
-        int64_t gi = C.off + g;
+  const int c = B.items[blockIdx.x].x;
+  const int f0 = B.items[blockIdx.x].y;
+  const BatchCase C = B.cases[c];
+  const int n = C.n;
+  // ---- stage the cells the item's faces read, f0 - H and up
+  for (int e = tid; e < RS; e += TB) {
+    const int g = f0 - K::H + e;
+    if (g >= 0 && g < n) {
+      const int64_t gi = C.off + g;
 #pragma unroll
-        for (int f = 0; f < FL::NQ; f++) sq[f * RS + e] = P.q[(int64_t)f * nn + gi];
-        if (PASS == PASS_CORR) sa0[e] = P.sn[(int64_t)FL::A * nn + gi];
-      }
+      for (int f = 0; f < FL::NQ; f++) sq[f * RS + e] = P.q[(int64_t)f * nn + gi];
+      if (K::NA0) sa0[e] = P.sn[(int64_t)FL::A * nn + gi];
     }
-    __syncthreads();
-    if (O2) {
-      for (int e = tid; e < SS; e += TB) {
-        int j = e - 1;
-        int gl = org + j - 1;
-        if (gl < 0 || gl + 1 >= n) continue;
-        int rl = j - 1 + K::H, rr = rl + 1;
-        // centre-to-centre distance with the reference's arithmetic (Element::distance)
-        double pl = (gl + 0.5) * C.dx, pr = (gl + 1 + 0.5) * C.dx, x = pl - pr;
-        double d = dsqrt(x * x);
+  }
+  __syncthreads();
+  // centre of cell g and centre-to-centre distance of cells g, g + 1 with the reference's arithmetic
+  // (Element::distance: sqrt(x x), which is |x| bit for bit)
+  auto centre = [&](int g) { return (g + 0.5) * C.dx; };
+  auto dist = [&](int g) { return fabs(centre(g) - centre(g + 1)); };
+  bool pone = true;
+  if (LSL) {
+    double pf = M.eos[0].pfloor;
 #pragma unroll
-        for (int k = 0; k < NP; k++) {
-          ssl[k * SS + e] = ndiv(sq[(FL::A + k) * RS + rr] - sq[(FL::A + k) * RS + rl], d);
-          ssl[(NP + k) * SS + e] = ndiv(sq[(FL::R + k) * RS + rr] - sq[(FL::R + k) * RS + rl], d);
-          double pR = eos_fix_p(M.eos[k], sq[FL::P * RS + rr]), pL = eos_fix_p(M.eos[k], sq[FL::P * RS + rl]);
-          ssl[(2 * NP + k) * SS + e] = ndiv(pR - pL, d);
-        }
-        ssl[(3 * NP) * SS + e] = ndiv(sq[FL::U * RS + rr] - sq[FL::U * RS + rl], d);
+    for (int k = 1; k < NP; k++) pf = dmax(pf, M.eos[k].pfloor);
+    for (int e = tid; e < SS; e += TB) {  // limited slopes of cell f0 - 1 + e
+      const int g = f0 - 1 + e;
+      if (g < 0 || g >= n) continue;
+      const int rc = e + 1;
+      if (g == 0 || g == n - 1) {  // no face beyond: every limited slope is zero
+#pragma unroll
+        for (int f = 0; f < FL::NSL; f++) ssl[f * SS + e] = 0.;
+        pone = pone && sq[FL::P * RS + rc] >= pf;
+        continue;
       }
-      __syncthreads();
+      const bool one = sq[FL::P * RS + rc - 1] >= pf && sq[FL::P * RS + rc] >= pf && sq[FL::P * RS + rc + 1] >= pf;
+      pone = pone && one;
+      const double dm = dist(g - 1), dp = dist(g);
+      cell_slopes<NP, 1, code_limiter(TYPES)>(M, sq, RS, rc - 1, rc, rc + 1, dm, nrcp(dm), dp, nrcp(dp), one, ssl, SS, e);
     }
-    double wmax = wave_none(false);
-    for (int j = tid; j <= TC; j += TB) {
-      int gl = org + j - 1;
+    pone = __syncthreads_and(pone);
+  } else if (O2) {
+    for (int e = tid; e < SS; e += TB) {  // slope e at face f0 - 1 + e
+      const int gl = f0 - 2 + e;
       if (gl < 0 || gl + 1 >= n) continue;
-      int rl = j - 1 + K::H, rr = rl + 1;
-      Thermo<NP> tl, tr;
-      double ug[3], vg[3];
-      if (!O2) {
-        cell_thermo<NP, 1>(M, sq, RS, rl, tl, ug);
-        cell_thermo<NP, 1>(M, sq, RS, rr, tr, vg);
-      } else {
-        const int f1 = j + 1;
-        const bool hasL = (gl - 1 >= 0), hasR = (gl + 2 < n);
-        const double* a0 = (PASS == PASS_CORR) ? sa0 : sq;
-        double aL = sq[FL::A * RS + rl], aR = sq[FL::A * RS + rr];
-        double aLL = hasL ? a0[rl - 1] : 0., aRR = hasR ? a0[rr + 1] : 0.;
-        double pl = (gl + 0.5) * C.dx, pf = pl + 0.5 * C.dx, pr = (gl + 1 + 0.5) * C.dx;
-        double y = pf - pl, z = pf - pr;
-        constexpr bool kThinc = (TYPES == EOS_DYNAMIC);
-        constexpr int kLim = code_limiter(TYPES);
-        reconstruct_side<NP, 1, kThinc, kLim>(M, P, sq, RS, rl, ssl, SS, f1, hasL ? j : -1, aL, aR, aLL, dsqrt(y * y), 1.,
-                                              tl, ug);
-        reconstruct_side<NP, 1, kThinc, kLim>(M, P, sq, RS, rr, ssl, SS, f1, hasR ? j + 2 : -1, aR, aL, aRR, dsqrt(z * z),
-                                              -1.,
-                                tr, vg);
-      }
-      double Fn[3];
-      Flux<NP> F;
-      hllc<NP>(M, tl, ug, tr, vg, false, C.lcfl, C.lcfl, wmax, Fn, F);
-      F.mom[0] = Fn[0];
+      const int rl = e, rr = e + 1;
+      const double d = dist(gl);
 #pragma unroll
       for (int k = 0; k < NP; k++) {
-        sfl[k * FS + j] = F.a[k];
-        sfl[(NP + k) * FS + j] = F.m[k];
-        sfl[(2 * NP + k) * FS + j] = F.en[k];
+        ssl[k * SS + e] = ndiv(sq[(FL::A + k) * RS + rr] - sq[(FL::A + k) * RS + rl], d);
+        ssl[(NP + k) * SS + e] = ndiv(sq[(FL::R + k) * RS + rr] - sq[(FL::R + k) * RS + rl], d);
+        double pR = eos_fix_p(M.eos[k], sq[FL::P * RS + rr]), pL = eos_fix_p(M.eos[k], sq[FL::P * RS + rl]);
+        ssl[(2 * NP + k) * SS + e] = ndiv(pR - pL, d);
       }
-      sfl[(3 * NP) * FS + j] = F.mom[0];
-      sfl[(3 * NP + 1) * FS + j] = F.E;
-      sfl[(3 * NP + 2) * FS + j] = F.sM;
-      sfl[(3 * NP + 3) * FS + j] = F.uStar;
-    }
-    __syncthreads();
-    const int g = org + tid;
-    const bool own = tid < TC && g < n;  // this thread's cell of the item
-    CellPrim<NP, 1> cp;
-    if (own) {
-      const int64_t cell = C.off + g;
-      double an[NP], rn[NP], pn[NP], aa[NP], am[NP], ae[NP], amom[1] = {0.}, aE = 0.;
-      double p0 = P.sn[(int64_t)FL::P * nn + cell];
-#pragma unroll
-      for (int k = 0; k < NP; k++) {
-        an[k] = P.sn[(int64_t)(FL::A + k) * nn + cell];
-        rn[k] = P.sn[(int64_t)(FL::R + k) * nn + cell];
-        pn[k] = eos_fix_p(M.eos[k], p0);
-        aa[k] = am[k] = ae[k] = 0.;
-      }
-#pragma unroll
-      for (int side = 0; side < 2; side++) {
-        int j = tid + side;
-        int gl = org + j - 1;
-        if (gl < 0 || gl + 1 >= n) continue;
-        Flux<NP> F;
-#pragma unroll
-        for (int k = 0; k < NP; k++) {
-          F.a[k] = sfl[k * FS + j];
-          F.m[k] = sfl[(NP + k) * FS + j];
-          F.en[k] = sfl[(2 * NP + k) * FS + j];
-        }
-        F.mom[0] = sfl[(3 * NP) * FS + j];
-        F.E = sfl[(3 * NP + 1) * FS + j];
-        F.sM = sfl[(3 * NP + 2) * FS + j];
-        F.uStar = sfl[(3 * NP + 3) * FS + j];
-        acc_face<NP, 1>(C.coefA, side == 0, F, an, pn, aa, am, ae, amom, aE);
-      }
-      if (g == 0) boundary_face<NP, 1>(M, P.q, nn, cell, 0, true, false, C.lcfl, C.coefA, wmax, an, pn, aa, am, ae, amom, aE);
-      if (g == n - 1)
-        boundary_face<NP, 1>(M, P.q, nn, cell, 0, false, false, C.lcfl, C.coefA, wmax, an, pn, aa, am, ae, amom, aE);
-      kapila_rebuild<NP, 1, PASS>(P, M, nn, cell, B.scal[c].dt, an, rn, pn, aa, am, ae, amom, aE, cp);
-    }
-    SeedGate<NP> sg;
-    const bool seeded = P.mlp != nullptr;  // uniform over the launch
-    if (seeded) seed_gate<NP, 1>(P, M, own, cp, sg);
-    if (own) {
-      const int64_t cell = C.off + g;
-      CellCounters cc;
-      if (seeded)
-        kapila_finish<NP, 1, PASS, false, true, (TYPES == EOS_DYNAMIC)>(P, M, nn, cell, cp, sg, cc);
-      else
-        kapila_finish<NP, 1, PASS, false, false, (TYPES == EOS_DYNAMIC)>(P, M, nn, cell, cp, sg, cc);
-      total.relax += cc.relax;
-      total.iters += cc.iters;
-      total.fallback += cc.fallback;
-      total.seeded += cc.seeded;
-      total.rejected += cc.rejected;
-      total.nonfinite += cc.nonfinite;
-      max_iters = max_iters > cc.iters ? max_iters : cc.iters;
-    }
-    // ---- segmented reduction: this item's faces belong to case c only
-    double v = wmax;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((tid & 31) == 0) red[tid >> 5] = v;
-    __syncthreads();
-    if (tid < 32) {
-      v = (tid < TB / 32) ? red[tid] : wave_none(false);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-      if (tid == 0) atomic_min_pos_double(&B.scal[c].dtmax_bits, wave_dtmax(v, false, C.lcfl));
+      ssl[(3 * NP) * SS + e] = ndiv(sq[FL::U * RS + rr] - sq[FL::U * RS + rl], d);
     }
     __syncthreads();
   }
-  // per-thread totals of all items this block processed; the per-bin histogram is not kept in
-  // batched mode (relax_calls / newton_evals / newton_max are)
-  block_counters(P.stats, total.relax, total.iters, total.fallback, total.seeded, total.rejected, total.nonfinite, 0u,
-                 max_iters, false);
+  double wmax = wave_none(false);
+  const int f = f0 + tid;
+  if (tid < TF && f <= n) {
+    Flux<NP> F;
+    double Fn[3];
+    if (f == 0 || f == n) {
+      // non-reflecting side: HLLC(cell, cell) in the side's frame (BoundCondNonReflecting::
+      // solveRiemannBoundary src/BoundConds/BoundCondNonReflecting.cpp:62)
+      const bool neg = f == 0;
+      Thermo<NP> t;
+      double ug[3], ul[3];
+      cell_thermo<NP, 1>(M, sq, RS, neg ? tid + K::H : tid + K::H - 1, t, ug);
+      to_local(0, neg, ug, ul);
+      hllc<NP>(M, t, ul, t, ul, false, C.lcfl, C.lcfl, wmax, Fn, F);
+      to_global(0, neg, Fn, F.mom);
+    } else {
+      const int gl = f - 1, rl = tid + K::H - 1, rr = rl + 1;
+      Thermo<NP> tl, tr;
+      double ug[3], vg[3];
+      const double pl = centre(gl), pf = pl + 0.5 * C.dx, pr = centre(gl + 1);
+      if (!O2) {
+        cell_thermo<NP, 1>(M, sq, RS, rl, tl, ug);
+        cell_thermo<NP, 1>(M, sq, RS, rr, tr, vg);
+      } else if (LSL) {
+        extrapolate_side<NP, 1>(M, sq, RS, rl, ssl, SS, tid, fabs(pf - pl), 1., pone, tl, ug);
+        extrapolate_side<NP, 1>(M, sq, RS, rr, ssl, SS, tid + 1, fabs(pf - pr), -1., pone, tr, vg);
+      } else {
+        const int f1 = tid + 1;
+        const bool hasL = (gl - 1 >= 0), hasR = (gl + 2 < n);
+        const double* a0 = K::NA0 ? sa0 : sq;
+        const double aL = sq[FL::A * RS + rl], aR = sq[FL::A * RS + rr];
+        const double aLL = hasL ? a0[rl - 1] : 0., aRR = hasR ? a0[rr + 1] : 0.;
+        constexpr bool kThinc = (TYPES == EOS_DYNAMIC);
+        constexpr int kLim = code_limiter(TYPES);
+        reconstruct_side<NP, 1, kThinc, kLim>(M, P, sq, RS, rl, ssl, SS, f1, hasL ? tid : -1, aL, aR, aLL,
+                                              fabs(pf - pl), 1., tl, ug);
+        reconstruct_side<NP, 1, kThinc, kLim>(M, P, sq, RS, rr, ssl, SS, f1, hasR ? tid + 2 : -1, aR, aL, aRR,
+                                              fabs(pf - pr), -1., tr, vg);
+      }
+      hllc<NP, O2>(M, tl, ug, tr, vg, false, C.lcfl, C.lcfl, wmax, Fn, F);
+      F.mom[0] = Fn[0];
+    }
+    double* out = B.flux + C.fbase + f;
+#pragma unroll
+    for (int k = 0; k < NP; k++) {
+      out[(int64_t)k * B.nfaces] = F.a[k];
+      out[(int64_t)(NP + k) * B.nfaces] = F.m[k];
+      out[(int64_t)(2 * NP + k) * B.nfaces] = F.en[k];
+    }
+    out[(int64_t)(3 * NP) * B.nfaces] = F.mom[0];
+    out[(int64_t)(3 * NP + 1) * B.nfaces] = F.E;
+    out[(int64_t)(3 * NP + 2) * B.nfaces] = F.sM;
+    out[(int64_t)(3 * NP + 3) * B.nfaces] = F.uStar;
+  }
+  // ---- segmented reduction: this item's faces belong to case c only
+  __shared__ double red[TB / 32];
+  double v = wmax;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if ((tid & 31) == 0) red[tid >> 5] = v;
+  __syncthreads();
+  if (tid == 0) {
+#pragma unroll
+    for (int w = 1; w < TB / 32; w++) v = dmax(v, red[w]);
+    atomic_min_pos_double(&B.scal[c].dtmax_bits, wave_dtmax(v, false, C.lcfl));
+  }
 }
 
-__global__ void k_batch_finalize(BatchScalars* s, const BatchCase* cases, int ncases, unsigned int* queue, int nq) {
+// One thread per cell of an item: the fluxes of its two faces, left added, right subtracted, sides of the case
+// last, then the cell update.
+template <int NP, int PASS, bool SEED, int TYPES>
+__global__ void __launch_bounds__(CELL_THREADS, SEED ? ECG_CELL_SEED_MINB : ECG_CELL_MINB)
+    k_batch_cells(BatchParams B, Model<NP> M0) {
+  const Model<NP> M = specialize_eos<NP, TYPES>(M0);
+  using FL = Fields<NP, 1>;
+  const StepParams& P = B.P;
+  const int64_t nn = P.n;
+  const int c = B.items[blockIdx.x].x;
+  const int g = B.items[blockIdx.x].y + (int)threadIdx.x;
+  const BatchCase C = B.cases[c];
+  const bool own = g < C.n;
+  const int64_t cell = C.off + g;
+  CellCounters cc;
+  CellPrim<NP, 1> cp;
+  if (own) {
+    double an[NP], rn[NP], pn[NP], aa[NP], am[NP], ae[NP], amom[1] = {0.}, aE = 0.;
+    const double p0 = P.sn[(int64_t)FL::P * nn + cell];
+#pragma unroll
+    for (int k = 0; k < NP; k++) {
+      an[k] = P.sn[(int64_t)(FL::A + k) * nn + cell];
+      rn[k] = P.sn[(int64_t)(FL::R + k) * nn + cell];
+      pn[k] = eos_fix_p(M.eos[k], p0);
+      aa[k] = am[k] = ae[k] = 0.;
+    }
+    const int64_t fid = C.fbase + g;
+    Flux<NP> FA, FB;  // the cell's lower and upper face
+    load_face_flux<NP, 1>(B.flux, B.nfaces, fid, FA, P.stats);
+    load_face_flux<NP, 1>(B.flux, B.nfaces, fid + 1, FB, P.stats);
+    if (g > 0) acc_face<NP, 1>(C.coefA, true, FA, an, pn, aa, am, ae, amom, aE);
+    if (g < C.n - 1) acc_face<NP, 1>(C.coefA, false, FB, an, pn, aa, am, ae, amom, aE);
+    if (g == 0) acc_face<NP, 1>(C.coefA, false, FA, an, pn, aa, am, ae, amom, aE);
+    if (g == C.n - 1) acc_face<NP, 1>(C.coefA, false, FB, an, pn, aa, am, ae, amom, aE);
+    kapila_rebuild<NP, 1, PASS>(P, M, nn, cell, B.scal[c].dt, an, rn, pn, aa, am, ae, amom, aE, cp);
+  }
+  SeedGate<NP> sg;
+  if (SEED) seed_gate<NP, 1>(P, M, own, cp, sg);
+  if (own) kapila_finish<NP, 1, PASS, false, SEED, (TYPES == EOS_DYNAMIC)>(P, M, nn, cell, cp, sg, cc);
+  // the per-bin histogram is not kept in batched mode (relax_calls / newton_evals / newton_max are)
+  block_counters(P.stats, cc.relax, cc.iters, cc.fallback, cc.seeded, cc.rejected, cc.nonfinite, 0u, cc.iters, false);
+}
+
+__global__ void k_batch_finalize(BatchScalars* s, const BatchCase* cases, int ncases) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c == 0)
-    for (int i = 0; i < nq; i++) queue[i] = 0u;
   if (c >= ncases) return;
   double dtmax = __longlong_as_double((long long)s[c].dtmax_bits);
   s[c].t += s[c].dt;
@@ -268,50 +262,53 @@ __global__ void k_batch_finalize(BatchScalars* s, const BatchCase* cases, int nc
   s[c].dtmax_bits = (unsigned long long)__double_as_longlong(1.e10);
 }
 
+// One pass: the face kernel over fitems, the cell kernel over citems; with prepare, the face kernel's shared
+// memory is configured.
 template <int NP, int TB, int PASS, int TYPES>
-static cudaError_t batch_one(const BatchParams& B, const ecg_eos* eos, double eps, int grid, cudaStream_t s,
-                             bool prepare, int* max_blocks) {
-  auto kern = k_batch<NP, TB, PASS, TYPES>;
-  const size_t base = BatchTile<NP, TB, PASS>::smem_bytes();
-  const size_t sm = base;
-  if (prepare) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)base);
-    if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(max_blocks, kern, TB, base);
-  }
+static cudaError_t batch_one(BatchParams B, const ecg_eos* eos, double eps, const int2* citems, int nf, int nc,
+                             cudaStream_t s, bool prepare) {
+  auto kern = k_batch_faces<NP, TB, PASS, TYPES>;
+  const size_t sm = BatchTile<NP, TB, PASS, TYPES>::smem_bytes();
+  if (prepare) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   Model<NP> M;
   for (int k = 0; k < NP; k++) M.eos[k] = make_eos_params(eos[k]);
   M.eps = eps;
-  kern<<<grid, TB, sm, s>>>(B, M);
+  kern<<<nf, TB, sm, s>>>(B, M);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  B.items = citems;
+  if (B.P.mlp != nullptr) k_batch_cells<NP, PASS, true, TYPES><<<nc, CELL_THREADS, 0, s>>>(B, M);
+  else k_batch_cells<NP, PASS, false, TYPES><<<nc, CELL_THREADS, 0, s>>>(B, M);
   return cudaGetLastError();
 }
 
 template <int NP, int TB, int TYPES = EOS_DYNAMIC>
-static cudaError_t batch_tb(int pass, const BatchParams& B, const ecg_eos* eos, double eps, int grid, cudaStream_t s,
-                            bool prepare, int* mb) {
-  if (pass == PASS_O1) return batch_one<NP, TB, PASS_O1, TYPES>(B, eos, eps, grid, s, prepare, mb);
-  if (pass == PASS_PRED) return batch_one<NP, TB, PASS_PRED, TYPES>(B, eos, eps, grid, s, prepare, mb);
-  return batch_one<NP, TB, PASS_CORR, TYPES>(B, eos, eps, grid, s, prepare, mb);
+static cudaError_t batch_tb(int pass, const BatchParams& B, const ecg_eos* eos, double eps, const int2* citems, int nf,
+                            int nc, cudaStream_t s, bool prepare) {
+  if constexpr (TYPES == EOS_DYNAMIC)  // the compiled-in configuration is a MUSCL one
+    if (pass == PASS_O1) return batch_one<NP, TB, PASS_O1, TYPES>(B, eos, eps, citems, nf, nc, s, prepare);
+  if (pass == PASS_PRED) return batch_one<NP, TB, PASS_PRED, TYPES>(B, eos, eps, citems, nf, nc, s, prepare);
+  return batch_one<NP, TB, PASS_CORR, TYPES>(B, eos, eps, citems, nf, nc, s, prepare);
 }
 
 // fast: two phases, SG liquid then ideal gas, no THINC -- the kernels with the EOS types compiled in
 static cudaError_t batch_launch(int np, int tb, int pass, const BatchParams& B, const ecg_eos* eos, double eps,
-                                int grid, cudaStream_t s, bool prepare, int* mb, bool fast) {
+                                const int2* citems, int nf, int nc, cudaStream_t s, bool prepare, bool fast) {
   // the batched workload's configuration: SG liquid, IG gas, van Leer everywhere
   constexpr int kSgIg = fast_code(eos_types_code<2>(ECG_EOS_SG, ECG_EOS_IG), ECG_LIM_VANLEER);
   if (np == 2 && fast) {
-    if (tb == 64) return batch_tb<2, 64, kSgIg>(pass, B, eos, eps, grid, s, prepare, mb);
-    if (tb == 128) return batch_tb<2, 128, kSgIg>(pass, B, eos, eps, grid, s, prepare, mb);
-    return batch_tb<2, 256, kSgIg>(pass, B, eos, eps, grid, s, prepare, mb);
+    if (tb == 64) return batch_tb<2, 64, kSgIg>(pass, B, eos, eps, citems, nf, nc, s, prepare);
+    if (tb == 128) return batch_tb<2, 128, kSgIg>(pass, B, eos, eps, citems, nf, nc, s, prepare);
+    return batch_tb<2, 256, kSgIg>(pass, B, eos, eps, citems, nf, nc, s, prepare);
   }
   if (np == 2) {
-    if (tb == 64) return batch_tb<2, 64>(pass, B, eos, eps, grid, s, prepare, mb);
-    if (tb == 128) return batch_tb<2, 128>(pass, B, eos, eps, grid, s, prepare, mb);
-    return batch_tb<2, 256>(pass, B, eos, eps, grid, s, prepare, mb);
+    if (tb == 64) return batch_tb<2, 64>(pass, B, eos, eps, citems, nf, nc, s, prepare);
+    if (tb == 128) return batch_tb<2, 128>(pass, B, eos, eps, citems, nf, nc, s, prepare);
+    return batch_tb<2, 256>(pass, B, eos, eps, citems, nf, nc, s, prepare);
   }
-  if (tb == 64) return batch_tb<3, 64>(pass, B, eos, eps, grid, s, prepare, mb);
-  if (tb == 128) return batch_tb<3, 128>(pass, B, eos, eps, grid, s, prepare, mb);
-  return batch_tb<3, 256>(pass, B, eos, eps, grid, s, prepare, mb);
+  if (tb == 64) return batch_tb<3, 64>(pass, B, eos, eps, citems, nf, nc, s, prepare);
+  if (tb == 128) return batch_tb<3, 128>(pass, B, eos, eps, citems, nf, nc, s, prepare);
+  return batch_tb<3, 256>(pass, B, eos, eps, citems, nf, nc, s, prepare);
 }
 
 }  // namespace ecg
@@ -335,11 +332,12 @@ struct ecg_batch {
   unsigned long long* dummy_dtmax = nullptr;
   double* dummy_dt = nullptr;
   DevStats* stats = nullptr;
-  unsigned int* queue = nullptr;
-  int2* items = nullptr;
-  int nitems = 0;
-  int tile = 0, threads = 0;
-  int grid = 0;
+  double* flux = nullptr;   // face fluxes, 3N + 4 per face
+  int64_t nfaces = 0;
+  int2* items = nullptr;    // face items of the current tile
+  int2* citems = nullptr;   // cell items
+  int nitems = 0, ncitems = 0;
+  int tile = 0;
   int cur = 0;
   int newton_cap = 100;
   MlpDev* mlp = nullptr;
@@ -366,15 +364,16 @@ void drop_graphs(ecg_batch* b) {
     }
 }
 
-ecg_status build_items(ecg_batch* b, int tile) {
+// (case, first entry) of every chunk of `chunk` of each case's n + extra entries
+ecg_status build_items(const ecg_batch* b, int chunk, int extra, int2** out, int* count) {
   std::vector<int2> it;
   for (int c = 0; c < b->ncases; c++)
-    for (int s = 0; s < b->hcases[c].n; s += tile - ECG_BATCH_ITEM_TRIM) it.push_back(make_int2(c, s));
-  cudaFree(b->items);
-  b->items = nullptr;
-  BCUDA(cudaMalloc(&b->items, sizeof(int2) * it.size()));
-  BCUDA(cudaMemcpy(b->items, it.data(), sizeof(int2) * it.size(), cudaMemcpyHostToDevice));
-  b->nitems = (int)it.size();
+    for (int s = 0; s < b->hcases[c].n + extra; s += chunk) it.push_back(make_int2(c, s));
+  cudaFree(*out);
+  *out = nullptr;
+  BCUDA(cudaMalloc(out, sizeof(int2) * it.size()));
+  BCUDA(cudaMemcpy(*out, it.data(), sizeof(int2) * it.size(), cudaMemcpyHostToDevice));
+  *count = (int)it.size();
   return ECG_OK;
 }
 
@@ -383,24 +382,15 @@ ecg_status set_shape(ecg_batch* b, int tile) {
     set_error("tile must be 64, 128 or 256 cells");
     return ECG_ERR_INVALID;
   }
-  int sms = 0, dev = 0;
-  BCUDA(cudaGetDevice(&dev));
-  BCUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  int occ = 1 << 30;
   BatchParams B{};
-  for (int pass = 0; pass < 3; pass++) {
-    int mb = 0;
-    BCUDA(batch_launch(b->np, tile, pass, B, b->c0.eos, b->eps, 0, b->stream, true, &mb, b->fast));
-    if ((b->order == 1 && pass == PASS_O1) || (b->order == 2 && pass != PASS_O1)) occ = std::min(occ, std::max(mb, 1));
-  }
+  for (int pass = 0; pass < 3; pass++)
+    BCUDA(batch_launch(b->np, tile, pass, B, b->c0.eos, b->eps, nullptr, 0, 0, b->stream, true, b->fast));
   b->tile = tile;
-  b->threads = tile;
-  b->grid = sms * occ;
   drop_graphs(b);
-  return build_items(b, tile);
+  return build_items(b, tile - 1, 1, &b->items, &b->nitems);
 }
 
-ecg_status launch_pass(ecg_batch* b, int pass, double* q, double* sn, double* out, unsigned int* queue) {
+ecg_status launch_pass(ecg_batch* b, int pass, double* q, double* sn, double* out) {
   BatchParams B{};
   B.P.done = b->done;
   B.P.q = q;
@@ -418,9 +408,10 @@ ecg_status launch_pass(ecg_batch* b, int pass, double* q, double* sn, double* ou
   B.cases = b->cases;
   B.scal = b->scal;
   B.items = b->items;
-  B.nitems = b->nitems;
-  B.queue = queue;
-  BCUDA(batch_launch(b->np, b->tile, pass, B, b->c0.eos, b->eps, b->grid, b->stream, false, nullptr, b->fast));
+  B.flux = b->flux;
+  B.nfaces = b->nfaces;
+  BCUDA(batch_launch(b->np, b->tile, pass, B, b->c0.eos, b->eps, b->citems, b->nitems, b->ncitems, b->stream, false,
+                     b->fast));
   return ECG_OK;
 }
 
@@ -429,13 +420,13 @@ ecg_status launch_step(ecg_batch* b, int parity) {
   double* s1 = b->state[1 - parity];
   ecg_status s;
   if (b->order == 1) {
-    s = launch_pass(b, PASS_O1, sn, sn, s1, b->queue);
+    s = launch_pass(b, PASS_O1, sn, sn, s1);
   } else {
-    s = launch_pass(b, PASS_PRED, sn, sn, b->half, b->queue);
-    if (s == ECG_OK) s = launch_pass(b, PASS_CORR, b->half, sn, s1, b->queue + 1);
+    s = launch_pass(b, PASS_PRED, sn, sn, b->half);
+    if (s == ECG_OK) s = launch_pass(b, PASS_CORR, b->half, sn, s1);
   }
   if (s != ECG_OK) return s;
-  k_batch_finalize<<<(b->ncases + 255) / 256, 256, 0, b->stream>>>(b->scal, b->cases, b->ncases, b->queue, 2);
+  k_batch_finalize<<<(b->ncases + 255) / 256, 256, 0, b->stream>>>(b->scal, b->cases, b->ncases);
   BCUDA(cudaGetLastError());
   return ECG_OK;
 }
@@ -522,6 +513,7 @@ extern "C" ecg_status ecg_batch_create(const ecg_case* cs, int32_t ncases, ecg_b
     const ecg_case& x = cs[c];
     BatchCase h{};
     h.off = off;
+    h.fbase = off + c;  // n + 1 faces per case
     h.n = x.ncells[0];
     double dX = x.length[0] / (double)x.ncells[0], dY = x.length[1] / (double)x.ncells[1],
            dZ = x.length[2] / (double)x.ncells[2];
@@ -533,6 +525,7 @@ extern "C" ecg_status ecg_batch_create(const ecg_case* cs, int32_t ncases, ecg_b
     off += h.n;
   }
   b->total = off;
+  b->nfaces = off + ncases;
   auto fail = [&](ecg_status s) {
     ecg_batch_destroy(b);
     return s;
@@ -551,7 +544,8 @@ extern "C" ecg_status ecg_batch_create(const ecg_case* cs, int32_t ncases, ecg_b
   if ((e = cudaMalloc(&b->dummy_dtmax, sizeof(unsigned long long))) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
   if ((e = cudaMalloc(&b->dummy_dt, sizeof(double))) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
   if ((e = cudaMalloc(&b->stats, sizeof(DevStats))) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
-  if ((e = cudaMalloc(&b->queue, 2 * sizeof(unsigned int))) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
+  if ((e = cudaMalloc(&b->flux, sizeof(double) * (size_t)(3 * b->np + 4) * (size_t)b->nfaces)) != cudaSuccess)
+    return fail(bfail(e, "cudaMalloc(face fluxes)"));
   cudaMemcpy(b->cases, b->hcases.data(), sizeof(BatchCase) * ncases, cudaMemcpyHostToDevice);
   std::vector<BatchScalars> hs(ncases);
   double big = 1.e10;
@@ -563,11 +557,11 @@ extern "C" ecg_status ecg_batch_create(const ecg_case* cs, int32_t ncases, ecg_b
   }
   cudaMemcpy(b->scal, hs.data(), sizeof(BatchScalars) * ncases, cudaMemcpyHostToDevice);
   cudaMemset(b->done, 0, sizeof(int));
-  cudaMemset(b->queue, 0, 2 * sizeof(unsigned int));
   cudaMemset(b->stats, 0, sizeof(DevStats));
   cudaMemset(b->state[0], 0, sb);
   cudaMemset(b->state[1], 0, sb);
-  ecg_status s = set_shape(b, 128);
+  ecg_status s = build_items(b, CELL_THREADS, 0, &b->citems, &b->ncitems);
+  if (s == ECG_OK) s = set_shape(b, 128);
   if (s != ECG_OK) return fail(s);
   *out = b;
   return ECG_OK;
@@ -587,8 +581,9 @@ extern "C" void ecg_batch_destroy(ecg_batch* b) {
   cudaFree(b->dummy_dtmax);
   cudaFree(b->dummy_dt);
   cudaFree(b->stats);
-  cudaFree(b->queue);
+  cudaFree(b->flux);
   cudaFree(b->items);
+  cudaFree(b->citems);
   cudaFree(b->mlp);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;

@@ -94,6 +94,15 @@ __device__ __forceinline__ double ndiv(double a, double b) {
   return (q1 == q1) ? q1 : a * y0;  // NaN only when an operand is zero, infinite or NaN
 }
 
+// The reciprocal ndiv divides by, for cdiv with a divisor shared by several quotients (b normal).
+__device__ __forceinline__ double nrcp(double b) {
+  const double y0 = rcp_approx(b);
+  double e = fma(-b, y0, 1.0);
+  double y = fma(y0, e, y0);
+  e = fma(-b, y, 1.0);
+  return fma(y, e, y);
+}
+
 // a / b for a divisor whose correctly rounded reciprocal y = RN(1/b) is at hand (EOS constants, computed on
 // the host): Markstein's correction alone.
 __device__ __forceinline__ double cdiv(double a, double b, double y) {

@@ -335,8 +335,8 @@ ecg_status ecg_trainer_set_norm(ecg_trainer* tr, const float* in_shift, const fl
 ecg_status ecg_trainer_set_norm_out1(ecg_trainer* tr, float out_shift, float out_scale);
 
 /* ------------------------------------------------------------------ batched independent cases */
-/* Many independent 1D cases of uneven cell counts advanced together by one persistent kernel per
- * pass that pulls (case, tile) work items from a device queue; each case keeps its own dt
+/* Many independent 1D cases of uneven cell counts advanced together, two launches per pass over all of
+ * them (face fluxes, cells); each case keeps its own dt
  * (segmented min-reduction) and time.  All cases must share model, phases, EOS, order and
  * limiters; their cell counts, lengths, CFL and initial states differ.  The reference runs such
  * cases one after another (src/main.cpp:82-133). */
@@ -349,8 +349,8 @@ ecg_status ecg_batch_download_prim(ecg_batch* b, double* const* fields, int64_t 
 /* Advance every case nsteps steps (each with its own dt); dt/t arrays of ncases (may be NULL). */
 ecg_status ecg_batch_step(ecg_batch* b, int32_t nsteps, double* dt, double* t, ecg_step_stats* stats);
 ecg_status ecg_batch_set_seed_model(ecg_batch* b, const ecg_mlp* mlp);
-/* Tile = threads per block (64, 128 or 256; 0 = autotuned); a work item covers tile - 1 cells of one
- * case, so its tile faces take one round of the block.  threads must be 0 or equal to tile. */
+/* Tile = threads per block of the face kernel (64, 128 or 256; 0 = autotuned); a work item covers
+ * tile - 1 faces of one case.  threads must be 0 or equal to tile. */
 ecg_status ecg_batch_set_shape(ecg_batch* b, int32_t tile, int32_t threads);
 ecg_status ecg_batch_autotune(ecg_batch* b, int32_t* tile, int32_t* threads);
 int64_t ecg_batch_total_cells(const ecg_batch* b);
