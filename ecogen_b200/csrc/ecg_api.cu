@@ -116,6 +116,7 @@ struct ecg_ctx {
   double* tmp = nullptr;      // download scratch (mixture pressure)
   double* flux[3] = {nullptr, nullptr, nullptr};  // face arrays of the split form (Kapila 2D / 3D)
   bool split = false;         // step passes in split form (face kernels + cell kernel)
+  FaceStreams fstreams{};     // auxiliary streams of the face kernels (split forms)
   FaceMaps fmaps{};           // tensor maps of the face kernels' TMA staging (fmaps.ok = 0: none)
   int staging = ECG_STAGING_TMA;
   DevScalars* scal = nullptr;
@@ -276,6 +277,7 @@ ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
   P.ptmu_seed_p = x->ptmu_seed_p;
   P.tsat_hist = x->tsat_hist;
   for (int a = 0; a < 3; a++) P.flux[a] = x->split ? x->flux[a] : nullptr;
+  P.fstreams = x->fstreams.fork ? &x->fstreams : nullptr;
   P.fmaps = (x->split && x->staging == ECG_STAGING_TMA && x->fmaps.ok) ? &x->fmaps : nullptr;
   double* sn = x->state[parity];
   double* s1 = x->state[1 - parity];
@@ -561,6 +563,12 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
       if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaMalloc(face fluxes)"));
     }
     x->split = true;
+    for (int a = 0; a + 1 < x->dim && e == cudaSuccess; a++) {
+      e = cudaStreamCreateWithFlags(&x->fstreams.s[a], cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->fstreams.join[a], cudaEventDisableTiming);
+    }
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->fstreams.fork, cudaEventDisableTiming);
+    if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaStreamCreate(face streams)"));
 #ifndef ECG_BOUNDS_CHECK
     // TMA staging of the face kernels' tiles where the layout allows it (the bounds-checked build
     // checks the kernels' own loads, so it stages them that way)
@@ -660,6 +668,11 @@ extern "C" void ecg_destroy(ecg_ctx* x) {
   cudaFree(x->rec_y);
   cudaFree(x->rec_count);
   cudaFree(x->tsat_hist);
+  for (int a = 0; a < 2; a++) {
+    if (x->fstreams.s[a]) cudaStreamDestroy(x->fstreams.s[a]);
+    if (x->fstreams.join[a]) cudaEventDestroy(x->fstreams.join[a]);
+  }
+  if (x->fstreams.fork) cudaEventDestroy(x->fstreams.fork);
   if (x->stream) cudaStreamDestroy(x->stream);
   delete x;
 }

@@ -165,8 +165,9 @@ __global__ void __launch_bounds__(TB, ECG_BATCH_SM_THREADS / TB) k_batch_faces(B
         cell_thermo<NP, 1>(M, sq, RS, rl, tl, ug);
         cell_thermo<NP, 1>(M, sq, RS, rr, tr, vg);
       } else if (LSL) {
-        extrapolate_side<NP, 1>(M, sq, RS, rl, ssl, SS, tid, fabs(pf - pl), 1., pone, tl, ug);
-        extrapolate_side<NP, 1>(M, sq, RS, rr, ssl, SS, tid + 1, fabs(pf - pr), -1., pone, tr, vg);
+        extrapolate_side<NP, 1>(M, sq, RS, rl, ssl, SS, tid, 0, 0, 0, fabs(pf - pl), 1., pone, tl, ug);
+        extrapolate_side<NP, 1>(M, sq, RS, rr, ssl, SS, tid + 1, 0, 0, 0, fabs(pf - pr), -1., pone, tr,
+                                vg);
       } else {
         const int f1 = tid + 1;
         const bool hasL = (gl - 1 >= 0), hasR = (gl + 2 < n);

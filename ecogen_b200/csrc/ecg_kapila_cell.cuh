@@ -123,11 +123,12 @@ __device__ __forceinline__ void cell_slopes(const Model<NP>& M, const double* sq
 }
 
 // One side of an internal face from the cell's limited slopes: reconstruct_side's extrapolation and clamps.
-// pone: no pressure of the block's cells is below a floor (one slope and one extrapolation for all phases).
+// u: the velocities of the planes pn (normal), p1, p2 (transverse).  pone: no pressure of the block's cells is
+// below a floor (one slope and one extrapolation for all phases).
 template <int NP, int DIM>
 __device__ __forceinline__ void extrapolate_side(const Model<NP>& M, const double* sq, int RS, int rc, const double* lsl,
-                                                 int LS, int ec, double dist, double sign, bool pone, Thermo<NP>& t,
-                                                 double u[3]) {
+                                                 int LS, int ec, int pn, int p1, int p2, double dist, double sign,
+                                                 bool pone, Thermo<NP>& t, double u[3]) {
   using FL = Fields<NP, DIM>;
   const double pc = sq[FL::P * RS + rc];
 #pragma unroll
@@ -149,9 +150,10 @@ __device__ __forceinline__ void extrapolate_side(const Model<NP>& M, const doubl
     for (int k = 0; k < NP; k++)
       t.p[k] = eos_fix_p(M.eos[k], eos_fix_p(M.eos[k], pc) + (sign * lsl[(2 * NP + k) * LS + ec]) * dist);
   }
-  u[0] = u[1] = u[2] = 0.;
-#pragma unroll
-  for (int d = 0; d < DIM; d++) u[d] = sq[(FL::U + d) * RS + rc] + (sign * lsl[(3 * NP + d) * LS + ec]) * dist;
+  auto vel = [&](int d) { return sq[(FL::U + d) * RS + rc] + (sign * lsl[(3 * NP + d) * LS + ec]) * dist; };
+  u[0] = vel(pn);
+  u[1] = DIM > 1 ? vel(p1) : 0.;
+  u[2] = DIM > 2 ? vel(p2) : 0.;
   fulfill<NP, true>(M, t);
 }
 

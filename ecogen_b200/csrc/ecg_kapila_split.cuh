@@ -1,5 +1,5 @@
-// Split form of a Kapila step pass for 2D and 3D meshes: one face-flux kernel per axis, then one cell
-// kernel.
+// Split form of a Kapila step pass for 2D and 3D meshes: one face-flux kernel per axis, side by side, then
+// one cell kernel.
 //
 // The fused pass (ecg_kapila_kernel.cuh) stages a tile per axis, computes its faces and accumulates
 // them in one kernel: every block runs the whole pass (both axes' slopes, reconstructions and HLLC
@@ -7,8 +7,7 @@
 // HLLC branch wait at the barrier for the ones sampling a star state, and the kernel's code (one copy
 // of the face work per axis) is larger than the instruction cache.  The split form trades HBM
 // traffic, of which the pass uses a few percent, for latency:
-//   k_kapila_faces<AX>  one thread per face normal to axis AX: stage the cells and the face slopes of a
-//                        block (one barrier), then reconstruct both sides and solve HLLC exactly as the
+//   k_kapila_faces       one thread per face: stage the cells and the slopes of a block (one barrier), then reconstruct both sides and solve HLLC exactly as the
 //                        fused pass does, including the domain sides (non-reflecting: HLLC(cell, cell) in
 //                        the side's frame; symmetry: the reflecting flux of the MUSCL buffer cell), and
 //                        store the face flux (3N + d + 3 doubles) in a face array of the axis;
@@ -21,32 +20,23 @@
 // Every flux is computed once, by the same device functions in the same operation order, and each cell
 // accumulates the same values in the same order, so the split and fused forms give identical bits.
 //
-// Face arrays (per axis, structure of arrays, NFL components of nfaces(AX) doubles): the face between
-// cells f-1 and f along AX (f = 0 and f = n_AX are the domain sides) of the line at the other
-// coordinates has index  f + (nx+1)(j + ny k)  (X),  i + nx (f + (ny+1) k)  (Y),  i + nx (j + ny f)  (Z),
-// so that consecutive threads of either kernel touch consecutive faces.
+// Face arrays: per axis, structure of arrays, NFL components of nfaces(AX) doubles (split_fid, ecg_faces.cuh).
 #pragma once
+#include "ecg_faces.cuh"
 #include "ecg_kapila_kernel.cuh"
-#include "ecg_tma.cuh"
 
 namespace ecg {
 
-__device__ __forceinline__ int64_t split_fid(const int n[3], int ax, int f, int i, int j, int k) {
-  if (ax == 0) return (int64_t)f + (int64_t)(n[0] + 1) * ((int64_t)j + (int64_t)n[1] * k);
-  if (ax == 1) return (int64_t)i + (int64_t)n[0] * ((int64_t)f + (int64_t)(n[1] + 1) * k);
-  return (int64_t)i + (int64_t)n[0] * ((int64_t)j + (int64_t)n[1] * f);
-}
-
-template <int NP, int DIM, int AX, int PASS, int TYPES>
+template <int NP, int DIM, int PASS, int TYPES>
 struct FaceKernelShape {
   using FL = Fields<NP, DIM>;
-  using FT = FaceTile<AX>;
   static constexpr bool O2 = (PASS != PASS_O1);
   // one limiter compiled in: limited slopes per cell (cell_slopes), no interface detector
   static constexpr bool LSL = O2 && code_limiter(TYPES) >= 0;
   static constexpr int NA0 = (PASS == PASS_CORR && !LSL) ? 1 : 0;  // separate time-n alpha_0 plane
-  static constexpr int SS = LSL ? FT::LS : FT::SS;                 // one slope plane
-  static constexpr size_t staged_bytes() { return sizeof(double) * (size_t)FT::RS * (FL::NQ + NA0); }
+  static constexpr int RS = FACE_RS;
+  static constexpr int SS = LSL ? FACE_LS : FACE_SS;               // one slope plane
+  static constexpr size_t staged_bytes() { return sizeof(double) * (size_t)RS * (FL::NQ + NA0); }
   // staged planes, slope planes, the staging mbarrier, and room to align the base to 128 bytes
   static constexpr size_t smem_bytes() {
     return staged_bytes() + (O2 ? sizeof(double) * (size_t)SS * FL::NSL : 0) + sizeof(uint64_t) + 128;
@@ -89,40 +79,50 @@ struct FaceKernelShape {
 constexpr int CELL_THREADS = 128;
 __host__ __device__ constexpr int cell_threads(bool ptmu) { return ptmu ? ECG_CELL_PTMU_THREADS : CELL_THREADS; }
 
+// The faces normal to AX, one block per tile.  The transverse velocities enter without the sign changes of
+// the face frames (src/Meshes/MeshCartesian.cpp:281-557); they only occur squared and as factors of their own
+// momentum flux, whose sign changes back.
 template <int NP, int DIM, int AX, int PASS, int TYPES>
-__global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D : ECG_FACE_MINB_3D)
-    k_kapila_faces(StepParams P, Geometry G, Model<NP> M0, double* __restrict__ flux,
-                   const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap ma0, int tma) {
+__global__ void __launch_bounds__(FACE_THREADS, DIM == 2 ? ECG_FACE_MINB_2D : ECG_FACE_MINB_3D)
+    k_kapila_faces(StepParams P, Geometry G, Model<NP> M0, const __grid_constant__ FaceLaunch L) {
   const Model<NP> M = specialize_eos<NP, TYPES>(M0);
-  using FT = FaceTile<AX>;
-  using KS = FaceKernelShape<NP, DIM, AX, PASS, TYPES>;
+  using KS = FaceKernelShape<NP, DIM, PASS, TYPES>;
   using FL = Fields<NP, DIM>;
   constexpr bool O2 = KS::O2, LSL = KS::LSL;
-  constexpr int RS = FT::RS, SS = KS::SS, CP = FT::CP;
+  constexpr int RS = KS::RS, SS = KS::SS, ax = AX;
   extern __shared__ unsigned char smem_raw[];
   double* smem = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
   double* sq = smem;                                // [NQ][RS]
   double* sa0 = sq + (size_t)FL::NQ * RS;           // [NA0][RS]
   double* ssl = sa0 + (size_t)KS::NA0 * RS;         // [NSL][SS]
   const double* a0 = KS::NA0 ? sa0 : sq;            // time-n alpha_0 plane
-
   if (*P.done) return;
   const int tid = threadIdx.x;
-  const int nax = G.n[AX];
-  const int ob = (AX == 0) ? 1 : 0;                 // the lines' axis
-  const int f0 = (int)(AX == 0 ? blockIdx.x : blockIdx.y) * FT::TF;
-  const int l0 = (int)(AX == 0 ? blockIdx.y : blockIdx.x) * FT::W;
-  const int third = (int)blockIdx.z;                // Z for X and Y faces, Y for Z faces
+  constexpr bool isx = ax == 0;
+  const FacePlace B = face_place<AX>();
+  const int f0 = B.f0, l0 = B.l0, third = B.third;
+  // tile: TF faces per line; a staged plane and a slope plane as [line][position] (X) or [position][line]
+  constexpr int TF = isx ? FaceTile<0>::TF : FaceTile<1>::TF;
+  constexpr int PS = isx ? 1 : FaceTile<1>::W;          // stride of a position (staged planes and slope planes)
+  constexpr int CL = isx ? FaceTile<0>::CP : 1;         // stride of a line, staged planes
+  constexpr int SL = isx ? (LSL ? FaceTile<0>::LP : FaceTile<0>::SP) : 1;  // ..., slope planes
+  constexpr int nsl = LSL ? (isx ? FaceTile<0>::LS : FaceTile<1>::LS) : (isx ? FaceTile<0>::SS : FaceTile<1>::SS);
+  const int nax = G.n[ax];
+  constexpr int ob = isx ? 1 : 0;                       // the lines' axis
   const int64_t nn = P.n;
-  // global cell coordinates of (line, position along AX)
-  auto coords = [&](int line, int gpos, int g[3]) {
-    g[AX] = gpos;
-    g[ob] = l0 + line;
-    g[AX == 2 ? 1 : 2] = third;
+  // (line, position) of entry e of a plane whose lines hold `len` entries
+  auto place = [&](int e, int len, int& line, int& pos) {
+    if (isx) {
+      line = e / len;
+      pos = e - line * len;
+    } else {
+      line = e % FaceTile<1>::W;
+      pos = e / FaceTile<1>::W;
+    }
   };
 
-  // ---- stage the cells f0-2 .. f0-3+CP of every line
-  if (tma) {
+  // ---- stage the cells from f0 - 2 of every line
+  if (L.tma) {
     // one tensor copy of the box (x, y[, z], field) for all primitive fields, one for the time-n
     // alpha_0 plane; cells outside the mesh arrive as zeros
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + KS::staged_bytes() / sizeof(double) +
@@ -131,27 +131,26 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
     __syncthreads();
     if (tid == 0) {
       mbar_expect_tx(bar, (uint32_t)KS::staged_bytes());
-      int o[3];  // box origin along x, y, z
-      o[AX] = f0 - 2;
-      o[ob] = l0;
-      o[AX == 2 ? 1 : 2] = third;
+      // box origin along x, y, z
+      const int ox = isx ? f0 - 2 : l0, oy = isx ? l0 : (ax == 1 ? f0 - 2 : third), oz = ax == 2 ? f0 - 2 : third;
       if (DIM == 3) {
-        tma_load_4d(sq, &mq, bar, o[0], o[1], o[2], 0);
-        if (KS::NA0) tma_load_4d(sa0, &ma0, bar, o[0], o[1], o[2], FL::A);
+        tma_load_4d(sq, &L.q, bar, ox, oy, oz, 0);
+        if (KS::NA0) tma_load_4d(sa0, &L.a0, bar, ox, oy, oz, FL::A);
       } else {
-        tma_load_3d(sq, &mq, bar, o[0], o[1], 0);
-        if (KS::NA0) tma_load_3d(sa0, &ma0, bar, o[0], o[1], FL::A);
+        tma_load_3d(sq, &L.q, bar, ox, oy, 0);
+        if (KS::NA0) tma_load_3d(sa0, &L.a0, bar, ox, oy, FL::A);
       }
     }
     // bounded wait; a copy that never lands is reported to the host (the step then fails)
     if (!mbar_wait_bounded(bar, 0, 1 << 22) && (tid & 31) == 0) atomicAdd(&P.stats->staging_timeouts, 1ull);
   } else {
-    for (int e = tid; e < RS; e += FT::NTH) {
-      const int line = AX == 0 ? e / CP : e % FT::W, pos = AX == 0 ? e % CP : e / FT::W;
-      int g[3];
-      coords(line, f0 - 2 + pos, g);
-      if (g[AX] >= 0 && g[AX] < nax && g[ob] < G.n[ob]) {
-        const int64_t c = (int64_t)g[0] + (int64_t)g[1] * G.n[0] + (int64_t)g[2] * G.n[0] * G.n[1];
+    for (int e = tid; e < RS; e += FACE_THREADS) {
+      int line, pos;
+      place(e, FaceTile<0>::CP, line, pos);
+      const int g = f0 - 2 + pos;
+      if (pos < TF + 3 && g >= 0 && g < nax && l0 + line < G.n[ob]) {
+        const int gx0 = isx ? g : l0 + line, gy0 = isx ? l0 + line : (ax == 1 ? g : third), gz0 = ax == 2 ? g : third;
+        const int64_t c = gx0 + (int64_t)G.n[0] * (gy0 + (int64_t)G.n[1] * gz0);
         if (!ECG_IN_BOUNDS(P.stats, c, nn)) continue;
 #pragma unroll
         for (int f = 0; f < FL::NQ; f++) sq[f * RS + e] = P.q[(int64_t)f * nn + c];
@@ -160,17 +159,20 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
     }
   }
   __syncthreads();
+  const double* dcc = G.dcc[ax];
   // ---- limited slopes (MUSCL, one limiter): cell f0 - 1 + s of every line, s in [0, TF]
   bool pone = true;  // no pressure read by this block's faces is below a phase's floor
   if (LSL) {
     double pf = M.eos[0].pfloor;
 #pragma unroll
     for (int k = 1; k < NP; k++) pf = dmax(pf, M.eos[k].pfloor);
-    for (int e = tid; e < SS; e += FT::NTH) {
-      const int line = AX == 0 ? e / FT::LP : e % FT::W, s = AX == 0 ? e % FT::LP : e / FT::W;
+    const double* rdcc = G.rdcc[ax];
+    for (int e = tid; e < nsl; e += FACE_THREADS) {
+      int line, s;
+      place(e, FaceTile<0>::LP, line, s);
       const int c = f0 - 1 + s;
       if (c < 0 || c >= nax || l0 + line >= G.n[ob]) continue;
-      const int rc = FT::cidx(line, s + 1);
+      const int rc = line * CL + (s + 1) * PS;
       if (c == 0 || c == nax - 1) {
         // no face beyond: the missing slope is zero, and so is every limited one, except the velocity
         // along the axis at a symmetry side, whose slope there is u over the centre-to-face coordinate
@@ -178,43 +180,42 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
 #pragma unroll
         for (int f = 0; f < FL::NSL; f++) ssl[f * SS + e] = 0.;
         const int sd = c == 0 ? 0 : 1;
-        const double wd = G.wslope[2 * AX + sd];
-        if (G.bc[2 * AX + sd] == ECG_BC_SYMMETRY && fabs(wd) > 1.e-8) {
-          const double* su = sq + (FL::U + AX) * RS;
-          const double so = sd ? ndiv(su[rc] - su[FT::cidx(line, s)], G.dcc[AX][c - 1])
-                               : ndiv(su[FT::cidx(line, s + 2)] - su[rc], G.dcc[AX][c]);
-          ssl[(3 * NP + AX) * SS + e] = limiter(code_limiter(TYPES), ndiv(su[rc], wd), so);
+        const double wd = G.wslope[2 * ax + sd];
+        if (G.bc[2 * ax + sd] == ECG_BC_SYMMETRY && fabs(wd) > 1.e-8) {
+          const double* su = sq + (FL::U + ax) * RS;
+          const double so = sd ? ndiv(su[rc] - su[rc - PS], dcc[c - 1]) : ndiv(su[rc + PS] - su[rc], dcc[c]);
+          ssl[(3 * NP + ax) * SS + e] = limiter(code_limiter(TYPES), ndiv(su[rc], wd), so);
         }
         pone = pone && sq[FL::P * RS + rc] >= pf;
         continue;
       }
-      const int prev = FT::cidx(line, s), next = FT::cidx(line, s + 2);
-      const bool one = sq[FL::P * RS + prev] >= pf && sq[FL::P * RS + rc] >= pf && sq[FL::P * RS + next] >= pf;
+      const bool one = sq[FL::P * RS + rc - PS] >= pf && sq[FL::P * RS + rc] >= pf && sq[FL::P * RS + rc + PS] >= pf;
       pone = pone && one;
-      cell_slopes<NP, DIM, code_limiter(TYPES)>(M, sq, RS, prev, rc, next, G.dcc[AX][c - 1], G.rdcc[AX][c - 1],
-                                                G.dcc[AX][c], G.rdcc[AX][c], one, ssl, SS, e);
+      cell_slopes<NP, DIM, code_limiter(TYPES)>(M, sq, RS, rc - PS, rc, rc + PS, dcc[c - 1], rdcc[c - 1], dcc[c], rdcc[c],
+                                                one, ssl, SS, e);
     }
     pone = __syncthreads_and(pone);
   }
   // ---- face slopes (MUSCL): slope s at face g = f0 - 1 + s, between cells g-1 and g
   if (O2 && !LSL) {
-    for (int e = tid; e < SS; e += FT::NTH) {
-      const int line = AX == 0 ? e / FT::SP : e % FT::W, s = AX == 0 ? e % FT::SP : e / FT::W;
+    for (int e = tid; e < nsl; e += FACE_THREADS) {
+      int line, s;
+      place(e, FaceTile<0>::SP, line, s);
       const int gl = f0 - 2 + s;  // left cell of the face
       if (l0 + line >= G.n[ob]) continue;
-      const int rl = FT::cidx(line, s), rr = FT::cidx(line, s + 1);
+      const int rl = line * CL + s * PS, rr = rl + PS;
       if (gl < 0 || gl + 1 >= nax) {
         // a side of the domain: slopes only on a symmetry side, the velocity along the axis over the
         // centre-to-face coordinate (BoundCondWallO2Cartesian::computeSlopes :84-108)
         const int sd = (gl == -1) ? 0 : ((gl == nax - 1) ? 1 : -1);
-        if (sd < 0 || G.bc[2 * AX + sd] != ECG_BC_SYMMETRY) continue;
+        if (sd < 0 || G.bc[2 * ax + sd] != ECG_BC_SYMMETRY) continue;
 #pragma unroll
         for (int f = 0; f < FL::NSL; f++) ssl[f * SS + e] = 0.;
-        const double wd = G.wslope[2 * AX + sd];
-        if (fabs(wd) > 1.e-8) ssl[(3 * NP + AX) * SS + e] = ndiv(sq[(FL::U + AX) * RS + (sd ? rl : rr)], wd);
+        const double wd = G.wslope[2 * ax + sd];
+        if (fabs(wd) > 1.e-8) ssl[(3 * NP + ax) * SS + e] = ndiv(sq[(FL::U + ax) * RS + (sd ? rl : rr)], wd);
         continue;
       }
-      const double d = G.dcc[AX][gl];
+      const double d = dcc[gl];
 #pragma unroll
       for (int k = 0; k < NP; k++) {
         ssl[k * SS + e] = ndiv(sq[(FL::A + k) * RS + rr] - sq[(FL::A + k) * RS + rl], d);
@@ -232,16 +233,28 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
   // ---- one face per thread
   double wmax = wave_none(G.stretched);
   {
-    const int line = AX == 0 ? tid / FT::TF : tid % FT::W, fl = AX == 0 ? tid % FT::TF : tid / FT::W;
+    int line, fl;
+    place(tid, FaceTile<0>::TF, line, fl);
     const int f = f0 + fl;
-    int g[3];
-    coords(line, f, g);
-    // (bounds-checked builds: the staged cells this face reads, positions fl .. fl + 3 of its line)
-    if (f <= nax && g[ob] < G.n[ob] && ECG_IN_BOUNDS(P.stats, FT::cidx(line, fl), RS) &&
-        ECG_IN_BOUNDS(P.stats, FT::cidx(line, fl + 3), RS)) {
+    const int lg = l0 + line;
+    // CFL length of the line's cell at position g
+    auto lcfl = [&](int g) {
+      return G.stretched ? cell_lcfl(G, isx ? g : lg, isx ? lg : (ax == 1 ? g : third), ax == 2 ? g : third) : G.lcfl;
+    };
+    const int rl = line * CL + (fl + 1) * PS, rr = rl + PS;  // the cells on its two sides
+    const int el = line * SL + fl * PS;                      // limited slopes of the left one; face slope below
+    // (bounds-checked builds: the staged cells this face reads)
+    if (f <= nax && lg < G.n[ob] && ECG_IN_BOUNDS(P.stats, rl - PS, RS) && ECG_IN_BOUNDS(P.stats, rr + PS, RS)) {
       Flux<NP> F;
       double Fn[3];
-      const int gl = f - 1;
+      // planes of the normal and the transverse velocities
+      constexpr int pn = ax, p1 = isx ? 1 : 0, p2 = ax == 2 ? 1 : 2;
+      auto local = [&](const double u[3], bool neg, double l[3]) {
+        l[0] = isx ? u[0] : (ax == 1 ? u[1] : u[2]);
+        l[1] = isx ? u[1] : u[0];
+        l[2] = ax == 2 ? u[1] : u[2];
+        if (neg) l[0] = -l[0];
+      };
       if (f == 0 || f == nax) {
         // a side: non-reflecting HLLC(cell, cell) in the side's frame (BoundCondNonReflecting::
         // solveRiemannBoundary src/BoundConds/BoundCondNonReflecting.cpp:62), or a symmetry side's
@@ -249,23 +262,20 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
         // MUSCL-extrapolated towards the side (BoundCondWallO2Cartesian::solveRiemann :111-141)
         const int sd = (f == 0) ? 0 : 1;
         const bool neg = sd == 0;
-        const int rc = FT::cidx(line, sd == 0 ? fl + 2 : fl + 1);
-        int gc[3] = {g[0], g[1], g[2]};  // the side's cell
-        gc[AX] = sd == 0 ? 0 : nax - 1;
-        const double lc = cell_lcfl(G, gc[0], gc[1], gc[2]);
+        const int rc = sd == 0 ? rr : rl;
+        const double lc = lcfl(sd == 0 ? 0 : nax - 1);
         Thermo<NP> t;
         double ug[3], ul[3];
-        if (G.bc[2 * AX + sd] == ECG_BC_SYMMETRY) {
+        if (G.bc[2 * ax + sd] == ECG_BC_SYMMETRY) {
           if (LSL) {
-            wall_side_limited<NP, DIM>(M, sq, RS, rc, ssl, SS, FT::lidx(line, sd == 0 ? fl + 1 : fl),
-                                       G.wdist[2 * AX + sd], t, ug);
+            wall_side_limited<NP, DIM>(M, sq, RS, rc, ssl, SS, sd == 0 ? el + PS : el, G.wdist[2 * ax + sd], t, ug);
           } else if (O2) {
-            const int fw = FT::sidx(line, fl + 1), fo = FT::sidx(line, sd == 0 ? fl + 2 : fl);
-            wall_side<NP, DIM>(M, P.lim, sq, RS, rc, ssl, SS, fw, fo, a0[rc], G.wdist[2 * AX + sd], t, ug);
+            wall_side<NP, DIM>(M, P.lim, sq, RS, rc, ssl, SS, el + PS, sd == 0 ? el + 2 * PS : el, a0[rc],
+                               G.wdist[2 * ax + sd], t, ug);
           } else {
             cell_thermo<NP, DIM>(M, sq, RS, rc, t, ug);
           }
-          to_local(AX, neg, ug, ul);
+          local(ug, neg, ul);
           const double pstar = wall_pstar<NP>(t, ul, G.stretched, lc, wmax);
 #pragma unroll
           for (int k = 0; k < NP; k++) F.a[k] = F.m[k] = F.en[k] = 0.;
@@ -277,64 +287,61 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
           Fn[2] = 0.;
         } else {
           cell_thermo<NP, DIM>(M, sq, RS, rc, t, ug);
-          to_local(AX, neg, ug, ul);
+          local(ug, neg, ul);
           hllc<NP>(M, t, ul, t, ul, G.stretched, lc, lc, wmax, Fn, F);
         }
-        to_global(AX, neg, Fn, F.mom);
+        if (neg) Fn[0] = -Fn[0];
       } else {
-        // internal face between cells gl and gl + 1 (positions fl + 1 and fl + 2)
-        const int rl = FT::cidx(line, fl + 1), rr = FT::cidx(line, fl + 2);
+        // internal face between cells gl and gl + 1
+        const int gl = f - 1;
         Thermo<NP> tl, tr;
-        double ug[3], vg[3];
-        if (!O2) {
-          cell_thermo<NP, DIM>(M, sq, RS, rl, tl, ug);
-          cell_thermo<NP, DIM>(M, sq, RS, rr, tr, vg);
-        } else if (LSL) {
-          extrapolate_side<NP, DIM>(M, sq, RS, rl, ssl, SS, FT::lidx(line, fl), G.dfl[AX][gl], 1., pone, tl, ug);
-          extrapolate_side<NP, DIM>(M, sq, RS, rr, ssl, SS, FT::lidx(line, fl + 1), G.dfr[AX][gl], -1., pone, tr, vg);
-        } else {
-          const int f1 = FT::sidx(line, fl + 1);  // this face
-          const bool hasL = (gl - 1 >= 0), hasR = (gl + 2 < nax);
-          // beyond a symmetry side the opposite slope is the side's and alphaCellAfterOppositeSide is the
-          // cell's own time-n alpha (CellO2Cartesian::computeLocalSlopes :68-71); a non-reflecting side
-          // has neither
-          const bool wL = !hasL && G.bc[2 * AX] == ECG_BC_SYMMETRY;
-          const bool wR = !hasR && G.bc[2 * AX + 1] == ECG_BC_SYMMETRY;
-          const int f2l = (hasL || wL) ? FT::sidx(line, fl) : -1;      // face (gl-1, gl)
-          const int f2r = (hasR || wR) ? FT::sidx(line, fl + 2) : -1;  // face (gl+1, gl+2)
-          const double aL = sq[FL::A * RS + rl], aR = sq[FL::A * RS + rr];
-          const double aLL = hasL ? a0[FT::cidx(line, fl)] : (wL ? a0[rl] : 0.);
-          const double aRR = hasR ? a0[FT::cidx(line, fl + 3)] : (wR ? a0[rr] : 0.);
-          constexpr bool kThinc = (TYPES == EOS_DYNAMIC);
-          constexpr int kLim = code_limiter(TYPES);
-          reconstruct_side<NP, DIM, kThinc, kLim>(M, P, sq, RS, rl, ssl, SS, f1, f2l, aL, aR, aLL, G.dfl[AX][gl], 1.,
-                                                  tl, ug);
-          reconstruct_side<NP, DIM, kThinc, kLim>(M, P, sq, RS, rr, ssl, SS, f1, f2r, aR, aL, aRR, G.dfr[AX][gl], -1.,
-                                                  tr, vg);
-        }
         double ul[3], ur[3];
-        to_local(AX, false, ug, ul);
-        to_local(AX, false, vg, ur);
-        int gf[3] = {g[0], g[1], g[2]};  // the face's left cell, then its right cell: their CFL lengths
-        gf[AX] = gl;
-        const double lL = cell_lcfl(G, gf[0], gf[1], gf[2]);
-        gf[AX] = gl + 1;
-        const double lR = cell_lcfl(G, gf[0], gf[1], gf[2]);
-        hllc<NP, O2>(M, tl, ul, tr, ur, G.stretched, lL, lR, wmax, Fn, F);
-        to_global(AX, false, Fn, F.mom);
+        if (LSL) {
+          extrapolate_side<NP, DIM>(M, sq, RS, rl, ssl, SS, el, pn, p1, p2, G.dfl[ax][gl], 1., pone, tl, ul);
+          extrapolate_side<NP, DIM>(M, sq, RS, rr, ssl, SS, el + PS, pn, p1, p2, G.dfr[ax][gl], -1., pone, tr, ur);
+        } else {
+          double ug[3], vg[3];
+          if (!O2) {
+            cell_thermo<NP, DIM>(M, sq, RS, rl, tl, ug);
+            cell_thermo<NP, DIM>(M, sq, RS, rr, tr, vg);
+          } else {
+            const int f1 = el + PS;  // this face
+            const bool hasL = (gl - 1 >= 0), hasR = (gl + 2 < nax);
+            // beyond a symmetry side the opposite slope is the side's and alphaCellAfterOppositeSide is the
+            // cell's own time-n alpha (CellO2Cartesian::computeLocalSlopes :68-71); a non-reflecting side
+            // has neither
+            const bool wL = !hasL && G.bc[2 * ax] == ECG_BC_SYMMETRY;
+            const bool wR = !hasR && G.bc[2 * ax + 1] == ECG_BC_SYMMETRY;
+            const int f2l = (hasL || wL) ? el : -1;           // face (gl-1, gl)
+            const int f2r = (hasR || wR) ? el + 2 * PS : -1;  // face (gl+1, gl+2)
+            const double aL = sq[FL::A * RS + rl], aR = sq[FL::A * RS + rr];
+            const double aLL = hasL ? a0[rl - PS] : (wL ? a0[rl] : 0.);
+            const double aRR = hasR ? a0[rr + PS] : (wR ? a0[rr] : 0.);
+            constexpr bool kThinc = (TYPES == EOS_DYNAMIC);
+            constexpr int kLim = code_limiter(TYPES);
+            reconstruct_side<NP, DIM, kThinc, kLim>(M, P, sq, RS, rl, ssl, SS, f1, f2l, aL, aR, aLL, G.dfl[ax][gl], 1.,
+                                                    tl, ug);
+            reconstruct_side<NP, DIM, kThinc, kLim>(M, P, sq, RS, rr, ssl, SS, f1, f2r, aR, aL, aRR, G.dfr[ax][gl],
+                                                    -1., tr, vg);
+          }
+          local(ug, false, ul);
+          local(vg, false, ur);
+        }
+        hllc<NP, O2>(M, tl, ul, tr, ur, G.stretched, lcfl(gl), lcfl(gl + 1), wmax, Fn, F);
       }
-      const int64_t nfa = split_nfaces(G.n, AX);
-      const int64_t fid = split_fid(G.n, AX, f, g[0], g[1], g[2]);
+      const int64_t nfa = split_nfaces(G.n, ax);
+      const int64_t fid = split_fid(G.n, ax, f, lg, isx ? lg : third, third);
       if (ECG_IN_BOUNDS(P.stats, fid, nfa)) {
-        double* out = flux + fid;
+        double* out = L.flux + fid;
 #pragma unroll
         for (int k = 0; k < NP; k++) {
           out[(int64_t)k * nfa] = F.a[k];
           out[(int64_t)(NP + k) * nfa] = F.m[k];
           out[(int64_t)(2 * NP + k) * nfa] = F.en[k];
         }
-#pragma unroll
-        for (int d = 0; d < DIM; d++) out[(int64_t)(3 * NP + d) * nfa] = F.mom[d];
+        out[(int64_t)(3 * NP + pn) * nfa] = Fn[0];
+        out[(int64_t)(3 * NP + p1) * nfa] = Fn[1];
+        if (DIM > 2) out[(int64_t)(3 * NP + p2) * nfa] = Fn[2];
         out[(int64_t)(3 * NP + DIM) * nfa] = F.E;
         out[(int64_t)(3 * NP + DIM + 1) * nfa] = F.sM;
         out[(int64_t)(3 * NP + DIM + 2) * nfa] = F.uStar;
@@ -343,17 +350,16 @@ __global__ void __launch_bounds__(FaceTile<AX>::NTH, DIM == 2 ? ECG_FACE_MINB_2D
   }
 
   // ---- dtMax: block reduction of the wave speeds, one atomic per block
-  __shared__ double red[32];
+  __shared__ double red[FACE_THREADS / 32];
   double v = wmax;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   if ((tid & 31) == 0) red[tid >> 5] = v;
   __syncthreads();
-  if (tid < 32) {
-    v = (tid < FT::NTH / 32) ? red[tid] : wave_none(G.stretched);
+  if (tid == 0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (tid == 0) atomic_min_pos_double(P.dtmax_bits, wave_dtmax(v, G.stretched, G.lcfl));
+    for (int w = 1; w < FACE_THREADS / 32; w++) v = dmax(v, red[w]);
+    atomic_min_pos_double(P.dtmax_bits, wave_dtmax(v, G.stretched, G.lcfl));
   }
 }
 
@@ -373,6 +379,24 @@ __device__ __forceinline__ void load_face_flux(const double* __restrict__ fl, in
   F.E = p[(int64_t)(3 * NP + DIM) * nfa];
   F.sM = p[(int64_t)(3 * NP + DIM + 1) * nfa];
   F.uStar = p[(int64_t)(3 * NP + DIM + 2) * nfa];
+}
+
+// L2 prefetches of the upper faces' fluxes of a warp's cells (rows of 32 doubles per component; the lower
+// faces' were read by earlier blocks, or are in the same rows along x): without them a warp met
+// the DRAM latency again for every face it accumulated (long-scoreboard stalls were 5.1 of 11.2 cycles between
+// issues at 128^3, DRAM at half its bandwidth).  Measured, cell kernels: 2D 2048^2 0.421 / 0.437 ms without,
+// 0.410 / 0.427 with every axis, 0.389 / 0.407 with Y only (the X loads follow at once); 3D 256^3 2.43 without,
+// 2.42 with Y and Z, 2.37 with every axis.  Prefetching for the block one wave ahead instead cost 30 % in 3D.
+template <int NP, int DIM>
+__device__ __forceinline__ void prefetch_face_fluxes(const Geometry& G, const double* const fa[3], const int g[3]) {
+  using FL = Fields<NP, DIM>;
+  const int c = threadIdx.x & 15;  // component; lanes 16..31 of a warp take the second 128 bytes of a row
+  static_assert(FL::NFL <= 16, "a lane per component and half row");
+#pragma unroll
+  for (int ax = DIM == 2 ? 1 : 0; ax < DIM; ax++) {
+    const int64_t fid = split_fid(G.n, ax, g[ax] + 1, g[0], g[1], g[2]) - c;
+    if (c < FL::NFL) asm volatile("prefetch.global.L2 [%0];" ::"l"(fa[ax] + fid + (int64_t)c * split_nfaces(G.n, ax)));
+  }
 }
 
 template <int NP, int DIM, int PASS, bool PTMU, bool SEED, int TYPES>
@@ -404,6 +428,8 @@ __global__ void __launch_bounds__(cell_threads(PTMU),
   CellCounters cc;
   CellPrim<NP, DIM> cp;
   if (active) {
+    const double* fa[3] = {fx, fy, fz};
+    prefetch_face_fluxes<NP, DIM>(G, fa, g);
     const double p0 = P.sn[(int64_t)FL::P * nn + cell];
 #pragma unroll
     for (int k = 0; k < NP; k++) {
@@ -411,7 +437,6 @@ __global__ void __launch_bounds__(cell_threads(PTMU),
       rn[k] = P.sn[(int64_t)(FL::R + k) * nn + cell];
       pn[k] = eos_fix_p(M.eos[k], p0);
     }
-    const double* fa[3] = {fx, fy, fz};
     // internal faces, axis by axis: the left face added, the right face subtracted
 #pragma unroll
     for (int ax = 0; ax < DIM; ax++) {
@@ -453,31 +478,12 @@ __global__ void __launch_bounds__(cell_threads(PTMU),
 
 template <int NP, int DIM, int AX, int PASS, int TYPES>
 cudaError_t launch_faces(const StepParams& P, const Geometry& G, const Model<NP>& M, cudaStream_t s, bool prepare) {
-  using FT = FaceTile<AX>;
+  using KS = FaceKernelShape<NP, DIM, PASS, TYPES>;
   auto kern = k_kapila_faces<NP, DIM, AX, PASS, TYPES>;
-  const size_t sm = FaceKernelShape<NP, DIM, AX, PASS, TYPES>::smem_bytes();
+  const size_t sm = KS::smem_bytes();
   if (prepare) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  // tensor maps of the buffers this pass reads (TMA staging), when the context built them
-  CUtensorMap mq{}, ma0{};
-  int tma = 0;
-  if (P.fmaps && P.fmaps->ok) {
-    const CUtensorMap *q = nullptr, *a = nullptr;
-    for (int b = 0; b < 3; b++) {
-      if (P.fmaps->buf[b] && P.fmaps->buf[b] == P.q) q = &P.fmaps->q[b][AX];
-      if (P.fmaps->buf[b] && P.fmaps->buf[b] == P.sn) a = &P.fmaps->a0[b][AX];
-    }
-    if (q && (!FaceKernelShape<NP, DIM, AX, PASS, TYPES>::NA0 || a)) {
-      mq = *q;
-      if (a) ma0 = *a;
-      tma = 1;
-    }
-  }
-  const int nax = G.n[AX], ob = AX == 0 ? 1 : 0, third = AX == 2 ? G.n[1] : G.n[2];
-  dim3 grid, blk(FT::NTH);
-  const unsigned gf = (unsigned)((nax + 1 + FT::TF - 1) / FT::TF), gl = (unsigned)((G.n[ob] + FT::W - 1) / FT::W);
-  if (AX == 0) grid = dim3(gf, gl, (unsigned)third);
-  else grid = dim3(gl, gf, (unsigned)third);
-  kern<<<grid, blk, sm, s>>>(P, G, M, P.flux[AX], mq, ma0, tma);
+  const FaceLaunch L = face_launch<AX>(P, KS::NA0 != 0);
+  kern<<<face_grid<AX>(G.n), FACE_THREADS, sm, s>>>(P, G, M, L);
   return cudaGetLastError();
 }
 
@@ -489,12 +495,9 @@ cudaError_t launch_split(const StepParams& P, const Geometry& G, const ecg_eos* 
   Model<NP> M;
   for (int k = 0; k < NP; k++) M.eos[k] = make_eos_params(eos[k]);
   M.eps = eps;
-  cudaError_t e = launch_faces<NP, DIM, 0, PASS, TYPES>(P, G, M, s, prepare);
-  if (e == cudaSuccess && P.split_ev && !prepare) e = cudaEventRecord(P.split_ev[0], s);
-  if (e == cudaSuccess) e = launch_faces<NP, DIM, 1, PASS, TYPES>(P, G, M, s, prepare);
-  if (e == cudaSuccess && P.split_ev && !prepare) e = cudaEventRecord(P.split_ev[1], s);
-  if (DIM > 2 && e == cudaSuccess) e = launch_faces<NP, DIM, (DIM > 2 ? 2 : 0), PASS, TYPES>(P, G, M, s, prepare);
-  if (DIM > 2 && e == cudaSuccess && P.split_ev && !prepare) e = cudaEventRecord(P.split_ev[2], s);
+  const cudaError_t e = face_axes<DIM>(P, s, prepare, [&](auto ax, cudaStream_t sa) {
+    return launch_faces<NP, DIM, decltype(ax)::value, PASS, TYPES>(P, G, M, sa, prepare);
+  });
   if (e != cudaSuccess || prepare) return e;
   constexpr int CT = cell_threads(PTMU);
   const unsigned blocks = (unsigned)((P.n + CT - 1) / CT);

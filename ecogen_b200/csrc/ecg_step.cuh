@@ -101,6 +101,13 @@ struct DevScalars {
   int done;                        // set once the stop condition holds; later steps are no-ops
 };
 
+// Auxiliary streams of a context's face kernels (axes 1 and 2) and the events that fork them from and join
+// them to its stream.
+struct FaceStreams {
+  cudaStream_t s[2];
+  cudaEvent_t fork, join[2];
+};
+
 struct StepParams {
   const int* done;      // device flag: skip the launch when set
   const double* q;      // primitives the fluxes are built from (S^n, or S^{n+1/2} in the corrector)
@@ -139,6 +146,7 @@ struct StepParams {
   // kernels run), and optional events recorded after each axis' face kernel (profiling)
   double* flux[3];
   cudaEvent_t* split_ev;
+  const struct FaceStreams* fstreams;  // auxiliary streams of the face kernels (nullptr: one after another)
   // host side: tensor maps of the face kernels' TMA staging (nullptr: the kernels load their tiles)
   const struct FaceMaps* fmaps;
 };

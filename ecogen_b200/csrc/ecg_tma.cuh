@@ -13,7 +13,7 @@
 // created, and reach the kernel as __grid_constant__ parameters.  A tiled copy needs a 16-byte aligned
 // base (cudaMalloc), strides that are multiples of 16 bytes (n_x even: the host builds no map
 // otherwise and the kernels load the tile themselves), an inner box extent that is a multiple of 16
-// bytes (20 doubles for X faces, 16 for Y and Z faces) and an x coordinate whose byte offset is a
+// bytes (22 doubles for X faces, 16 for Y and Z faces) and an x coordinate whose byte offset is a
 // multiple of 16: f0 - 2 with f0 a multiple of the X chunk (16), or the first of 16 x lines.  Every copy
 // reads this GPU's own memory into its own CTA; there is no multicast.
 #pragma once
@@ -24,42 +24,39 @@
 
 namespace ecg {
 
-// Block of the face kernel of axis AX: TF faces along AX times W lines along the fastest other axis
-// (Y lines for X faces, X lines for Y and Z faces), one thread per face; the block's third coordinate
-// is blockIdx.z.  Shared planes are laid out so that the linear thread order is the storage order,
-// and so that a staged plane is the box a tensor copy writes: X faces [line][CP cells], Y and Z faces
-// [CP cells][W lines].  A line of X faces has n_x + 1 faces, so its last chunk holds a single face:
-// chunks of 16 faces keep more lanes busy than chunks of 32 on short lines (257 faces at 256^3: 94 %
-// against 89 %).
-#ifndef ECG_XFACE_TF
-#define ECG_XFACE_TF 16
-#endif
+// Block of the face kernel for the faces of axis AX: TF faces along AX times W lines along the fastest other
+// axis (Y lines for X faces, X lines for Y and Z faces), one thread per face, at one third coordinate.
+// Shared planes are laid out so that the linear thread order is the storage order, and so that a staged
+// plane is the box a tensor copy writes: X faces [line][CP cells], Y and Z faces [CP cells][W lines].  The
+// planes have the same size for every axis, so that one kernel addresses them with constant offsets.
+// A line of X faces has n_x + 1 faces, so its last chunk holds a single face: chunks of 16 faces keep more
+// lanes busy than chunks of 32 on short lines (257 faces at 256^3: 94 % against 89 %).
+constexpr int FACE_THREADS = 128;
 template <int AX>
 struct FaceTile {
-  static constexpr int TF = (AX == 0) ? ECG_XFACE_TF : 8;
-  static constexpr int W = (AX == 0) ? 128 / ECG_XFACE_TF : 16;
-  static constexpr int NTH = TF * W;
-  // staged cells per line, from f0-2: TF + 3 are read (f0-2 .. f0+TF); X lines stage one more so a
-  // staged row is a multiple of 16 bytes
-  static constexpr int CP = (AX == 0) ? TF + 4 : TF + 3;
+  static constexpr int TF = (AX == 0) ? 16 : 8;
+  static constexpr int W = FACE_THREADS / TF;
+  // staged cells per line, from f0-2: TF + 3 are read (f0-2 .. f0+TF); X lines stage three more so a
+  // staged row is a multiple of 16 bytes and a plane as large as the other axes'
+  static constexpr int CP = (AX == 0) ? TF + 6 : TF + 3;
   static constexpr int SP = TF + 2;  // slopes per line: faces f0-1 .. f0+TF
   static constexpr int RS = W * CP;  // one staged plane
-  static constexpr int SS = W * SP;  // one slope plane
+  static constexpr int SS = W * SP;  // slopes
   static constexpr int LP = TF + 1;  // limited slopes per line: cells f0-1 .. f0+TF-1
-  static constexpr int LS = W * LP;  // one plane of them
-  __host__ __device__ static constexpr int cidx(int line, int pos) { return AX == 0 ? line * CP + pos : pos * W + line; }
-  __host__ __device__ static constexpr int sidx(int line, int s) { return AX == 0 ? line * SP + s : s * W + line; }
-  __host__ __device__ static constexpr int lidx(int line, int s) { return AX == 0 ? line * LP + s : s * W + line; }
+  static constexpr int LS = W * LP;  // limited slopes
   // extent of the staged box along x, y, z (the tensor's first three dimensions)
   static constexpr int box(int d) {
     return AX == 0 ? (d == 0 ? CP : (d == 1 ? W : 1)) : (d == 0 ? W : (d == AX ? CP : 1));
   }
 };
+constexpr int FACE_RS = FaceTile<1>::RS;  // stride of the staged planes, of the face slopes' and limited slopes' planes
+constexpr int FACE_SS = FaceTile<1>::SS > FaceTile<0>::SS ? FaceTile<1>::SS : FaceTile<0>::SS;
+constexpr int FACE_LS = FaceTile<1>::LS > FaceTile<0>::LS ? FaceTile<1>::LS : FaceTile<0>::LS;
+static_assert(FaceTile<0>::RS == FACE_RS, "the staged planes of every axis have one size");
 static_assert((FaceTile<0>::CP * sizeof(double)) % 16 == 0 && (FaceTile<1>::W * sizeof(double)) % 16 == 0,
               "the inner extent of a staged box must be a multiple of 16 bytes");
 static_assert(FaceTile<0>::TF % 2 == 0 && FaceTile<1>::W % 2 == 0, "box x origins must be 16-byte aligned");
-static_assert((FaceTile<0>::RS * sizeof(double)) % 128 == 0 && (FaceTile<1>::RS * sizeof(double)) % 128 == 0,
-              "staged planes keep the 128-byte alignment of the shared-memory base");
+static_assert((FACE_RS * sizeof(double)) % 128 == 0, "staged planes keep the 128-byte alignment of the shared-memory base");
 
 // Host-side table of a context's tensor maps: for each state buffer (the two ping-pong states and the
 // MUSCL half-step state) and axis, the box of every primitive field and the box of field 0 alone (the
