@@ -114,8 +114,9 @@ struct ecg_ctx {
   double* half = nullptr;     // MUSCL half-step primitives
   double* dist = nullptr;     // distance tables (3 axes x 3 tables)
   double* tmp = nullptr;      // download scratch (mixture pressure)
-  double* flux[3] = {nullptr, nullptr, nullptr};  // face arrays of the split form (Kapila 2D / 3D)
-  bool split = false;         // step passes in split form (face kernels + cell kernel)
+  double* flux[3] = {nullptr, nullptr, nullptr};  // face arrays of the split form (2D / 3D)
+  bool split = false;         // Kapila step passes in split form (face kernels + cell kernel)
+  bool flow = false;          // Euler or PTUEq passes in split form (no choice of form for these models)
   FaceStreams fstreams{};     // auxiliary streams of the face kernels (split forms)
   FaceMaps fmaps{};           // tensor maps of the face kernels' TMA staging (fmaps.ok = 0: none)
   int staging = ECG_STAGING_TMA;
@@ -276,9 +277,9 @@ ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
   P.pcrit = x->pcrit;
   P.ptmu_seed_p = x->ptmu_seed_p;
   P.tsat_hist = x->tsat_hist;
-  for (int a = 0; a < 3; a++) P.flux[a] = x->split ? x->flux[a] : nullptr;
+  for (int a = 0; a < 3; a++) P.flux[a] = (x->split || x->flow) ? x->flux[a] : nullptr;
   P.fstreams = x->fstreams.fork ? &x->fstreams : nullptr;
-  P.fmaps = (x->split && x->staging == ECG_STAGING_TMA && x->fmaps.ok) ? &x->fmaps : nullptr;
+  P.fmaps = ((x->split || x->flow) && x->staging == ECG_STAGING_TMA && x->fmaps.ok) ? &x->fmaps : nullptr;
   double* sn = x->state[parity];
   double* s1 = x->state[1 - parity];
   const bool euler = x->c.model == ECG_MODEL_EULER;
@@ -554,15 +555,19 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
   }
   e = cudaMalloc(&x->tmp, sizeof(double) * (size_t)(ptueq ? 2 : 1) * (size_t)x->n);  // download scratch
   if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaMalloc(tmp)"));
-  if (!euler && !ptueq && x->dim >= 2 && c->ntransports == 0) {
-    // face arrays of the split form: 3N + d + 3 flux components per face, faces of each axis including
-    // the domain sides
-    const int nfl = 3 * x->np + x->dim + 3;
+  // Euler (one limiter slot is read) and PTUEq run in split form when one limiter decides every slope
+  const bool one_limiter = c->limiter[1] == c->limiter[0] && c->limiter[2] == c->limiter[0] &&
+                           c->limiter[3] == c->limiter[0] && c->limiter[0] != ECG_LIM_THINC;
+  x->flow = x->dim >= 2 && c->ntransports == 0 && (euler || (ptueq && (c->order == 1 || one_limiter)));
+  if ((!euler && !ptueq && x->dim >= 2 && c->ntransports == 0) || x->flow) {
+    // face arrays of the split form: the flux components (Kapila 3N + d + 3, Euler d + 2, PTUEq d + 3) of every
+    // face of each axis, the domain sides included
+    const int nfl = euler ? x->dim + 2 : (ptueq ? x->dim + 3 : 3 * x->np + x->dim + 3);
     for (int a = 0; a < x->dim; a++) {
       e = cudaMalloc(&x->flux[a], sizeof(double) * (size_t)nfl * (size_t)split_nfaces(c->ncells, a));
       if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaMalloc(face fluxes)"));
     }
-    x->split = true;
+    x->split = !x->flow;
     for (int a = 0; a + 1 < x->dim && e == cudaSuccess; a++) {
       e = cudaStreamCreateWithFlags(&x->fstreams.s[a], cudaStreamNonBlocking);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->fstreams.join[a], cudaEventDisableTiming);
@@ -571,9 +576,10 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
     if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaStreamCreate(face streams)"));
 #ifndef ECG_BOUNDS_CHECK
     // TMA staging of the face kernels' tiles where the layout allows it (the bounds-checked build
-    // checks the kernels' own loads, so it stages them that way)
+    // checks the kernels' own loads, so it stages them that way).  Staged planes: all but E, which the
+    // first-order Euler pass reads too.
     const double* bufs[3] = {x->state[0], x->state[1], x->half};
-    build_face_maps(x->fmaps, bufs, x->dim, c->ncells, x->nq);
+    build_face_maps(x->fmaps, bufs, x->dim, c->ncells, x->nq + (euler && c->order == 1 ? 1 : 0));
 #endif
   }
   std::vector<double> h, sz[3], ctr[3];
@@ -682,8 +688,8 @@ extern "C" void* ecg_stream(const ecg_ctx* x) { return x ? (void*)x->stream : nu
 
 extern "C" ecg_status ecg_set_step_form(ecg_ctx* x, int32_t form) {
   if (!x || (form != ECG_FORM_FUSED && form != ECG_FORM_SPLIT)) { set_error("bad step form"); return ECG_ERR_INVALID; }
-  if (form == ECG_FORM_SPLIT && !x->flux[0]) { set_error("no split form for this case (1D, Euler, PTUEq or transports)"); return ECG_ERR_UNSUPPORTED; }
-  x->split = form == ECG_FORM_SPLIT;
+  if (form == ECG_FORM_SPLIT && (!x->flux[0] || x->flow)) { set_error("no split form for this case (1D, Euler, PTUEq or transports)"); return ECG_ERR_UNSUPPORTED; }
+  if (!x->flow) x->split = form == ECG_FORM_SPLIT;
   x->graph_dirty = true;
   return ECG_OK;
 }

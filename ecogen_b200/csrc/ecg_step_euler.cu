@@ -8,7 +8,7 @@
 // (src/Models/Euler/PhaseEuler.cpp:105), and so it is here.
 #include <cuda_runtime.h>
 
-#include "ecg_step.cuh"
+#include "ecg_flow_split.cuh"
 
 namespace ecg {
 
@@ -52,6 +52,13 @@ __device__ __forceinline__ void euler_complete(const EosParams& q, double eps, E
   s.c = eos_c(q, eps, s.rho, s.p);
   s.E = e + 0.5 * (s.u[0] * s.u[0] + s.u[1] * s.u[1] + s.u[2] * s.u[2]);
 }
+
+#ifndef ECG_EULER_FACE_MINB
+#define ECG_EULER_FACE_MINB 8
+#endif
+#ifndef ECG_EULER_CELL_MINB
+#define ECG_EULER_CELL_MINB 8
+#endif
 
 // ModEuler::solveRiemannIntern src/Models/Euler/ModEuler.cpp:105-225 (strict sL > 0 / sR < 0).
 __device__ __forceinline__ void hllc_euler(const EulerSide& L, const double ul[3], const EulerSide& R,
@@ -99,6 +106,111 @@ __device__ __forceinline__ void hllc_euler(const EulerSide& L, const double ul[3
     FE = (rhoStar * Estar + pStar) * sM;
   }
 }
+
+// FluxEuler::buildCons, Cell::timeEvolution, FluxEuler::buildPrim of a cell from its accumulated fluxes.
+template <int DIM, int PASS>
+__device__ __forceinline__ void euler_update(const StepParams& P, const EosParams& q, double eps, int64_t nn,
+                                             int64_t cell, double am, const double* amom, double aE) {
+  const double dt = *P.dt;
+  const double scale = (PASS == PASS_PRED) ? 0.5 * dt : dt;
+  const double rn = P.sn[cell];
+  const double En = P.sn[(int64_t)(2 + DIM) * nn + cell];
+  am = am * scale + 1. * rn;
+  double u[DIM], usq = 0.;
+#pragma unroll
+  for (int d = 0; d < DIM; d++) u[d] = amom[d] * scale + 1. * (rn * P.sn[(int64_t)(2 + d) * nn + cell]);
+  aE = aE * scale + 1. * (rn * En);
+#pragma unroll
+  for (int d = 0; d < DIM; d++) {
+    u[d] = ndiv(u[d], am);
+    if (fabs(u[d]) < 1.e-8) u[d] = 0.;
+    usq += u[d] * u[d];
+  }
+  const double E = ndiv(aE, am);
+  const double p = eos_p(q, eps, am, E - 0.5 * usq);
+  P.out[cell] = am;
+  P.out[nn + cell] = p;
+#pragma unroll
+  for (int d = 0; d < DIM; d++) P.out[(int64_t)(2 + d) * nn + cell] = u[d];
+  if (PASS != PASS_PRED) P.out[(int64_t)(2 + DIM) * nn + cell] = E;
+}
+
+// The model in split form (ecg_flow_split.cuh); the energy of a completed side sums |u|^2 in the absolute
+// frame's order.
+struct EulerFlow {
+  struct Eos {
+    EosParams q;
+    double eps;
+  };
+  struct Side {
+    EulerSide s;  // s.u unused: the face-frame velocities are ul
+    double c, ul[3];
+  };
+  static constexpr int NM = 1, U = 2, STORED = 1, FACE_MINB = ECG_EULER_FACE_MINB, CELL_MINB = ECG_EULER_CELL_MINB;
+  static __device__ __forceinline__ void complete(const Eos& M, int ax, Side& A) {
+    const double n2 = A.ul[0] * A.ul[0], t1 = A.ul[1] * A.ul[1], t2 = A.ul[2] * A.ul[2];
+    const double e = eos_e(M.q, M.eps, A.s.rho, A.s.p);
+    A.c = A.s.c = eos_c(M.q, M.eps, A.s.rho, A.s.p);
+    A.s.E = e + 0.5 * (ax == 2 ? (t1 + t2) + n2 : (n2 + t1) + t2);
+  }
+  template <int DIM>
+  static __device__ __forceinline__ void fields(const double* sq, int RS, int rc, int pn, int p1, int p2, Side& A) {
+    A.s.rho = sq[rc];
+    A.s.p = sq[RS + rc];
+    A.ul[0] = sq[(U + pn) * RS + rc];
+    A.ul[1] = sq[(U + p1) * RS + rc];
+    A.ul[2] = DIM > 2 ? sq[(U + p2) * RS + rc] : 0.;
+  }
+  template <int DIM>
+  static __device__ __forceinline__ void load(const Eos& M, const double* sq, int RS, int rc, int ax, int pn, int p1,
+                                              int p2, bool stored, Side& A) {
+    fields<DIM>(sq, RS, rc, pn, p1, p2, A);
+    complete(M, ax, A);
+    if (stored) A.s.E = sq[(U + DIM) * RS + rc];  // no fulfillState on interior first-order faces
+  }
+  // global limiter (the interface detector never fires for Euler), extrapolation
+  template <int DIM>
+  static __device__ __forceinline__ void shift(const double* ssl, int SS, int e, int pn, int p1, int p2, double dist,
+                                               double sign, Side& A) {
+    A.s.rho += (sign * ssl[e]) * dist;
+    A.s.p += (sign * ssl[SS + e]) * dist;
+    A.ul[0] += (sign * ssl[(U + pn) * SS + e]) * dist;
+    A.ul[1] += (sign * ssl[(U + p1) * SS + e]) * dist;
+    if (DIM > 2) A.ul[2] += (sign * ssl[(U + p2) * SS + e]) * dist;
+  }
+  template <int DIM>
+  static __device__ __forceinline__ void extrapolate(const Eos& M, const double* sq, int RS, int rc, const double* ssl,
+                                                     int SS, int e, int ax, int pn, int p1, int p2, double dist,
+                                                     double sign, Side& A) {
+    fields<DIM>(sq, RS, rc, pn, p1, p2, A);
+    shift<DIM>(ssl, SS, e, pn, p1, p2, dist, sign, A);
+    if (A.s.rho < 1.e-10) A.s.rho = 1.e-10;
+    A.s.p = eos_fix_p(M.q, A.s.p);
+    eos_rho_max(M.q, A.s.rho);
+    complete(M, ax, A);
+  }
+  // BoundCondWallO2Cartesian::solveRiemann :111-141: extrapolation by the signed distance without clamps
+  template <int DIM, bool O2>
+  static __device__ __forceinline__ void wall(const Eos& M, const double* sq, int RS, int rc, const double* ssl, int SS,
+                                              int e, int ax, int pn, int p1, int p2, double dist, Side& A) {
+    fields<DIM>(sq, RS, rc, pn, p1, p2, A);
+    if (O2) shift<DIM>(ssl, SS, e, pn, p1, p2, dist, 1., A);
+    complete(M, ax, A);
+  }
+  // ModEuler::solveRiemannWall src/Models/Euler/ModEuler.cpp:368-409
+  static __device__ __forceinline__ double wall_flux(const Side& A, double sL) {
+    return A.s.rho * A.ul[0] * (A.ul[0] - sL) + A.s.p;
+  }
+  static __device__ __forceinline__ void hllc(const Side& A, const Side& B, bool stretched, double dxL, double dxR,
+                                              double& wmax, double Fm[1], double Fn[3], double& FE) {
+    hllc_euler(A.s, A.ul, B.s, B.ul, stretched, dxL, dxR, wmax, Fm[0], Fn, FE);
+  }
+  template <int DIM, int PASS>
+  static __device__ __forceinline__ void update(const StepParams& P, const Eos& M, int64_t nn, int64_t cell,
+                                                const double* acc) {
+    euler_update<DIM, PASS>(P, M.q, M.eps, nn, cell, acc[0], acc + 1, acc[1 + DIM]);
+  }
+};
 
 // Register budget: ECG_EULER_MINB2D > 0 asks the compiler for that many resident blocks per SM in 2D;
 // 0 leaves the register count to the compiler.  Measured on a 2048^2 blast (MUSCL + van Leer,
@@ -394,30 +506,8 @@ __global__ void __launch_bounds__(EulerStep<DIM, PASS, NTM>::NTH,
         at[t] -= -cA * tn[t] * sMb;
       }
     }
-    // FluxEuler::buildCons, Cell::timeEvolution, FluxEuler::buildPrim
-    const double dt = *P.dt;
-    const double scale = (PASS == PASS_PRED) ? 0.5 * dt : dt;
-    double rn = P.sn[cell];
-    double En = P.sn[(int64_t)(2 + DIM) * nn + cell];
-    am = am * scale + 1. * rn;
-    double u[DIM], usq = 0.;
-#pragma unroll
-    for (int d = 0; d < DIM; d++) amom[d] = amom[d] * scale + 1. * (rn * P.sn[(int64_t)(2 + d) * nn + cell]);
-    aE = aE * scale + 1. * (rn * En);
-#pragma unroll
-    for (int d = 0; d < DIM; d++) {
-      u[d] = ndiv(amom[d], am);
-      if (fabs(u[d]) < 1.e-8) u[d] = 0.;
-      usq += u[d] * u[d];
-    }
-    double E = ndiv(aE, am);
-    double e = E - 0.5 * usq;
-    double p = eos_p(q, eps, am, e);
-    P.out[cell] = am;
-    P.out[nn + cell] = p;
-#pragma unroll
-    for (int d = 0; d < DIM; d++) P.out[(int64_t)(2 + d) * nn + cell] = u[d];
-    if (PASS != PASS_PRED) P.out[(int64_t)(2 + DIM) * nn + cell] = E;
+    euler_update<DIM, PASS>(P, q, eps, nn, cell, am, amom, aE);
+    const double scale = (PASS == PASS_PRED) ? 0.5 * *P.dt : *P.dt;
 #pragma unroll
     for (int t = 0; t < NTM; t++)  // Cell::timeEvolution / CellO2::predictionOrdre2
       if (t < P.ntr) P.out[(int64_t)(NS + t) * nn + cell] = tn[t] + at[t] * scale;
@@ -463,6 +553,15 @@ static cudaError_t euler_dim(int pass, const StepParams& P, const Geometry& G, c
                              cudaStream_t s, bool prepare) {
   if (P.ntr > 2) return cudaErrorNotSupported;
   if (P.ntr > 0) return euler_dim_tr<DIM, 2>(pass, P, G, eos, eps, s, prepare);  // up to two passive transports
+  if constexpr (DIM >= 2) {
+    const EulerFlow::Eos M{make_eos_params(eos[0]), eps};
+    if (prepare) {
+      const cudaError_t e = flow_pass<EulerFlow, DIM>(pass, P, G, M, s, true);
+      if (e != cudaSuccess) return e;
+    } else if (P.flux[0] != nullptr) {
+      return flow_pass<EulerFlow, DIM>(pass, P, G, M, s, false);
+    }
+  }
   return euler_dim_tr<DIM, 0>(pass, P, G, eos, eps, s, prepare);
 }
 

@@ -13,7 +13,7 @@
 // MixPTUEq::computeMixtureVariables (src/Models/PTUEq/MixPTUEq.cpp:293-313) compute them.
 #include <cuda_runtime.h>
 
-#include "ecg_step.cuh"
+#include "ecg_flow_split.cuh"
 
 namespace ecg {
 
@@ -145,6 +145,143 @@ __device__ __forceinline__ void hllc_pt(const PtSide& L, const double ul[3], con
     FE = (rhoStar * EStar + pStar) * sM;
   }
 }
+
+#ifndef ECG_PTUEQ_FACE_MINB
+#define ECG_PTUEQ_FACE_MINB 8
+#endif
+#ifndef ECG_PTUEQ_CELL_MINB
+#define ECG_PTUEQ_CELL_MINB 8
+#endif
+
+// Update of a cell from its accumulated fluxes.
+template <int DIM, int PASS>
+__device__ __forceinline__ void pt_update(const StepParams& P, const PtEos& M, int64_t nn, int64_t cell,
+                                          const double* am, const double* amom, double aE) {
+  constexpr int FP = 2, FT = 3, FU = 4;
+  // ---- FluxPTUEq::buildCons (time-n state), Cell::timeEvolution, FluxPTUEq::buildPrim (:125-160) with
+  // MixPTUEq::computePressure (:93-122, Le Martelot's analytic p of two IG/SG phases) and
+  // computeTemperature (:126-145)
+  const double dt = *P.dt;
+  const double scale = (PASS == PASS_PRED) ? 0.5 * dt : dt;
+  PtSide n0;
+  n0.a[0] = P.sn[cell];
+  n0.a[1] = P.sn[nn + cell];
+  n0.p = P.sn[(int64_t)FP * nn + cell];
+  n0.T = P.sn[(int64_t)FT * nn + cell];
+  const double En = P.sn[(int64_t)(FU + DIM) * nn + cell];
+  double rhon = 0.;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    n0.r[k] = pt_rho(M.e[k], n0.p, n0.T);
+    rhon += n0.a[k] * n0.r[k];
+  }
+  double m[2];
+#pragma unroll
+  for (int k = 0; k < 2; k++) m[k] = am[k] * scale + 1. * (n0.a[k] * n0.r[k]);
+  double mom[DIM];
+#pragma unroll
+  for (int d = 0; d < DIM; d++) mom[d] = amom[d] * scale + 1. * (rhon * P.sn[(int64_t)(FU + d) * nn + cell]);
+  const double rE = aE * scale + 1. * (rhon * En);
+  const double rhoMel = 0. + m[0] + m[1];
+  double u[3] = {0., 0., 0.};
+#pragma unroll
+  for (int d = 0; d < DIM; d++) {
+    u[d] = ndiv(mom[d], rhoMel);
+    if (fabs(u[d]) < 1.e-8) u[d] = 0.;
+  }
+  const double ie = ndiv(rE, rhoMel) - 0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+  const EosParams& E1 = M.e[0];
+  const EosParams& E2 = M.e[1];
+  const double pInf1 = pt_pinf(E1), pInf2 = pt_pinf(E2);
+  const double Y1 = ndiv(m[0], rhoMel), Y2 = ndiv(m[1], rhoMel);
+  const double q = Y1 * E1.eref + Y2 * E2.eref;
+  const double cvMel = Y1 * E1.cv + Y2 * E2.cv;
+  const double A1 = ndiv(Y1 * (E1.gamma - 1.) * E1.cv, cvMel) * (rhoMel * (ie - q) - pInf1);
+  const double A2 = ndiv(Y2 * (E2.gamma - 1.) * E2.cv, cvMel) * (rhoMel * (ie - q) - pInf2);
+  const double p = 0.5 * (A1 + A2 - (pInf1 + pInf2)) +
+                   dsqrt(0.25 * (A2 - A1 - (pInf2 - pInf1)) * (A2 - A1 - (pInf2 - pInf1)) + A1 * A2);
+  double Tm = 0.;
+  Tm += ndiv(ndiv(m[0], rhoMel) * (E1.gamma - 1.) * E1.cv, p + pInf1);
+  Tm += ndiv(ndiv(m[1], rhoMel) * (E2.gamma - 1.) * E2.cv, p + pInf2);
+  Tm = ndiv(1., Tm * rhoMel);
+  P.out[cell] = ndiv(m[0], pt_rho(E1, p, Tm));
+  P.out[nn + cell] = ndiv(m[1], pt_rho(E2, p, Tm));
+  P.out[(int64_t)FP * nn + cell] = p;
+  P.out[(int64_t)FT * nn + cell] = Tm;
+#pragma unroll
+  for (int d = 0; d < DIM; d++) P.out[(int64_t)(FU + d) * nn + cell] = u[d];
+  if (PASS != PASS_PRED) P.out[(int64_t)(FU + DIM) * nn + cell] = ndiv(rE, rhoMel);
+}
+
+// The model in split form (ecg_flow_split.cuh).
+struct PtFlow {
+  using Eos = PtEos;
+  struct Side {
+    PtSide s;  // s.u unused: the face-frame velocities are ul
+    double c, ul[3];
+  };
+  static constexpr int NM = 2, U = 4, STORED = 0, FACE_MINB = ECG_PTUEQ_FACE_MINB, CELL_MINB = ECG_PTUEQ_CELL_MINB;
+  static __device__ __forceinline__ void complete(const Eos& M, Side& A) {
+    pt_complete(M, A.s);
+    A.c = A.s.c;
+  }
+  template <int DIM>
+  static __device__ __forceinline__ void fields(const double* sq, int RS, int rc, int pn, int p1, int p2, Side& A) {
+    A.s.a[0] = sq[rc];
+    A.s.a[1] = sq[RS + rc];
+    A.s.p = sq[2 * RS + rc];
+    A.s.T = sq[3 * RS + rc];
+    A.ul[0] = sq[(U + pn) * RS + rc];
+    A.ul[1] = sq[(U + p1) * RS + rc];
+    A.ul[2] = DIM > 2 ? sq[(U + p2) * RS + rc] : 0.;
+  }
+  template <int DIM>
+  static __device__ __forceinline__ void load(const Eos& M, const double* sq, int RS, int rc, int, int pn, int p1,
+                                              int p2, bool, Side& A) {
+    fields<DIM>(sq, RS, rc, pn, p1, p2, A);
+    complete(M, A);
+  }
+  // extrapolation and PhasePTUEq::verifyAndCorrectPhase (alpha in [1e-10, 1 - 1e-10])
+  template <int DIM>
+  static __device__ __forceinline__ void extrapolate(const Eos& M, const double* sq, int RS, int rc, const double* ssl,
+                                                     int SS, int e, int, int pn, int p1, int p2, double dist,
+                                                     double sign, Side& A) {
+    fields<DIM>(sq, RS, rc, pn, p1, p2, A);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      double a = A.s.a[k] + (sign * ssl[k * SS + e]) * dist;
+      if (a < 1e-10) a = 1e-10;
+      if (a > 1. - 1e-10) a = 1. - 1e-10;
+      A.s.a[k] = a;
+    }
+    A.s.p += (sign * ssl[2 * SS + e]) * dist;
+    A.s.T += (sign * ssl[3 * SS + e]) * dist;
+    A.ul[0] += (sign * ssl[(U + pn) * SS + e]) * dist;
+    A.ul[1] += (sign * ssl[(U + p1) * SS + e]) * dist;
+    if (DIM > 2) A.ul[2] += (sign * ssl[(U + p2) * SS + e]) * dist;
+    complete(M, A);
+  }
+  // symmetry sides are first order only
+  template <int DIM, bool O2>
+  static __device__ __forceinline__ void wall(const Eos& M, const double* sq, int RS, int rc, const double*, int, int,
+                                              int, int pn, int p1, int p2, double, Side& A) {
+    fields<DIM>(sq, RS, rc, pn, p1, p2, A);
+    complete(M, A);
+  }
+  // ModPTUEq::solveRiemannWall src/Models/PTUEq/ModPTUEq.cpp:233-265
+  static __device__ __forceinline__ double wall_flux(const Side& A, double sL) {
+    return A.s.rho * (A.ul[0] - sL) * A.ul[0] + A.s.p;
+  }
+  static __device__ __forceinline__ void hllc(const Side& A, const Side& B, bool stretched, double dxL, double dxR,
+                                              double& wmax, double Fm[2], double Fn[3], double& FE) {
+    hllc_pt(A.s, A.ul, B.s, B.ul, stretched, dxL, dxR, wmax, Fm, Fn, FE);
+  }
+  template <int DIM, int PASS>
+  static __device__ __forceinline__ void update(const StepParams& P, const Eos& M, int64_t nn, int64_t cell,
+                                                const double* acc) {
+    pt_update<DIM, PASS>(P, M, nn, cell, acc, acc + 2, acc[2 + DIM]);
+  }
+};
 
 // Register budget: the resident-block target of the tile shape (TileShape::MINB), as the Kapila
 // kernels, with 8 blocks in 2D (ECG_PTUEQ_MINB2D); ECG_PTUEQ_NO_MINB leaves the register count to the
@@ -387,59 +524,7 @@ __global__ void ECG_PTUEQ_BOUNDS(DIM, PASS) k_ptueq_step(StepParams P, Geometry 
       for (int d = 0; d < DIM; d++) amom[d] -= cA * Fg[d];
       aE -= cA * FE;
     }
-    // ---- FluxPTUEq::buildCons (time-n state), Cell::timeEvolution, FluxPTUEq::buildPrim (:125-160) with
-    // MixPTUEq::computePressure (:93-122, Le Martelot's analytic p of two IG/SG phases) and
-    // computeTemperature (:126-145)
-    const double dt = *P.dt;
-    const double scale = (PASS == PASS_PRED) ? 0.5 * dt : dt;
-    PtSide n0;
-    n0.a[0] = P.sn[cell];
-    n0.a[1] = P.sn[nn + cell];
-    n0.p = P.sn[(int64_t)FP * nn + cell];
-    n0.T = P.sn[(int64_t)FT * nn + cell];
-    const double En = P.sn[(int64_t)(FU + DIM) * nn + cell];
-    double rhon = 0.;
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      n0.r[k] = pt_rho(M.e[k], n0.p, n0.T);
-      rhon += n0.a[k] * n0.r[k];
-    }
-    double m[2];
-#pragma unroll
-    for (int k = 0; k < 2; k++) m[k] = am[k] * scale + 1. * (n0.a[k] * n0.r[k]);
-    double mom[DIM];
-#pragma unroll
-    for (int d = 0; d < DIM; d++) mom[d] = amom[d] * scale + 1. * (rhon * P.sn[(int64_t)(FU + d) * nn + cell]);
-    const double rE = aE * scale + 1. * (rhon * En);
-    const double rhoMel = 0. + m[0] + m[1];
-    double u[3] = {0., 0., 0.};
-#pragma unroll
-    for (int d = 0; d < DIM; d++) {
-      u[d] = ndiv(mom[d], rhoMel);
-      if (fabs(u[d]) < 1.e-8) u[d] = 0.;
-    }
-    const double ie = ndiv(rE, rhoMel) - 0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
-    const EosParams& E1 = M.e[0];
-    const EosParams& E2 = M.e[1];
-    const double pInf1 = pt_pinf(E1), pInf2 = pt_pinf(E2);
-    const double Y1 = ndiv(m[0], rhoMel), Y2 = ndiv(m[1], rhoMel);
-    const double q = Y1 * E1.eref + Y2 * E2.eref;
-    const double cvMel = Y1 * E1.cv + Y2 * E2.cv;
-    const double A1 = ndiv(Y1 * (E1.gamma - 1.) * E1.cv, cvMel) * (rhoMel * (ie - q) - pInf1);
-    const double A2 = ndiv(Y2 * (E2.gamma - 1.) * E2.cv, cvMel) * (rhoMel * (ie - q) - pInf2);
-    const double p = 0.5 * (A1 + A2 - (pInf1 + pInf2)) +
-                     dsqrt(0.25 * (A2 - A1 - (pInf2 - pInf1)) * (A2 - A1 - (pInf2 - pInf1)) + A1 * A2);
-    double Tm = 0.;
-    Tm += ndiv(ndiv(m[0], rhoMel) * (E1.gamma - 1.) * E1.cv, p + pInf1);
-    Tm += ndiv(ndiv(m[1], rhoMel) * (E2.gamma - 1.) * E2.cv, p + pInf2);
-    Tm = ndiv(1., Tm * rhoMel);
-    P.out[cell] = ndiv(m[0], pt_rho(E1, p, Tm));
-    P.out[nn + cell] = ndiv(m[1], pt_rho(E2, p, Tm));
-    P.out[(int64_t)FP * nn + cell] = p;
-    P.out[(int64_t)FT * nn + cell] = Tm;
-#pragma unroll
-    for (int d = 0; d < DIM; d++) P.out[(int64_t)(FU + d) * nn + cell] = u[d];
-    if (PASS != PASS_PRED) P.out[(int64_t)(FU + DIM) * nn + cell] = ndiv(rE, rhoMel);
+    pt_update<DIM, PASS>(P, M, nn, cell, am, amom, aE);
   }
   __shared__ double red[32];
   double v = wmax;
@@ -474,6 +559,16 @@ static cudaError_t ptueq_one(const StepParams& P, const Geometry& G, const ecg_e
 template <int DIM>
 static cudaError_t ptueq_dim(int pass, const StepParams& P, const Geometry& G, const ecg_eos* eos, cudaStream_t s,
                              bool prepare) {
+  if constexpr (DIM >= 2) {
+    PtEos M;
+    for (int k = 0; k < 2; k++) M.e[k] = make_eos_params(eos[k]);
+    if (prepare) {
+      const cudaError_t e = flow_pass<PtFlow, DIM>(pass, P, G, M, s, true);
+      if (e != cudaSuccess) return e;
+    } else if (P.flux[0] != nullptr) {
+      return flow_pass<PtFlow, DIM>(pass, P, G, M, s, false);
+    }
+  }
   if (pass == PASS_O1) return ptueq_one<DIM, PASS_O1>(P, G, eos, s, prepare);
   if (pass == PASS_PRED) return ptueq_one<DIM, PASS_PRED>(P, G, eos, s, prepare);
   return ptueq_one<DIM, PASS_CORR>(P, G, eos, s, prepare);
