@@ -416,24 +416,34 @@ __device__ __forceinline__ bool relax_pinf(const Model<NP>& M, double a[NP], dou
     else st.rejected = true;
   }
   double aS[NP], rS[NP];
-  double f = 0., df = 1., drhodp = 0.;
-  int iteration = 0;
-  do {
-    iteration++;
-    ps -= ndiv(f, df);
-#pragma unroll
-    for (int k = 0; k < NP; k++) ps = eos_fix_p(M.eos[k], ps);
-    f = -1.;
-    df = 0.;
-#pragma unroll
-    for (int k = 0; k < NP; k++) {
-      rS[k] = eos_rho_pfinal(M.eos[k], M.eps, p[k], r[k], ps, &drhodp);
-      aS[k] = ndiv(a[k] * r[k], rS[k]);
-      double dalpha = ndiv(a[k] * r[k] * drhodp, rS[k] * rS[k]);
-      f += aS[k];
-      df -= dalpha;
+  // the first evaluation is at the start itself (f / df = 0 / 1 before it)
+  NewtonState s{ps, 0., 1., 1, 1.};
+  bool quick = pinf_quick<NP>(M, a, r, s, p, aS, rS);
+  while (quick && fabs(s.f) > 1e-10 && s.it < max_iter) {
+    const double d = qdiv(s.f, s.df, s.ydf);
+    if (!(d == d)) {
+      quick = false;
+      break;
     }
-  } while (fabs(f) > 1e-10 && iteration < max_iter);
+    s.it++;
+    s.ps -= d;
+    quick = pinf_quick<NP>(M, a, r, s, p, aS, rS);
+  }
+  if (!quick) {  // the whole iteration in the general form (the iterates up to here are its own, bit for bit)
+    s.ps = ps;
+    s.it = 0;
+    s.f = 0.;
+    s.df = 1.;
+    do {
+      s.it++;
+      s.ps -= ndiv(s.f, s.df);
+#pragma unroll
+      for (int k = 0; k < NP; k++) s.ps = eos_fix_p(M.eos[k], s.ps);
+      pinf_eval_general<NP>(M, a, r, s, p, aS, rS);
+    } while (fabs(s.f) > 1e-10 && s.it < max_iter);
+  }
+  const int iteration = s.it;
+  ps = s.ps;
   st.iters = iteration;
   if (iteration < max_iter || accept) {  // accept: a capped iteration keeps its last iterate
 #pragma unroll
@@ -478,16 +488,6 @@ __device__ __forceinline__ bool relax_pinf(const Model<NP>& M, double a[NP], dou
 
 // ------------------------------------------------------------------ relaxation (p-T-mu, 2 phases)
 
-// Pieces of the same relaxation for the seeded kernels, which gate the learned seed on the first
-// evaluation: a Newton state after k evaluations, one evaluation at an iterate (verifyAndModifyPressure
-// of every phase, then f = sum_k alpha_k rho_k / rho_k*(p) - 1 and its derivative) and the
-// interface-pressure fallback (RelaxationP::NewtonRaphson src/Relaxations/RelaxationP.cpp:43-68,
-// RelaxationPInfinite.cpp:43-97).  The arithmetic is relax_pinf's, operation for operation.
-struct NewtonState {
-  double ps, f, df;
-  int it;
-};
-
 template <int NP>
 __device__ __forceinline__ bool pinf_applies(const Model<NP>& M, const double a[NP]) {
   if (M.eps > 1.e-20) {
@@ -497,24 +497,101 @@ __device__ __forceinline__ bool pinf_applies(const Model<NP>& M, const double a[
   }
   return true;
 }
+// A Newton state after `it` evaluations at the iterates up to ps (RelaxationP::NewtonRaphson
+// src/Relaxations/RelaxationP.cpp:43-68): f = sum_k alpha_k rho_k / rho_k*(ps) - 1, its derivative df, and an
+// approximate reciprocal ydf of df (NaN: none).
+struct NewtonState {
+  double ps, f, df;
+  int it;
+  double ydf;
+};
 
+// One evaluation, term by term (the general form).
 template <int NP>
-__device__ __forceinline__ void pinf_eval(const Model<NP>& M, const double a[NP], const double r[NP], NewtonState& s,
-                                          const double p[NP], double aS[NP], double rS[NP]) {
+__device__ __forceinline__ void pinf_eval_general(const Model<NP>& M, const double a[NP], const double r[NP],
+                                                      NewtonState& s, const double p[NP], double aS[NP],
+                                                      double rS[NP]) {
   double drhodp = 0.;
-#pragma unroll
-  for (int k = 0; k < NP; k++) s.ps = eos_fix_p(M.eos[k], s.ps);
   s.f = -1.;
   s.df = 0.;
 #pragma unroll
   for (int k = 0; k < NP; k++) {
     rS[k] = eos_rho_pfinal(M.eos[k], M.eps, p[k], r[k], s.ps, &drhodp);
     aS[k] = ndiv(a[k] * r[k], rS[k]);
-    double dalpha = ndiv(a[k] * r[k] * drhodp, rS[k] * rS[k]);
+    const double dalpha = ndiv(a[k] * r[k] * drhodp, rS[k] * rS[k]);
     s.f += aS[k];
     s.df -= dalpha;
   }
+  s.ydf = __longlong_as_double(0x7ff8000000000000ll);
 }
+
+// One evaluation at s.ps, after verifyAndModifyPressure of every phase.
+//
+// The iteration is a serial chain, up to 60 evaluations long in the cells of a contact, and those cells set the
+// time of a small mesh's step.  Term by term it holds three dependent divisions, each a reciprocal sequence
+// (an approximation and two Newton steps) and a correction.  The quotients and their order are the same here,
+// but the reciprocals come from values at hand before the exact divisors: with rho* = rho num / denom,
+// 1/denom and 1/(rho num) start side by side, 1/rho* is denom (1/(rho num)), the squares' reciprocals are the
+// reciprocals' squares, and 1/df is taken from the derivative assembled from them, while f and df themselves
+// are still being rounded.  A quotient corrected with a reciprocal of a few ulps' error is RN(a / b) unless
+// a / b lies within 2^-47 ulp of a midpoint (the residual is exact, the correction a product of two errors).
+// Measured with the same bits (one B200, mid-run states, per step): tube of 1000 cells, whose contact cells need
+// 55 evaluations, 25.4 -> 23.1 us; cell kernels of 191 x 103 cells 32 / 34 -> 23 / 23 us, of 2048^2 0.41 / 0.43
+// -> 0.36 / 0.37 ms, of 256^3 (three phases, at most 6 evaluations) 2.36 / 2.38 -> 2.24 / 2.27 ms.  With the
+// general form as a branch inside the loop the three-phase cell kernel spilled 192 bytes and took 2.46 ms.
+// Returns false where the general form has to run: for NASG phases, and where a divisor lies near its floor or
+// an operand is zero, infinite or NaN (f or df is NaN then).
+template <int NP>
+__device__ __forceinline__ bool pinf_quick(const Model<NP>& M, const double a[NP], const double r[NP], NewtonState& s,
+                                          const double p[NP], double aS[NP], double rS[NP]) {
+#pragma unroll
+  for (int k = 0; k < NP; k++) s.ps = eos_fix_p(M.eos[k], s.ps);
+  const double ps = s.ps;
+  double f = -1., df = 0., dfa = 0.;
+  bool plain = true;
+  const double low = M.eps > 0. ? 1.e-7 : 1.e-140;  // above it eos_rho_pfinal's floors of denom and denom^2 do nothing
+#pragma unroll
+  for (int k = 0; k < NP; k++) {
+    const EosParams& q = M.eos[k];
+    plain = plain && q.type != ECG_EOS_NASG;
+    const double pi = q.type == ECG_EOS_IG ? 0. : q.pinf;
+    const double num = q.type == ECG_EOS_IG ? q.gamma * ps : q.gamma * (ps + pi);
+    const double denom = num + p[k] - ps;
+    plain = plain && denom > low;
+    const double rn = r[k] * num, d2 = denom * denom, ar = a[k] * r[k];
+    const double c = q.type == ECG_EOS_IG ? r[k] * q.gamma * p[k] : r[k] * q.gamma * (p[k] + pi);
+    const double yd = nrcp(denom), yn = nrcp(rn);
+    const double yr = denom * yn, yd2 = yd * yd, yr2 = yr * yr;
+    dfa -= (ar * c) * (yd2 * yr2);
+    const double rho = qdiv(rn, denom, yd);
+    const double drhodp = qdiv(c, d2, yd2);
+    const double as = qdiv(ar, rho, yr);
+    const double dalpha = qdiv(ar * drhodp, rho * rho, yr2);
+    rS[k] = rho;
+    aS[k] = as;
+    f += as;
+    df -= dalpha;
+  }
+  s.f = f;
+  s.df = df;
+  s.ydf = nrcp(dfa);
+  return plain && f == f && df == df;
+}
+
+// One evaluation in either form (the seeded kernels').
+template <int NP>
+__device__ __forceinline__ void pinf_eval(const Model<NP>& M, const double a[NP], const double r[NP], NewtonState& s,
+                                          const double p[NP], double aS[NP], double rS[NP]) {
+  if (!pinf_quick<NP>(M, a, r, s, p, aS, rS)) pinf_eval_general<NP>(M, a, r, s, p, aS, rS);
+}
+
+// The Newton step f / df of the seeded kernels.
+__device__ __forceinline__ double newton_step(const NewtonState& s) {
+  double d = qdiv(s.f, s.df, s.ydf);
+  if (!(d == d)) d = ndiv(s.f, s.df);
+  return d;
+}
+
 
 // First evaluation at the plain start sum_k alpha_k p_k (relax_pinf's first iteration).
 template <int NP>
@@ -523,7 +600,7 @@ __device__ __forceinline__ void pinf_first(const Model<NP>& M, const double a[NP
   double ps = 0.;
 #pragma unroll
   for (int k = 0; k < NP; k++) ps += a[k] * p[k];
-  s.ps = ps - 0. / 1.;
+  s.ps = ps;
   s.it = 1;
   pinf_eval<NP>(M, a, r, s, p, aS, rS);
 }
@@ -535,7 +612,7 @@ __device__ __forceinline__ void pinf_finish(const Model<NP>& M, double a[NP], do
                                             int max_iter, bool accept = false) {
   while (fabs(s.f) > 1e-10 && s.it < max_iter) {
     s.it++;
-    s.ps -= ndiv(s.f, s.df);
+    s.ps -= newton_step(s);
     pinf_eval<NP>(M, a, r, s, p, aS, rS);
   }
   st.iters = s.it;
@@ -557,6 +634,7 @@ __device__ __forceinline__ void pinf_finish(const Model<NP>& M, double a[NP], do
 #pragma unroll
     for (int j = 0; j < NP; j++)
       if (j != k) sumZj += zk[j];
+  double drhodp = 0.;
     pI += sumZj * (p[k] - 0.);
   }
   pI = ndiv(pI, sumZk * (NP - 1));

@@ -103,6 +103,13 @@ __device__ __forceinline__ double nrcp(double b) {
   return fma(y, e, y);
 }
 
+// a / b with a reciprocal y of b that is a few ulps off: RN(a / b) unless a / b lies within 2^-47 ulp of a
+// midpoint.  NaN when an operand is zero (b), infinite or NaN.
+__device__ __forceinline__ double qdiv(double a, double b, double y) {
+  const double q = a * y;
+  return fma(-fma(b, q, -a), y, q);
+}
+
 // a / b for a divisor whose correctly rounded reciprocal y = RN(1/b) is at hand (EOS constants, computed on
 // the host): Markstein's correction alone.
 __device__ __forceinline__ double cdiv(double a, double b, double y) {

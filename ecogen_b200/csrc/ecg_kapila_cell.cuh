@@ -562,7 +562,7 @@ __device__ __forceinline__ void kapila_finish(const StepParams& P, const Model<N
 #pragma unroll
         for (int k = 1; k < NP; k++) { lo = dmin(lo, pk[k]); hi = dmax(hi, pk[k]); }
         if (isfinite(g.seed) && g.seed >= lo && g.seed <= hi) {
-          s.ps = g.seed - 0. / 1.;
+          s.ps = g.seed;
           s.it += 1;
           pinf_eval<NP>(M, a, r, s, pk, aS, rS);
           rs.seeded = true;
