@@ -274,6 +274,7 @@ ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
   P.ptmu = x->c.ptmu;
   P.ptmu_liq = x->c.ptmu_liquid;
   P.ptmu_vap = x->c.ptmu_vapor;
+  if (P.ptmu) P.pt_mu = make_ptmu_params(x->c.eos[P.ptmu_liq], x->c.eos[P.ptmu_vap]);
   P.pcrit = x->pcrit;
   P.ptmu_seed_p = x->ptmu_seed_p;
   P.tsat_hist = x->tsat_hist;

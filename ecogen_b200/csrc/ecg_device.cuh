@@ -382,121 +382,6 @@ struct RelaxStats {
   bool rejected;  // the learned seed was rejected (plain start used)
 };
 
-// RelaxationPInfinite::relaxation src/Relaxations/RelaxationPInfinite.cpp:43-97 with
-// RelaxationP::NewtonRaphson src/Relaxations/RelaxationP.cpp:43-68.  a/r/p are the phase state
-// after buildPrim (p per phase); the phase sound speeds of that state are needed only by the
-// interface-pressure fallback, RelaxationP::computeInterfacePressure :72, recomputed there from
-// the same rho_k, p_k as PhaseUEq::extendedCalculusPhase does).  On return a/r hold
-// the relaxed state and pstar the relaxed pressure; returns false if the relaxation was skipped.
-template <int NP>
-__device__ __forceinline__ bool relax_pinf(const Model<NP>& M, double a[NP], double r[NP], const double p[NP],
-                                           double& pstar, RelaxStats& st, double seed, bool use_seed,
-                                           int max_iter, bool accept = false) {
-  st.iters = 0;
-  st.fallback = false;
-  st.seeded = false;
-  st.rejected = false;
-  if (M.eps > 1.e-20) {
-    bool relax = true;
-#pragma unroll
-    for (int k = 0; k < NP; k++)
-      if (a[k] > (1. - 1.e-5)) relax = false;
-    if (!relax) return false;
-  }
-  double ps = 0.;
-#pragma unroll
-  for (int k = 0; k < NP; k++) ps += a[k] * p[k];
-  if (use_seed) {
-    // A learned initial guess replaces sum_k alpha_k p_k only when it is finite and inside the
-    // bracket of the phase pressures; otherwise it is rejected and the plain start is kept.
-    double lo = p[0], hi = p[0];
-#pragma unroll
-    for (int k = 1; k < NP; k++) { lo = dmin(lo, p[k]); hi = dmax(hi, p[k]); }
-    if (isfinite(seed) && seed >= lo && seed <= hi) { ps = seed; st.seeded = true; }
-    else st.rejected = true;
-  }
-  double aS[NP], rS[NP];
-  // the first evaluation is at the start itself (f / df = 0 / 1 before it)
-  NewtonState s{ps, 0., 1., 1, 1.};
-  bool quick = pinf_quick<NP>(M, a, r, s, p, aS, rS);
-  while (quick && fabs(s.f) > 1e-10 && s.it < max_iter) {
-    const double d = qdiv(s.f, s.df, s.ydf);
-    if (!(d == d)) {
-      quick = false;
-      break;
-    }
-    s.it++;
-    s.ps -= d;
-    quick = pinf_quick<NP>(M, a, r, s, p, aS, rS);
-  }
-  if (!quick) {  // the whole iteration in the general form (the iterates up to here are its own, bit for bit)
-    s.ps = ps;
-    s.it = 0;
-    s.f = 0.;
-    s.df = 1.;
-    do {
-      s.it++;
-      s.ps -= ndiv(s.f, s.df);
-#pragma unroll
-      for (int k = 0; k < NP; k++) s.ps = eos_fix_p(M.eos[k], s.ps);
-      pinf_eval_general<NP>(M, a, r, s, p, aS, rS);
-    } while (fabs(s.f) > 1e-10 && s.it < max_iter);
-  }
-  const int iteration = s.it;
-  ps = s.ps;
-  st.iters = iteration;
-  if (iteration < max_iter || accept) {  // accept: a capped iteration keeps its last iterate
-#pragma unroll
-    for (int k = 0; k < NP; k++) { a[k] = aS[k]; r[k] = rS[k]; }
-    pstar = ps;
-    return true;
-  }
-  st.fallback = true;
-  double zk[NP], pI = 0., sumZk = 0.;
-#pragma unroll
-  for (int k = 0; k < NP; k++) zk[k] = r[k] * eos_c(M.eos[k], M.eps, r[k], p[k]);
-#pragma unroll
-  for (int k = 0; k < NP; k++) {
-    sumZk += zk[k];
-    double sumZj = 0.;
-#pragma unroll
-    for (int j = 0; j < NP; j++)
-      if (j != k) sumZj += zk[j];
-    pI += sumZj * (p[k] - 0.);
-  }
-  pI = ndiv(pI, sumZk * (NP - 1));
-#pragma unroll
-  for (int k = 0; k < NP; k++) pI = eos_fix_p(M.eos[k], pI);
-#pragma unroll
-  for (int k = 0; k < NP; k++) {
-    double rr = eos_rho_pfinal(M.eos[k], M.eps, p[k], r[k], pI, &drhodp);
-    a[k] = ndiv(a[k] * r[k], rr);
-    r[k] = rr;
-  }
-  pstar = pI;
-  return true;
-}
-
-
-// ------------------------------------------------------------------ logarithm of the saturation solve
-// The saturation temperature solve (Mixture::computeTsat) branches on tight tests (pure-phase
-// hypotheses, |f| > 1e-10), so a last-ulp difference between the device's log and the host libm's can
-// change a cell's path.  It takes its logarithms from elog (ecg_pow.cuh): ln x carried as a
-// double-double from a 128-row table and rounded once, i.e. the correctly rounded logarithm except
-// within about 2^-75 of a midpoint; on the solve's arguments (temperatures, pressures) it equals the
-// host glibc log on every one of 8e6 tested values.
-
-// ------------------------------------------------------------------ relaxation (p-T-mu, 2 phases)
-
-template <int NP>
-__device__ __forceinline__ bool pinf_applies(const Model<NP>& M, const double a[NP]) {
-  if (M.eps > 1.e-20) {
-#pragma unroll
-    for (int k = 0; k < NP; k++)
-      if (a[k] > (1. - 1.e-5)) return false;
-  }
-  return true;
-}
 // A Newton state after `it` evaluations at the iterates up to ps (RelaxationP::NewtonRaphson
 // src/Relaxations/RelaxationP.cpp:43-68): f = sum_k alpha_k rho_k / rho_k*(ps) - 1, its derivative df, and an
 // approximate reciprocal ydf of df (NaN: none).
@@ -592,6 +477,122 @@ __device__ __forceinline__ double newton_step(const NewtonState& s) {
   return d;
 }
 
+// RelaxationPInfinite::relaxation src/Relaxations/RelaxationPInfinite.cpp:43-97 with
+// RelaxationP::NewtonRaphson src/Relaxations/RelaxationP.cpp:43-68.  a/r/p are the phase state
+// after buildPrim (p per phase); the phase sound speeds of that state are needed only by the
+// interface-pressure fallback, RelaxationP::computeInterfacePressure :72, recomputed there from
+// the same rho_k, p_k as PhaseUEq::extendedCalculusPhase does).  On return a/r hold
+// the relaxed state and pstar the relaxed pressure; returns false if the relaxation was skipped.
+template <int NP>
+__device__ __forceinline__ bool relax_pinf(const Model<NP>& M, double a[NP], double r[NP], const double p[NP],
+                                           double& pstar, RelaxStats& st, double seed, bool use_seed,
+                                           int max_iter, bool accept = false) {
+  st.iters = 0;
+  st.fallback = false;
+  st.seeded = false;
+  st.rejected = false;
+  if (M.eps > 1.e-20) {
+    bool relax = true;
+#pragma unroll
+    for (int k = 0; k < NP; k++)
+      if (a[k] > (1. - 1.e-5)) relax = false;
+    if (!relax) return false;
+  }
+  double ps = 0.;
+#pragma unroll
+  for (int k = 0; k < NP; k++) ps += a[k] * p[k];
+  if (use_seed) {
+    // A learned initial guess replaces sum_k alpha_k p_k only when it is finite and inside the
+    // bracket of the phase pressures; otherwise it is rejected and the plain start is kept.
+    double lo = p[0], hi = p[0];
+#pragma unroll
+    for (int k = 1; k < NP; k++) { lo = dmin(lo, p[k]); hi = dmax(hi, p[k]); }
+    if (isfinite(seed) && seed >= lo && seed <= hi) { ps = seed; st.seeded = true; }
+    else st.rejected = true;
+  }
+  double aS[NP], rS[NP];
+  // the first evaluation is at the start itself (f / df = 0 / 1 before it)
+  NewtonState s{ps, 0., 1., 1, 1.};
+  bool quick = pinf_quick<NP>(M, a, r, s, p, aS, rS);
+  while (quick && fabs(s.f) > 1e-10 && s.it < max_iter) {
+    const double d = qdiv(s.f, s.df, s.ydf);
+    if (!(d == d)) {
+      quick = false;
+      break;
+    }
+    s.it++;
+    s.ps -= d;
+    quick = pinf_quick<NP>(M, a, r, s, p, aS, rS);
+  }
+  if (!quick) {  // the whole iteration in the general form (the iterates up to here are its own, bit for bit)
+    s.ps = ps;
+    s.it = 0;
+    s.f = 0.;
+    s.df = 1.;
+    do {
+      s.it++;
+      s.ps -= ndiv(s.f, s.df);
+#pragma unroll
+      for (int k = 0; k < NP; k++) s.ps = eos_fix_p(M.eos[k], s.ps);
+      pinf_eval_general<NP>(M, a, r, s, p, aS, rS);
+    } while (fabs(s.f) > 1e-10 && s.it < max_iter);
+  }
+  const int iteration = s.it;
+  ps = s.ps;
+  st.iters = iteration;
+  if (iteration < max_iter || accept) {  // accept: a capped iteration keeps its last iterate
+#pragma unroll
+    for (int k = 0; k < NP; k++) { a[k] = aS[k]; r[k] = rS[k]; }
+    pstar = ps;
+    return true;
+  }
+  st.fallback = true;
+  double drhodp = 0.;
+  double zk[NP], pI = 0., sumZk = 0.;
+#pragma unroll
+  for (int k = 0; k < NP; k++) zk[k] = r[k] * eos_c(M.eos[k], M.eps, r[k], p[k]);
+#pragma unroll
+  for (int k = 0; k < NP; k++) {
+    sumZk += zk[k];
+    double sumZj = 0.;
+#pragma unroll
+    for (int j = 0; j < NP; j++)
+      if (j != k) sumZj += zk[j];
+    pI += sumZj * (p[k] - 0.);
+  }
+  pI = ndiv(pI, sumZk * (NP - 1));
+#pragma unroll
+  for (int k = 0; k < NP; k++) pI = eos_fix_p(M.eos[k], pI);
+#pragma unroll
+  for (int k = 0; k < NP; k++) {
+    double rr = eos_rho_pfinal(M.eos[k], M.eps, p[k], r[k], pI, &drhodp);
+    a[k] = ndiv(a[k] * r[k], rr);
+    r[k] = rr;
+  }
+  pstar = pI;
+  return true;
+}
+
+
+// ------------------------------------------------------------------ logarithm of the saturation solve
+// The saturation temperature solve (Mixture::computeTsat) branches on tight tests (pure-phase
+// hypotheses, |f| > 1e-10), so a last-ulp difference between the device's log and the host libm's can
+// change a cell's path.  It takes its logarithms from elog (ecg_pow.cuh): ln x carried as a
+// double-double from a 128-row table and rounded once, i.e. the correctly rounded logarithm except
+// within about 2^-75 of a midpoint; on the solve's arguments (temperatures, pressures) it equals the
+// host glibc log on every one of 8e6 tested values.
+
+// ------------------------------------------------------------------ relaxation (p-T-mu, 2 phases)
+
+template <int NP>
+__device__ __forceinline__ bool pinf_applies(const Model<NP>& M, const double a[NP]) {
+  if (M.eps > 1.e-20) {
+#pragma unroll
+    for (int k = 0; k < NP; k++)
+      if (a[k] > (1. - 1.e-5)) return false;
+  }
+  return true;
+}
 
 // First evaluation at the plain start sum_k alpha_k p_k (relax_pinf's first iteration).
 template <int NP>
@@ -634,7 +635,6 @@ __device__ __forceinline__ void pinf_finish(const Model<NP>& M, double a[NP], do
 #pragma unroll
     for (int j = 0; j < NP; j++)
       if (j != k) sumZj += zk[j];
-  double drhodp = 0.;
     pI += sumZj * (p[k] - 0.);
   }
   pI = ndiv(pI, sumZk * (NP - 1));
@@ -668,40 +668,44 @@ struct PtmuCount {
 // start right of it jumps left of it in one step, possibly past T = 0.  So a start is taken only inside
 // (0, 0.5 B / C), and an iterate that leaves (0, B / C) sends the iteration back to the cold start
 // (at most once); either way it converges to the root the reference's iteration finds.
-__device__ __forceinline__ double compute_tsat(const EosParams& L, const EosParams& V, double p, double* dTsat,
-                                               bool& err, PtmuCount* pc = nullptr, double T0 = -1.) {
-  double gL = L.gamma, piL = (L.type == ECG_EOS_IG) ? 0. : L.pinf, cvL = L.cv, e0L = L.eref, s0L = L.sref;
-  double gV = V.gamma, piV = (V.type == ECG_EOS_IG) ? 0. : V.pinf, cvV = V.cv, e0V = V.eref, s0V = V.sref;
-  double A = ndiv(gL * cvL - gV * cvV + s0V - s0L, gV * cvV - cvV);
-  double B = ndiv(e0L - e0V, gV * cvV - cvV);
-  double C = ndiv(gV * cvV - gL * cvL, gV * cvV - cvV);
-  double D = ndiv(gL * cvL - cvL, gV * cvV - cvV);
+__device__ __forceinline__ double compute_tsat(const PtmuParams& t, double p, double* dTsat, bool& err,
+                                               PtmuCount* pc = nullptr, double T0 = -1.) {
+  const double piL = (t.liq.type == ECG_EOS_IG) ? 0. : t.liq.pinf, piV = (t.vap.type == ECG_EOS_IG) ? 0. : t.vap.pinf;
   int iteration = 0;
-  bool seeded = T0 > 0. && T0 < ndiv(0.5 * B, C);
-  double Tsat = seeded ? T0 : ndiv(0.1 * B, C), f = 0., df = 1.;
+  bool seeded = T0 > 0. && T0 < t.half;
+  double Tsat = seeded ? T0 : t.cold, f = 0., df = 1., step = 0.;
   // ln(p + pInf) of both phases do not depend on the iterate: evaluated once per solve (the same
   // values enter the same sum, so f has the bits of the reference's per-iteration evaluation)
-  const double lnV = elog(p + piV), lnL = elog(p + piL);
+  const double lnV = elog(p + piV), lnL = t.D * elog(p + piL);
   do {
-    Tsat -= ndiv(f, df);
-    if (seeded && !(Tsat > 0. && Tsat < ndiv(B, C))) {  // a seeded iterate left the root's branch
+    Tsat -= step;
+    if (seeded && !(Tsat > 0. && Tsat < t.branch)) {  // a seeded iterate left the root's branch
       seeded = false;
-      Tsat = ndiv(0.1 * B, C);
+      Tsat = t.cold;
     }
     iteration++;
     if (iteration > 50) {
       err = true;
       break;
     }
-    f = A + ndiv(B, Tsat) + C * elog(Tsat) - lnV + D * lnL;
-    df = ndiv(C, Tsat) - ndiv(B, Tsat * Tsat);
+    // B/T, C/T and B/T^2 from one reciprocal (1/T^2 is its square); zero, infinite and NaN iterates make the
+    // derivative NaN and take the general quotients
+    const double y = nrcp(Tsat), T2 = Tsat * Tsat;
+    double bT = qdiv(t.B, Tsat, y);
+    df = qdiv(t.C, Tsat, y) - qdiv(t.B, T2, y * y);
+    if (!(df == df)) {
+      bT = ndiv(t.B, Tsat);
+      df = ndiv(t.C, Tsat) - ndiv(t.B, T2);
+    }
+    f = t.A + bT + t.C * elog(Tsat) - lnV + lnL;
+    step = ndiv(f, df);
   } while (fabs(f) > 1e-10);
   if (pc) {
     pc->tsat_calls++;
     pc->tsat_iters += (unsigned int)iteration;
     pc->tsat_max = max(pc->tsat_max, (unsigned int)iteration);
   }
-  double dfdp = ndiv(-1., p + piV) + ndiv(D, p + piL);
+  double dfdp = ndiv(-1., p + piV) + ndiv(t.D, p + piL);
   *dTsat = ndiv(-dfdp, df);
   return Tsat;
 }
@@ -743,11 +747,17 @@ __device__ __forceinline__ double eos_rhoe_sat(const EosParams& q, double p, dou
 // iteration on p* starts at p_seed instead of sum_k alpha_k p_k.  Every loop still stops at
 // |f| <= 1e-10.
 template <int NP>
-__device__ __forceinline__ bool relax_ptmu(const Model<NP>& M, int liq, int vap, double pcrit, double a[NP],
+__device__ __forceinline__ bool relax_ptmu(const Model<NP>& M, const PtmuParams& t, int liq, double pcrit, double a[NP],
                                            double r[NP], double p[NP], double rhomix, double emix, bool& err,
                                            PtmuCount* pc = nullptr, double p_seed = -1., double T_seed = -1.) {
-  const EosParams& EL = M.eos[liq];
-  const EosParams& EV = M.eos[vap];
+  const EosParams& EL = t.liq;
+  const EosParams& EV = t.vap;
+  const bool first = liq == 0;  // the liquid is phase 0 (two phases; no run-time index into the phase arrays)
+  // (liquid, vapour) values of a phase array
+  auto put = [&](double x[NP], double l, double v) {
+    x[0] = first ? l : v;
+    x[1] = first ? v : l;
+  };
   double pStar = 0., Tsat, dTsat = 0.;
 #pragma unroll
   for (int k = 0; k < NP; k++) pStar += a[k] * p[k];
@@ -756,24 +766,22 @@ __device__ __forceinline__ bool relax_ptmu(const Model<NP>& M, int liq, int vap,
   double pv = eos_p(EV, M.eps, rho, emix);
   double Tv = eos_T(EV, M.eps, rho, pv);
   if (pv > 0) {
-    Tsat = compute_tsat(EL, EV, pv, &dTsat, err, pc);
+    Tsat = compute_tsat(t, pv, &dTsat, err, pc);
     if (Tv >= Tsat) {
-      a[vap] = 1.;
-      a[liq] = 0.;
-      r[vap] = rho;
-      p[vap] = pv;
+      put(a, 0., 1.);
+      put(r, first ? r[0] : r[1], rho);
+      put(p, first ? p[0] : p[1], pv);
       return true;
     }
   }
   double pl = eos_p(EL, M.eps, rho, emix);
   double Tl = eos_T(EL, M.eps, rho, pl);
   if (pl > 0.) {
-    Tsat = compute_tsat(EL, EV, pl, &dTsat, err, pc);
+    Tsat = compute_tsat(t, pl, &dTsat, err, pc);
     if (Tl <= Tsat) {
-      a[liq] = 1.;
-      a[vap] = 0.;
-      r[liq] = rho;
-      p[liq] = pl;
+      put(a, 1., 0.);
+      put(r, rho, first ? r[1] : r[0]);
+      put(p, pl, first ? p[1] : p[0]);
       return true;
     }
   }
@@ -792,7 +800,7 @@ __device__ __forceinline__ bool relax_ptmu(const Model<NP>& M, int liq, int vap,
     }
 #pragma unroll
     for (int k = 0; k < NP; k++) pStar = eos_fix_p(M.eos[k], pStar);
-    Tsat = compute_tsat(EL, EV, pStar, &dTsat, err, pc, Tstart);
+    Tsat = compute_tsat(t, pStar, &dTsat, err, pc, Tstart);
     if (T_seed > 0.) Tstart = Tsat;
     rhoLSat = eos_rho_sat(EL, M.eps, pStar, Tsat, dTsat, &drhoLSat);
     rhoVSat = eos_rho_sat(EV, M.eps, pStar, Tsat, dTsat, &drhoVSat);
@@ -816,12 +824,9 @@ __device__ __forceinline__ bool relax_ptmu(const Model<NP>& M, int liq, int vap,
     pc->pstar = pStar;
     pc->tsat = Tsat;
   }
-  a[liq] = aLSat;
-  r[liq] = rhoLSat;
-  p[liq] = pStar;
-  a[vap] = aVSat;
-  r[vap] = rhoVSat;
-  p[vap] = pStar;
+  put(a, aLSat, aVSat);
+  put(r, rhoLSat, rhoVSat);
+  put(p, pStar, pStar);
   return true;
 }
 

@@ -585,12 +585,17 @@ __device__ __forceinline__ void kapila_finish(const StepParams& P, const Model<N
     // mixture internal energy of the rebuilt state (MixUEq::computeMixtureVariables :136), which
     // RelaxationPTMu reads before any fulfillState
     const double emix = rebuilt_emix<NP>(M, a0, r0, p0, rhomix);
+    PtmuParams T = P.pt_mu;
+    if (!XPT) {  // EOS types compiled in: both phases' type is the first one's
+      T.liq.type = M.eos[0].type;
+      T.vap.type = M.eos[0].type;
+    }
     bool err = false;
     const double ps = SEED ? g.ptmu_p : -1.;
     // T_sat start: the network's (seeded kernels), else the cell's previous converged T_sat when the
     // warm start is on (a value <= 0: no solve yet, cold start), else the reference's cold start
     const double Ts = SEED ? g.ptmu_T : (P.tsat_hist != nullptr ? P.tsat_hist[cell] : -1.);
-    if (relax_ptmu<NP>(M, P.ptmu_liq, P.ptmu_vap, P.pcrit, a, r, pk, rhomix, emix, err, &cc.pc, ps, Ts)) {
+    if (relax_ptmu<NP>(M, T, P.ptmu_liq, P.pcrit, a, r, pk, rhomix, emix, err, &cc.pc, ps, Ts)) {
       rhomix = 0.;
 #pragma unroll
       for (int k = 0; k < NP; k++) rhomix += a[k] * r[k];

@@ -193,6 +193,7 @@ extern "C" ecg_status ecg_step_noalloc(const ecg_case* c, const double* state_in
   P.ptmu = c->ptmu;
   P.ptmu_liq = c->ptmu_liquid;
   P.ptmu_vap = c->ptmu_vapor;
+  if (P.ptmu) P.pt_mu = make_ptmu_params(c->eos[P.ptmu_liq], c->eos[P.ptmu_vap]);
   if (c->ptmu) {
     const ecg_eos& L = c->eos[c->ptmu_liquid];
     const ecg_eos& V = c->eos[c->ptmu_vapor];

@@ -30,7 +30,7 @@
 // host build against glibc and 300-bit arithmetic, tests/test_gpu_pow.py the device build against the host
 // build bit for bit.
 //
-// Domain: x in [2^-60, 2^60] and 0 < y <= 10, which holds every density ratio and EOS gamma of the
+// Domain: x in [2^-60, 2^61) and y in [2^-60, 8), which holds every density ratio and EOS gamma of the
 // step; any other argument (zero, negative, infinite, NaN, far outside that range) goes to CUDA's pow,
 // which keeps its special values.
 #pragma once
@@ -116,7 +116,8 @@ ECG_POW_FN void epow_log(double x, double& Lh, double& Ll) {
 // correctly rounded (300-bit arithmetic); tests/test_pow.py.  x outside the positive normal range goes to
 // the library's log.
 ECG_POW_FN double elog(double x) {
-  if (!(x >= 0x1p-1022 && x <= 0x1.fffffffffffffp1023)) return log_outside(x);
+  // positive and normal, by the exponent field (sign 0, exponent 1 .. 2046)
+  if ((uint32_t)(pow_bits(x) >> 52) - 1u >= 2046u) return log_outside(x);
   double Lh, Ll;
   epow_log(x, Lh, Ll);
   return Lh;
@@ -124,7 +125,9 @@ ECG_POW_FN double elog(double x) {
 
 // x^y by the tables (see above); pow_fma is the fused multiply-add of the device or of the host libm
 ECG_EPOW_FN double epow(double x, double y) {
-  if (!(x >= 0x1p-60 && x <= 0x1p60 && y > 0. && y <= 10.)) return pow_outside(x, y);
+  // by the exponent fields (sign 0): x in [2^-60, 2^61), y in [2^-60, 8)
+  if ((uint32_t)(pow_bits(x) >> 52) - (1023u - 60u) > 120u || (uint32_t)(pow_bits(y) >> 52) - (1023u - 60u) > 62u)
+    return pow_outside(x, y);
   double Lh, Ll;
   epow_log(x, Lh, Ll);
   // ---- Y = y ln x = Yh + Yl

@@ -131,6 +131,7 @@ struct StepParams {
   int rec_min_evals;
   // p-T-mu relaxation
   int ptmu, ptmu_liq, ptmu_vap;
+  PtmuParams pt_mu;
   double pcrit;
   int ptmu_seed_p;  // seeded p-T-mu: 1 = the network's p* starts the saturation Newton too (else T only)
   double* tsat_hist;  // p-T-mu warm start: per-cell T_sat of the cell's last saturation solve (nullptr: off)
