@@ -70,8 +70,88 @@ struct BatchTile {
   }
 };
 
+// Centre of cell g, with the reference's arithmetic.
+__device__ __forceinline__ double batch_centre(const BatchCase& C, int g) { return (g + 0.5) * C.dx; }
+
+template <int NP>
+__device__ __forceinline__ void store_batch_face(const BatchParams& B, int64_t fid, double mom, const Flux<NP>& F) {
+  double* out = B.flux + fid;
+#pragma unroll
+  for (int k = 0; k < NP; k++) {
+    out[(int64_t)k * B.nfaces] = F.a[k];
+    out[(int64_t)(NP + k) * B.nfaces] = F.m[k];
+    out[(int64_t)(2 * NP + k) * B.nfaces] = F.en[k];
+  }
+  out[(int64_t)(3 * NP) * B.nfaces] = mom;
+  out[(int64_t)(3 * NP + 1) * B.nfaces] = F.E;
+  out[(int64_t)(3 * NP + 2) * B.nfaces] = F.sM;
+  out[(int64_t)(3 * NP + 3) * B.nfaces] = F.uStar;
+}
+
+// The two sides of internal face f, face i of the item; FULFILL: their closure too.
+template <int NP, int TB, int PASS, int TYPES, bool FULFILL>
+__device__ __forceinline__ void batch_sides(const StepParams& P, const Model<NP>& M, const double* sq, const BatchCase& C,
+                                            int f, int i, bool pone, Thermo<NP>& tl, double ul[3], Thermo<NP>& tr,
+                                            double ur[3]) {
+  using FL = Fields<NP, 1>;
+  using K = BatchTile<NP, TB, PASS, TYPES>;
+  constexpr int RS = K::RL, SS = K::SS;
+  const double* a0 = K::NA0 ? sq + (size_t)FL::NQ * RS : sq;
+  const double* ssl = sq + (size_t)(FL::NQ + K::NA0) * RS;
+  const int gl = f - 1, rl = i + K::H - 1, rr = rl + 1;
+  const double pl = batch_centre(C, gl), pf = pl + 0.5 * C.dx, pr = batch_centre(C, gl + 1);
+  if (!K::O2) {
+    cell_thermo<NP, 1, FULFILL>(M, sq, RS, rl, tl, ul);
+    cell_thermo<NP, 1, FULFILL>(M, sq, RS, rr, tr, ur);
+  } else if (K::LSL) {
+    extrapolate_side<NP, 1, FULFILL>(M, sq, RS, rl, ssl, SS, i, 0, 0, 0, fabs(pf - pl), 1., pone, tl, ul);
+    extrapolate_side<NP, 1, FULFILL>(M, sq, RS, rr, ssl, SS, i + 1, 0, 0, 0, fabs(pf - pr), -1., pone, tr, ur);
+  } else {
+    const int f1 = i + 1;
+    const bool hasL = (gl - 1 >= 0), hasR = (gl + 2 < C.n);
+    const double aL = sq[FL::A * RS + rl], aR = sq[FL::A * RS + rr];
+    const double aLL = hasL ? a0[rl - 1] : 0., aRR = hasR ? a0[rr + 1] : 0.;
+    constexpr bool kThinc = (TYPES == EOS_DYNAMIC);
+    constexpr int kLim = code_limiter(TYPES);
+    reconstruct_side<NP, 1, kThinc, kLim, FULFILL>(M, P, sq, RS, rl, ssl, SS, f1, hasL ? i : -1, aL, aR, aLL,
+                                                   fabs(pf - pl), 1., tl, ul);
+    reconstruct_side<NP, 1, kThinc, kLim, FULFILL>(M, P, sq, RS, rr, ssl, SS, f1, hasR ? i + 2 : -1, aR, aL, aRR,
+                                                   fabs(pf - pr), -1., tr, ur);
+  }
+}
+
+// Any face of an item, sides of the case included, solved by fulfill and hllc and stored; returns its wave value.
 template <int NP, int TB, int PASS, int TYPES>
-__global__ void __launch_bounds__(TB, ECG_BATCH_SM_THREADS / TB) k_batch_faces(BatchParams B, Model<NP> M0) {
+static __device__ __noinline__ double batch_face_general(const BatchParams& B, const Model<NP>& M0, const double* sq,
+                                                         const BatchCase C, int f, int i, bool pone) {
+  const Model<NP> M = specialize_eos<NP, TYPES>(M0);
+  using K = BatchTile<NP, TB, PASS, TYPES>;
+  double wmax = wave_none(false), Fn[3];
+  Flux<NP> F;
+  if (f == 0 || f == C.n) {
+    // non-reflecting side: HLLC(cell, cell) in the side's frame (BoundCondNonReflecting::
+    // solveRiemannBoundary src/BoundConds/BoundCondNonReflecting.cpp:62)
+    const bool neg = f == 0;
+    Thermo<NP> t;
+    double ug[3], ul[3], mom[3];
+    cell_thermo<NP, 1>(M, sq, K::RL, neg ? i + K::H : i + K::H - 1, t, ug);
+    to_local(0, neg, ug, ul);
+    hllc<NP>(M, t, ul, t, ul, false, C.lcfl, C.lcfl, wmax, Fn, F);
+    to_global(0, neg, Fn, mom);
+    Fn[0] = mom[0];
+  } else {
+    Thermo<NP> tl, tr;
+    double ul[3], ur[3];
+    batch_sides<NP, TB, PASS, TYPES, true>(B.P, M, sq, C, f, i, pone, tl, ul, tr, ur);
+    hllc<NP, K::O2>(M, tl, ul, tr, ur, false, C.lcfl, C.lcfl, wmax, Fn, F);
+  }
+  store_batch_face<NP>(B, C.fbase + f, Fn[0], F);
+  return wmax;
+}
+
+template <int NP, int TB, int PASS, int TYPES>
+__global__ void __launch_bounds__(TB, ECG_BATCH_SM_THREADS / TB) k_batch_faces(const __grid_constant__ BatchParams B,
+                                                                                  const __grid_constant__ Model<NP> M0) {
   const Model<NP> M = specialize_eos<NP, TYPES>(M0);  // EOS types compiled in for the shipped workload
   using FL = Fields<NP, 1>;
   using K = BatchTile<NP, TB, PASS, TYPES>;
@@ -99,10 +179,9 @@ __global__ void __launch_bounds__(TB, ECG_BATCH_SM_THREADS / TB) k_batch_faces(B
     }
   }
   __syncthreads();
-  // centre of cell g and centre-to-centre distance of cells g, g + 1 with the reference's arithmetic
-  // (Element::distance: sqrt(x x), which is |x| bit for bit)
-  auto centre = [&](int g) { return (g + 0.5) * C.dx; };
-  auto dist = [&](int g) { return fabs(centre(g) - centre(g + 1)); };
+  // centre-to-centre distance of cells g, g + 1 with the reference's arithmetic (Element::distance: sqrt(x x),
+  // which is |x| bit for bit)
+  auto dist = [&](int g) { return fabs(batch_centre(C, g) - batch_centre(C, g + 1)); };
   bool pone = true;
   if (LSL) {
     double pf = M.eos[0].pfloor;
@@ -144,57 +223,26 @@ __global__ void __launch_bounds__(TB, ECG_BATCH_SM_THREADS / TB) k_batch_faces(B
   double wmax = wave_none(false);
   const int f = f0 + tid;
   if (tid < TF && f <= n) {
+    Thermo<NP> tl, tr;
+    double ul[3], ur[3], Fn[3];
     Flux<NP> F;
-    double Fn[3];
-    if (f == 0 || f == n) {
-      // non-reflecting side: HLLC(cell, cell) in the side's frame (BoundCondNonReflecting::
-      // solveRiemannBoundary src/BoundConds/BoundCondNonReflecting.cpp:62)
-      const bool neg = f == 0;
-      Thermo<NP> t;
-      double ug[3], ul[3];
-      cell_thermo<NP, 1>(M, sq, RS, neg ? tid + K::H : tid + K::H - 1, t, ug);
-      to_local(0, neg, ug, ul);
-      hllc<NP>(M, t, ul, t, ul, false, C.lcfl, C.lcfl, wmax, Fn, F);
-      to_global(0, neg, Fn, F.mom);
-    } else {
-      const int gl = f - 1, rl = tid + K::H - 1, rr = rl + 1;
-      Thermo<NP> tl, tr;
-      double ug[3], vg[3];
-      const double pl = centre(gl), pf = pl + 0.5 * C.dx, pr = centre(gl + 1);
-      if (!O2) {
-        cell_thermo<NP, 1>(M, sq, RS, rl, tl, ug);
-        cell_thermo<NP, 1>(M, sq, RS, rr, tr, vg);
-      } else if (LSL) {
-        extrapolate_side<NP, 1>(M, sq, RS, rl, ssl, SS, tid, 0, 0, 0, fabs(pf - pl), 1., pone, tl, ug);
-        extrapolate_side<NP, 1>(M, sq, RS, rr, ssl, SS, tid + 1, 0, 0, 0, fabs(pf - pr), -1., pone, tr,
-                                vg);
-      } else {
-        const int f1 = tid + 1;
-        const bool hasL = (gl - 1 >= 0), hasR = (gl + 2 < n);
-        const double* a0 = K::NA0 ? sa0 : sq;
-        const double aL = sq[FL::A * RS + rl], aR = sq[FL::A * RS + rr];
-        const double aLL = hasL ? a0[rl - 1] : 0., aRR = hasR ? a0[rr + 1] : 0.;
-        constexpr bool kThinc = (TYPES == EOS_DYNAMIC);
-        constexpr int kLim = code_limiter(TYPES);
-        reconstruct_side<NP, 1, kThinc, kLim>(M, P, sq, RS, rl, ssl, SS, f1, hasL ? tid : -1, aL, aR, aLL,
-                                              fabs(pf - pl), 1., tl, ug);
-        reconstruct_side<NP, 1, kThinc, kLim>(M, P, sq, RS, rr, ssl, SS, f1, hasR ? tid + 2 : -1, aR, aL, aRR,
-                                              fabs(pf - pr), -1., tr, vg);
-      }
-      hllc<NP, O2>(M, tl, ug, tr, vg, false, C.lcfl, C.lcfl, wmax, Fn, F);
-      F.mom[0] = Fn[0];
-    }
-    double* out = B.flux + C.fbase + f;
+    bool ok = true;
+    if (f > 0 && f < n) {
+      batch_sides<NP, TB, PASS, TYPES, false>(P, M, sq, C, f, tid, pone, tl, ul, tr, ur);
+    } else {  // a non-reflecting side: HLLC(cell, cell) in the side's frame, with the other faces of the warp
+      cell_thermo<NP, 1, false>(M, sq, RS, f == 0 ? tid + K::H : tid + K::H - 1, tl, ul);
+      if (f == 0) ul[0] = -ul[0];
+      tr = tl;
 #pragma unroll
-    for (int k = 0; k < NP; k++) {
-      out[(int64_t)k * B.nfaces] = F.a[k];
-      out[(int64_t)(NP + k) * B.nfaces] = F.m[k];
-      out[(int64_t)(2 * NP + k) * B.nfaces] = F.en[k];
+      for (int i = 0; i < 3; i++) ur[i] = ul[i];
+#pragma unroll
+      for (int k = 0; k < NP; k++) ok = ok && tl.r[k] >= 1.e-15;
     }
-    out[(int64_t)(3 * NP) * B.nfaces] = F.mom[0];
-    out[(int64_t)(3 * NP + 1) * B.nfaces] = F.E;
-    out[(int64_t)(3 * NP + 2) * B.nfaces] = F.sM;
-    out[(int64_t)(3 * NP + 3) * B.nfaces] = F.uStar;
+    const bool solved = hllc_quick<NP, !O2>(M, tl, ul, tr, ur, false, C.lcfl, C.lcfl, wmax, Fn, F, ok);
+    if (f == 0) Fn[0] = -Fn[0];
+    if (solved) store_batch_face<NP>(B, C.fbase + f, Fn[0], F);
+    // operands out of hllc_quick's range
+    if (!solved) wmax = dmax(wmax, batch_face_general<NP, TB, PASS, TYPES>(B, M0, sq, C, f, tid, pone));
   }
   // ---- segmented reduction: this item's faces belong to case c only
   __shared__ double red[TB / 32];

@@ -119,8 +119,8 @@ __device__ __forceinline__ double cdiv(double a, double b, double y) {
   return (q1 == q1) ? q1 : q;
 }
 
-// sqrt(x), correctly rounded (see above)
-__device__ __forceinline__ double dsqrt(double x) {
+// sqrt(x), correctly rounded (see above), for positive finite x; NaN otherwise
+__device__ __forceinline__ double qsqrt(double x) {
   const double y0 = rsqrt_approx(x);
   double g = x * y0, h = 0.5 * y0;
   double r = fma(-g, h, 0.5);
@@ -129,8 +129,12 @@ __device__ __forceinline__ double dsqrt(double x) {
   r = fma(-g, h, 0.5);
   g = fma(g, r, g);
   h = fma(h, r, h);
-  const double d = fma(-g, g, x);
-  const double s = fma(d, h, g);
+  return fma(fma(-g, g, x), h, g);
+}
+
+// sqrt(x), correctly rounded (see above)
+__device__ __forceinline__ double dsqrt(double x) {
+  const double s = qsqrt(x);
   // s is NaN exactly for zero, negative, infinite and NaN operands; of these +-0 and +inf are their own roots
   return (s == s || x < 0.) ? s : x;
 }

@@ -21,7 +21,7 @@ struct CellCounters {
 // (CellInterfaceO2Cartesian.cpp:132-150 left side, :164-181 right side, whose final expressions
 // differ and are kept as they are) alpha_0 and alpha_1 = 1 - alpha_0 of an interface cell are then
 // replaced by the hyperbolic-tangent reconstruction.
-template <int NP, int DIM, bool THINC = true, int LIMC = -1>
+template <int NP, int DIM, bool THINC = true, int LIMC = -1, bool FULFILL = true>
 __device__ ECG_RECON_INLINE void reconstruct_side(const Model<NP>& M, const StepParams& P, const double* sq, int RS,
                                                  int rc, const double* ssl, int SS, int f1, int f2, double alphaCell,
                                                  double alphaOther, double alphaAfter, double dist, double sign,
@@ -81,7 +81,7 @@ __device__ ECG_RECON_INLINE void reconstruct_side(const Model<NP>& M, const Step
     t.a[0] = na;
     t.a[1] = 1. - na;
   }
-  fulfill<NP, true>(M, t);
+  if (FULFILL) fulfill<NP, true>(M, t);
 }
 
 // ---- limited slopes per cell (one limiter in all four slots)
@@ -122,10 +122,11 @@ __device__ __forceinline__ void cell_slopes(const Model<NP>& M, const double* sq
         lim(sq[(FL::U + d) * RS + prev], sq[(FL::U + d) * RS + rc], sq[(FL::U + d) * RS + next]);
 }
 
+// FULFILL: the side's closure too (hllc_quick computes it itself).
 // One side of an internal face from the cell's limited slopes: reconstruct_side's extrapolation and clamps.
 // u: the velocities of the planes pn (normal), p1, p2 (transverse).  pone: no pressure of the block's cells is
 // below a floor (one slope and one extrapolation for all phases).
-template <int NP, int DIM>
+template <int NP, int DIM, bool FULFILL = true>
 __device__ __forceinline__ void extrapolate_side(const Model<NP>& M, const double* sq, int RS, int rc, const double* lsl,
                                                  int LS, int ec, int pn, int p1, int p2, double dist, double sign,
                                                  bool pone, Thermo<NP>& t, double u[3]) {
@@ -154,7 +155,7 @@ __device__ __forceinline__ void extrapolate_side(const Model<NP>& M, const doubl
   u[0] = vel(pn);
   u[1] = DIM > 1 ? vel(p1) : 0.;
   u[2] = DIM > 2 ? vel(p2) : 0.;
-  fulfill<NP, true>(M, t);
+  if (FULFILL) fulfill<NP, true>(M, t);
 }
 
 // The buffer cell of a symmetry side (wall_side) from the cell's limited slopes.
@@ -175,7 +176,7 @@ __device__ __forceinline__ void wall_side_limited(const Model<NP>& M, const doub
   fulfill<NP>(M, t);
 }
 
-template <int NP, int DIM>
+template <int NP, int DIM, bool FULFILL = true>
 __device__ __forceinline__ void cell_thermo(const Model<NP>& M, const double* sq, int RS, int rc, Thermo<NP>& t,
                                             double u[3]) {
   using FL = Fields<NP, DIM>;
@@ -188,7 +189,7 @@ __device__ __forceinline__ void cell_thermo(const Model<NP>& M, const double* sq
   u[0] = u[1] = u[2] = 0.;
 #pragma unroll
   for (int d = 0; d < DIM; d++) u[d] = sq[(FL::U + d) * RS + rc];
-  fulfill<NP>(M, t);
+  if (FULFILL) fulfill<NP>(M, t);
 }
 
 template <int NP, int DIM>

@@ -79,12 +79,164 @@ struct FaceKernelShape {
 constexpr int CELL_THREADS = 128;
 __host__ __device__ constexpr int cell_threads(bool ptmu) { return ptmu ? ECG_CELL_PTMU_THREADS : CELL_THREADS; }
 
+// A face of a block: its position along the axis, line and third coordinate, the staged cell left of it, that
+// cell's limited slopes (or the face slope left of it), and whether no staged pressure is below a floor.
+struct FaceAt {
+  int f, lg, third, rl, el;
+  bool pone;
+};
+
+// CFL length of the cell at position g of the line.
+template <int AX>
+__device__ __forceinline__ double face_lcfl(const Geometry& G, int g, int lg, int third) {
+  return cell_lcfl(G, AX == 0 ? g : lg, AX == 0 ? lg : (AX == 1 ? g : third), AX == 2 ? g : third);
+}
+
+// Face-frame velocity (normal, transverse) of a global one; neg: the frame of a minus side.
+template <int AX>
+__device__ __forceinline__ void face_frame(const double u[3], bool neg, double l[3]) {
+  l[0] = neg ? -u[AX] : u[AX];
+  l[1] = AX == 0 ? u[1] : u[0];
+  l[2] = AX == 2 ? u[1] : u[2];
+}
+
+template <int NP, int DIM, int AX>
+__device__ __forceinline__ void store_face(const StepParams& P, const Geometry& G, double* flux, int f, int lg,
+                                           int third, const double Fn[3], const Flux<NP>& F) {
+  const int64_t nfa = split_nfaces(G.n, AX);
+  const int64_t fid = split_fid(G.n, AX, f, lg, AX == 0 ? lg : third, third);
+  if (!ECG_IN_BOUNDS(P.stats, fid, nfa)) return;
+  constexpr int p1 = AX == 0 ? 1 : 0, p2 = AX == 2 ? 1 : 2;  // planes of the transverse momenta
+  double* out = flux + fid;
+#pragma unroll
+  for (int k = 0; k < NP; k++) {
+    out[(int64_t)k * nfa] = F.a[k];
+    out[(int64_t)(NP + k) * nfa] = F.m[k];
+    out[(int64_t)(2 * NP + k) * nfa] = F.en[k];
+  }
+  out[(int64_t)(3 * NP + AX) * nfa] = Fn[0];
+  out[(int64_t)(3 * NP + p1) * nfa] = Fn[1];
+  if (DIM > 2) out[(int64_t)(3 * NP + p2) * nfa] = Fn[2];
+  out[(int64_t)(3 * NP + DIM) * nfa] = F.E;
+  out[(int64_t)(3 * NP + DIM + 1) * nfa] = F.sM;
+  out[(int64_t)(3 * NP + DIM + 2) * nfa] = F.uStar;
+}
+
+// The two sides of an internal face, from the block's staged planes; FULFILL: their closure too.
+template <int NP, int DIM, int AX, int PASS, int TYPES, bool FULFILL>
+__device__ __forceinline__ void face_sides(const StepParams& P, const Geometry& G, const Model<NP>& M, const double* sq,
+                                           const FaceAt& A, Thermo<NP>& tl, double ul[3], Thermo<NP>& tr,
+                                           double ur[3]) {
+  using KS = FaceKernelShape<NP, DIM, PASS, TYPES>;
+  using FL = Fields<NP, DIM>;
+  constexpr int RS = KS::RS, SS = KS::SS, PS = AX == 0 ? 1 : FaceTile<1>::W;
+  constexpr int p1 = AX == 0 ? 1 : 0, p2 = AX == 2 ? 1 : 2;
+  const double* a0 = KS::NA0 ? sq + (size_t)FL::NQ * RS : sq;  // time-n alpha_0 plane
+  const double* ssl = sq + (size_t)(FL::NQ + KS::NA0) * RS;
+  const int gl = A.f - 1, rl = A.rl, rr = rl + PS, nax = G.n[AX];
+  if (KS::LSL) {
+    extrapolate_side<NP, DIM, FULFILL>(M, sq, RS, rl, ssl, SS, A.el, AX, p1, p2, G.dfl[AX][gl], 1., A.pone, tl, ul);
+    extrapolate_side<NP, DIM, FULFILL>(M, sq, RS, rr, ssl, SS, A.el + PS, AX, p1, p2, G.dfr[AX][gl], -1., A.pone, tr, ur);
+    return;
+  }
+  double ug[3], vg[3];
+  if (!KS::O2) {
+    cell_thermo<NP, DIM, FULFILL>(M, sq, RS, rl, tl, ug);
+    cell_thermo<NP, DIM, FULFILL>(M, sq, RS, rr, tr, vg);
+  } else {
+    const int f1 = A.el + PS;  // this face
+    const bool hasL = (gl - 1 >= 0), hasR = (gl + 2 < nax);
+    // beyond a symmetry side the opposite slope is the side's and alphaCellAfterOppositeSide is the
+    // cell's own time-n alpha (CellO2Cartesian::computeLocalSlopes :68-71); a non-reflecting side
+    // has neither
+    const bool wL = !hasL && G.bc[2 * AX] == ECG_BC_SYMMETRY;
+    const bool wR = !hasR && G.bc[2 * AX + 1] == ECG_BC_SYMMETRY;
+    const int f2l = (hasL || wL) ? A.el : -1;           // face (gl-1, gl)
+    const int f2r = (hasR || wR) ? A.el + 2 * PS : -1;  // face (gl+1, gl+2)
+    const double aL = sq[FL::A * RS + rl], aR = sq[FL::A * RS + rr];
+    const double aLL = hasL ? a0[rl - PS] : (wL ? a0[rl] : 0.);
+    const double aRR = hasR ? a0[rr + PS] : (wR ? a0[rr] : 0.);
+    constexpr bool kThinc = (TYPES == EOS_DYNAMIC);
+    constexpr int kLim = code_limiter(TYPES);
+    reconstruct_side<NP, DIM, kThinc, kLim, FULFILL>(M, P, sq, RS, rl, ssl, SS, f1, f2l, aL, aR, aLL, G.dfl[AX][gl], 1.,
+                                                     tl, ug);
+    reconstruct_side<NP, DIM, kThinc, kLim, FULFILL>(M, P, sq, RS, rr, ssl, SS, f1, f2r, aR, aL, aRR, G.dfr[AX][gl],
+                                                     -1., tr, vg);
+  }
+  face_frame<AX>(ug, false, ul);
+  face_frame<AX>(vg, false, ur);
+}
+
+// Any face of a block, domain sides included, solved by fulfill and hllc and stored; returns its wave value
+// (wave_add).  Out of line: the kernel holds the ordinary face only, and calls this for symmetry sides and
+// for the faces hllc_quick leaves.
+template <int NP, int DIM, int AX, int PASS, int TYPES>
+static __device__ __noinline__ double face_general(const StepParams& P, const Geometry& G, const Model<NP>& M0,
+                                                   double* flux, const double* sq, const FaceAt A) {
+  const Model<NP> M = specialize_eos<NP, TYPES>(M0);
+  using KS = FaceKernelShape<NP, DIM, PASS, TYPES>;
+  using FL = Fields<NP, DIM>;
+  constexpr bool O2 = KS::O2;
+  constexpr int RS = KS::RS, SS = KS::SS, PS = AX == 0 ? 1 : FaceTile<1>::W;
+  const double* a0 = KS::NA0 ? sq + (size_t)FL::NQ * RS : sq;
+  const double* ssl = sq + (size_t)(FL::NQ + KS::NA0) * RS;
+  const int nax = G.n[AX];
+  double wmax = wave_none(G.stretched), Fn[3];
+  Flux<NP> F;
+  if (A.f == 0 || A.f == nax) {
+    // a side: non-reflecting HLLC(cell, cell) in the side's frame (BoundCondNonReflecting::
+    // solveRiemannBoundary src/BoundConds/BoundCondNonReflecting.cpp:62), or a symmetry side's
+    // reflecting flux (ModUEq::solveRiemannWall src/Models/UEq/ModUEq.cpp:452) of the buffer cell,
+    // MUSCL-extrapolated towards the side (BoundCondWallO2Cartesian::solveRiemann :111-141)
+    const int sd = (A.f == 0) ? 0 : 1;
+    const bool neg = sd == 0;
+    const int rc = sd == 0 ? A.rl + PS : A.rl;
+    const double lc = face_lcfl<AX>(G, sd == 0 ? 0 : nax - 1, A.lg, A.third);
+    Thermo<NP> t;
+    double ug[3], ul[3];
+    if (G.bc[2 * AX + sd] == ECG_BC_SYMMETRY) {
+      if (KS::LSL) {
+        wall_side_limited<NP, DIM>(M, sq, RS, rc, ssl, SS, sd == 0 ? A.el + PS : A.el, G.wdist[2 * AX + sd], t, ug);
+      } else if (O2) {
+        wall_side<NP, DIM>(M, P.lim, sq, RS, rc, ssl, SS, A.el + PS, sd == 0 ? A.el + 2 * PS : A.el, a0[rc],
+                           G.wdist[2 * AX + sd], t, ug);
+      } else {
+        cell_thermo<NP, DIM>(M, sq, RS, rc, t, ug);
+      }
+      face_frame<AX>(ug, neg, ul);
+      const double pstar = wall_pstar<NP>(t, ul, G.stretched, lc, wmax);
+#pragma unroll
+      for (int k = 0; k < NP; k++) F.a[k] = F.m[k] = F.en[k] = 0.;
+      F.E = 0.;
+      F.sM = 0.;
+      F.uStar = 0.;
+      Fn[0] = pstar;
+      Fn[1] = 0.;
+      Fn[2] = 0.;
+    } else {
+      cell_thermo<NP, DIM>(M, sq, RS, rc, t, ug);
+      face_frame<AX>(ug, neg, ul);
+      hllc<NP>(M, t, ul, t, ul, G.stretched, lc, lc, wmax, Fn, F);
+    }
+    if (neg) Fn[0] = -Fn[0];
+  } else {
+    Thermo<NP> tl, tr;
+    double ul[3], ur[3];
+    face_sides<NP, DIM, AX, PASS, TYPES, true>(P, G, M, sq, A, tl, ul, tr, ur);
+    hllc<NP, O2>(M, tl, ul, tr, ur, G.stretched, face_lcfl<AX>(G, A.f - 1, A.lg, A.third),
+                 face_lcfl<AX>(G, A.f, A.lg, A.third), wmax, Fn, F);
+  }
+  store_face<NP, DIM, AX>(P, G, flux, A.f, A.lg, A.third, Fn, F);
+  return wmax;
+}
+
 // The faces normal to AX, one block per tile.  The transverse velocities enter without the sign changes of
 // the face frames (src/Meshes/MeshCartesian.cpp:281-557); they only occur squared and as factors of their own
 // momentum flux, whose sign changes back.
 template <int NP, int DIM, int AX, int PASS, int TYPES>
 __global__ void __launch_bounds__(FACE_THREADS, DIM == 2 ? ECG_FACE_MINB_2D : ECG_FACE_MINB_3D)
-    k_kapila_faces(StepParams P, Geometry G, Model<NP> M0, const __grid_constant__ FaceLaunch L) {
+    k_kapila_faces(const __grid_constant__ StepParams P, const __grid_constant__ Geometry G,
+                   const __grid_constant__ Model<NP> M0, const __grid_constant__ FaceLaunch L) {
   const Model<NP> M = specialize_eos<NP, TYPES>(M0);
   using KS = FaceKernelShape<NP, DIM, PASS, TYPES>;
   using FL = Fields<NP, DIM>;
@@ -237,115 +389,38 @@ __global__ void __launch_bounds__(FACE_THREADS, DIM == 2 ? ECG_FACE_MINB_2D : EC
     place(tid, FaceTile<0>::TF, line, fl);
     const int f = f0 + fl;
     const int lg = l0 + line;
-    // CFL length of the line's cell at position g
-    auto lcfl = [&](int g) {
-      return G.stretched ? cell_lcfl(G, isx ? g : lg, isx ? lg : (ax == 1 ? g : third), ax == 2 ? g : third) : G.lcfl;
-    };
     const int rl = line * CL + (fl + 1) * PS, rr = rl + PS;  // the cells on its two sides
     const int el = line * SL + fl * PS;                      // limited slopes of the left one; face slope below
     // (bounds-checked builds: the staged cells this face reads)
     if (f <= nax && lg < G.n[ob] && ECG_IN_BOUNDS(P.stats, rl - PS, RS) && ECG_IN_BOUNDS(P.stats, rr + PS, RS)) {
-      Flux<NP> F;
-      double Fn[3];
-      // planes of the normal and the transverse velocities
-      constexpr int pn = ax, p1 = isx ? 1 : 0, p2 = ax == 2 ? 1 : 2;
-      auto local = [&](const double u[3], bool neg, double l[3]) {
-        l[0] = isx ? u[0] : (ax == 1 ? u[1] : u[2]);
-        l[1] = isx ? u[1] : u[0];
-        l[2] = ax == 2 ? u[1] : u[2];
-        if (neg) l[0] = -l[0];
-      };
-      if (f == 0 || f == nax) {
-        // a side: non-reflecting HLLC(cell, cell) in the side's frame (BoundCondNonReflecting::
-        // solveRiemannBoundary src/BoundConds/BoundCondNonReflecting.cpp:62), or a symmetry side's
-        // reflecting flux (ModUEq::solveRiemannWall src/Models/UEq/ModUEq.cpp:452) of the buffer cell,
-        // MUSCL-extrapolated towards the side (BoundCondWallO2Cartesian::solveRiemann :111-141)
-        const int sd = (f == 0) ? 0 : 1;
-        const bool neg = sd == 0;
-        const int rc = sd == 0 ? rr : rl;
-        const double lc = lcfl(sd == 0 ? 0 : nax - 1);
-        Thermo<NP> t;
-        double ug[3], ul[3];
-        if (G.bc[2 * ax + sd] == ECG_BC_SYMMETRY) {
-          if (LSL) {
-            wall_side_limited<NP, DIM>(M, sq, RS, rc, ssl, SS, sd == 0 ? el + PS : el, G.wdist[2 * ax + sd], t, ug);
-          } else if (O2) {
-            wall_side<NP, DIM>(M, P.lim, sq, RS, rc, ssl, SS, el + PS, sd == 0 ? el + 2 * PS : el, a0[rc],
-                               G.wdist[2 * ax + sd], t, ug);
-          } else {
-            cell_thermo<NP, DIM>(M, sq, RS, rc, t, ug);
-          }
-          local(ug, neg, ul);
-          const double pstar = wall_pstar<NP>(t, ul, G.stretched, lc, wmax);
-#pragma unroll
-          for (int k = 0; k < NP; k++) F.a[k] = F.m[k] = F.en[k] = 0.;
-          F.E = 0.;
-          F.sM = 0.;
-          F.uStar = 0.;
-          Fn[0] = pstar;
-          Fn[1] = 0.;
-          Fn[2] = 0.;
-        } else {
-          cell_thermo<NP, DIM>(M, sq, RS, rc, t, ug);
-          local(ug, neg, ul);
-          hllc<NP>(M, t, ul, t, ul, G.stretched, lc, lc, wmax, Fn, F);
-        }
-        if (neg) Fn[0] = -Fn[0];
-      } else {
-        // internal face between cells gl and gl + 1
-        const int gl = f - 1;
+      FaceAt at{f, lg, third, rl, el, pone};
+      bool solved = false;
+      const bool inner = f > 0 && f < nax;
+      if (inner || G.bc[2 * AX + (f == 0 ? 0 : 1)] == ECG_BC_NONREFLECTING) {
         Thermo<NP> tl, tr;
-        double ul[3], ur[3];
-        if (LSL) {
-          extrapolate_side<NP, DIM>(M, sq, RS, rl, ssl, SS, el, pn, p1, p2, G.dfl[ax][gl], 1., pone, tl, ul);
-          extrapolate_side<NP, DIM>(M, sq, RS, rr, ssl, SS, el + PS, pn, p1, p2, G.dfr[ax][gl], -1., pone, tr, ur);
-        } else {
-          double ug[3], vg[3];
-          if (!O2) {
-            cell_thermo<NP, DIM>(M, sq, RS, rl, tl, ug);
-            cell_thermo<NP, DIM>(M, sq, RS, rr, tr, vg);
-          } else {
-            const int f1 = el + PS;  // this face
-            const bool hasL = (gl - 1 >= 0), hasR = (gl + 2 < nax);
-            // beyond a symmetry side the opposite slope is the side's and alphaCellAfterOppositeSide is the
-            // cell's own time-n alpha (CellO2Cartesian::computeLocalSlopes :68-71); a non-reflecting side
-            // has neither
-            const bool wL = !hasL && G.bc[2 * ax] == ECG_BC_SYMMETRY;
-            const bool wR = !hasR && G.bc[2 * ax + 1] == ECG_BC_SYMMETRY;
-            const int f2l = (hasL || wL) ? el : -1;           // face (gl-1, gl)
-            const int f2r = (hasR || wR) ? el + 2 * PS : -1;  // face (gl+1, gl+2)
-            const double aL = sq[FL::A * RS + rl], aR = sq[FL::A * RS + rr];
-            const double aLL = hasL ? a0[rl - PS] : (wL ? a0[rl] : 0.);
-            const double aRR = hasR ? a0[rr + PS] : (wR ? a0[rr] : 0.);
-            constexpr bool kThinc = (TYPES == EOS_DYNAMIC);
-            constexpr int kLim = code_limiter(TYPES);
-            reconstruct_side<NP, DIM, kThinc, kLim>(M, P, sq, RS, rl, ssl, SS, f1, f2l, aL, aR, aLL, G.dfl[ax][gl], 1.,
-                                                    tl, ug);
-            reconstruct_side<NP, DIM, kThinc, kLim>(M, P, sq, RS, rr, ssl, SS, f1, f2r, aR, aL, aRR, G.dfr[ax][gl],
-                                                    -1., tr, vg);
-          }
-          local(ug, false, ul);
-          local(vg, false, ur);
-        }
-        hllc<NP, O2>(M, tl, ul, tr, ur, G.stretched, lcfl(gl), lcfl(gl + 1), wmax, Fn, F);
-      }
-      const int64_t nfa = split_nfaces(G.n, ax);
-      const int64_t fid = split_fid(G.n, ax, f, lg, isx ? lg : third, third);
-      if (ECG_IN_BOUNDS(P.stats, fid, nfa)) {
-        double* out = L.flux + fid;
+        double ul[3], ur[3], Fn[3];
+        Flux<NP> F;
+        bool ok = true;
+        if (inner) {
+          face_sides<NP, DIM, AX, PASS, TYPES, false>(P, G, M, sq, at, tl, ul, tr, ur);
+        } else {  // a non-reflecting side: HLLC(cell, cell) in the side's frame, with the other faces of the warp
+          double ug[3];
+          cell_thermo<NP, DIM, false>(M, sq, RS, f == 0 ? rr : rl, tl, ug);
+          face_frame<AX>(ug, f == 0, ul);
+          tr = tl;
 #pragma unroll
-        for (int k = 0; k < NP; k++) {
-          out[(int64_t)k * nfa] = F.a[k];
-          out[(int64_t)(NP + k) * nfa] = F.m[k];
-          out[(int64_t)(2 * NP + k) * nfa] = F.en[k];
+          for (int i = 0; i < 3; i++) ur[i] = ul[i];
+#pragma unroll
+          for (int k = 0; k < NP; k++) ok = ok && tl.r[k] >= 1.e-15;
         }
-        out[(int64_t)(3 * NP + pn) * nfa] = Fn[0];
-        out[(int64_t)(3 * NP + p1) * nfa] = Fn[1];
-        if (DIM > 2) out[(int64_t)(3 * NP + p2) * nfa] = Fn[2];
-        out[(int64_t)(3 * NP + DIM) * nfa] = F.E;
-        out[(int64_t)(3 * NP + DIM + 1) * nfa] = F.sM;
-        out[(int64_t)(3 * NP + DIM + 2) * nfa] = F.uStar;
+        const double lL = G.stretched ? face_lcfl<AX>(G, f > 0 ? f - 1 : 0, lg, third) : G.lcfl;
+        const double lR = G.stretched ? face_lcfl<AX>(G, f < nax ? f : nax - 1, lg, third) : G.lcfl;
+        solved = hllc_quick<NP, !O2>(M, tl, ul, tr, ur, G.stretched, lL, lR, wmax, Fn, F, ok);
+        if (f == 0) Fn[0] = -Fn[0];
+        if (solved) store_face<NP, DIM, AX>(P, G, L.flux, f, lg, third, Fn, F);
       }
+      // a symmetry side, or operands out of hllc_quick's range
+      if (!solved) wmax = dmax(wmax, face_general<NP, DIM, AX, PASS, TYPES>(P, G, M0, L.flux, sq, at));
     }
   }
 
