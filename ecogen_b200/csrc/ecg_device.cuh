@@ -343,7 +343,8 @@ __device__ ECG_HLLC_INLINE void hllc(const Model<NP>& M, const Thermo<NP>& L, co
 // face by fulfill and hllc.  Measured with the same bits (one B200, mid-run states): face kernels 2D 2048^2
 // 0.311 / 0.291 -> 0.303 / 0.286 ms, 3D 256^3 1.91 / 1.64 / 1.64 -> 1.79 / 1.61 / 1.62 ms (X faces with the
 // domain sides solved beside the others), THINC 1000 x 601 0.099 / 0.094 -> 0.073 / 0.066 ms (the general face
-// and its sides out of line); 4096 tubes 3.28 -> 3.05 ms per step.  LOW: the densities may lie below the floors (sides not clamped by phase_fix_ar).
+// and its sides out of line); 4096 tubes 3.28 -> 3.05 ms per step.  LOW: the densities and pressures may lie below the
+// floors (sides not clamped by phase_fix_ar and eos_fix_p).
 template <int NP>
 __device__ __forceinline__ void fulfill_quick(const Model<NP>& M, Thermo<NP>& t) {
   double c[NP];
@@ -377,7 +378,8 @@ __device__ __forceinline__ bool hllc_quick(const Model<NP>& M, Thermo<NP>& L, co
 #pragma unroll
   for (int k = 0; k < NP; k++) {
     ok = ok && M.eos[k].type != ECG_EOS_NASG;
-    if (LOW) ok = ok && L.r[k] >= 1.e-15 && R.r[k] >= 1.e-15;
+    if (LOW)
+      ok = ok && L.r[k] >= 1.e-15 && R.r[k] >= 1.e-15 && L.p[k] >= M.eos[k].pfloor && R.p[k] >= M.eos[k].pfloor;
   }
   fulfill_quick<NP>(M, L);
   fulfill_quick<NP>(M, R);
@@ -441,7 +443,7 @@ __device__ __forceinline__ bool hllc_quick(const Model<NP>& M, Thermo<NP>& L, co
     F.E = (rhoStar * EStar + pStar) * sM;
     F.uStar = sM;
   }
-  double t = F.E + (cL + cR);
+  double t = F.E + (cL + cR) + F.sM;
 #pragma unroll
   for (int k = 0; k < NP; k++) t += F.en[k];
   if (!(ok && t == t)) return false;
@@ -540,7 +542,7 @@ __device__ __forceinline__ void pinf_eval_general(const Model<NP>& M, const doub
 // -> 0.36 / 0.37 ms, of 256^3 (three phases, at most 6 evaluations) 2.36 / 2.38 -> 2.24 / 2.27 ms.  With the
 // general form as a branch inside the loop the three-phase cell kernel spilled 192 bytes and took 2.46 ms.
 // Returns false where the general form has to run: for NASG phases, and where a divisor lies near its floor or
-// an operand is zero, infinite or NaN (f or df is NaN then).
+// an operand is zero, infinite or NaN (f or df is NaN then), or where the terms of df cancel.
 template <int NP>
 __device__ __forceinline__ bool pinf_quick(const Model<NP>& M, const double a[NP], const double r[NP], NewtonState& s,
                                           const double p[NP], double aS[NP], double rS[NP]) {
@@ -575,7 +577,9 @@ __device__ __forceinline__ bool pinf_quick(const Model<NP>& M, const double a[NP
   s.f = f;
   s.df = df;
   s.ydf = nrcp(dfa);
-  return plain && f == f && df == df;
+  // df sums terms of one sign (densities, volume fractions and p + pInf are positive), so 1/dfa is 1/df to a few
+  // ulps; checked all the same
+  return plain && f == f && fabs(fma(df, s.ydf, -1.)) < 1.e-12;
 }
 
 // One evaluation in either form (the seeded kernels').
