@@ -17,7 +17,8 @@
 // interface detector decides nothing, and each limiter is symmetric in its slopes) and it has neither THINC
 // nor passive transports; otherwise the fused kernels run.  Why it is faster: the fused pass computed the
 // faces and slopes of a tile's border twice, limited every slope twice and met a barrier per phase and axis.
-// Measured on one B200 (mid-run states, per step): PTUEq 2048^2 1.93 -> 1.23 ms, Euler 2048^2 1.11 -> 0.80 ms;
+// Measured on one B200 (mid-run states, per step): PTUEq 2048^2 1.93 -> 1.23 ms, Euler 2048^2 1.11 -> 0.80 ms (1.19 and 0.72 ms with the
+// register budgets below);
 // the same bits in every field.
 #pragma once
 #include "ecg_faces.cuh"
@@ -39,7 +40,7 @@ struct FlowShape {
 // The faces normal to AX, one block per tile.  LIMC >= 0: the limiter, compiled in; -1: P.lim[0], read at run
 // time.
 template <class MD, int DIM, int AX, int PASS, int LIMC>
-__global__ void __launch_bounds__(FACE_THREADS, MD::FACE_MINB)
+__global__ void __launch_bounds__(FACE_THREADS, DIM == 2 ? MD::FACE_MINB : 8)
     k_flow_faces(StepParams P, Geometry G, typename MD::Eos M, const __grid_constant__ FaceLaunch L) {
   using KS = FlowShape<MD, DIM, PASS>;
   constexpr bool O2 = KS::O2, isx = AX == 0;
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(FACE_THREADS, MD::FACE_MINB)
 // One thread per cell: its faces' fluxes in the reference's order (axis by axis the left face added, the right
 // one subtracted; then the domain sides), then the model's update.
 template <class MD, int DIM, int PASS>
-__global__ void __launch_bounds__(128, MD::CELL_MINB)
+__global__ void __launch_bounds__(128, DIM == 2 ? MD::CELL_MINB : 8)
     k_flow_cells(StepParams P, Geometry G, typename MD::Eos M, FaceArrays FA) {
   constexpr int NFL = MD::NM + DIM + 1;
   if (*P.done) return;

@@ -43,14 +43,14 @@ struct FaceKernelShape {
   }
 };
 
-// Resident blocks per SM asked of the face and cell kernels (registers 65536 / (128 x MINB)).  Measured
-// on one B200 with the branch-free division (per-kernel CUDA events, 100 steps): 3D three-phase cavity
-// 256^3: face kernels at 6 blocks (80 registers) 2.35 / 2.11 ms (X / Y faces), at 5 2.43 / 2.13 ms;
-// cell kernel at 6 blocks 2.96 ms, at 5 (96 registers, fewer spills) 2.90 ms; 2D shock-bubble 2048^2:
-// face kernels at 8 blocks 0.353 / 0.328 ms, at 7 0.354 / 0.322 ms; cell kernel at 6 0.393 ms, at 5
-// 0.390 ms.
+// Resident blocks per SM asked of the face and cell kernels (registers 65536 / (128 x MINB)).  Measured on one
+// B200 (per-kernel CUDA events, mid-run states; X / Y faces, cells of the predictor): 2D two-phase 2048^2 face
+// kernels at 7 blocks 304 / 287 us, at 8 (64 registers) 288 / 270, at 9 302 / 281; cell kernel at 5 blocks 360 us,
+// at 6 (80 registers) 346, but 26 us against 23 on 191 x 103 cells, where the spills of the Newton loop are not
+// hidden; at 4 384 us.  3D three-phase 256^3 face kernels at 5 blocks 1.83 / 1.65 ms, at 6 (80 registers) 1.82 /
+// 1.64, at 7 1.94 / 1.70; cell kernel at 5 2.26 ms, at 6 3.50, at 4 2.45.
 #ifndef ECG_FACE_MINB_2D
-#define ECG_FACE_MINB_2D 7
+#define ECG_FACE_MINB_2D 8
 #endif
 #ifndef ECG_FACE_MINB_3D
 #define ECG_FACE_MINB_3D 6

@@ -53,11 +53,13 @@ __device__ __forceinline__ void euler_complete(const EosParams& q, double eps, E
   s.E = e + 0.5 * (s.u[0] * s.u[0] + s.u[1] * s.u[1] + s.u[2] * s.u[2]);
 }
 
+// Resident blocks per SM of the split form's 2D kernels (3D: 8).  Measured on the 2048^2 blast (us per step; face,
+// cell blocks): 8, 8 801; 9, 10 766; 10, 12 744; 12, 8 732; 12, 10 (40 and 48 registers) 720; 14, 12 721.
 #ifndef ECG_EULER_FACE_MINB
-#define ECG_EULER_FACE_MINB 8
+#define ECG_EULER_FACE_MINB 12
 #endif
 #ifndef ECG_EULER_CELL_MINB
-#define ECG_EULER_CELL_MINB 8
+#define ECG_EULER_CELL_MINB 10
 #endif
 
 // ModEuler::solveRiemannIntern src/Models/Euler/ModEuler.cpp:105-225 (strict sL > 0 / sR < 0).

@@ -146,11 +146,13 @@ __device__ __forceinline__ void hllc_pt(const PtSide& L, const double ul[3], con
   }
 }
 
+// Resident blocks per SM of the split form's 2D kernels (3D: 8).  Measured on the 2048^2 bubble (us per step; face,
+// cell blocks): 8, 8 1229; 9, 9 1197; 9, 10 1190; 10, 10 (48 registers) 1186; 10, 8 1205; 8, 12 1218.
 #ifndef ECG_PTUEQ_FACE_MINB
-#define ECG_PTUEQ_FACE_MINB 8
+#define ECG_PTUEQ_FACE_MINB 10
 #endif
 #ifndef ECG_PTUEQ_CELL_MINB
-#define ECG_PTUEQ_CELL_MINB 8
+#define ECG_PTUEQ_CELL_MINB 10
 #endif
 
 // Update of a cell from its accumulated fluxes.
