@@ -33,16 +33,11 @@ cudaError_t euler_launch(int dim, int pass, const StepParams& P, const Geometry&
 cudaError_t ptueq_launch(int dim, int pass, const StepParams& P, const Geometry& G, const ecg_eos* eos, cudaStream_t s,
                          bool prepare);
 
-__global__ void k_finalize(DevScalars* s) {
-  // Run::solver src/Run.cpp:417-440: t += dt, iteration++, stop test, dt = cfl * dtMax
-  if (s->done) return;
-  double dtmax = __longlong_as_double((long long)s->dtmax_bits);
-  s->t += s->dt;
-  s->it += 1;
-  if (s->mode == 1 && s->it >= s->max_it) s->done = 1;
-  if (s->mode == 2 && s->t >= s->t_end) s->done = 1;
-  s->dt = s->cfl * dtmax;
-  s->dtmax_bits = (unsigned long long)__double_as_longlong(1.e10);
+__global__ void k_finalize(const DevScalars* from, DevScalars* to) { step_finalize(from, to); }
+
+cudaError_t launch_step_end(const DevScalars* from, DevScalars* to, cudaStream_t s) {
+  k_finalize<<<1, 1, 0, s>>>(from, to);
+  return cudaGetLastError();
 }
 
 // Mixture pressure sum_k alpha_k p_k of the stored state (what the reference writes as
@@ -120,7 +115,9 @@ struct ecg_ctx {
   FaceStreams fstreams{};     // auxiliary streams of the face kernels (split forms)
   FaceMaps fmaps{};           // tensor maps of the face kernels' TMA staging (fmaps.ok = 0: none)
   int staging = ECG_STAGING_TMA;
-  DevScalars* scal = nullptr;
+  DevScalars* scal = nullptr;      // two, by state parity (DevScalars)
+  unsigned int* fin_count = nullptr;  // blocks done of the fused pass that ends a step
+  StepEnd step_end[2]{};           // the end of the steps from state[0] / state[1] (split forms)
   DevStats* stats = nullptr;
   // pinned host staging of the scalars and counters an ecg_step call exchanges (asynchronous copies,
   // one synchronisation per call)
@@ -254,10 +251,11 @@ void distance_tables(const ecg_case& c, const std::vector<double>* sz, const std
 
 ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
   StepParams P{};
-  P.done = &x->scal->done;
+  DevScalars* sc = x->scal + parity;
+  P.done = &sc->done;
   P.n = x->n;
-  P.dt = &x->scal->dt;
-  P.dtmax_bits = &x->scal->dtmax_bits;
+  P.dt = &sc->dt;
+  P.dtmax_bits = &sc->dtmax_bits;
   P.stats = x->stats;
   for (int i = 0; i < 4; i++) P.lim[i] = x->c.limiter[i];
   P.newton_cap = x->newton_cap;
@@ -291,12 +289,26 @@ ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
     return kapila_launch(x->np, x->dim, x->c.ptmu != 0, pass, P, x->geo, x->c.eos, x->eps, x->stream, false);
   };
   cudaError_t e;
+  P.chained = ev ? 0 : 1;
+  const bool beside = !ev && (x->split || x->flow);
+  // what the last pass of the step does beside its own work (profiled steps end in a launch of their own)
+  auto last = [&] {
+    if (ev) return;
+    if (beside) {
+      P.end = &x->step_end[parity];
+    } else {
+      P.fin_from = sc;
+      P.fin_to = x->scal + (1 - parity);
+      P.fin_count = x->fin_count;
+    }
+  };
   if (ev) cudaEventRecord(ev[0], x->stream);
   if (x->c.order == 1) {
     P.q = sn;
     P.sn = sn;
     P.out = s1;
     P.split_ev = (ev && x->split) ? ev + 4 : nullptr;
+    last();
     e = run(PASS_O1);
     if (e != cudaSuccess) return cuda_fail(e, "step kernel");
     if (ev) cudaEventRecord(ev[1], x->stream);
@@ -311,14 +323,16 @@ ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
     P.q = x->half;
     P.out = s1;
     P.split_ev = (ev && x->split) ? ev + 7 : nullptr;
+    last();
     e = run(PASS_CORR);
     if (e != cudaSuccess) return cuda_fail(e, "corrector kernel");
   }
   if (ev) cudaEventRecord(ev[2], x->stream);
-  k_finalize<<<1, 1, 0, x->stream>>>(x->scal);
-  if (ev) cudaEventRecord(ev[3], x->stream);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "finalize kernel");
+  if (ev) {
+    e = launch_step_end(sc, x->scal + (1 - parity), x->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "finalize kernel");
+    cudaEventRecord(ev[3], x->stream);
+  }
   return ECG_OK;
 }
 
@@ -573,7 +587,8 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
       e = cudaStreamCreateWithFlags(&x->fstreams.s[a], cudaStreamNonBlocking);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->fstreams.join[a], cudaEventDisableTiming);
     }
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->fstreams.fork, cudaEventDisableTiming);
+    for (cudaEvent_t* ev : {&x->fstreams.fork, &x->fstreams.end_fork, &x->fstreams.end_join})
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
     if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaStreamCreate(face streams)"));
 #ifndef ECG_BOUNDS_CHECK
     // TMA staging of the face kernels' tiles where the layout allows it (the bounds-checked build
@@ -622,10 +637,12 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
     pc /= (L.gamma - 1.) * L.cv - (V.gamma - 1.) * V.cv;
     x->pcrit = pc;
   }
-  e = cudaMalloc(&x->scal, sizeof(DevScalars));
+  e = cudaMalloc(&x->scal, 2 * sizeof(DevScalars));
   if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaMalloc(scalars)"));
   e = cudaMalloc(&x->stats, sizeof(DevStats));
-  if (e == cudaSuccess) e = cudaMallocHost(&x->h_scal, sizeof(DevScalars));
+  if (e == cudaSuccess) e = cudaMalloc(&x->fin_count, sizeof(unsigned int));
+  if (e == cudaSuccess) e = cudaMemset(x->fin_count, 0, sizeof(unsigned int));
+  if (e == cudaSuccess) e = cudaMallocHost(&x->h_scal, 2 * sizeof(DevScalars));
   if (e == cudaSuccess) e = cudaMallocHost(&x->h_stats, sizeof(DevStats));
   if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaMalloc(stats)"));
   DevScalars s0{};
@@ -634,7 +651,10 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
   s0.dtmax_bits = (unsigned long long)0;
   double big = 1.e10;
   std::memcpy(&s0.dtmax_bits, &big, sizeof(double));
-  cudaMemcpy(x->scal, &s0, sizeof(s0), cudaMemcpyHostToDevice);
+  for (int i = 0; i < 2; i++) cudaMemcpy(x->scal + i, &s0, sizeof(s0), cudaMemcpyHostToDevice);
+  if (x->fstreams.fork)
+    for (int i = 0; i < 2; i++)
+      x->step_end[i] = {x->scal + i, x->scal + (1 - i), x->fstreams.s[0], x->fstreams.end_fork, x->fstreams.end_join};
   cudaMemset(x->stats, 0, sizeof(DevStats));
   // kernel attributes (dynamic shared memory) for every pass of this case shape
   for (int pass = 0; pass < 3; pass++) {
@@ -667,6 +687,7 @@ extern "C" void ecg_destroy(ecg_ctx* x) {
   cudaFree(x->tmp);
   for (int a = 0; a < 3; a++) cudaFree(x->flux[a]);
   cudaFree(x->scal);
+  cudaFree(x->fin_count);
   cudaFree(x->stats);
   cudaFreeHost(x->h_scal);
   cudaFreeHost(x->h_stats);
@@ -679,7 +700,8 @@ extern "C" void ecg_destroy(ecg_ctx* x) {
     if (x->fstreams.s[a]) cudaStreamDestroy(x->fstreams.s[a]);
     if (x->fstreams.join[a]) cudaEventDestroy(x->fstreams.join[a]);
   }
-  if (x->fstreams.fork) cudaEventDestroy(x->fstreams.fork);
+  for (cudaEvent_t ev : {x->fstreams.fork, x->fstreams.end_fork, x->fstreams.end_join})
+    if (ev) cudaEventDestroy(ev);
   if (x->stream) cudaStreamDestroy(x->stream);
   delete x;
 }
@@ -897,8 +919,9 @@ static ecg_status step_common(ecg_ctx* x, int mode, int32_t nsteps, double* dt, 
   h.max_it = x->c.max_iterations;
   h.mode = mode;
   h.done = (mode == 1 && h.it >= h.max_it) || (mode == 2 && h.t >= h.t_end);
-  *x->h_scal = h;  // the previous call synchronised, so the staging buffer is free
-  ECG_CUDA(cudaMemcpyAsync(x->scal, x->h_scal, sizeof(h), cudaMemcpyHostToDevice, x->stream));
+  // the previous call synchronised, so the staging buffer is free; both parities' scalars start from the caller's
+  x->h_scal[0] = x->h_scal[1] = h;
+  ECG_CUDA(cudaMemcpyAsync(x->scal, x->h_scal, 2 * sizeof(h), cudaMemcpyHostToDevice, x->stream));
   ECG_CUDA(cudaMemsetAsync(x->stats, 0, sizeof(DevStats), x->stream));
   const int cur0 = x->cur;  // a step that finds the stop flag set writes nothing, so the state that
                             // holds the result is decided by the number of steps actually taken
@@ -952,12 +975,13 @@ static ecg_status step_common(ecg_ctx* x, int mode, int32_t nsteps, double* dt, 
       ecg_status s = advance(x, chunk);
       if (s != ECG_OK) return s;
       DevScalars r{};
-      ECG_CUDA(cudaMemcpyAsync(&r, x->scal, sizeof(r), cudaMemcpyDeviceToHost, x->stream));
+      ECG_CUDA(cudaMemcpyAsync(&r, x->scal + x->cur, sizeof(r), cudaMemcpyDeviceToHost, x->stream));
       ECG_CUDA(cudaStreamSynchronize(x->stream));
       if (r.done) break;
     }
   }
-  ECG_CUDA(cudaMemcpyAsync(x->h_scal, x->scal, sizeof(DevScalars), cudaMemcpyDeviceToHost, x->stream));
+  // x->cur: the parity after the launched steps, whose scalars the last one wrote
+  ECG_CUDA(cudaMemcpyAsync(x->h_scal, x->scal + x->cur, sizeof(DevScalars), cudaMemcpyDeviceToHost, x->stream));
   ECG_CUDA(cudaMemcpyAsync(x->h_stats, x->stats, sizeof(DevStats), cudaMemcpyDeviceToHost, x->stream));
   ECG_CUDA(cudaStreamSynchronize(x->stream));
   const DevScalars r = *x->h_scal;

@@ -102,4 +102,19 @@ inline cudaError_t face_axes(const StepParams& P, cudaStream_t s, bool prepare, 
   return e;
 }
 
+// The end of the step beside its last cell kernel: the wave speeds are complete once the face kernels are, and
+// the cell kernel reads the scalars of its own parity.
+cudaError_t launch_step_end(const DevScalars* from, DevScalars* to, cudaStream_t s);
+inline cudaError_t end_begin(const StepParams& P, cudaStream_t s) {
+  if (!P.end) return cudaSuccess;
+  cudaError_t e = cudaEventRecord(P.end->fork, s);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(P.end->s, P.end->fork, 0);
+  if (e == cudaSuccess) e = launch_step_end(P.end->from, P.end->to, P.end->s);
+  if (e == cudaSuccess) e = cudaEventRecord(P.end->join, P.end->s);
+  return e;
+}
+inline cudaError_t end_join(const StepParams& P, cudaStream_t s) {
+  return P.end ? cudaStreamWaitEvent(s, P.end->join, 0) : cudaSuccess;
+}
+
 }  // namespace ecg

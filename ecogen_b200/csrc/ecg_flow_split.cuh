@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(FACE_THREADS, DIM == 2 ? MD::FACE_MINB : 8)
   extern __shared__ unsigned char smem_raw[];
   double* sq = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);  // [NQ][RS]
   double* ssl = sq + (size_t)NQ * RS;                                                                      // [NSL][SS]
-  if (*P.done) return;
+  const int done = *P.done;
   const int tid = threadIdx.x;
   const FacePlace B = face_place<AX>();
   const int f0 = B.f0, l0 = B.l0, third = B.third;
@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(FACE_THREADS, DIM == 2 ? MD::FACE_MINB : 8)
       }
     }
   }
+  if (done) return;  // tested here: the staging does not wait for it
   __syncthreads();
   // ---- limited slopes: cell f0 - 1 + s of every line, s in [0, TF]
   if (O2) {
@@ -205,7 +206,7 @@ template <class MD, int DIM, int PASS>
 __global__ void __launch_bounds__(128, DIM == 2 ? MD::CELL_MINB : 8)
     k_flow_cells(StepParams P, Geometry G, typename MD::Eos M, FaceArrays FA) {
   constexpr int NFL = MD::NM + DIM + 1;
-  if (*P.done) return;
+  const int done = *P.done;
   const int64_t nn = P.n;
   const int64_t cell = (int64_t)blockIdx.x * 128 + threadIdx.x;
   if (cell >= nn) return;
@@ -244,6 +245,7 @@ __global__ void __launch_bounds__(128, DIM == 2 ? MD::CELL_MINB : 8)
 #pragma unroll
     for (int i = 0; i < NFL; i++) acc[i] -= cA * FA.flux[ax][(int64_t)i * nfa + fid];
   }
+  if (done) return;
   MD::template update<DIM, PASS>(P, M, nn, cell, acc);
 }
 
@@ -266,8 +268,11 @@ cudaError_t launch_flow(const StepParams& P, const Geometry& G, const typename M
   if (e != cudaSuccess || prepare) return e;
   FaceArrays FA{};
   for (int ax = 0; ax < DIM; ax++) FA.flux[ax] = P.flux[ax];
+  const cudaError_t ee = end_begin(P, s);
+  if (ee != cudaSuccess) return ee;
   k_flow_cells<MD, DIM, PASS><<<(unsigned)((P.n + 127) / 128), 128, 0, s>>>(P, G, M, FA);
-  return cudaGetLastError();
+  const cudaError_t ec = cudaGetLastError();
+  return ec == cudaSuccess ? end_join(P, s) : ec;
 }
 
 // One pass of a model in split form (the caller has checked P.flux).

@@ -66,7 +66,11 @@ __global__ void __launch_bounds__(KapilaStep<NP, DIM, PASS, NTM>::NTH,
   double* sfl = ssl + (K::O2 ? (size_t)(FL::NSL + NTM) * SS : 0);  // [NFL + NTM][FS]
   constexpr int NTA = NTM > 0 ? NTM : 1;
 
-  if (*P.done) return;  // stop condition reached earlier in a captured step sequence
+  if (DIM == 1) {
+    chain_wait();
+    chain_next();
+  }
+  const int done = *P.done;  // stop condition reached earlier in a captured step sequence
   const int tid = threadIdx.x;
   const int org[3] = {(int)blockIdx.x * TS::X, (int)blockIdx.y * TS::Y, (int)blockIdx.z * TS::Z};
   const int lc[3] = {tid % TS::X, (tid / TS::X) % TS::Y, tid / (TS::X * TS::Y)};
@@ -133,6 +137,10 @@ __global__ void __launch_bounds__(KapilaStep<NP, DIM, PASS, NTM>::NTH,
         for (int j = 0; j < NTM; j++)
           if (j < P.ntr) str[j * RS + e] = P.q[(int64_t)(FL::NS + j) * nn + c];
       }
+    }
+    if (ax == 0 && done) {  // tested here: the first loads do not wait for it
+      step_skipped(P);
+      return;
     }
     __syncthreads();
     // ---- face slopes (MUSCL): face j between local cells j-1 and j, j in [-1, T+1]
@@ -351,25 +359,22 @@ __global__ void __launch_bounds__(KapilaStep<NP, DIM, PASS, NTM>::NTH,
   if (SEED && !PTMU) seed_gate<NP, DIM>(P, M, active, cp, sg);
   if (SEED && PTMU) ptmu_seed_gate<NP, DIM>(P, M, active, cp, sg, cc);
   if (active) kapila_finish<NP, DIM, PASS, PTMU, SEED, (TYPES == EOS_DYNAMIC)>(P, M, nn, cell, cp, sg, cc);
-  block_counters(P.stats, cc.relax, cc.iters, cc.fallback, cc.seeded, cc.rejected, cc.nonfinite, cc.ptmu, cc.iters, true);
-  if (PTMU)
-    block_ptmu_counters(P.stats, cc.pc.solve, cc.pc.outer, cc.pc.tsat_calls, cc.pc.tsat_iters, cc.pc.tsat_max,
-                        cc.pc.seeded, cc.pc.rejected);
-
-  // ---- dtMax: block min, one atomic per block
-  __shared__ double red[32];
+  // ---- dtMax: block reduction of the wave speeds (over the counters' barrier), one atomic per block
+  __shared__ double red[K::NTH / 32];
   double v = wmax;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   if ((tid & 31) == 0) red[tid >> 5] = v;
-  __syncthreads();
-  if (tid < 32) {
-    v = (tid < K::NTH / 32) ? red[tid] : wave_none(G.stretched);
+  block_counters(P.stats, cc.relax, cc.iters, cc.fallback, cc.seeded, cc.rejected, cc.nonfinite, cc.ptmu, cc.iters, true);
+  if (PTMU)
+    block_ptmu_counters(P.stats, cc.pc.solve, cc.pc.outer, cc.pc.tsat_calls, cc.pc.tsat_iters, cc.pc.tsat_max,
+                        cc.pc.seeded, cc.pc.rejected);
+  if (tid == 0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (tid == 0) atomic_min_pos_double(P.dtmax_bits, wave_dtmax(v, G.stretched, G.lcfl));
+    for (int w = 1; w < K::NTH / 32; w++) v = dmax(v, red[w]);
+    atomic_min_pos_double(P.dtmax_bits, wave_dtmax(v, G.stretched, G.lcfl));
+    step_end(P);
   }
 }
 
 }  // namespace ecg
-

@@ -21,8 +21,7 @@ cudaError_t launch_one(const StepParams& P, const Geometry& G, const ecg_eos* eo
   for (int k = 0; k < NP; k++) M.eos[k] = make_eos_params(eos[k]);
   M.eps = eps;
   dim3 grid((G.n[0] + TS::X - 1) / TS::X, (G.n[1] + TS::Y - 1) / TS::Y, (G.n[2] + TS::Z - 1) / TS::Z);
-  kern<<<grid, K::NTH, sm, s>>>(P, G, M);
-  return cudaGetLastError();
+  return launch_chained(kern, grid, dim3(K::NTH), sm, s, DIM == 1 && P.chained, P, G, M);
 }
 
 // One pass of one kernel variant: the split form (face kernels + cell kernel) for 2D and 3D cases whose

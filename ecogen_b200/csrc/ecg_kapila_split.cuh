@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(FACE_THREADS, DIM == 2 ? ECG_FACE_MINB_2D : EC
   double* sa0 = sq + (size_t)FL::NQ * RS;           // [NA0][RS]
   double* ssl = sa0 + (size_t)KS::NA0 * RS;         // [NSL][SS]
   const double* a0 = KS::NA0 ? sa0 : sq;            // time-n alpha_0 plane
-  if (*P.done) return;
+  const int done = *P.done;
   const int tid = threadIdx.x;
   constexpr bool isx = ax == 0;
   const FacePlace B = face_place<AX>();
@@ -310,6 +310,7 @@ __global__ void __launch_bounds__(FACE_THREADS, DIM == 2 ? ECG_FACE_MINB_2D : EC
       }
     }
   }
+  if (done) return;  // tested here: the staging does not wait for it
   __syncthreads();
   const double* dcc = G.dcc[ax];
   // ---- limited slopes (MUSCL, one limiter): cell f0 - 1 + s of every line, s in [0, TF]
@@ -481,7 +482,7 @@ __global__ void __launch_bounds__(cell_threads(PTMU),
                    const double* __restrict__ fy, const double* __restrict__ fz) {
   const Model<NP> M = specialize_eos<NP, TYPES>(M0);
   using FL = Fields<NP, DIM>;
-  if (*P.done) return;
+  const int done = *P.done;
   const int64_t nn = P.n;
   const int64_t cell = (int64_t)blockIdx.x * cell_threads(PTMU) + threadIdx.x;
   const bool active = cell < nn;
@@ -502,8 +503,8 @@ __global__ void __launch_bounds__(cell_threads(PTMU),
   for (int d = 0; d < DIM; d++) amom[d] = 0.;
   CellCounters cc;
   CellPrim<NP, DIM> cp;
+  const double* fa[3] = {fx, fy, fz};
   if (active) {
-    const double* fa[3] = {fx, fy, fz};
     prefetch_face_fluxes<NP, DIM>(G, fa, g);
     const double p0 = P.sn[(int64_t)FL::P * nn + cell];
 #pragma unroll
@@ -512,6 +513,9 @@ __global__ void __launch_bounds__(cell_threads(PTMU),
       rn[k] = P.sn[(int64_t)(FL::R + k) * nn + cell];
       pn[k] = eos_fix_p(M.eos[k], p0);
     }
+  }
+  if (done) return;  // tested here: the first loads do not wait for it
+  if (active) {
     // internal faces, axis by axis: the left face added, the right face subtracted
 #pragma unroll
     for (int ax = 0; ax < DIM; ax++) {
@@ -574,11 +578,14 @@ cudaError_t launch_split(const StepParams& P, const Geometry& G, const ecg_eos* 
     return launch_faces<NP, DIM, decltype(ax)::value, PASS, TYPES>(P, G, M, sa, prepare);
   });
   if (e != cudaSuccess || prepare) return e;
+  const cudaError_t ee = end_begin(P, s);
+  if (ee != cudaSuccess) return ee;
   constexpr int CT = cell_threads(PTMU);
   const unsigned blocks = (unsigned)((P.n + CT - 1) / CT);
   k_kapila_cells<NP, DIM, PASS, PTMU, SEED, TYPES><<<blocks, CT, 0, s>>>(P, G, M, P.flux[0], P.flux[1],
                                                                                  DIM > 2 ? P.flux[2] : nullptr);
-  return cudaGetLastError();
+  const cudaError_t ec = cudaGetLastError();
+  return ec == cudaSuccess ? end_join(P, s) : ec;
 }
 
 }  // namespace ecg

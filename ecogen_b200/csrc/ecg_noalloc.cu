@@ -22,7 +22,7 @@ cudaError_t kapila_launch(int np, int dim, bool ptmu, int pass, const StepParams
                           const ecg_eos* eos, double eps, cudaStream_t s, bool prepare);
 cudaError_t euler_launch(int dim, int pass, const StepParams& P, const Geometry& G, const ecg_eos* eos, double eps,
                          cudaStream_t s, bool prepare);
-__global__ void k_finalize(DevScalars* s);
+__global__ void k_finalize(const DevScalars* from, DevScalars* to);
 
 namespace {
 
@@ -238,7 +238,7 @@ extern "C" ecg_status ecg_step_noalloc(const ecg_case* c, const double* state_in
     }
   }
   if (e == cudaSuccess) {
-    k_finalize<<<1, 1, 0, s>>>(&S->scal);
+    k_finalize<<<1, 1, 0, s>>>(&S->scal, &S->scal);
     e = cudaGetLastError();
   }
   DevScalars r{};

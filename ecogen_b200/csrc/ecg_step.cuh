@@ -36,9 +36,12 @@ enum { PASS_O1 = 0, PASS_PRED = 1, PASS_CORR = 2 };
 // 8x14 / 128 / 7 (72) 949 M; 8x14 / 128 / 8 (64) 883 M; 16x7 / 128 / 7 868 M; 8x7 / 64 / 14 719 M.
 // 1D single cases (the 1000-cell tube of the reference's CPU-sized configuration) run a few blocks
 // and are latency-bound: fewer spills matter more than resident warps.  Measured on that tube
-// (cell-updates/s): 3 blocks per SM (80 registers) 48.6 M, 2 (128 registers) 51.8 M, 1 52.8 M.
+// (cell-updates/s, blocks of 256 threads): 3 blocks per SM (80 registers) 48.6 M, 2 (128 registers) 51.8 M,
+// 1 52.8 M.  Blocks of 128 threads keep that budget with one warp per scheduler.
+// Measured with the chained launches, the step ended by the last block and one barrier for the counters (mid-run
+// tube of 1000 cells, us per step): 22.9 -> 18.9; 4093 cells in MUSCL 44.5 -> 42.8.
 #ifndef ECG_TILE1D_MINB
-#define ECG_TILE1D_MINB 2
+#define ECG_TILE1D_MINB 4
 #endif
 #ifndef ECG_TILE2D_X
 #define ECG_TILE2D_X 8
@@ -67,7 +70,7 @@ enum { PASS_O1 = 0, PASS_PRED = 1, PASS_CORR = 2 };
 template <int DIM>
 struct TileShape;
 template <>
-struct TileShape<1> { static constexpr int X = 255, Y = 1, Z = 1, THREADS = 256, MINB = ECG_TILE1D_MINB; };
+struct TileShape<1> { static constexpr int X = 127, Y = 1, Z = 1, THREADS = 128, MINB = ECG_TILE1D_MINB; };
 template <>
 struct TileShape<2> {
   static constexpr int X = ECG_TILE2D_X, Y = ECG_TILE2D_Y, Z = 1, THREADS = ECG_TILE2D_THREADS, MINB = ECG_TILE2D_MINB;
@@ -89,7 +92,9 @@ struct Fields {
   static constexpr int NFL = 3 * NP + DIM + 3;   // flux components: a_k, m_k, e_k, mom_d, E, sM, uStar
 };
 
-// Device scalars of a context's time loop (Run::solver src/Run.cpp:385-490).
+// Device scalars of a context's time loop (Run::solver src/Run.cpp:385-490).  A context holds two, by the
+// parity of its state buffers: a step reads the scalars beside the state it reads and its end writes the ones
+// beside the state it wrote, so the end needs only the step's wave speeds and can run beside its last kernel.
 struct DevScalars {
   double dt;                       // step being taken (1e-15 before the first step, src/Run.cpp:38)
   double t;                        // physical time
@@ -106,6 +111,16 @@ struct DevScalars {
 struct FaceStreams {
   cudaStream_t s[2];
   cudaEvent_t fork, join[2];
+  cudaEvent_t end_fork, end_join;  // of the end of the step beside its last cell kernel
+};
+
+// The end of a step that runs beside its last cell kernel (split forms): the scalars it reads and writes, its
+// stream and the events that fork it from and join it to the step's stream.
+struct StepEnd {
+  const DevScalars* from;
+  DevScalars* to;
+  cudaStream_t s;
+  cudaEvent_t fork, join;
 };
 
 struct StepParams {
@@ -147,6 +162,13 @@ struct StepParams {
   // kernels run), and optional events recorded after each axis' face kernel (profiling)
   double* flux[3];
   cudaEvent_t* split_ev;
+  // the end of the step (k_finalize), on the last pass of a step that is not profiled: run beside the cell
+  // kernel (split forms), or by the last block of the pass (fused kernels: fin_from != nullptr)
+  const struct StepEnd* end;
+  const DevScalars* fin_from;
+  DevScalars* fin_to;
+  unsigned int* fin_count;  // blocks of the pass that are done; wraps to 0
+  int chained;              // 1D passes: launched so that a pass' blocks start while the one before drains
   const struct FaceStreams* fstreams;  // auxiliary streams of the face kernels (nullptr: one after another)
   // host side: tensor maps of the face kernels' TMA staging (nullptr: the kernels load their tiles)
   const struct FaceMaps* fmaps;
@@ -210,40 +232,106 @@ __device__ __forceinline__ void atomic_min_pos_double(unsigned long long* addr, 
 }
 
 
-// Reduces the per-thread relaxation counters of a block (warp reductions, then shared atomics)
-// and adds them to the device counters with one global atomic per counter and block.
-// Every thread of the block must call it.
+// Run::solver src/Run.cpp:417-440: t += dt, iteration++, stop test, dt = cfl * dtMax; after the stop the
+// scalars are copied on unchanged.
+__device__ __forceinline__ void step_finalize(const DevScalars* from, DevScalars* to) {
+  DevScalars s = *from;
+  const double dtmax = __longlong_as_double((long long)__ldcg(&from->dtmax_bits));  // past L1: atomics wrote it
+  if (!s.done) {
+    s.t += s.dt;
+    s.it += 1;
+    if (s.mode == 1 && s.it >= s.max_it) s.done = 1;
+    if (s.mode == 2 && s.t >= s.t_end) s.done = 1;
+    s.dt = s.cfl * dtmax;
+  }
+  s.dtmax_bits = (unsigned long long)__double_as_longlong(1.e10);
+  *to = s;
+}
+
+// Called by thread 0 of every block of a fused pass after the block's wave speeds went into dtmax_bits (and
+// its threads have read dt): the last block to arrive ends the step.
+__device__ __forceinline__ void step_end(const StepParams& P) {
+  if (P.fin_from == nullptr) return;
+  __threadfence();
+  const unsigned int n = gridDim.x * gridDim.y * gridDim.z;
+  if (atomicInc(P.fin_count, n - 1) == n - 1) {
+    __threadfence();
+    step_finalize(P.fin_from, P.fin_to);
+  }
+}
+
+// A fused pass after the stop: nothing is advanced, but the scalars pass on.
+__device__ __forceinline__ void step_skipped(const StepParams& P) {
+  if (P.fin_from != nullptr && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
+    step_finalize(P.fin_from, P.fin_to);
+}
+
+// Programmatic dependent launch (chained passes): wait for the kernels before, and let the next one start.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Launches a kernel, with chained as a programmatic dependent of the one before it in the stream (its blocks
+// may start once every block of that kernel runs, and wait for its end in chain_wait).
+template <class... KA, class... A>
+inline cudaError_t launch_chained(void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool chained,
+                                  A... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kern, KA(args)...);
+}
+
+// Reduces the per-thread relaxation counters of a block (a row of shared counters per warp, one barrier) and
+// adds them to the device counters with one global atomic per counter and block.  Every thread of the block
+// must call it.
 __device__ __forceinline__ void block_counters(DevStats* st, unsigned int relax, unsigned int iters,
                                                unsigned int fallback, unsigned int seeded, unsigned int rejected,
                                                unsigned int nonfinite, unsigned int ptmu, unsigned int max_iters,
                                                bool hist) {
-  __shared__ unsigned int sc[24];
-  const int tid = threadIdx.x;
-  if (tid < 24) sc[tid] = 0u;
-  __syncthreads();
+  __shared__ unsigned int sc[8][24];  // up to 256 threads
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = (int)(blockDim.x >> 5);
   const unsigned full = 0xffffffffu;
-  unsigned int v[7] = {relax, iters, fallback, seeded, rejected, nonfinite, ptmu};
+  const unsigned int nr = __reduce_add_sync(full, relax), ni = __reduce_add_sync(full, iters);
+  const unsigned int mx = __reduce_max_sync(full, max_iters);
+  unsigned int v = lane == 0 ? nr : (lane == 1 ? ni : (lane == 7 ? mx : 0u));
+  if (__any_sync(full, fallback | seeded | rejected | nonfinite | ptmu)) {
+    const unsigned int o[5] = {fallback, seeded, rejected, nonfinite, ptmu};
 #pragma unroll
-  for (int i = 0; i < 7; i++) {
-    unsigned int w = __reduce_add_sync(full, v[i]);
-    if ((tid & 31) == 0 && w) atomicAdd(&sc[i], w);
+    for (int i = 0; i < 5; i++) {
+      const unsigned int w = __reduce_add_sync(full, o[i]);
+      if (lane == 2 + i) v = w;
+    }
   }
-  unsigned int mx = __reduce_max_sync(full, max_iters);
-  if ((tid & 31) == 0 && mx) atomicMax(&sc[7], mx);
-  if (hist && relax) atomicAdd(&sc[8 + (iters < 16 ? (iters >= 1 ? iters - 1 : 0) : 15)], 1u);
+  if (lane < 24) sc[warp][lane] = v;
+  if (hist) {
+    __syncwarp();
+    const unsigned int bin = relax ? (iters < 16 ? (iters >= 1 ? iters - 1 : 0) : 15) : 16;
+    const unsigned int same = __match_any_sync(full, bin);
+    if (bin < 16 && (int)__ffs(same) - 1 == lane) sc[warp][8 + bin] = (unsigned)__popc(same);
+  }
   __syncthreads();
-  if (tid < 24 && sc[tid]) {
-    unsigned long long x = sc[tid];
-    switch (tid) {
-      case 0: atomicAdd(&st->relax_calls, x); break;
-      case 1: atomicAdd(&st->newton_evals, x); break;
-      case 2: atomicAdd(&st->newton_fallback, x); break;
-      case 3: atomicAdd(&st->seeded, x); break;
-      case 4: atomicAdd(&st->seed_rejected, x); break;
-      case 5: atomicAdd(&st->nonfinite, x); break;
-      case 6: atomicAdd(&st->ptmu_errors, x); break;
-      case 7: atomicMax(&st->newton_max, x); break;
-      default: atomicAdd(&st->hist[tid - 8], x); break;
+  if (tid < 24) {
+    unsigned long long x = sc[0][tid];
+    for (int w = 1; w < nw; w++) x = tid == 7 ? (x > sc[w][tid] ? x : sc[w][tid]) : x + sc[w][tid];
+    if (x) {
+      switch (tid) {
+        case 0: atomicAdd(&st->relax_calls, x); break;
+        case 1: atomicAdd(&st->newton_evals, x); break;
+        case 2: atomicAdd(&st->newton_fallback, x); break;
+        case 3: atomicAdd(&st->seeded, x); break;
+        case 4: atomicAdd(&st->seed_rejected, x); break;
+        case 5: atomicAdd(&st->nonfinite, x); break;
+        case 6: atomicAdd(&st->ptmu_errors, x); break;
+        case 7: atomicMax(&st->newton_max, x); break;
+        default: atomicAdd(&st->hist[tid - 8], x); break;
+      }
     }
   }
 }

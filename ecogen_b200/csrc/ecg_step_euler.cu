@@ -228,7 +228,14 @@ __global__ void __launch_bounds__(EulerStep<DIM, PASS, NTM>::NTH,
     k_euler_step(StepParams P, Geometry G, EosParams q, double eps) {
   using K = EulerStep<DIM, PASS, NTM>;
   using TS = TileShape<DIM>;
-  if (*P.done) return;
+  if (DIM == 1) {
+    chain_wait();
+    chain_next();
+  }
+  if (*P.done) {
+    step_skipped(P);
+    return;
+  }
   extern __shared__ double smem[];
   constexpr int RS = K::RMAX();
   constexpr int SS = (K::SMAX() > 0) ? K::SMAX() : 1;
@@ -514,17 +521,17 @@ __global__ void __launch_bounds__(EulerStep<DIM, PASS, NTM>::NTH,
     for (int t = 0; t < NTM; t++)  // Cell::timeEvolution / CellO2::predictionOrdre2
       if (t < P.ntr) P.out[(int64_t)(NS + t) * nn + cell] = tn[t] + at[t] * scale;
   }
-  __shared__ double red[32];
+  __shared__ double red[K::NTH / 32];
   double v = wmax;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   if ((tid & 31) == 0) red[tid >> 5] = v;
   __syncthreads();
-  if (tid < 32) {
-    v = (tid < K::NTH / 32) ? red[tid] : wave_none(G.stretched);
+  if (tid == 0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (tid == 0) atomic_min_pos_double(P.dtmax_bits, wave_dtmax(v, G.stretched, G.lcfl));
+    for (int w = 1; w < K::NTH / 32; w++) v = dmax(v, red[w]);
+    atomic_min_pos_double(P.dtmax_bits, wave_dtmax(v, G.stretched, G.lcfl));
+    step_end(P);
   }
 }
 
@@ -538,8 +545,7 @@ static cudaError_t euler_one(const StepParams& P, const Geometry& G, const ecg_e
   if (prepare) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   const EosParams q = make_eos_params(eos[0]);
   dim3 grid((G.n[0] + TS::X - 1) / TS::X, (G.n[1] + TS::Y - 1) / TS::Y, (G.n[2] + TS::Z - 1) / TS::Z);
-  kern<<<grid, K::NTH, sm, s>>>(P, G, q, eps);
-  return cudaGetLastError();
+  return launch_chained(kern, grid, dim3(K::NTH), sm, s, DIM == 1 && P.chained, P, G, q, eps);
 }
 
 template <int DIM, int NTM>

@@ -304,7 +304,14 @@ template <int DIM, int PASS>
 __global__ void ECG_PTUEQ_BOUNDS(DIM, PASS) k_ptueq_step(StepParams P, Geometry G, PtEos M) {
   using K = PtStep<DIM, PASS>;
   using TS = TileShape<DIM>;
-  if (*P.done) return;
+  if (DIM == 1) {
+    chain_wait();
+    chain_next();
+  }
+  if (*P.done) {
+    step_skipped(P);
+    return;
+  }
   extern __shared__ double smem[];
   constexpr int RS = K::RMAX();
   constexpr int SS = (K::SMAX() > 0) ? K::SMAX() : 1;
@@ -528,17 +535,17 @@ __global__ void ECG_PTUEQ_BOUNDS(DIM, PASS) k_ptueq_step(StepParams P, Geometry 
     }
     pt_update<DIM, PASS>(P, M, nn, cell, am, amom, aE);
   }
-  __shared__ double red[32];
+  __shared__ double red[K::NTH / 32];
   double v = wmax;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   if ((tid & 31) == 0) red[tid >> 5] = v;
   __syncthreads();
-  if (tid < 32) {
-    v = (tid < K::NTH / 32) ? red[tid] : wave_none(G.stretched);
+  if (tid == 0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (tid == 0) atomic_min_pos_double(P.dtmax_bits, wave_dtmax(v, G.stretched, G.lcfl));
+    for (int w = 1; w < K::NTH / 32; w++) v = dmax(v, red[w]);
+    atomic_min_pos_double(P.dtmax_bits, wave_dtmax(v, G.stretched, G.lcfl));
+    step_end(P);
   }
 }
 
@@ -554,8 +561,7 @@ static cudaError_t ptueq_one(const StepParams& P, const Geometry& G, const ecg_e
   for (int k = 0; k < 2; k++)
     M.e[k] = make_eos_params(eos[k]);
   dim3 grid((G.n[0] + TS::X - 1) / TS::X, (G.n[1] + TS::Y - 1) / TS::Y, (G.n[2] + TS::Z - 1) / TS::Z);
-  kern<<<grid, K::NTH, sm, s>>>(P, G, M);
-  return cudaGetLastError();
+  return launch_chained(kern, grid, dim3(K::NTH), sm, s, DIM == 1 && P.chained, P, G, M);
 }
 
 template <int DIM>
