@@ -25,6 +25,13 @@ struct FaceLaunch {
   int tma;
 };
 
+// Copies of a cell kernel's later inputs into shared slots of the thread's own, issued before its first load
+// (cp.async: no registers held, no barrier needed).
+__device__ __forceinline__ void cell_copy(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cell_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // The face arrays a cell kernel reads.
 struct FaceArrays {
   const double* flux[3];

@@ -333,12 +333,14 @@ struct CellPrim {
 
 // The cell update that follows the flux accumulation of one pass (everything after the face loop
 // of solveHyperbolic for one cell), first half: U^n, time evolution and buildPrim.  aa/am/ae/amom/aE
-// hold sum_faces coefA*F (+ the non-conservative terms); an/rn/pn are the time-n alpha_k, rho_k, p_k.
+// hold sum_faces coefA*F (+ the non-conservative terms); an/rn/pn are the time-n alpha_k, rho_k, p_k; ue, where
+// given, the time-n velocities and E (copied ahead, `stride` apart).
 template <int NP, int DIM, int PASS>
 __device__ __forceinline__ void kapila_rebuild(const StepParams& P, const Model<NP>& M, int64_t nn, int64_t cell,
                                                double dt, const double an[NP], const double rn[NP],
                                                const double pn[NP], double aa[NP], double am[NP], double ae[NP],
-                                               double amom[DIM], double aE, CellPrim<NP, DIM>& cp) {
+                                               double amom[DIM], double aE, CellPrim<NP, DIM>& cp,
+                                               const double* ue = nullptr, int stride = 0) {
   using FL = Fields<NP, DIM>;
   // ---- U^n (FluxUEq::buildCons src/Models/UEq/FluxUEq.cpp:147) and time evolution
   //      (Cell::timeEvolution src/Order1/Cell.cpp:286: m_cons*dt then + U^n)
@@ -357,10 +359,10 @@ __device__ __forceinline__ void kapila_rebuild(const StepParams& P, const Model<
   double un[DIM];
 #pragma unroll
   for (int d = 0; d < DIM; d++) {
-    un[d] = P.sn[(int64_t)(FL::U + d) * nn + cell];
+    un[d] = ue ? ue[d * stride] : P.sn[(int64_t)(FL::U + d) * nn + cell];
     amom[d] = amom[d] * scale + 1. * (rhon * un[d]);
   }
-  double En = P.sn[(int64_t)FL::E * nn + cell];
+  double En = ue ? ue[DIM * stride] : P.sn[(int64_t)FL::E * nn + cell];
   aE = aE * scale + 1. * (rhon * En);
 
   // ---- buildPrim (FluxUEq::buildPrim src/Models/UEq/FluxUEq.cpp:161-209)

@@ -69,12 +69,13 @@ struct FaceKernelShape {
 // iterations, and in 4-warp blocks the warps that finish first waited at the block's counter reduction
 // for the slowest one (barrier stalls were 5.6 of 12.4 cycles between issues on the 1024^2 expansion),
 // holding their slots; a one-warp block frees its slot for the next block as soon as it is done.
-// 16 such blocks per SM keep the 128-register budget of 4 blocks of 4 warps.
+// 24 such blocks per SM (80 registers, no spill in the loops): measured on the 1024^2 expansion, cell kernel at 16
+// blocks 0.392 ms, at 20 0.395, at 24 0.360, at 32 0.373.
 #ifndef ECG_CELL_PTMU_THREADS
 #define ECG_CELL_PTMU_THREADS 32
 #endif
 #ifndef ECG_CELL_PTMU_MINB
-#define ECG_CELL_PTMU_MINB (512 / ECG_CELL_PTMU_THREADS)
+#define ECG_CELL_PTMU_MINB (768 / ECG_CELL_PTMU_THREADS)
 #endif
 constexpr int CELL_THREADS = 128;
 __host__ __device__ constexpr int cell_threads(bool ptmu) { return ptmu ? ECG_CELL_PTMU_THREADS : CELL_THREADS; }
@@ -457,19 +458,22 @@ __device__ __forceinline__ void load_face_flux(const double* __restrict__ fl, in
   F.uStar = p[(int64_t)(3 * NP + DIM + 2) * nfa];
 }
 
-// L2 prefetches of the upper faces' fluxes of a warp's cells (rows of 32 doubles per component; the lower
-// faces' were read by earlier blocks, or are in the same rows along x): without them a warp met
-// the DRAM latency again for every face it accumulated (long-scoreboard stalls were 5.1 of 11.2 cycles between
-// issues at 128^3, DRAM at half its bandwidth).  Measured, cell kernels: 2D 2048^2 0.421 / 0.437 ms without,
-// 0.410 / 0.427 with every axis, 0.389 / 0.407 with Y only (the X loads follow at once); 3D 256^3 2.43 without,
-// 2.42 with Y and Z, 2.37 with every axis.  Prefetching for the block one wave ahead instead cost 30 % in 3D.
+// How the cell kernel's loads overlap.  Accumulating face after face, a warp met the DRAM latency four (2D) to
+// seven times (long-scoreboard stalls were 4.9 of 10.5 cycles between issues in 2D, DRAM at 37 %).  2D: each
+// thread copies what it needs last, the Y faces' fluxes and the time-n u and E, into shared memory before its
+// first load (cp.async: no registers held, 25 doubles a thread, five blocks of 128 per SM).  3D: such copies of one
+// axis take 35 KB a block from L1, so a lane per component prefetches the rows of the upper faces into L2 instead
+// (the lower faces' were read by earlier blocks, or are in the same rows along x).  Measured on one B200, cell
+// kernels of predictor and corrector: 2D 2048^2 0.421 / 0.437 ms with neither, 0.369 / 0.381 with prefetches of the
+// Y rows and the other steps, 0.323 / 0.333 with the copies; 3D 256^3 2.43 ms with neither, 2.31 / 2.33 with
+// prefetches and the other steps, 2.39 / 2.47 with copies.  Prefetching for the block one wave ahead cost 30 % in 3D.
 template <int NP, int DIM>
 __device__ __forceinline__ void prefetch_face_fluxes(const Geometry& G, const double* const fa[3], const int g[3]) {
   using FL = Fields<NP, DIM>;
   const int c = threadIdx.x & 15;  // component; lanes 16..31 of a warp take the second 128 bytes of a row
   static_assert(FL::NFL <= 16, "a lane per component and half row");
 #pragma unroll
-  for (int ax = DIM == 2 ? 1 : 0; ax < DIM; ax++) {
+  for (int ax = 0; ax < DIM; ax++) {
     const int64_t fid = split_fid(G.n, ax, g[ax] + 1, g[0], g[1], g[2]) - c;
     if (c < FL::NFL) asm volatile("prefetch.global.L2 [%0];" ::"l"(fa[ax] + fid + (int64_t)c * split_nfaces(G.n, ax)));
   }
@@ -504,8 +508,27 @@ __global__ void __launch_bounds__(cell_threads(PTMU),
   CellCounters cc;
   CellPrim<NP, DIM> cp;
   const double* fa[3] = {fx, fy, fz};
+  // 2D: the fluxes of the last axis' two faces, u and E of the time-n state, copied ahead into a shared slot of
+  // the thread's own (no barrier)
+  constexpr bool AHEAD = DIM == 2;
+  constexpr int CT = cell_threads(PTMU), LA = DIM - 1;
+  __shared__ double stage[AHEAD ? 2 * FL::NFL + DIM + 1 : 1][CT];
   if (active) {
-    prefetch_face_fluxes<NP, DIM>(G, fa, g);
+    if (AHEAD) {
+      const int64_t nfa = split_nfaces(G.n, LA);
+      const double* lo = fa[LA] + split_fid(G.n, LA, g[LA], g[0], g[1], g[2]);
+      const double* hi = fa[LA] + split_fid(G.n, LA, g[LA] + 1, g[0], g[1], g[2]);
+#pragma unroll
+      for (int i = 0; i < (AHEAD ? FL::NFL : 0); i++) {
+        cell_copy(&stage[i][threadIdx.x], lo + (int64_t)i * nfa);
+        cell_copy(&stage[FL::NFL + i][threadIdx.x], hi + (int64_t)i * nfa);
+      }
+#pragma unroll
+      for (int d = 0; d < (AHEAD ? DIM + 1 : 0); d++)
+        cell_copy(&stage[2 * FL::NFL + d][threadIdx.x], P.sn + (int64_t)(FL::U + d) * nn + cell);
+    } else {
+      prefetch_face_fluxes<NP, DIM>(G, fa, g);
+    }
     const double p0 = P.sn[(int64_t)FL::P * nn + cell];
 #pragma unroll
     for (int k = 0; k < NP; k++) {
@@ -514,7 +537,10 @@ __global__ void __launch_bounds__(cell_threads(PTMU),
       pn[k] = eos_fix_p(M.eos[k], p0);
     }
   }
-  if (done) return;  // tested here: the first loads do not wait for it
+  if (done) {  // tested here: the first loads do not wait for it
+    if (AHEAD) cell_copies_wait();
+    return;
+  }
   if (active) {
     // internal faces, axis by axis: the left face added, the right face subtracted
 #pragma unroll
@@ -522,12 +548,16 @@ __global__ void __launch_bounds__(cell_threads(PTMU),
       const int64_t nfa = split_nfaces(G.n, ax);
       const double cA = cell_coefA(G, ax, g[0], g[1], g[2]);
       Flux<NP> F;
+      const bool ahead = AHEAD && ax == LA;
+      if (ahead) cell_copies_wait();
       if (g[ax] >= 1) {
-        load_face_flux<NP, DIM>(fa[ax], nfa, split_fid(G.n, ax, g[ax], g[0], g[1], g[2]), F, P.stats);
+        if (ahead) load_face_flux<NP, DIM>(&stage[0][threadIdx.x], CT, 0, F, P.stats);
+        else load_face_flux<NP, DIM>(fa[ax], nfa, split_fid(G.n, ax, g[ax], g[0], g[1], g[2]), F, P.stats);
         acc_face<NP, DIM>(cA, true, F, an, pn, aa, am, ae, amom, aE);
       }
       if (g[ax] + 1 <= G.n[ax] - 1) {
-        load_face_flux<NP, DIM>(fa[ax], nfa, split_fid(G.n, ax, g[ax] + 1, g[0], g[1], g[2]), F, P.stats);
+        if (ahead) load_face_flux<NP, DIM>(&stage[AHEAD ? FL::NFL : 0][threadIdx.x], CT, 0, F, P.stats);
+        else load_face_flux<NP, DIM>(fa[ax], nfa, split_fid(G.n, ax, g[ax] + 1, g[0], g[1], g[2]), F, P.stats);
         acc_face<NP, DIM>(cA, false, F, an, pn, aa, am, ae, amom, aE);
       }
     }
@@ -543,7 +573,8 @@ __global__ void __launch_bounds__(cell_threads(PTMU),
                               F, P.stats);
       acc_face<NP, DIM>(cell_coefA(G, ax, g[0], g[1], g[2]), false, F, an, pn, aa, am, ae, amom, aE);
     }
-    kapila_rebuild<NP, DIM, PASS>(P, M, nn, cell, *P.dt, an, rn, pn, aa, am, ae, amom, aE, cp);
+    kapila_rebuild<NP, DIM, PASS>(P, M, nn, cell, *P.dt, an, rn, pn, aa, am, ae, amom, aE, cp,
+                                  AHEAD ? &stage[AHEAD ? 2 * FL::NFL : 0][threadIdx.x] : nullptr, CT);
   }
   SeedGate<NP> sg;
   if (SEED && !PTMU) seed_gate<NP, DIM>(P, M, active, cp, sg);

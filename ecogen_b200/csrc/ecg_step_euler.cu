@@ -109,18 +109,20 @@ __device__ __forceinline__ void hllc_euler(const EulerSide& L, const double ul[3
   }
 }
 
-// FluxEuler::buildCons, Cell::timeEvolution, FluxEuler::buildPrim of a cell from its accumulated fluxes.
+// FluxEuler::buildCons, Cell::timeEvolution, FluxEuler::buildPrim of a cell from its accumulated fluxes and its
+// time-n fields (sn, `stride` apart).
 template <int DIM, int PASS>
 __device__ __forceinline__ void euler_update(const StepParams& P, const EosParams& q, double eps, int64_t nn,
-                                             int64_t cell, double am, const double* amom, double aE) {
+                                             int64_t cell, double am, const double* amom, double aE, const double* sn,
+                                             int64_t stride) {
   const double dt = *P.dt;
   const double scale = (PASS == PASS_PRED) ? 0.5 * dt : dt;
-  const double rn = P.sn[cell];
-  const double En = P.sn[(int64_t)(2 + DIM) * nn + cell];
+  const double rn = sn[0];
+  const double En = sn[(2 + DIM) * stride];
   am = am * scale + 1. * rn;
   double u[DIM], usq = 0.;
 #pragma unroll
-  for (int d = 0; d < DIM; d++) u[d] = amom[d] * scale + 1. * (rn * P.sn[(int64_t)(2 + d) * nn + cell]);
+  for (int d = 0; d < DIM; d++) u[d] = amom[d] * scale + 1. * (rn * sn[(2 + d) * stride]);
   aE = aE * scale + 1. * (rn * En);
 #pragma unroll
   for (int d = 0; d < DIM; d++) {
@@ -209,8 +211,8 @@ struct EulerFlow {
   }
   template <int DIM, int PASS>
   static __device__ __forceinline__ void update(const StepParams& P, const Eos& M, int64_t nn, int64_t cell,
-                                                const double* acc) {
-    euler_update<DIM, PASS>(P, M.q, M.eps, nn, cell, acc[0], acc + 1, acc[1 + DIM]);
+                                                const double* acc, const double* sn, int64_t stride) {
+    euler_update<DIM, PASS>(P, M.q, M.eps, nn, cell, acc[0], acc + 1, acc[1 + DIM], sn, stride);
   }
 };
 
@@ -515,7 +517,7 @@ __global__ void __launch_bounds__(EulerStep<DIM, PASS, NTM>::NTH,
         at[t] -= -cA * tn[t] * sMb;
       }
     }
-    euler_update<DIM, PASS>(P, q, eps, nn, cell, am, amom, aE);
+    euler_update<DIM, PASS>(P, q, eps, nn, cell, am, amom, aE, P.sn + cell, nn);
     const double scale = (PASS == PASS_PRED) ? 0.5 * *P.dt : *P.dt;
 #pragma unroll
     for (int t = 0; t < NTM; t++)  // Cell::timeEvolution / CellO2::predictionOrdre2

@@ -155,10 +155,11 @@ __device__ __forceinline__ void hllc_pt(const PtSide& L, const double ul[3], con
 #define ECG_PTUEQ_CELL_MINB 10
 #endif
 
-// Update of a cell from its accumulated fluxes.
+// Update of a cell from its accumulated fluxes and its time-n fields (sn, `stride` apart).
 template <int DIM, int PASS>
 __device__ __forceinline__ void pt_update(const StepParams& P, const PtEos& M, int64_t nn, int64_t cell,
-                                          const double* am, const double* amom, double aE) {
+                                          const double* am, const double* amom, double aE, const double* sn,
+                                          int64_t stride) {
   constexpr int FP = 2, FT = 3, FU = 4;
   // ---- FluxPTUEq::buildCons (time-n state), Cell::timeEvolution, FluxPTUEq::buildPrim (:125-160) with
   // MixPTUEq::computePressure (:93-122, Le Martelot's analytic p of two IG/SG phases) and
@@ -166,11 +167,11 @@ __device__ __forceinline__ void pt_update(const StepParams& P, const PtEos& M, i
   const double dt = *P.dt;
   const double scale = (PASS == PASS_PRED) ? 0.5 * dt : dt;
   PtSide n0;
-  n0.a[0] = P.sn[cell];
-  n0.a[1] = P.sn[nn + cell];
-  n0.p = P.sn[(int64_t)FP * nn + cell];
-  n0.T = P.sn[(int64_t)FT * nn + cell];
-  const double En = P.sn[(int64_t)(FU + DIM) * nn + cell];
+  n0.a[0] = sn[0];
+  n0.a[1] = sn[stride];
+  n0.p = sn[FP * stride];
+  n0.T = sn[FT * stride];
+  const double En = sn[(FU + DIM) * stride];
   double rhon = 0.;
 #pragma unroll
   for (int k = 0; k < 2; k++) {
@@ -182,7 +183,7 @@ __device__ __forceinline__ void pt_update(const StepParams& P, const PtEos& M, i
   for (int k = 0; k < 2; k++) m[k] = am[k] * scale + 1. * (n0.a[k] * n0.r[k]);
   double mom[DIM];
 #pragma unroll
-  for (int d = 0; d < DIM; d++) mom[d] = amom[d] * scale + 1. * (rhon * P.sn[(int64_t)(FU + d) * nn + cell]);
+  for (int d = 0; d < DIM; d++) mom[d] = amom[d] * scale + 1. * (rhon * sn[(FU + d) * stride]);
   const double rE = aE * scale + 1. * (rhon * En);
   const double rhoMel = 0. + m[0] + m[1];
   double u[3] = {0., 0., 0.};
@@ -280,8 +281,8 @@ struct PtFlow {
   }
   template <int DIM, int PASS>
   static __device__ __forceinline__ void update(const StepParams& P, const Eos& M, int64_t nn, int64_t cell,
-                                                const double* acc) {
-    pt_update<DIM, PASS>(P, M, nn, cell, acc, acc + 2, acc[2 + DIM]);
+                                                const double* acc, const double* sn, int64_t stride) {
+    pt_update<DIM, PASS>(P, M, nn, cell, acc, acc + 2, acc[2 + DIM], sn, stride);
   }
 };
 
@@ -533,7 +534,7 @@ __global__ void ECG_PTUEQ_BOUNDS(DIM, PASS) k_ptueq_step(StepParams P, Geometry 
       for (int d = 0; d < DIM; d++) amom[d] -= cA * Fg[d];
       aE -= cA * FE;
     }
-    pt_update<DIM, PASS>(P, M, nn, cell, am, amom, aE);
+    pt_update<DIM, PASS>(P, M, nn, cell, am, amom, aE, P.sn + cell, nn);
   }
   __shared__ double red[K::NTH / 32];
   double v = wmax;
