@@ -289,8 +289,12 @@ inline cudaError_t launch_chained(void (*kern)(KA...), dim3 grid, dim3 block, si
 }
 
 // Reduces the per-thread relaxation counters of a block (a row of shared counters per warp, one barrier) and
-// adds them to the device counters with one global atomic per counter and block.  Every thread of the block
-// must call it.
+// adds them to the device counters with one global atomic per counter and block, a lane each at consecutive
+// addresses, so that a block sends a few requests instead of one per counter: all blocks add to the same lines.
+// Measured, one instruction against one per counter (cell kernels, one B200): 2D 2048^2 0.325 / 0.335 -> 0.320 /
+// 0.326 ms, 3D 256^3 2.35 / 2.36 -> 2.30 / 2.31 ms, p-T-mu 1024^2 0.359 -> 0.347 ms (no atomics at all: 0.310 / 0.318,
+// 2.28 / 2.29, 0.347; cell blocks of 64 threads 0.338 / 0.390 and 2.47 ms with one per counter, of 32 0.70 and 4.39 ms).
+// Every thread of the block must call it.
 __device__ __forceinline__ void block_counters(DevStats* st, unsigned int relax, unsigned int iters,
                                                unsigned int fallback, unsigned int seeded, unsigned int rejected,
                                                unsigned int nonfinite, unsigned int ptmu, unsigned int max_iters,
@@ -321,17 +325,8 @@ __device__ __forceinline__ void block_counters(DevStats* st, unsigned int relax,
     unsigned long long x = sc[0][tid];
     for (int w = 1; w < nw; w++) x = tid == 7 ? (x > sc[w][tid] ? x : sc[w][tid]) : x + sc[w][tid];
     if (x) {
-      switch (tid) {
-        case 0: atomicAdd(&st->relax_calls, x); break;
-        case 1: atomicAdd(&st->newton_evals, x); break;
-        case 2: atomicAdd(&st->newton_fallback, x); break;
-        case 3: atomicAdd(&st->seeded, x); break;
-        case 4: atomicAdd(&st->seed_rejected, x); break;
-        case 5: atomicAdd(&st->nonfinite, x); break;
-        case 6: atomicAdd(&st->ptmu_errors, x); break;
-        case 7: atomicMax(&st->newton_max, x); break;
-        default: atomicAdd(&st->hist[tid - 8], x); break;
-      }
+      if (tid == 7) atomicMax(&st->newton_max, x);
+      else atomicAdd(&st->relax_calls + tid, x);  // one instruction for the block's counters: consecutive addresses
     }
   }
 }
@@ -365,17 +360,8 @@ __device__ __forceinline__ void block_ptmu_counters(DevStats* st, unsigned int s
   __syncthreads();
   if (tid < 24 && sp[tid]) {
     const unsigned long long x = sp[tid];
-    switch (tid) {
-      case 22: atomicAdd(&st->ptmu_seeded, x); break;
-      case 23: atomicAdd(&st->ptmu_seed_rejected, x); break;
-      case 0: atomicAdd(&st->ptmu_solves, x); break;
-      case 1: atomicAdd(&st->ptmu_outer, x); break;
-      case 2: atomicAdd(&st->ptmu_tsat_calls, x); break;
-      case 3: atomicAdd(&st->ptmu_tsat_iters, x); break;
-      case 4: atomicMax(&st->ptmu_outer_max, x); break;
-      case 5: atomicMax(&st->ptmu_tsat_max, x); break;
-      default: atomicAdd(&st->ptmu_hist[tid - 6], x); break;
-    }
+    if (tid == 4 || tid == 5) atomicMax(&st->ptmu_solves + tid, x);
+    else atomicAdd(&st->ptmu_solves + tid, x);
   }
 }
 

@@ -107,14 +107,15 @@ inline void side_geometry(const ecg_case& c, const std::vector<double>* sz, cons
   }
 }
 
-// Device counters filled by the step kernels.
+// Device counters filled by the step kernels.  The first 24, and the 24 of the p-T-mu relaxation, are in the order in
+// which a block adds them, one lane each (block_counters, block_ptmu_counters).
 struct DevStats {
-  unsigned long long relax_calls, newton_evals, newton_fallback, seeded, seed_rejected, ptmu_errors, nonfinite;
+  unsigned long long relax_calls, newton_evals, newton_fallback, seeded, seed_rejected, nonfinite, ptmu_errors;
   unsigned long long newton_max;
   unsigned long long hist[16];
   // p-T-mu relaxation: saturation solves, their p* iterations (sum, max, histogram), T_sat solves and
   // their iterations (sum, max)
-  unsigned long long ptmu_solves, ptmu_outer, ptmu_outer_max, ptmu_tsat_calls, ptmu_tsat_iters, ptmu_tsat_max;
+  unsigned long long ptmu_solves, ptmu_outer, ptmu_tsat_calls, ptmu_tsat_iters, ptmu_outer_max, ptmu_tsat_max;
   unsigned long long ptmu_hist[16];
   unsigned long long ptmu_seeded, ptmu_seed_rejected;
   unsigned long long bounds_violations;  // bounds-checked builds: accesses outside their buffer (skipped)
