@@ -4,8 +4,16 @@
 #include <cstdint>
 
 #include "ecg_internal.h"
+#include "ecg_pow.cuh"
+#include "ecg_types.h"
 
 namespace ecg {
+
+void ptmu_cold_terms(PtmuParams& t) {
+  const double T = t.cold;
+  t.f0 = t.A + t.B / T + t.C * elog(T);
+  t.df0 = t.C / T - t.B / (T * T);
+}
 
 // Checks a case against what the library runs (ecg_create and ecg_step_noalloc accept the same cases).
 ecg_status validate_case(const ecg_case* c) {

@@ -43,7 +43,13 @@ inline EosParams make_eos_params(const ecg_eos& e) {
 struct PtmuParams {
   EosParams liq, vap;
   double A, B, C, D, cold, half, branch;
+  // the first evaluation of a cold start, the same in every solve but for the pressures' logarithms:
+  // A + B/cold + C ln(cold), and the derivative there
+  double f0, df0;
 };
+
+// f0 and df0 (ecg_case.cpp: the logarithm is the host build of the kernels' elog, bit for bit the device's).
+void ptmu_cold_terms(PtmuParams& t);
 
 inline PtmuParams make_ptmu_params(const ecg_eos& l, const ecg_eos& v) {
   PtmuParams t{};
@@ -57,6 +63,7 @@ inline PtmuParams make_ptmu_params(const ecg_eos& l, const ecg_eos& v) {
   t.cold = 0.1 * t.B / t.C;
   t.half = 0.5 * t.B / t.C;
   t.branch = t.B / t.C;
+  ptmu_cold_terms(t);
   return t;
 }
 
