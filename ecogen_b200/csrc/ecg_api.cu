@@ -138,6 +138,7 @@ struct ecg_ctx {
   Geometry geo{};
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // two-step sequences starting from state[0] / state[1]
   bool graph_dirty = true;
+  int direct_steps = 0;  // steps launched one by one since the graphs were dropped
 };
 
 namespace {
@@ -343,6 +344,7 @@ void drop_graphs(ecg_ctx* x) {
       x->graph[i] = nullptr;
     }
   x->graph_dirty = false;
+  x->direct_steps = 0;
 }
 
 // Captures two consecutive steps starting from state[parity] (the pair returns to state[parity]).
@@ -363,8 +365,22 @@ ecg_status build_graph(ecg_ctx* x, int parity) {
   return ECG_OK;
 }
 
+// Steps a context launches one by one before it captures its graphs.  A graph saves host time per launch but its
+// capture and instantiation cost 0.2 to 0.6 ms, which a few small steps do not earn back.  Measured (one B200, a
+// context's first call / a repeated one, us), graphs from the first step against none: 80 x 70 cells, 4 steps 678 / 319
+// against 389 / 369; 32 x 30 x 28, 4 steps 1046 / 475 against 547 / 490; Euler 90 x 100, 3 steps 463 / 149 against
+// 245 / 194; 191 x 103, 20 steps 1734 / 1405 against 1591 / 1555; 1D 1000 cells, 16 steps 419 / 273 against 283 / 263.
+// So a graph earns its cost after some tens of steps.
+#ifndef ECG_GRAPH_AFTER
+#define ECG_GRAPH_AFTER 32
+#endif
 ecg_status advance(ecg_ctx* x, int nsteps) {
   if (x->graph_dirty) drop_graphs(x);
+  for (; nsteps > 0 && x->direct_steps < ECG_GRAPH_AFTER; nsteps--, x->direct_steps++) {
+    ecg_status s = launch_step(x, x->cur);
+    if (s != ECG_OK) return s;
+    x->cur = 1 - x->cur;
+  }
   while (nsteps >= 2) {
     if (!x->graph[x->cur]) {
       ecg_status s = build_graph(x, x->cur);
