@@ -151,11 +151,20 @@ def kernel_bytes_per_cell(case, form: str, slot: str) -> int:
     return 8 * (case.dim * nfl + ns + (ns - 1 if pred else ns))
 
 
+def flow_split(case) -> bool:
+    """Euler and PTUEq passes that run as face kernels and a cell kernel (2D and 3D without transports, with one limiter
+    in every slot), timed in one slot per pass."""
+    euler, ptueq = case.model.upper() == "EULER", getattr(case, "ptueq", False)
+    return (euler or ptueq) and case.dim >= 2 and not getattr(case, "transports", None)
+
+
 def kernel_label(case, form: str, slot: str) -> str:
     euler, ptueq = case.model.upper() == "EULER", getattr(case, "ptueq", False)
-    base = "k_euler_step" if euler else ("k_ptueq_step" if ptueq else "k_kapila_step")
     pas = ("MUSCL corrector" if slot.startswith("pass2") else
            ("MUSCL predictor" if case.second_order else "first-order step"))
+    if flow_split(case):  # one slot for the kernels of a pass
+        return f"k_flow_faces + k_flow_cells ({pas})"
+    base = "k_euler_step" if euler else ("k_ptueq_step" if ptueq else "k_kapila_step")
     if form == "split" and case.dim >= 2 and not euler and not ptueq:
         if "_faces_" in slot:
             return f"k_kapila_faces, {slot[-1].upper()} faces ({pas})"
@@ -164,36 +173,39 @@ def kernel_label(case, form: str, slot: str) -> str:
 
 
 def launches_per_step(case, form: str) -> int:
+    """Kernels of one step: split passes launch a face kernel per axis and a cell kernel, and the step ends in a
+    launch beside the last of them; a fused pass is one kernel, and the last one ends the step."""
     passes = 2 if case.second_order else 1
-    per_pass = (case.dim + 1) if (form == "split" and case.dim >= 2) else 1
-    return passes * per_pass + 1
+    if (form == "split" and case.dim >= 2) or flow_split(case):
+        return passes * (case.dim + 1) + 1
+    return passes
 
 
 # DRAM bytes per cell of the step kernels measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum
 # of one launch / cells: 2D two-phase MUSCL at 1536^2, 3D three-phase MUSCL at 128^3, 2D PTUEq MUSCL at
-# 1536^2, 2D p-T-mu at 1536^2, 2D Euler at 2048^2).  The kernels stream the state once, so traffic
-# scales with the cell count.
+# 1536^2, 2D p-T-mu at 1536^2, 2D Euler at 2048^2; PTUEq and Euler: the face and cell kernels of a pass).  The
+# kernels stream their arrays once, so traffic scales with the cell count.
 NCU_TRAFFIC_PER_CELL = {("kapila", 2, 2, True, "fused", "pass2_cells"): 190.96,
                         ("kapila", 2, 2, True, "fused", "pass1_cells"): 125.14,
                         ("kapila", 3, 3, True, "fused", "pass2_cells"): 250.27,
                         ("kapila", 3, 3, True, "fused", "pass1_cells"): 155.89,
-                        ("ptueq", 2, 2, True, "fused", "pass2_cells"): 150.78,
-                        ("ptueq", 2, 2, True, "fused", "pass1_cells"): 91.56,
+                        ("ptueq", 2, 2, True, "fused", "pass2_cells"): 328.,
+                        ("ptueq", 2, 2, True, "fused", "pass1_cells"): 322.,
                         ("kapila_ptmu", 2, 2, True, "fused", "pass2_cells"): 181.05,
                         ("kapila_ptmu", 2, 2, True, "fused", "pass1_cells"): 112.08,
-                        ("euler", 1, 2, True, "fused", "pass2_cells"): 98.52,
-                        ("euler", 1, 2, True, "fused", "pass1_cells"): 64.92}
+                        ("euler", 1, 2, True, "fused", "pass2_cells"): 247.,
+                        ("euler", 1, 2, True, "fused", "pass1_cells"): 240.}
 # Split form: DRAM bytes per unit of the kernel (faces of its axis for a face kernel, cells for the cell
 # kernel), ncu on one launch at 1536^2 (2D two-phase), 128^3 (3D three-phase) and 1024^2 (p-T-mu); the
 # traffic of a launch grows with its units, so a full-size launch is the per-unit figure times its units.
 _SPLIT_NCU = {  # (model, phases, dim): {slot: (FP64 thread instructions per unit, DRAM bytes per unit)}
-    ("kapila", 2, 2): {"pass1_faces_x": (742, 124), "pass1_faces_y": (751, 123), "pass1_cells": (498, 290),
-                       "pass2_faces_x": (742, 133), "pass2_faces_y": (751, 132), "pass2_cells": (498, 297)},
-    ("kapila", 3, 3): {"pass1_faces_x": (988, 184), "pass1_faces_y": (1003, 183), "pass1_faces_z": (997, 181),
-                       "pass1_cells": (879, 534), "pass2_faces_x": (982, 191), "pass2_faces_y": (1005, 191),
-                       "pass2_faces_z": (999, 190), "pass2_cells": (899, 542)},
-    ("kapila_ptmu", 2, 2): {"pass1_faces_x": (753, 96), "pass1_faces_y": (763, 95), "pass1_cells": (1722, 303),
-                            "pass2_faces_x": (753, 105), "pass2_faces_y": (763, 106), "pass2_cells": (1731, 310)},
+    ("kapila", 2, 2): {"pass1_faces_x": (595, 125), "pass1_faces_y": (601, 125), "pass1_cells": (420, 290),
+                       "pass2_faces_x": (595, 126), "pass2_faces_y": (601, 125), "pass2_cells": (419, 297)},
+    ("kapila", 3, 3): {"pass1_faces_x": (807, 186), "pass1_faces_y": (814, 184), "pass1_faces_z": (814, 183),
+                       "pass1_cells": (747, 531), "pass2_faces_x": (808, 185), "pass2_faces_y": (815, 184),
+                       "pass2_faces_z": (815, 183), "pass2_cells": (760, 537)},
+    ("kapila_ptmu", 2, 2): {"pass1_faces_x": (597, 99), "pass1_faces_y": (603, 100), "pass1_cells": (1290, 320),
+                            "pass2_faces_x": (597, 100), "pass2_faces_y": (603, 100), "pass2_cells": (1291, 329)},
 }
 for (_m, _np, _d), _slots in _SPLIT_NCU.items():
     for _slot, (_fp, _dram) in _slots.items():
@@ -396,7 +408,7 @@ def reference_sample(steps: int, warmup: int, iters: int | None = None, procs: i
 
 
 def bench_batch(args, rank, world, local):
-    """Batched independent 1D shock tubes (persistent work-queue kernel, per-case dt)."""
+    """Batched independent 1D shock tubes (a face and a cell kernel per pass, per-case dt)."""
     import ctypes as C
 
     import torch
@@ -501,9 +513,9 @@ def bench_batch(args, rank, world, local):
                            "parallelism": f"replicas{world}"},
                 "roofline": {"bound": "hbm", "achieved": B * value / 1e9, "peak": peak, "unit": "GB/s",
                              "frac": B * value / 1e9 / peak, "traffic": None, "peak_kind": kind,
-                             "kernel": "k_batch (predictor + corrector of one step)",
+                             "kernel": "k_batch_faces + k_batch_cells (predictor + corrector of one step)",
                              "ncu_bytes_per_cell_update": NCU_BATCH_BYTES_PER_CELL_UPDATE},
-                "e2e": e2e, "gpu_launches": args.steps * 3, "clocks": clk.summary(),
+                "e2e": e2e, "gpu_launches": args.steps * 5, "clocks": clk.summary(),
                 "newton": {"relax_calls": st.relax_calls, "evals": st.newton_evals, "max": st.newton_max}}
         if seeded is not None:
             line["mlp_seeded"] = seeded
