@@ -2,10 +2,11 @@
 //
 // A context owns, on one GPU, two copies of the state S (ping-pong: a step reads S^n and writes
 // S^{n+1}), the MUSCL half-step state, the mesh distance tables, device scalars (dt, t, dtMax,
-// stop flag) and counters, and one stream.  Every step is a fixed launch sequence
-//   first order : step(O1) -> finalize
-//   MUSCL       : step(PRED) -> step(CORR) -> finalize
-// whose only data-dependent quantity (dt) lives in device memory, so sequences of steps are
+// stop flag, by parity of S) and counters, and one stream, with auxiliary ones that fork from it and join it
+// within a step.  Every step is a fixed launch sequence
+//   first order : step(O1), which ends the step
+//   MUSCL       : step(PRED) -> step(CORR), which ends the step
+// whose only data-dependent quantity (dt) lives in device memory, so the steps after a context's first ones are
 // captured once as CUDA graphs and replayed without host round trips.
 #include <cuda_runtime.h>
 
