@@ -132,69 +132,59 @@ KERNEL_SLOTS = ["pass1_faces_x", "pass1_faces_y", "pass1_faces_z", "pass1_cells"
                 "pass2_faces_x", "pass2_faces_y", "pass2_faces_z", "pass2_cells", "update"]
 
 
+def model_of(case) -> str:
+    return "euler" if case.model.upper() == "EULER" else ("ptueq" if getattr(case, "ptueq", False) else "kapila")
+
+
 def kernel_bytes_per_cell(case, form: str, slot: str) -> int:
     """Algorithmic bytes per cell of one launch of a step kernel.
 
     Fused form: the pass's bytes (pass_bytes_per_cell).  Split form, face kernel of one axis: read the
-    pass's input state (NS - 1 fields; the corrector also the time-n alpha_0), write one flux
-    (3N + d + 3 doubles) per face; cell kernel: read the d faces' fluxes per cell, S^n (NS), write the
-    output state (NS, the predictor NS - 1)."""
+    pass's input state (NS - 1 fields; a first-order Euler pass reads E too), write the flux of one face
+    (Kapila 3N + d + 3 doubles, Euler d + 2, PTUEq d + 3); cell kernel: read the d faces' fluxes per cell,
+    S^n (NS), write the output state (NS, the predictor NS - 1)."""
     ns = state_fields(case)
     pb = pass_bytes_per_cell(case)
     if form != "split" or case.dim < 2:
         return pb["pass2" if slot.startswith("pass2") else "pass1"]
-    nfl = 3 * case.nphases + case.dim + 3
-    corr = slot.startswith("pass2")
+    model = model_of(case)
+    nfl = case.dim + {"euler": 2, "ptueq": 3, "kapila": 3 * case.nphases + 3}[model]
     pred = slot.startswith("pass1") and case.second_order
     if "_faces_" in slot:
-        return 8 * ((ns - 1) + (1 if corr else 0) + nfl)
+        return 8 * (ns - 1 + (1 if model == "euler" and not case.second_order else 0) + nfl)
     return 8 * (case.dim * nfl + ns + (ns - 1 if pred else ns))
 
 
-def flow_split(case) -> bool:
-    """Euler and PTUEq passes that run as face kernels and a cell kernel (2D and 3D without transports, with one limiter
-    in every slot), timed in one slot per pass."""
-    euler, ptueq = case.model.upper() == "EULER", getattr(case, "ptueq", False)
-    return (euler or ptueq) and case.dim >= 2 and not getattr(case, "transports", None)
-
-
 def kernel_label(case, form: str, slot: str) -> str:
-    euler, ptueq = case.model.upper() == "EULER", getattr(case, "ptueq", False)
+    model = model_of(case)
     pas = ("MUSCL corrector" if slot.startswith("pass2") else
            ("MUSCL predictor" if case.second_order else "first-order step"))
-    if flow_split(case):  # one slot for the kernels of a pass
-        return f"k_flow_faces + k_flow_cells ({pas})"
-    base = "k_euler_step" if euler else ("k_ptueq_step" if ptueq else "k_kapila_step")
-    if form == "split" and case.dim >= 2 and not euler and not ptueq:
+    if form == "split" and case.dim >= 2:
+        kernel = "k_kapila" if model == "kapila" else "k_flow"
         if "_faces_" in slot:
-            return f"k_kapila_faces, {slot[-1].upper()} faces ({pas})"
-        return f"k_kapila_cells ({pas})"
-    return f"{base} ({pas})"
+            return f"{kernel}_faces, {slot[-1].upper()} faces ({pas})"
+        return f"{kernel}_cells ({pas})"
+    return f"k_{model}_step ({pas})"
 
 
 def launches_per_step(case, form: str) -> int:
     """Kernels of one step: split passes launch a face kernel per axis and a cell kernel, and the step ends in a
     launch beside the last of them; a fused pass is one kernel, and the last one ends the step."""
     passes = 2 if case.second_order else 1
-    if (form == "split" and case.dim >= 2) or flow_split(case):
+    if form == "split" and case.dim >= 2:
         return passes * (case.dim + 1) + 1
     return passes
 
 
 # DRAM bytes per cell of the step kernels measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum
-# of one launch / cells: 2D two-phase MUSCL at 1536^2, 3D three-phase MUSCL at 128^3, 2D PTUEq MUSCL at
-# 1536^2, 2D p-T-mu at 1536^2, 2D Euler at 2048^2; PTUEq and Euler: the face and cell kernels of a pass).  The
+# of one launch / cells: 2D two-phase MUSCL at 1536^2, 3D three-phase MUSCL at 128^3, 2D p-T-mu at 1536^2).  The
 # kernels stream their arrays once, so traffic scales with the cell count.
 NCU_TRAFFIC_PER_CELL = {("kapila", 2, 2, True, "fused", "pass2_cells"): 190.96,
                         ("kapila", 2, 2, True, "fused", "pass1_cells"): 125.14,
                         ("kapila", 3, 3, True, "fused", "pass2_cells"): 250.27,
                         ("kapila", 3, 3, True, "fused", "pass1_cells"): 155.89,
-                        ("ptueq", 2, 2, True, "fused", "pass2_cells"): 328.,
-                        ("ptueq", 2, 2, True, "fused", "pass1_cells"): 322.,
                         ("kapila_ptmu", 2, 2, True, "fused", "pass2_cells"): 181.05,
-                        ("kapila_ptmu", 2, 2, True, "fused", "pass1_cells"): 112.08,
-                        ("euler", 1, 2, True, "fused", "pass2_cells"): 247.,
-                        ("euler", 1, 2, True, "fused", "pass1_cells"): 240.}
+                        ("kapila_ptmu", 2, 2, True, "fused", "pass1_cells"): 112.08}
 # Split form: DRAM bytes per unit of the kernel (faces of its axis for a face kernel, cells for the cell
 # kernel), ncu on one launch at 1536^2 (2D two-phase), 128^3 (3D three-phase) and 1024^2 (p-T-mu); the
 # traffic of a launch grows with its units, so a full-size launch is the per-unit figure times its units.
@@ -536,7 +526,7 @@ def main():
     ap.add_argument("--size", type=int, default=None)
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--form", default="default", choices=["default", "split", "fused"],
-                    help="form of the 2D / 3D Kapila passes (ecg_set_step_form); default: the library's")
+                    help="form of the 2D / 3D passes (ecg_set_step_form); default: the library's")
     ap.add_argument("--staging", default="default", choices=["default", "tma", "plain"],
                     help="face-kernel tile staging of the split form (default: TMA where the mesh allows)")
     args = ap.parse_args()
@@ -787,7 +777,7 @@ def main():
         top_bytes = kernel_bytes_per_cell(case, form, top)
         units = kernel_units(case, form, top)
         achieved = top_bytes * units / (top_ms * 1e-3) / 1e9
-        model_key = "euler" if case.model.upper() == "EULER" else ("ptueq" if case.ptueq else "kapila")
+        model_key = model_of(case)
         if model_key == "kapila" and case.ptmu is not None:
             model_key = "kapila_ptmu"
         tkey = (model_key, case.nphases, case.dim, bool(case.second_order), form, top)

@@ -111,8 +111,7 @@ struct ecg_ctx {
   double* dist = nullptr;     // distance tables (3 axes x 3 tables)
   double* tmp = nullptr;      // download scratch (mixture pressure)
   double* flux[3] = {nullptr, nullptr, nullptr};  // face arrays of the split form (2D / 3D)
-  bool split = false;         // Kapila step passes in split form (face kernels + cell kernel)
-  bool flow = false;          // Euler or PTUEq passes in split form (no choice of form for these models)
+  bool split = false;         // step passes in split form (face kernels + cell kernel)
   FaceStreams fstreams{};     // auxiliary streams of the face kernels (split forms)
   FaceMaps fmaps{};           // tensor maps of the face kernels' TMA staging (fmaps.ok = 0: none)
   int staging = ECG_STAGING_TMA;
@@ -278,9 +277,9 @@ ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
   P.pcrit = x->pcrit;
   P.ptmu_seed_p = x->ptmu_seed_p;
   P.tsat_hist = x->tsat_hist;
-  for (int a = 0; a < 3; a++) P.flux[a] = (x->split || x->flow) ? x->flux[a] : nullptr;
+  for (int a = 0; a < 3; a++) P.flux[a] = x->split ? x->flux[a] : nullptr;
   P.fstreams = x->fstreams.fork ? &x->fstreams : nullptr;
-  P.fmaps = ((x->split || x->flow) && x->staging == ECG_STAGING_TMA && x->fmaps.ok) ? &x->fmaps : nullptr;
+  P.fmaps = (x->split && x->staging == ECG_STAGING_TMA && x->fmaps.ok) ? &x->fmaps : nullptr;
   double* sn = x->state[parity];
   double* s1 = x->state[1 - parity];
   const bool euler = x->c.model == ECG_MODEL_EULER;
@@ -292,7 +291,7 @@ ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
   };
   cudaError_t e;
   P.chained = ev ? 0 : 1;
-  const bool beside = !ev && (x->split || x->flow);
+  const bool beside = !ev && x->split;
   // what the last pass of the step does beside its own work (profiled steps end in a launch of their own)
   auto last = [&] {
     if (ev) return;
@@ -587,11 +586,10 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
   }
   e = cudaMalloc(&x->tmp, sizeof(double) * (size_t)(ptueq ? 2 : 1) * (size_t)x->n);  // download scratch
   if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaMalloc(tmp)"));
-  // Euler (one limiter slot is read) and PTUEq run in split form when one limiter decides every slope
+  // PTUEq has a split form when one limiter decides every slope (Euler reads one limiter slot)
   const bool one_limiter = c->limiter[1] == c->limiter[0] && c->limiter[2] == c->limiter[0] &&
                            c->limiter[3] == c->limiter[0] && c->limiter[0] != ECG_LIM_THINC;
-  x->flow = x->dim >= 2 && c->ntransports == 0 && (euler || (ptueq && (c->order == 1 || one_limiter)));
-  if ((!euler && !ptueq && x->dim >= 2 && c->ntransports == 0) || x->flow) {
+  if (x->dim >= 2 && c->ntransports == 0 && (!ptueq || c->order == 1 || one_limiter)) {
     // face arrays of the split form: the flux components (Kapila 3N + d + 3, Euler d + 2, PTUEq d + 3) of every
     // face of each axis, the domain sides included
     const int nfl = euler ? x->dim + 2 : (ptueq ? x->dim + 3 : 3 * x->np + x->dim + 3);
@@ -599,7 +597,7 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
       e = cudaMalloc(&x->flux[a], sizeof(double) * (size_t)nfl * (size_t)split_nfaces(c->ncells, a));
       if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaMalloc(face fluxes)"));
     }
-    x->split = !x->flow;
+    x->split = true;
     for (int a = 0; a + 1 < x->dim && e == cudaSuccess; a++) {
       e = cudaStreamCreateWithFlags(&x->fstreams.s[a], cudaStreamNonBlocking);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->fstreams.join[a], cudaEventDisableTiming);
@@ -728,8 +726,8 @@ extern "C" void* ecg_stream(const ecg_ctx* x) { return x ? (void*)x->stream : nu
 
 extern "C" ecg_status ecg_set_step_form(ecg_ctx* x, int32_t form) {
   if (!x || (form != ECG_FORM_FUSED && form != ECG_FORM_SPLIT)) { set_error("bad step form"); return ECG_ERR_INVALID; }
-  if (form == ECG_FORM_SPLIT && (!x->flux[0] || x->flow)) { set_error("no split form for this case (1D, Euler, PTUEq or transports)"); return ECG_ERR_UNSUPPORTED; }
-  if (!x->flow) x->split = form == ECG_FORM_SPLIT;
+  if (form == ECG_FORM_SPLIT && !x->flux[0]) { set_error("no split form for this case (1D, transports, or PTUEq with several limiters or THINC)"); return ECG_ERR_UNSUPPORTED; }
+  x->split = form == ECG_FORM_SPLIT;
   x->graph_dirty = true;
   return ECG_OK;
 }

@@ -192,12 +192,13 @@ ecg_status ecg_step_profiled(ecg_ctx* ctx, int32_t nsteps, double* dt, double* t
  * time goes to its cell-kernel slot ([3] or [7]); entries of kernels that do not run stay 0. */
 ecg_status ecg_step_profiled_kernels(ecg_ctx* ctx, int32_t nsteps, double* dt, double* t, ecg_step_stats* stats,
                                      double* kernel_ms);
-/* Form of the Kapila step passes on 2D and 3D meshes.  ECG_FORM_SPLIT (the default where it applies):
+/* Form of the step passes on 2D and 3D meshes.  ECG_FORM_SPLIT (the default where it applies):
  * per axis a face-flux kernel writing every face's flux to a face array of the context, then one cell
  * kernel accumulating them in the reference's face order; ECG_FORM_FUSED: one kernel per pass that
  * stages a tile per axis in shared memory.  Both compute every flux with the same arithmetic and
- * accumulate in the same order, so they give the same bits.  1D cases and passive transports run fused
- * only, and the Euler and PTUEq models leave no choice (ECG_ERR_UNSUPPORTED for ECG_FORM_SPLIT). */
+ * accumulate in the same order, so they give the same bits.  1D cases, passive transports, and PTUEq in
+ * MUSCL with limiter slots that differ or with THINC run fused only (ECG_ERR_UNSUPPORTED for
+ * ECG_FORM_SPLIT). */
 enum { ECG_FORM_FUSED = 0, ECG_FORM_SPLIT = 1 };
 ecg_status ecg_set_step_form(ecg_ctx* ctx, int32_t form);
 int32_t ecg_step_form(const ecg_ctx* ctx);
