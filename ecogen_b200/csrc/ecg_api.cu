@@ -337,6 +337,51 @@ ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
   return ECG_OK;
 }
 
+// Sets a context up for the split form where the case has one: the face arrays, the auxiliary streams and the
+// tensor maps.  Where the face arrays do not fit the GPU's free memory the context keeps the fused kernels, which
+// need none (doubles per cell in MUSCL, fused / split: Euler 3D 19 / 34, PTUEq 3D 26 / 44, Kapila 3D of three
+// phases 34 / 79).
+cudaError_t make_split_form(ecg_ctx* x) {
+  const ecg_case& c = x->c;
+  const bool euler = c.model == ECG_MODEL_EULER, ptueq = c.model == ECG_MODEL_PTUEQ;
+  // PTUEq has a split form when one limiter decides every slope (Euler reads one limiter slot)
+  const bool one_limiter = c.limiter[1] == c.limiter[0] && c.limiter[2] == c.limiter[0] &&
+                           c.limiter[3] == c.limiter[0] && c.limiter[0] != ECG_LIM_THINC;
+  if (x->dim < 2 || c.ntransports != 0 || (ptueq && c.order != 1 && !one_limiter)) return cudaSuccess;
+  // the flux components (Kapila 3N + d + 3, Euler d + 2, PTUEq d + 3) of every face of each axis, the domain
+  // sides included
+  const int nfl = euler ? x->dim + 2 : (ptueq ? x->dim + 3 : 3 * x->np + x->dim + 3);
+  cudaError_t e = cudaSuccess;
+  for (int a = 0; a < x->dim && e == cudaSuccess; a++)
+    e = cudaMalloc(&x->flux[a], sizeof(double) * (size_t)nfl * (size_t)split_nfaces(c.ncells, a));
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();  // the launches to come do not report it
+    for (int a = 0; a < x->dim; a++) {
+      cudaFree(x->flux[a]);
+      x->flux[a] = nullptr;
+    }
+    return cudaSuccess;
+  }
+  for (int a = 0; a + 1 < x->dim && e == cudaSuccess; a++) {
+    e = cudaStreamCreateWithFlags(&x->fstreams.s[a], cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->fstreams.join[a], cudaEventDisableTiming);
+  }
+  for (cudaEvent_t* ev : {&x->fstreams.fork, &x->fstreams.end_fork, &x->fstreams.end_join})
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+  if (e != cudaSuccess) return e;
+  for (int i = 0; i < 2; i++)
+    x->step_end[i] = {x->scal + i, x->scal + (1 - i), x->fstreams.s[0], x->fstreams.end_fork, x->fstreams.end_join};
+#ifndef ECG_BOUNDS_CHECK
+  // TMA staging of the face kernels' tiles where the layout allows it (the bounds-checked build
+  // checks the kernels' own loads, so it stages them that way).  Staged planes: all but E, which the
+  // first-order Euler pass reads too.
+  const double* bufs[3] = {x->state[0], x->state[1], x->half};
+  build_face_maps(x->fmaps, bufs, x->dim, c.ncells, x->nq + (euler && c.order == 1 ? 1 : 0));
+#endif
+  x->split = true;
+  return cudaSuccess;
+}
+
 void drop_graphs(ecg_ctx* x) {
   for (int i = 0; i < 2; i++)
     if (x->graph[i]) {
@@ -586,33 +631,6 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
   }
   e = cudaMalloc(&x->tmp, sizeof(double) * (size_t)(ptueq ? 2 : 1) * (size_t)x->n);  // download scratch
   if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaMalloc(tmp)"));
-  // PTUEq has a split form when one limiter decides every slope (Euler reads one limiter slot)
-  const bool one_limiter = c->limiter[1] == c->limiter[0] && c->limiter[2] == c->limiter[0] &&
-                           c->limiter[3] == c->limiter[0] && c->limiter[0] != ECG_LIM_THINC;
-  if (x->dim >= 2 && c->ntransports == 0 && (!ptueq || c->order == 1 || one_limiter)) {
-    // face arrays of the split form: the flux components (Kapila 3N + d + 3, Euler d + 2, PTUEq d + 3) of every
-    // face of each axis, the domain sides included
-    const int nfl = euler ? x->dim + 2 : (ptueq ? x->dim + 3 : 3 * x->np + x->dim + 3);
-    for (int a = 0; a < x->dim; a++) {
-      e = cudaMalloc(&x->flux[a], sizeof(double) * (size_t)nfl * (size_t)split_nfaces(c->ncells, a));
-      if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaMalloc(face fluxes)"));
-    }
-    x->split = true;
-    for (int a = 0; a + 1 < x->dim && e == cudaSuccess; a++) {
-      e = cudaStreamCreateWithFlags(&x->fstreams.s[a], cudaStreamNonBlocking);
-      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->fstreams.join[a], cudaEventDisableTiming);
-    }
-    for (cudaEvent_t* ev : {&x->fstreams.fork, &x->fstreams.end_fork, &x->fstreams.end_join})
-      if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
-    if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaStreamCreate(face streams)"));
-#ifndef ECG_BOUNDS_CHECK
-    // TMA staging of the face kernels' tiles where the layout allows it (the bounds-checked build
-    // checks the kernels' own loads, so it stages them that way).  Staged planes: all but E, which the
-    // first-order Euler pass reads too.
-    const double* bufs[3] = {x->state[0], x->state[1], x->half};
-    build_face_maps(x->fmaps, bufs, x->dim, c->ncells, x->nq + (euler && c->order == 1 ? 1 : 0));
-#endif
-  }
   std::vector<double> h, sz[3], ctr[3];
   for (int a = 0; a < 3; a++) axis_cells(*c, a, sz[a], ctr[a]);
   distance_tables(*c, sz, ctr, h);
@@ -667,10 +685,9 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
   double big = 1.e10;
   std::memcpy(&s0.dtmax_bits, &big, sizeof(double));
   for (int i = 0; i < 2; i++) cudaMemcpy(x->scal + i, &s0, sizeof(s0), cudaMemcpyHostToDevice);
-  if (x->fstreams.fork)
-    for (int i = 0; i < 2; i++)
-      x->step_end[i] = {x->scal + i, x->scal + (1 - i), x->fstreams.s[0], x->fstreams.end_fork, x->fstreams.end_join};
   cudaMemset(x->stats, 0, sizeof(DevStats));
+  e = make_split_form(x);  // last: what the fused kernels need has its memory by now
+  if (e != cudaSuccess) return fail_free(cuda_fail(e, "face arrays"));
   // kernel attributes (dynamic shared memory) for every pass of this case shape
   for (int pass = 0; pass < 3; pass++) {
     StepParams P{};
@@ -726,7 +743,7 @@ extern "C" void* ecg_stream(const ecg_ctx* x) { return x ? (void*)x->stream : nu
 
 extern "C" ecg_status ecg_set_step_form(ecg_ctx* x, int32_t form) {
   if (!x || (form != ECG_FORM_FUSED && form != ECG_FORM_SPLIT)) { set_error("bad step form"); return ECG_ERR_INVALID; }
-  if (form == ECG_FORM_SPLIT && !x->flux[0]) { set_error("no split form for this case (1D, transports, or PTUEq with several limiters or THINC)"); return ECG_ERR_UNSUPPORTED; }
+  if (form == ECG_FORM_SPLIT && !x->flux[0]) { set_error("no split form for this case (1D, transports, PTUEq with several limiters or THINC, or too little memory)"); return ECG_ERR_UNSUPPORTED; }
   x->split = form == ECG_FORM_SPLIT;
   x->graph_dirty = true;
   return ECG_OK;
