@@ -17,6 +17,7 @@
 #include <string>
 #include <vector>
 
+#include "ecg_faces.cuh"
 #include "ecg_internal.h"
 #include "ecg_mlp_device.cuh"
 #include "ecg_step.cuh"
@@ -337,9 +338,17 @@ ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
   return ECG_OK;
 }
 
+// Whether the face kernels' grids hold a mesh: their lines and third coordinates are the grid's second and third
+// dimensions, of 65535 blocks at most (2D: 524,279 cells along y; 3D: 65,535 along y and z).  The fused kernels' tiles
+// reach further (2D: 917,490; 3D: 393,210).
+bool face_grids_fit(const int n[3], int dim) {
+  auto fits = [](dim3 g) { return g.y <= 65535 && g.z <= 65535; };
+  return fits(face_grid<0>(n)) && fits(face_grid<1>(n)) && (dim < 3 || fits(face_grid<2>(n)));
+}
+
 // Sets a context up for the split form where the case has one: the face arrays, the auxiliary streams and the
-// tensor maps.  Where the face arrays do not fit the GPU's free memory the context keeps the fused kernels, which
-// need none (doubles per cell in MUSCL, fused / split: Euler 3D 19 / 34, PTUEq 3D 26 / 44, Kapila 3D of three
+// tensor maps.  Where the mesh is too long for the face kernels' grids, or the face arrays do not fit the GPU's free
+// memory, the context keeps the fused kernels, which need no face arrays (doubles per cell in MUSCL, fused / split: Euler 3D 19 / 34, PTUEq 3D 26 / 44, Kapila 3D of three
 // phases 34 / 79).
 cudaError_t make_split_form(ecg_ctx* x) {
   const ecg_case& c = x->c;
@@ -348,6 +357,7 @@ cudaError_t make_split_form(ecg_ctx* x) {
   const bool one_limiter = c.limiter[1] == c.limiter[0] && c.limiter[2] == c.limiter[0] &&
                            c.limiter[3] == c.limiter[0] && c.limiter[0] != ECG_LIM_THINC;
   if (x->dim < 2 || c.ntransports != 0 || (ptueq && c.order != 1 && !one_limiter)) return cudaSuccess;
+  if (!face_grids_fit(c.ncells, x->dim)) return cudaSuccess;
   // the flux components (Kapila 3N + d + 3, Euler d + 2, PTUEq d + 3) of every face of each axis, the domain
   // sides included
   const int nfl = euler ? x->dim + 2 : (ptueq ? x->dim + 3 : 3 * x->np + x->dim + 3);
@@ -743,7 +753,7 @@ extern "C" void* ecg_stream(const ecg_ctx* x) { return x ? (void*)x->stream : nu
 
 extern "C" ecg_status ecg_set_step_form(ecg_ctx* x, int32_t form) {
   if (!x || (form != ECG_FORM_FUSED && form != ECG_FORM_SPLIT)) { set_error("bad step form"); return ECG_ERR_INVALID; }
-  if (form == ECG_FORM_SPLIT && !x->flux[0]) { set_error("no split form for this case (1D, transports, PTUEq with several limiters or THINC, or too little memory)"); return ECG_ERR_UNSUPPORTED; }
+  if (form == ECG_FORM_SPLIT && !x->flux[0]) { set_error("no split form for this case (1D, transports, PTUEq with several limiters or THINC, a mesh beyond the face kernels' grids, or too little memory)"); return ECG_ERR_UNSUPPORTED; }
   x->split = form == ECG_FORM_SPLIT;
   x->graph_dirty = true;
   return ECG_OK;

@@ -198,7 +198,8 @@ ecg_status ecg_step_profiled_kernels(ecg_ctx* ctx, int32_t nsteps, double* dt, d
  * stages a tile per axis in shared memory.  Both compute every flux with the same arithmetic and
  * accumulate in the same order, so they give the same bits.  1D cases, passive transports, and PTUEq in
  * MUSCL with limiter slots that differ or with THINC run fused only (ECG_ERR_UNSUPPORTED for
- * ECG_FORM_SPLIT), and so does a case whose face arrays do not fit the GPU's free memory. */
+ * ECG_FORM_SPLIT), and so does a case whose face arrays do not fit the GPU's free memory or whose mesh
+ * has more than 524,279 cells along y (2D), or more than 65,535 along y or z (3D). */
 enum { ECG_FORM_FUSED = 0, ECG_FORM_SPLIT = 1 };
 ecg_status ecg_set_step_form(ecg_ctx* ctx, int32_t form);
 int32_t ecg_step_form(const ecg_ctx* ctx);
