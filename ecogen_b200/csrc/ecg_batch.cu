@@ -2,9 +2,9 @@
 //
 // The reference runs independent cases one after the other (src/main.cpp:82-133), each with its
 // own time loop.  Here all cases live in one concatenated structure-of-arrays state (case c owns
-// cells [off_c, off_c + n_c) and faces [off_c + c, off_c + c + n_c]), every pass (first order, or MUSCL
-// predictor then corrector) is two launches over lists of (case, first face) and (case, first cell) items,
-// one block per item, and each case keeps its own dt: the fastest wave of an item's faces merges into the
+// cells [off_c, off_c + n_c)), every pass (first order, or MUSCL predictor then corrector) is two launches
+// over lists of (case, first face) and (case, first cell) items, one block per item (where the face fluxes do
+// not all fit the free memory: two launches per piece of the batch), and each case keeps its own dt: the fastest wave of an item's faces merges into the
 // case's slot with one atomicMin (a segmented min-reduction), then a per-case update sets
 // dt_c = cfl_c dtMax_c.  The step sequence is captured once as a CUDA graph.  The faces of an item (the
 // tile) are picked by a small autotuner that times each candidate on a copy of the state.
@@ -36,7 +36,6 @@ namespace ecg {
 
 struct BatchCase {
   int64_t off;
-  int64_t fbase;  // first face
   int n;
   double dx, coefA, lcfl, cfl;
 };
@@ -47,10 +46,11 @@ struct BatchScalars {
   long long it;
 };
 
-// A block's piece of a case: `first` face or cell of case c, whose place and size stand here too, so that the
-// block's loads start one access earlier than through BatchCase.
+// A block's piece of a case: the faces or cells of case c from `first` on, up to face `end` or cell `end` - 1.  The
+// case's size and place stand here too, so that the block's loads start one access earlier than through BatchCase;
+// face f's fluxes are at fbase + f.
 struct __align__(16) BatchItem {
-  int c, first, n, pad;
+  int c, first, n, end;
   int64_t off, fbase;
 };
 
@@ -59,7 +59,7 @@ struct BatchParams {
   const BatchCase* cases;
   BatchScalars* scal;
   const BatchItem* items;    // face items of the face kernel, cell items of the cell kernel
-  double* flux;              // face fluxes, stride nfaces
+  double* flux;              // face fluxes of a piece of the batch, stride nfaces
   int64_t nfaces;
 };
 
@@ -132,7 +132,7 @@ __device__ __forceinline__ void batch_sides(const StepParams& P, const Model<NP>
 // Any face of an item, sides of the case included, solved by fulfill and hllc and stored; returns its wave value.
 template <int NP, int TB, int PASS, int TYPES>
 static __device__ __noinline__ double batch_face_general(const BatchParams& B, const Model<NP>& M0, const double* sq,
-                                                         const BatchCase C, int f, int i, bool pone) {
+                                                         const BatchCase C, int64_t fid, int f, int i, bool pone) {
   const Model<NP> M = specialize_eos<NP, TYPES>(M0);
   using K = BatchTile<NP, TB, PASS, TYPES>;
   double wmax = wave_none(false), Fn[3];
@@ -154,7 +154,7 @@ static __device__ __noinline__ double batch_face_general(const BatchParams& B, c
     batch_sides<NP, TB, PASS, TYPES, true>(B.P, M, sq, C, C.n, f, i, pone, tl, ul, tr, ur);
     hllc<NP, K::O2>(M, tl, ul, tr, ur, false, C.lcfl, C.lcfl, wmax, Fn, F);
   }
-  store_batch_face<NP>(B, C.fbase + f, Fn[0], F);
+  store_batch_face<NP>(B, fid, Fn[0], F);
   return wmax;
 }
 
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(TB, ECG_BATCH_SM_THREADS / TB) k_batch_faces(c
   }
   double wmax = wave_none(false);
   const int f = f0 + tid;
-  if (tid < TF && f <= n) {
+  if (tid < TF && f <= I.end) {
     Thermo<NP> tl, tr;
     double ul[3], ur[3], Fn[3];
     Flux<NP> F;
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(TB, ECG_BATCH_SM_THREADS / TB) k_batch_faces(c
     if (f == 0) Fn[0] = -Fn[0];
     if (solved) store_batch_face<NP>(B, I.fbase + f, Fn[0], F);
     // operands out of hllc_quick's range
-    if (!solved) wmax = dmax(wmax, batch_face_general<NP, TB, PASS, TYPES>(B, M0, sq, C, f, tid, pone));
+    if (!solved) wmax = dmax(wmax, batch_face_general<NP, TB, PASS, TYPES>(B, M0, sq, C, I.fbase + f, f, tid, pone));
   }
   // ---- segmented reduction: this item's faces belong to case c only
   __shared__ double red[TB / 32];
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(CELL_THREADS, SEED ? ECG_CELL_SEED_MINB : ECG_
   const BatchItem I = B.items[blockIdx.x];
   const BatchCase& C = B.cases[I.c];
   const int c = I.c, g = I.first + (int)threadIdx.x;
-  const bool own = g < I.n;
+  const bool own = g < I.end;
   const int64_t cell = I.off + g;
   __shared__ double ue[2][CELL_THREADS];  // the time-n u and E, copied ahead
   CellCounters cc;
@@ -381,6 +381,12 @@ static cudaError_t batch_launch(int np, int tb, int pass, const BatchParams& B, 
 
 using namespace ecg;
 
+// The items of a part of the batch whose face fluxes fit the flux array: a pass runs its face kernel and its cell
+// kernel piece by piece.
+struct BatchPiece {
+  int item0, nitems, citem0, ncitems;
+};
+
 struct ecg_batch {
   ecg_case c0;
   bool fast = false;  // kernels with the EOS types compiled in apply
@@ -399,10 +405,10 @@ struct ecg_batch {
   double* dummy_dt = nullptr;
   DevStats* stats = nullptr;
   double* flux = nullptr;   // face fluxes, 3N + 4 per face
-  int64_t nfaces = 0;
-  BatchItem* items = nullptr;   // face items of the current tile
-  BatchItem* citems = nullptr;  // cell items
-  int nitems = 0, ncitems = 0;
+  int64_t nfaces = 0;       // faces it holds: all of them where memory allows
+  BatchItem* items = nullptr;   // face items of the current tile, piece after piece
+  BatchItem* citems = nullptr;  // cell items, piece after piece
+  std::vector<BatchPiece> pieces;
   int tile = 0;
   int cur = 0;
   int newton_cap = 100;
@@ -430,19 +436,75 @@ void drop_graphs(ecg_batch* b) {
     }
 }
 
-// (case, first entry) of every chunk of `chunk` of each case's n + extra entries
-ecg_status build_items(const ecg_batch* b, int chunk, int extra, BatchItem** out, int* count) {
-  std::vector<BatchItem> it;
-  for (int c = 0; c < b->ncases; c++) {
-    const BatchCase& h = b->hcases[c];
-    for (int s = 0; s < h.n + extra; s += chunk) it.push_back({c, s, h.n, 0, h.off, h.fbase});
-  }
-  cudaFree(*out);
-  *out = nullptr;
+ecg_status upload_items(const std::vector<BatchItem>& it, BatchItem** out) {
   BCUDA(cudaMalloc(out, sizeof(BatchItem) * it.size()));
   BCUDA(cudaMemcpy(*out, it.data(), sizeof(BatchItem) * it.size(), cudaMemcpyHostToDevice));
-  *count = (int)it.size();
   return ECG_OK;
+}
+
+// Lays the batch out in pieces of at most nfaces faces: runs of whole cases, a case that does not fit the rest of a
+// piece cut at a multiple of CELL_THREADS cells.  The face at a cut belongs to both pieces (its flux and its wave
+// speed are computed twice, to the same values).
+ecg_status build_items(ecg_batch* b, int tile) {
+  std::vector<BatchItem> it, ct;
+  std::vector<BatchPiece> pieces;
+  BatchPiece p{0, 0, 0, 0};
+  int64_t used = 0;  // faces of the current piece
+  auto close = [&] {
+    p.nitems = (int)it.size() - p.item0;
+    p.ncitems = (int)ct.size() - p.citem0;
+    if (p.ncitems) pieces.push_back(p);
+    p = {(int)it.size(), 0, (int)ct.size(), 0};
+    used = 0;
+  };
+  for (int c = 0; c < b->ncases; c++) {
+    const BatchCase& h = b->hcases[c];
+    for (int s = 0; s < h.n;) {
+      int64_t m = std::min<int64_t>(h.n - s, b->nfaces - used - 1);  // cells from s on whose faces fit
+      if (m < h.n - s) m -= m % CELL_THREADS;
+      if (m <= 0) {
+        close();
+        continue;
+      }
+      const int e = s + (int)m;
+      const int64_t fbase = used - s;
+      for (int f = s; f <= e; f += tile - 1) it.push_back({c, f, h.n, e, h.off, fbase});
+      for (int g = s; g < e; g += CELL_THREADS) ct.push_back({c, g, h.n, e, h.off, fbase});
+      used += m + 1;
+      s = e;
+    }
+  }
+  close();
+  cudaFree(b->items);
+  cudaFree(b->citems);
+  b->items = b->citems = nullptr;
+  b->pieces.clear();
+  ecg_status st = upload_items(it, &b->items);
+  if (st == ECG_OK) st = upload_items(ct, &b->citems);
+  if (st == ECG_OK) b->pieces = pieces;
+  return st;
+}
+
+// The flux array for all faces of the batch or, where they do not fit the GPU's free memory, for as many as leave as
+// much again for the rest (a two-phase MUSCL batch: 21 doubles per cell and 10 per face).
+cudaError_t alloc_flux(ecg_batch* b) {
+  auto alloc = [&](int64_t faces) {
+    const cudaError_t e = cudaMalloc(&b->flux, sizeof(double) * (size_t)(3 * b->np + 4) * (size_t)faces);
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // the launches to come do not report it
+      b->flux = nullptr;
+    }
+    b->nfaces = faces;
+    return e;
+  };
+  int64_t faces = b->total + b->ncases;
+  cudaError_t e = alloc(faces);
+  if (e != cudaErrorMemoryAllocation) return e;
+  constexpr int64_t kLeast = 1 << 14;
+  while (e == cudaErrorMemoryAllocation && faces > 2 * kLeast) e = alloc(faces /= 2);
+  if (e != cudaSuccess) return e;
+  cudaFree(b->flux);
+  return alloc(faces / 2);
 }
 
 ecg_status set_shape(ecg_batch* b, int tile) {
@@ -455,7 +517,7 @@ ecg_status set_shape(ecg_batch* b, int tile) {
     BCUDA(batch_launch(b->np, tile, pass, B, b->c0.eos, b->eps, nullptr, 0, 0, b->stream, true, b->fast));
   b->tile = tile;
   drop_graphs(b);
-  return build_items(b, tile - 1, 1, &b->items, &b->nitems);
+  return build_items(b, tile);
 }
 
 ecg_status launch_pass(ecg_batch* b, int pass, double* q, double* sn, double* out) {
@@ -475,11 +537,17 @@ ecg_status launch_pass(ecg_batch* b, int pass, double* q, double* sn, double* ou
   B.P.mlp = b->mlp;
   B.cases = b->cases;
   B.scal = b->scal;
-  B.items = b->items;
   B.flux = b->flux;
   B.nfaces = b->nfaces;
-  BCUDA(batch_launch(b->np, b->tile, pass, B, b->c0.eos, b->eps, b->citems, b->nitems, b->ncitems, b->stream, false,
-                     b->fast));
+  if (b->pieces.empty()) {
+    set_error("the batch's shape could not be set");
+    return ECG_ERR_INVALID;
+  }
+  for (const BatchPiece& p : b->pieces) {
+    B.items = b->items + p.item0;
+    BCUDA(batch_launch(b->np, b->tile, pass, B, b->c0.eos, b->eps, b->citems + p.citem0, p.nitems, p.ncitems, b->stream,
+                       false, b->fast));
+  }
   return ECG_OK;
 }
 
@@ -581,7 +649,6 @@ extern "C" ecg_status ecg_batch_create(const ecg_case* cs, int32_t ncases, ecg_b
     const ecg_case& x = cs[c];
     BatchCase h{};
     h.off = off;
-    h.fbase = off + c;  // n + 1 faces per case
     h.n = x.ncells[0];
     double dX = x.length[0] / (double)x.ncells[0], dY = x.length[1] / (double)x.ncells[1],
            dZ = x.length[2] / (double)x.ncells[2];
@@ -593,7 +660,6 @@ extern "C" ecg_status ecg_batch_create(const ecg_case* cs, int32_t ncases, ecg_b
     off += h.n;
   }
   b->total = off;
-  b->nfaces = off + ncases;
   auto fail = [&](ecg_status s) {
     ecg_batch_destroy(b);
     return s;
@@ -612,8 +678,7 @@ extern "C" ecg_status ecg_batch_create(const ecg_case* cs, int32_t ncases, ecg_b
   if ((e = cudaMalloc(&b->dummy_dtmax, sizeof(unsigned long long))) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
   if ((e = cudaMalloc(&b->dummy_dt, sizeof(double))) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
   if ((e = cudaMalloc(&b->stats, sizeof(DevStats))) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
-  if ((e = cudaMalloc(&b->flux, sizeof(double) * (size_t)(3 * b->np + 4) * (size_t)b->nfaces)) != cudaSuccess)
-    return fail(bfail(e, "cudaMalloc(face fluxes)"));
+  if ((e = alloc_flux(b)) != cudaSuccess) return fail(bfail(e, "cudaMalloc(face fluxes)"));
   cudaMemcpy(b->cases, b->hcases.data(), sizeof(BatchCase) * ncases, cudaMemcpyHostToDevice);
   std::vector<BatchScalars> hs(ncases);
   double big = 1.e10;
@@ -628,8 +693,7 @@ extern "C" ecg_status ecg_batch_create(const ecg_case* cs, int32_t ncases, ecg_b
   cudaMemset(b->stats, 0, sizeof(DevStats));
   cudaMemset(b->state[0], 0, sb);
   cudaMemset(b->state[1], 0, sb);
-  ecg_status s = build_items(b, CELL_THREADS, 0, &b->citems, &b->ncitems);
-  if (s == ECG_OK) s = set_shape(b, 128);
+  ecg_status s = set_shape(b, 128);
   if (s != ECG_OK) return fail(s);
   *out = b;
   return ECG_OK;
