@@ -251,7 +251,8 @@ void distance_tables(const ecg_case& c, const std::vector<double>* sz, const std
   }
 }
 
-ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
+// The parameters of a step from state[parity], less its passes' buffers and its end.
+StepParams step_params(const ecg_ctx* x, int parity) {
   StepParams P{};
   DevScalars* sc = x->scal + parity;
   P.done = &sc->done;
@@ -281,15 +282,34 @@ ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
   for (int a = 0; a < 3; a++) P.flux[a] = x->split ? x->flux[a] : nullptr;
   P.fstreams = x->fstreams.fork ? &x->fstreams : nullptr;
   P.fmaps = (x->split && x->staging == ECG_STAGING_TMA && x->fmaps.ok) ? &x->fmaps : nullptr;
+  return P;
+}
+
+// Launches one pass or, with prepare, configures the kernels it would launch.
+cudaError_t run_pass(const ecg_ctx* x, int pass, const StepParams& P, bool prepare) {
+  if (x->c.model == ECG_MODEL_EULER)
+    return euler_launch(x->dim, pass, P, x->geo, x->c.eos, x->eps, x->stream, prepare);
+  if (x->c.model == ECG_MODEL_PTUEQ) return ptueq_launch(x->dim, pass, P, x->geo, x->c.eos, x->stream, prepare);
+  return kapila_launch(x->np, x->dim, x->c.ptmu != 0, pass, P, x->geo, x->c.eos, x->eps, x->stream, prepare);
+}
+
+// Configures (dynamic shared memory) the kernels of the context's passes in its present form, with or without a
+// seed.  The first touch of a kernel loads it, so no other kernel is touched.  Measured (one B200, creation of the
+// first context of a process, ms; every variant of every pass configured / these): tube of 1000 cells 35.9 / 34.5,
+// p-T-mu 256^2 70 / 64, PTUEq 256^2 20.5 / 19.7.
+cudaError_t configure(const ecg_ctx* x) {
+  const StepParams P = step_params(x, 0);
+  if (x->c.order == 1) return run_pass(x, PASS_O1, P, true);
+  const cudaError_t e = run_pass(x, PASS_PRED, P, true);
+  return e == cudaSuccess ? run_pass(x, PASS_CORR, P, true) : e;
+}
+
+ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
+  StepParams P = step_params(x, parity);
+  DevScalars* sc = x->scal + parity;
   double* sn = x->state[parity];
   double* s1 = x->state[1 - parity];
-  const bool euler = x->c.model == ECG_MODEL_EULER;
-  const bool ptueq = x->c.model == ECG_MODEL_PTUEQ;
-  auto run = [&](int pass) -> cudaError_t {
-    if (euler) return euler_launch(x->dim, pass, P, x->geo, x->c.eos, x->eps, x->stream, false);
-    if (ptueq) return ptueq_launch(x->dim, pass, P, x->geo, x->c.eos, x->stream, false);
-    return kapila_launch(x->np, x->dim, x->c.ptmu != 0, pass, P, x->geo, x->c.eos, x->eps, x->stream, false);
-  };
+  auto run = [&](int pass) { return run_pass(x, pass, P, false); };
   cudaError_t e;
   P.chained = ev ? 0 : 1;
   const bool beside = !ev && x->split;
@@ -698,20 +718,13 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
   cudaMemset(x->stats, 0, sizeof(DevStats));
   e = make_split_form(x);  // last: what the fused kernels need has its memory by now
   if (e != cudaSuccess) return fail_free(cuda_fail(e, "face arrays"));
-  // kernel attributes (dynamic shared memory) for every pass of this case shape
-  for (int pass = 0; pass < 3; pass++) {
-    StepParams P{};
-    P.ntr = c->ntransports;
-    cudaError_t pe = euler   ? euler_launch(x->dim, pass, P, x->geo, c->eos, x->eps, x->stream, true)
-                     : ptueq ? ptueq_launch(x->dim, pass, P, x->geo, c->eos, x->stream, true)
-                             : kapila_launch(x->np, x->dim, c->ptmu != 0, pass, P, x->geo, c->eos, x->eps, x->stream, true);
-    if (pe == cudaErrorNotSupported) {
-      set_error("no kernel built for this model / phases / dimension");
-      ecg_destroy(x);
-      return ECG_ERR_UNSUPPORTED;
-    }
-    if (pe != cudaSuccess) return fail_free(cuda_fail(pe, "cudaFuncSetAttribute"));
+  e = configure(x);
+  if (e == cudaErrorNotSupported) {
+    set_error("no kernel built for this model / phases / dimension");
+    ecg_destroy(x);
+    return ECG_ERR_UNSUPPORTED;
   }
+  if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaFuncSetAttribute"));
   e = cudaStreamSynchronize(x->stream);
   if (e != cudaSuccess) return fail_free(cuda_fail(e, "create"));
   *out = x;
@@ -756,6 +769,7 @@ extern "C" ecg_status ecg_set_step_form(ecg_ctx* x, int32_t form) {
   if (form == ECG_FORM_SPLIT && !x->flux[0]) { set_error("no split form for this case (1D, transports, PTUEq with several limiters or THINC, a mesh beyond the face kernels' grids, or too little memory)"); return ECG_ERR_UNSUPPORTED; }
   x->split = form == ECG_FORM_SPLIT;
   x->graph_dirty = true;
+  ECG_CUDA(configure(x));
   return ECG_OK;
 }
 
@@ -1073,11 +1087,14 @@ extern "C" ecg_status ecg_set_seed_model(ecg_ctx* x, const ecg_mlp* m) {
   if (!m) {
     cudaFree(x->mlp);
     x->mlp = nullptr;
+    ECG_CUDA(configure(x));
     return ECG_OK;
   }
   if (x->c.model != ECG_MODEL_KAPILA) { set_error("the seed model applies to Kapila relaxation"); return ECG_ERR_UNSUPPORTED; }
   if (x->c.ntransports > 0) { set_error("the seeded kernels run without passive transports"); return ECG_ERR_UNSUPPORTED; }
-  return mlp_upload(m, x->np, x->c.ptmu != 0, &x->mlp, x->stream);
+  const ecg_status s = mlp_upload(m, x->np, x->c.ptmu != 0, &x->mlp, x->stream);
+  if (s == ECG_OK) ECG_CUDA(configure(x));
+  return s;
 }
 
 extern "C" ecg_status ecg_set_ptmu_warm_start(ecg_ctx* x, int32_t on) {

@@ -409,7 +409,7 @@ struct ecg_batch {
   BatchItem* items = nullptr;   // face items of the current tile, piece after piece
   BatchItem* citems = nullptr;  // cell items, piece after piece
   std::vector<BatchPiece> pieces;
-  int tile = 0;
+  int tile = 128;
   int cur = 0;
   int newton_cap = 100;
   MlpDev* mlp = nullptr;
@@ -513,8 +513,9 @@ ecg_status set_shape(ecg_batch* b, int tile) {
     return ECG_ERR_INVALID;
   }
   BatchParams B{};
-  for (int pass = 0; pass < 3; pass++)
-    BCUDA(batch_launch(b->np, tile, pass, B, b->c0.eos, b->eps, nullptr, 0, 0, b->stream, true, b->fast));
+  for (int pass : {PASS_O1, PASS_PRED, PASS_CORR})
+    if ((pass == PASS_O1) == (b->order == 1))
+      BCUDA(batch_launch(b->np, tile, pass, B, b->c0.eos, b->eps, nullptr, 0, 0, b->stream, true, b->fast));
   b->tile = tile;
   drop_graphs(b);
   return build_items(b, tile);
@@ -539,10 +540,6 @@ ecg_status launch_pass(ecg_batch* b, int pass, double* q, double* sn, double* ou
   B.scal = b->scal;
   B.flux = b->flux;
   B.nfaces = b->nfaces;
-  if (b->pieces.empty()) {
-    set_error("the batch's shape could not be set");
-    return ECG_ERR_INVALID;
-  }
   for (const BatchPiece& p : b->pieces) {
     B.items = b->items + p.item0;
     BCUDA(batch_launch(b->np, b->tile, pass, B, b->c0.eos, b->eps, b->citems + p.citem0, p.nitems, p.ncitems, b->stream,
@@ -568,6 +565,10 @@ ecg_status launch_step(ecg_batch* b, int parity) {
 }
 
 ecg_status advance(ecg_batch* b, int nsteps) {
+  if (b->pieces.empty()) {  // no shape asked for yet
+    const ecg_status s = set_shape(b, b->tile);
+    if (s != ECG_OK) return s;
+  }
   while (nsteps >= 2) {
     if (!b->graph[b->cur]) {
       cudaGraph_t g = nullptr;
@@ -693,8 +694,6 @@ extern "C" ecg_status ecg_batch_create(const ecg_case* cs, int32_t ncases, ecg_b
   cudaMemset(b->stats, 0, sizeof(DevStats));
   cudaMemset(b->state[0], 0, sb);
   cudaMemset(b->state[1], 0, sb);
-  ecg_status s = set_shape(b, 128);
-  if (s != ECG_OK) return fail(s);
   *out = b;
   return ECG_OK;
 }

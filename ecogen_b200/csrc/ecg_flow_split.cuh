@@ -298,18 +298,11 @@ cudaError_t flow_pass(int pass, const StepParams& P, const Geometry& G, const ty
                       bool prepare) {
   const bool vl = P.lim[0] == ECG_LIM_VANLEER;  // the limiter of the shipped workloads, compiled in
   if (pass == PASS_O1) return launch_flow<MD, DIM, PASS_O1, -1>(P, G, M, s, prepare);
-  if (pass == PASS_PRED) {
-    if (prepare || vl) {
-      const cudaError_t e = launch_flow<MD, DIM, PASS_PRED, ECG_LIM_VANLEER>(P, G, M, s, prepare);
-      if (!prepare || e != cudaSuccess) return e;
-    }
-    return launch_flow<MD, DIM, PASS_PRED, -1>(P, G, M, s, prepare);
-  }
-  if (prepare || vl) {
-    const cudaError_t e = launch_flow<MD, DIM, PASS_CORR, ECG_LIM_VANLEER>(P, G, M, s, prepare);
-    if (!prepare || e != cudaSuccess) return e;
-  }
-  return launch_flow<MD, DIM, PASS_CORR, -1>(P, G, M, s, prepare);
+  if (pass == PASS_PRED)
+    return vl ? launch_flow<MD, DIM, PASS_PRED, ECG_LIM_VANLEER>(P, G, M, s, prepare)
+              : launch_flow<MD, DIM, PASS_PRED, -1>(P, G, M, s, prepare);
+  return vl ? launch_flow<MD, DIM, PASS_CORR, ECG_LIM_VANLEER>(P, G, M, s, prepare)
+            : launch_flow<MD, DIM, PASS_CORR, -1>(P, G, M, s, prepare);
 }
 
 }  // namespace ecg

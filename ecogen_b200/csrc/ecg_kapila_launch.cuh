@@ -26,18 +26,13 @@ cudaError_t launch_one(const StepParams& P, const Geometry& G, const ecg_eos* eo
 
 // One pass of one kernel variant: the split form (face kernels + cell kernel) for 2D and 3D cases whose
 // context holds face arrays, the fused kernel otherwise (1D, passive transports, the allocation-free
-// entry point).  With prepare both forms are configured.
+// entry point).  With prepare that form is configured.
 template <int NP, int DIM, int PASS, bool PTMU, bool SEED, int TYPES, int NTM>
 cudaError_t launch_form(const StepParams& P, const Geometry& G, const ecg_eos* eos, double eps, cudaStream_t s,
                         bool prepare) {
   constexpr bool kSplit = DIM >= 2 && NTM == 0;
-  if (prepare) {
-    cudaError_t e = launch_one<NP, DIM, PASS, PTMU, SEED, TYPES, NTM>(P, G, eos, eps, s, true);
-    if (kSplit && e == cudaSuccess) e = launch_split<NP, DIM, PASS, PTMU, SEED, TYPES>(P, G, eos, eps, s, true);
-    return e;
-  }
-  if (kSplit && P.flux[0] != nullptr) return launch_split<NP, DIM, PASS, PTMU, SEED, TYPES>(P, G, eos, eps, s, false);
-  return launch_one<NP, DIM, PASS, PTMU, SEED, TYPES, NTM>(P, G, eos, eps, s, false);
+  if (kSplit && P.flux[0] != nullptr) return launch_split<NP, DIM, PASS, PTMU, SEED, TYPES>(P, G, eos, eps, s, prepare);
+  return launch_one<NP, DIM, PASS, PTMU, SEED, TYPES, NTM>(P, G, eos, eps, s, prepare);
 }
 
 template <int NP, int DIM, bool PTMU, bool SEED, int TYPES = EOS_DYNAMIC, int NTM = 0>
@@ -85,7 +80,7 @@ template <int NP, int DIM, bool PTMU>
 cudaError_t launch_pass(int pass, const StepParams& P, const Geometry& G, const ecg_eos* eos, double eps,
                                cudaStream_t s, bool prepare) {
   // kernels with the learned seed are separate variants, so that the plain kernels carry none of
-  // its registers; with prepare both are configured
+  // its registers
 #ifndef ECG_NO_EOS_SPECIALIZATION
   constexpr bool kFast = true;
 #else
@@ -98,29 +93,25 @@ cudaError_t launch_pass(int pass, const StepParams& P, const Geometry& G, const 
   // EOS types compiled in (limiters at run time), and EOS types plus the workload's limiter
   constexpr int kEos = kFast ? fast_code(workload_types<NP, PTMU>(), -1) : EOS_DYNAMIC;
   constexpr int kEosLim = kFast ? fast_code(workload_types<NP, PTMU>(), eos_fast_limiter<NP>()) : EOS_DYNAMIC;
-  if (prepare) {
+  if (prepare && P.prepare_all) {
     cudaError_t e = launch_pass_seed<NP, DIM, PTMU, false>(pass, P, G, eos, eps, s, true);
     if (e == cudaSuccess && kFast) e = launch_pass_seed<NP, DIM, PTMU, false, kEos>(pass, P, G, eos, eps, s, true);
     if (e == cudaSuccess && kFast) e = launch_pass_seed<NP, DIM, PTMU, false, kEosLim>(pass, P, G, eos, eps, s, true);
-    if (e != cudaSuccess) return e;
-    e = launch_pass_seed<NP, DIM, PTMU, true>(pass, P, G, eos, eps, s, true);
-    if (e == cudaSuccess && kFast) e = launch_pass_seed<NP, DIM, PTMU, true, kEos>(pass, P, G, eos, eps, s, true);
-    if (e == cudaSuccess && kFast) e = launch_pass_seed<NP, DIM, PTMU, true, kEosLim>(pass, P, G, eos, eps, s, true);
     return e;
   }
   const bool fast_eos = kFast && !P.thinc && !P.pt && eos_is_fast<NP, PTMU>(eos);
   const int L = eos_fast_limiter<NP>();
   const bool fast_lim = P.lim[0] == L && P.lim[1] == L && P.lim[2] == L && P.lim[3] == L;
   if (P.mlp != nullptr) {  // the seeded kernels get the same compile-time configurations as the plain ones
-    if (fast_eos && fast_lim) return launch_pass_seed<NP, DIM, PTMU, true, kEosLim>(pass, P, G, eos, eps, s, false);
-    if (fast_eos) return launch_pass_seed<NP, DIM, PTMU, true, kEos>(pass, P, G, eos, eps, s, false);
-    return launch_pass_seed<NP, DIM, PTMU, true>(pass, P, G, eos, eps, s, false);
+    if (fast_eos && fast_lim) return launch_pass_seed<NP, DIM, PTMU, true, kEosLim>(pass, P, G, eos, eps, s, prepare);
+    if (fast_eos) return launch_pass_seed<NP, DIM, PTMU, true, kEos>(pass, P, G, eos, eps, s, prepare);
+    return launch_pass_seed<NP, DIM, PTMU, true>(pass, P, G, eos, eps, s, prepare);
   }
   if (fast_eos) {
-    if (fast_lim) return launch_pass_seed<NP, DIM, PTMU, false, kEosLim>(pass, P, G, eos, eps, s, false);
-    return launch_pass_seed<NP, DIM, PTMU, false, kEos>(pass, P, G, eos, eps, s, false);
+    if (fast_lim) return launch_pass_seed<NP, DIM, PTMU, false, kEosLim>(pass, P, G, eos, eps, s, prepare);
+    return launch_pass_seed<NP, DIM, PTMU, false, kEos>(pass, P, G, eos, eps, s, prepare);
   }
-  return launch_pass_seed<NP, DIM, PTMU, false>(pass, P, G, eos, eps, s, false);
+  return launch_pass_seed<NP, DIM, PTMU, false>(pass, P, G, eos, eps, s, prepare);
 }
 
 

@@ -205,6 +205,7 @@ extern "C" ecg_status ecg_step_noalloc(const ecg_case* c, const double* state_in
     if (euler) return euler_launch(dim, pass, P, G, c->eos, eps, s, prepare);
     return kapila_launch(c->nphases, dim, c->ptmu != 0, pass, P, G, c->eos, eps, s, prepare);
   };
+  P.prepare_all = 1;
   for (int pass = 0; pass < 3; pass++) {
     cudaError_t e = run(pass, true);
     if (e == cudaErrorNotSupported) {

@@ -172,6 +172,9 @@ struct StepParams {
   const struct FaceStreams* fstreams;  // auxiliary streams of the face kernels (nullptr: one after another)
   // host side: tensor maps of the face kernels' TMA staging (nullptr: the kernels load their tiles)
   const struct FaceMaps* fmaps;
+  // host side, with prepare: every EOS and limiter variant is configured, not only this case's (the allocation-free
+  // entry point, whose first call loads what later calls of other cases run)
+  int prepare_all;
 };
 
 // Host side of the THINC parameters (CellInterfaceO2Cartesian::solveRiemann's beta = 1.6).

@@ -565,12 +565,7 @@ static cudaError_t euler_dim(int pass, const StepParams& P, const Geometry& G, c
   if (P.ntr > 0) return euler_dim_tr<DIM, 2>(pass, P, G, eos, eps, s, prepare);  // up to two passive transports
   if constexpr (DIM >= 2) {
     const EulerFlow::Eos M{make_eos_params(eos[0]), eps};
-    if (prepare) {
-      const cudaError_t e = flow_pass<EulerFlow, DIM>(pass, P, G, M, s, true);
-      if (e != cudaSuccess) return e;
-    } else if (P.flux[0] != nullptr) {
-      return flow_pass<EulerFlow, DIM>(pass, P, G, M, s, false);
-    }
+    if (P.flux[0] != nullptr) return flow_pass<EulerFlow, DIM>(pass, P, G, M, s, prepare);
   }
   return euler_dim_tr<DIM, 0>(pass, P, G, eos, eps, s, prepare);
 }

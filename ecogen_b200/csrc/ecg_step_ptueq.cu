@@ -571,12 +571,7 @@ static cudaError_t ptueq_dim(int pass, const StepParams& P, const Geometry& G, c
   if constexpr (DIM >= 2) {
     PtEos M;
     for (int k = 0; k < 2; k++) M.e[k] = make_eos_params(eos[k]);
-    if (prepare) {
-      const cudaError_t e = flow_pass<PtFlow, DIM>(pass, P, G, M, s, true);
-      if (e != cudaSuccess) return e;
-    } else if (P.flux[0] != nullptr) {
-      return flow_pass<PtFlow, DIM>(pass, P, G, M, s, false);
-    }
+    if (P.flux[0] != nullptr) return flow_pass<PtFlow, DIM>(pass, P, G, M, s, prepare);
   }
   if (pass == PASS_O1) return ptueq_one<DIM, PASS_O1>(P, G, eos, s, prepare);
   if (pass == PASS_PRED) return ptueq_one<DIM, PASS_PRED>(P, G, eos, s, prepare);

@@ -85,3 +85,26 @@ def test_cases_that_run_fused_only_say_so(transports, tmp_path):
     with pytest.raises(api.EcgError):
         ctx.set_step_form(api.FORM_SPLIT)
     ctx.close()
+
+
+def test_kernels_are_configured_whatever_the_order_of_settings(tmp_path):
+    """A context configures the kernels of its present form and seed: every combination of the two, reached in either
+    order, steps and gives the plain split form's bits where no seed is installed."""
+    from ecogen_b200 import seed as seedmod
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    model = seedmod.SeedModel.load(os.path.join(root, "ecogen_b200", "models", "seed_np3.npz"))
+    spec = cases.cavity_collapse_3d(n=14, iterations=6, ninclusions=3, radius_cells=(2.0, 4.0))
+    ctx, f = _context(spec, tmp_path)
+    ref = _six(ctx, f)
+    model.install(ctx)
+    ctx.set_step_form(api.FORM_FUSED)
+    seeded = _six(ctx, f)
+    ctx.set_seed_model(None)
+    _same(ref, _six(ctx, f))
+    model.install(ctx)
+    ctx.set_step_form(api.FORM_SPLIT)
+    _same(seeded, _six(ctx, f))
+    ctx.set_seed_model(None)
+    ctx.set_step_form(api.FORM_FUSED)
+    _same(ref, _six(ctx, f))
+    ctx.close()
