@@ -100,6 +100,13 @@ __global__ void k_euler_derived(const double* __restrict__ S, int64_t n, ecg_eos
 
 using namespace ecg;
 
+// The small device data of a context.
+struct DevBlock {
+  DevScalars scal[2];                   // by state parity
+  alignas(128) DevStats stats;          // (cache lines of their own: different kernels' atomics)
+  alignas(128) unsigned int fin_count;  // blocks done of the fused pass that ends a step
+};
+
 struct ecg_ctx {
   ecg_case c;
   int dim = 1, np = 2, nstate = 0, nq = 0;
@@ -111,19 +118,15 @@ struct ecg_ctx {
   double* half = nullptr;     // MUSCL half-step primitives
   double* dist = nullptr;     // distance tables (3 axes x 3 tables)
   double* tmp = nullptr;      // download scratch (mixture pressure)
-  double* flux[3] = {nullptr, nullptr, nullptr};  // face arrays of the split form (2D / 3D)
+  double* flux[3] = {nullptr, nullptr, nullptr};  // face arrays of the split form (2D / 3D), one allocation
   bool split = false;         // step passes in split form (face kernels + cell kernel)
   FaceStreams fstreams{};     // auxiliary streams of the face kernels (split forms)
   FaceMaps fmaps{};           // tensor maps of the face kernels' TMA staging (fmaps.ok = 0: none)
   int staging = ECG_STAGING_TMA;
-  DevScalars* scal = nullptr;      // two, by state parity (DevScalars)
-  unsigned int* fin_count = nullptr;  // blocks done of the fused pass that ends a step
+  DevBlock* dev = nullptr;
   StepEnd step_end[2]{};           // the end of the steps from state[0] / state[1] (split forms)
-  DevStats* stats = nullptr;
-  // pinned host staging of the scalars and counters an ecg_step call exchanges (asynchronous copies,
-  // one synchronisation per call)
-  DevScalars* h_scal = nullptr;
-  DevStats* h_stats = nullptr;
+  DevBlock* host = nullptr;  // pinned staging of the scalars and counters an ecg_step call exchanges (asynchronous
+                             // copies, one synchronisation per call)
   int cur = 0;
   int newton_cap = 100;
   int newton_accept = 0;
@@ -254,12 +257,12 @@ void distance_tables(const ecg_case& c, const std::vector<double>* sz, const std
 // The parameters of a step from state[parity], less its passes' buffers and its end.
 StepParams step_params(const ecg_ctx* x, int parity) {
   StepParams P{};
-  DevScalars* sc = x->scal + parity;
+  DevScalars* sc = x->dev->scal + parity;
   P.done = &sc->done;
   P.n = x->n;
   P.dt = &sc->dt;
   P.dtmax_bits = &sc->dtmax_bits;
-  P.stats = x->stats;
+  P.stats = &x->dev->stats;
   for (int i = 0; i < 4; i++) P.lim[i] = x->c.limiter[i];
   P.newton_cap = x->newton_cap;
   P.newton_accept = x->newton_accept;
@@ -306,7 +309,7 @@ cudaError_t configure(const ecg_ctx* x) {
 
 ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
   StepParams P = step_params(x, parity);
-  DevScalars* sc = x->scal + parity;
+  DevScalars* sc = x->dev->scal + parity;
   double* sn = x->state[parity];
   double* s1 = x->state[1 - parity];
   auto run = [&](int pass) { return run_pass(x, pass, P, false); };
@@ -320,8 +323,8 @@ ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
       P.end = &x->step_end[parity];
     } else {
       P.fin_from = sc;
-      P.fin_to = x->scal + (1 - parity);
-      P.fin_count = x->fin_count;
+      P.fin_to = x->dev->scal + (1 - parity);
+      P.fin_count = &x->dev->fin_count;
     }
   };
   if (ev) cudaEventRecord(ev[0], x->stream);
@@ -351,7 +354,7 @@ ecg_status launch_step(ecg_ctx* x, int parity, cudaEvent_t* ev = nullptr) {
   }
   if (ev) cudaEventRecord(ev[2], x->stream);
   if (ev) {
-    e = launch_step_end(sc, x->scal + (1 - parity), x->stream);
+    e = launch_step_end(sc, x->dev->scal + (1 - parity), x->stream);
     if (e != cudaSuccess) return cuda_fail(e, "finalize kernel");
     cudaEventRecord(ev[3], x->stream);
   }
@@ -381,17 +384,16 @@ cudaError_t make_split_form(ecg_ctx* x) {
   // the flux components (Kapila 3N + d + 3, Euler d + 2, PTUEq d + 3) of every face of each axis, the domain
   // sides included
   const int nfl = euler ? x->dim + 2 : (ptueq ? x->dim + 3 : 3 * x->np + x->dim + 3);
-  cudaError_t e = cudaSuccess;
-  for (int a = 0; a < x->dim && e == cudaSuccess; a++)
-    e = cudaMalloc(&x->flux[a], sizeof(double) * (size_t)nfl * (size_t)split_nfaces(c.ncells, a));
+  size_t at[4] = {0, 0, 0, 0};  // each axis' array on a 256-byte boundary
+  for (int a = 0; a < x->dim; a++) at[a + 1] = at[a] + ((size_t)nfl * (size_t)split_nfaces(c.ncells, a) + 31) / 32 * 32;
+  double* mem = nullptr;
+  cudaError_t e = cudaMalloc(&mem, sizeof(double) * at[x->dim]);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();  // the launches to come do not report it
-    for (int a = 0; a < x->dim; a++) {
-      cudaFree(x->flux[a]);
-      x->flux[a] = nullptr;
-    }
     return cudaSuccess;
   }
+  if (e != cudaSuccess) return e;
+  for (int a = 0; a < x->dim; a++) x->flux[a] = mem + at[a];
   for (int a = 0; a + 1 < x->dim && e == cudaSuccess; a++) {
     e = cudaStreamCreateWithFlags(&x->fstreams.s[a], cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->fstreams.join[a], cudaEventDisableTiming);
@@ -400,7 +402,7 @@ cudaError_t make_split_form(ecg_ctx* x) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
   if (e != cudaSuccess) return e;
   for (int i = 0; i < 2; i++)
-    x->step_end[i] = {x->scal + i, x->scal + (1 - i), x->fstreams.s[0], x->fstreams.end_fork, x->fstreams.end_join};
+    x->step_end[i] = {x->dev->scal + i, x->dev->scal + (1 - i), x->fstreams.s[0], x->fstreams.end_fork, x->fstreams.end_join};
 #ifndef ECG_BOUNDS_CHECK
   // TMA staging of the face kernels' tiles where the layout allows it (the bounds-checked build
   // checks the kernels' own loads, so it stages them that way).  Staged planes: all but E, which the
@@ -700,22 +702,18 @@ extern "C" ecg_status ecg_create(const ecg_case* c, ecg_ctx** out) {
     pc /= (L.gamma - 1.) * L.cv - (V.gamma - 1.) * V.cv;
     x->pcrit = pc;
   }
-  e = cudaMalloc(&x->scal, 2 * sizeof(DevScalars));
+  e = cudaMalloc(&x->dev, sizeof(DevBlock));
+  if (e == cudaSuccess) e = cudaMallocHost(&x->host, sizeof(DevBlock));
   if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaMalloc(scalars)"));
-  e = cudaMalloc(&x->stats, sizeof(DevStats));
-  if (e == cudaSuccess) e = cudaMalloc(&x->fin_count, sizeof(unsigned int));
-  if (e == cudaSuccess) e = cudaMemset(x->fin_count, 0, sizeof(unsigned int));
-  if (e == cudaSuccess) e = cudaMallocHost(&x->h_scal, 2 * sizeof(DevScalars));
-  if (e == cudaSuccess) e = cudaMallocHost(&x->h_stats, sizeof(DevStats));
-  if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaMalloc(stats)"));
-  DevScalars s0{};
+  std::memset(x->host, 0, sizeof(DevBlock));
+  DevScalars& s0 = x->host->scal[0];
   s0.dt = 1.e-15;
   s0.cfl = c->cfl;
-  s0.dtmax_bits = (unsigned long long)0;
-  double big = 1.e10;
+  const double big = 1.e10;
   std::memcpy(&s0.dtmax_bits, &big, sizeof(double));
-  for (int i = 0; i < 2; i++) cudaMemcpy(x->scal + i, &s0, sizeof(s0), cudaMemcpyHostToDevice);
-  cudaMemset(x->stats, 0, sizeof(DevStats));
+  x->host->scal[1] = s0;
+  e = cudaMemcpyAsync(x->dev, x->host, sizeof(DevBlock), cudaMemcpyHostToDevice, x->stream);
+  if (e != cudaSuccess) return fail_free(cuda_fail(e, "cudaMemcpy(scalars)"));
   e = make_split_form(x);  // last: what the fused kernels need has its memory by now
   if (e != cudaSuccess) return fail_free(cuda_fail(e, "face arrays"));
   e = configure(x);
@@ -740,12 +738,9 @@ extern "C" void ecg_destroy(ecg_ctx* x) {
   cudaFree(x->half);
   cudaFree(x->dist);
   cudaFree(x->tmp);
-  for (int a = 0; a < 3; a++) cudaFree(x->flux[a]);
-  cudaFree(x->scal);
-  cudaFree(x->fin_count);
-  cudaFree(x->stats);
-  cudaFreeHost(x->h_scal);
-  cudaFreeHost(x->h_stats);
+  cudaFree(x->flux[0]);
+  cudaFree(x->dev);
+  cudaFreeHost(x->host);
   cudaFree(x->mlp);
   cudaFree(x->rec_x);
   cudaFree(x->rec_y);
@@ -976,9 +971,9 @@ static ecg_status step_common(ecg_ctx* x, int mode, int32_t nsteps, double* dt, 
   h.mode = mode;
   h.done = (mode == 1 && h.it >= h.max_it) || (mode == 2 && h.t >= h.t_end);
   // the previous call synchronised, so the staging buffer is free; both parities' scalars start from the caller's
-  x->h_scal[0] = x->h_scal[1] = h;
-  ECG_CUDA(cudaMemcpyAsync(x->scal, x->h_scal, 2 * sizeof(h), cudaMemcpyHostToDevice, x->stream));
-  ECG_CUDA(cudaMemsetAsync(x->stats, 0, sizeof(DevStats), x->stream));
+  x->host->scal[0] = x->host->scal[1] = h;
+  ECG_CUDA(cudaMemcpyAsync(x->dev->scal, x->host->scal, 2 * sizeof(h), cudaMemcpyHostToDevice, x->stream));
+  ECG_CUDA(cudaMemsetAsync(&x->dev->stats, 0, sizeof(DevStats), x->stream));
   const int cur0 = x->cur;  // a step that finds the stop flag set writes nothing, so the state that
                             // holds the result is decided by the number of steps actually taken
   int64_t done_steps = 0;
@@ -1031,17 +1026,17 @@ static ecg_status step_common(ecg_ctx* x, int mode, int32_t nsteps, double* dt, 
       ecg_status s = advance(x, chunk);
       if (s != ECG_OK) return s;
       DevScalars r{};
-      ECG_CUDA(cudaMemcpyAsync(&r, x->scal + x->cur, sizeof(r), cudaMemcpyDeviceToHost, x->stream));
+      ECG_CUDA(cudaMemcpyAsync(&r, x->dev->scal + x->cur, sizeof(r), cudaMemcpyDeviceToHost, x->stream));
       ECG_CUDA(cudaStreamSynchronize(x->stream));
       if (r.done) break;
     }
   }
   // x->cur: the parity after the launched steps, whose scalars the last one wrote
-  ECG_CUDA(cudaMemcpyAsync(x->h_scal, x->scal + x->cur, sizeof(DevScalars), cudaMemcpyDeviceToHost, x->stream));
-  ECG_CUDA(cudaMemcpyAsync(x->h_stats, x->stats, sizeof(DevStats), cudaMemcpyDeviceToHost, x->stream));
+  ECG_CUDA(cudaMemcpyAsync(x->host->scal, x->dev->scal + x->cur, sizeof(DevScalars), cudaMemcpyDeviceToHost, x->stream));
+  ECG_CUDA(cudaMemcpyAsync(&x->host->stats, &x->dev->stats, sizeof(DevStats), cudaMemcpyDeviceToHost, x->stream));
   ECG_CUDA(cudaStreamSynchronize(x->stream));
-  const DevScalars r = *x->h_scal;
-  const DevStats ds = *x->h_stats;
+  const DevScalars r = x->host->scal[0];
+  const DevStats ds = x->host->stats;
   done_steps = r.it - h.it;
   x->cur = cur0 ^ (int)(done_steps & 1);
   *dt = r.dt;

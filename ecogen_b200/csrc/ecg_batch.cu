@@ -400,9 +400,6 @@ struct ecg_batch {
   double* state[2] = {nullptr, nullptr};
   double* half = nullptr;
   double* tmp = nullptr;
-  int* done = nullptr;
-  unsigned long long* dummy_dtmax = nullptr;
-  double* dummy_dt = nullptr;
   DevStats* stats = nullptr;
   double* flux = nullptr;   // face fluxes, 3N + 4 per face
   int64_t nfaces = 0;       // faces it holds: all of them where memory allows
@@ -523,13 +520,10 @@ ecg_status set_shape(ecg_batch* b, int tile) {
 
 ecg_status launch_pass(ecg_batch* b, int pass, double* q, double* sn, double* out) {
   BatchParams B{};
-  B.P.done = b->done;
   B.P.q = q;
   B.P.sn = sn;
   B.P.out = out;
   B.P.n = b->total;
-  B.P.dt = b->dummy_dt;
-  B.P.dtmax_bits = b->dummy_dtmax;
   B.P.stats = b->stats;
   for (int i = 0; i < 4; i++) B.P.lim[i] = b->c0.limiter[i];
   B.P.newton_cap = b->newton_cap;
@@ -675,9 +669,6 @@ extern "C" ecg_status ecg_batch_create(const ecg_case* cs, int32_t ncases, ecg_b
   if ((e = cudaMalloc(&b->tmp, sizeof(double) * (size_t)b->total)) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
   if ((e = cudaMalloc(&b->cases, sizeof(BatchCase) * ncases)) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
   if ((e = cudaMalloc(&b->scal, sizeof(BatchScalars) * ncases)) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
-  if ((e = cudaMalloc(&b->done, sizeof(int))) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
-  if ((e = cudaMalloc(&b->dummy_dtmax, sizeof(unsigned long long))) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
-  if ((e = cudaMalloc(&b->dummy_dt, sizeof(double))) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
   if ((e = cudaMalloc(&b->stats, sizeof(DevStats))) != cudaSuccess) return fail(bfail(e, "cudaMalloc"));
   if ((e = alloc_flux(b)) != cudaSuccess) return fail(bfail(e, "cudaMalloc(face fluxes)"));
   cudaMemcpy(b->cases, b->hcases.data(), sizeof(BatchCase) * ncases, cudaMemcpyHostToDevice);
@@ -690,10 +681,11 @@ extern "C" ecg_status ecg_batch_create(const ecg_case* cs, int32_t ncases, ecg_b
     s.it = 0;
   }
   cudaMemcpy(b->scal, hs.data(), sizeof(BatchScalars) * ncases, cudaMemcpyHostToDevice);
-  cudaMemset(b->done, 0, sizeof(int));
-  cudaMemset(b->stats, 0, sizeof(DevStats));
-  cudaMemset(b->state[0], 0, sb);
-  cudaMemset(b->state[1], 0, sb);
+  // ordered before the batch's work, which all runs on its stream
+  cudaMemsetAsync(b->stats, 0, sizeof(DevStats), b->stream);
+  cudaMemsetAsync(b->state[0], 0, sb, b->stream);
+  cudaMemsetAsync(b->state[1], 0, sb, b->stream);
+  if ((e = cudaStreamSynchronize(b->stream)) != cudaSuccess) return fail(bfail(e, "create"));
   *out = b;
   return ECG_OK;
 }
@@ -708,9 +700,6 @@ extern "C" void ecg_batch_destroy(ecg_batch* b) {
   cudaFree(b->tmp);
   cudaFree(b->cases);
   cudaFree(b->scal);
-  cudaFree(b->done);
-  cudaFree(b->dummy_dtmax);
-  cudaFree(b->dummy_dt);
   cudaFree(b->stats);
   cudaFree(b->flux);
   cudaFree(b->items);

@@ -52,7 +52,7 @@ def test_context_without_room_for_face_arrays_runs_fused(model, tmp_path):
     ctx.step(1)
     ctx.close()
     cells = n[0] * n[1] * n[2]
-    room = 0.6 * faces * 8 * cells  # the first face array fits, the last does not
+    room = 0.6 * faces * 8 * cells  # some of the face arrays would fit
     with Scarce(int(planes * 8 * cells + room)):
         ctx = api.Context(inp.case)
         assert ctx.step_form == api.FORM_FUSED
