@@ -1,7 +1,7 @@
 // Split form of an Euler or PTUEq step pass on 2D and 3D meshes: one face-flux kernel per axis, side by side,
 // then one cell kernel (see ecg_kapila_split.cuh, whose tiles, staging and face arrays these kernels
-// share; the reference lines of the physics stand at the functions they call, in ecg_step_euler.cu and
-// ecg_step_ptueq.cu, which include this file).
+// share; the reference lines of the physics stand at the functions they call, in ecg_euler.cuh and
+// ecg_ptueq.cuh, which include this file).
 //
 // A model M supplies: Eos (its parameters), Side (a completed face side), NM mass fluxes, U (the plane of the
 // first velocity; planes 0 .. U + DIM - 1 are the reconstructed fields, in the state's order), STORED (planes
