@@ -137,7 +137,7 @@ KERNEL_SLOTS = ["pass1_faces_x", "pass1_faces_y", "pass1_faces_z", "pass1_cells"
 GRAPH_AFTER = 32
 
 
-def warm(ctx, fields, warmup: int):
+def warm_up(ctx, fields, warmup: int):
     """The state `warmup` steps after `fields`, in a context whose graphs exist, so that a timed region holds neither
     their capture nor steps launched one by one."""
     ctx.upload(fields)
@@ -606,7 +606,7 @@ def main():
         return c
 
     ctx = new_context()
-    warm(ctx, fields0, args.warmup)
+    warm_up(ctx, fields0, args.warmup)
     stream = torch.cuda.ExternalStream(api.lib().ecg_stream(ctx.h))
 
     # ---- device-timed region: K steps replayed from captured graphs, events on the context stream
@@ -635,7 +635,7 @@ def main():
         ref_ctx.step(args.warmup)
         ctx3 = new_context()
         model.install(ctx3)
-        warm(ctx3, fields0, args.warmup)
+        warm_up(ctx3, fields0, args.warmup)
         stream3 = torch.cuda.ExternalStream(api.lib().ecg_stream(ctx3.h))
         torch.cuda.synchronize()
         s0, s1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -665,7 +665,7 @@ def main():
             ctx4 = new_context()
             model.install(ctx4)
             ctx4.set_ptmu_seed(api.PTMU_SEED_P_T)
-            warm(ctx4, fields0, args.warmup)
+            warm_up(ctx4, fields0, args.warmup)
             stream4 = torch.cuda.ExternalStream(api.lib().ecg_stream(ctx4.h))
             torch.cuda.synchronize()
             q0, q1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -694,7 +694,7 @@ def main():
                 cctx = new_context()
                 cctx.set_newton_cap(cap)
                 cctx.set_newton_cap_mode(api.CAP_ACCEPT)
-                warm(cctx, fields0, args.warmup)
+                warm_up(cctx, fields0, args.warmup)
                 cstream = torch.cuda.ExternalStream(api.lib().ecg_stream(cctx.h))
                 torch.cuda.synchronize()
                 c0, c1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -717,7 +717,7 @@ def main():
         ref_w.step(args.warmup)
         ctxw = new_context()
         ctxw.set_ptmu_warm_start(True)
-        warm(ctxw, fields0, args.warmup)
+        warm_up(ctxw, fields0, args.warmup)
         streamw = torch.cuda.ExternalStream(api.lib().ecg_stream(ctxw.h))
         torch.cuda.synchronize()
         w0, w1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

@@ -1,4 +1,4 @@
-"""The benchmark's warm-up (bench.warm) against the library's rule for graphs: the timed steps replay graphs that
+"""The benchmark's warm-up (bench.warm_up) against the library's rule for graphs: the timed steps replay graphs that
 exist, from the state the contract asks for."""
 import ctypes as C
 import os
@@ -40,7 +40,7 @@ class _Fake:
 @pytest.mark.parametrize("warmup", [0, 3, 4, 5, 50])
 def test_timed_steps_replay_existing_graphs(warmup):
     ctx = _Fake()
-    bench.warm(ctx, "fields", warmup)
+    bench.warm_up(ctx, "fields", warmup)
     assert ctx.since_upload == warmup and ctx.iteration == warmup and ctx.t.value == warmup
     assert (warmup == 0) == (ctx.dt.value == 1e-15)
     assert ctx.step(200) == (0, 0)
