@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(CELL_THREADS, SEED ? ECG_CELL_SEED_MINB : ECG_
   if (SEED) seed_gate<NP, 1>(P, M, own, cp, sg);
   if (own) kapila_finish<NP, 1, PASS, false, SEED, (TYPES == EOS_DYNAMIC)>(P, M, nn, cell, cp, sg, cc);
   // the per-bin histogram is not kept in batched mode (relax_calls / newton_evals / newton_max are)
-  block_counters(P.stats, cc.relax, cc.iters, cc.fallback, cc.seeded, cc.rejected, cc.nonfinite, 0u, cc.iters, false);
+  block_counters<CELL_THREADS>(P.stats, cc.relax, cc.iters, cc.fallback, cc.seeded, cc.rejected, cc.nonfinite, 0u, cc.iters, false);
 }
 
 __global__ void k_batch_finalize(BatchScalars* s, const BatchCase* cases, int ncases) {

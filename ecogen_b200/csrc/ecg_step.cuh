@@ -297,13 +297,16 @@ inline cudaError_t launch_chained(void (*kern)(KA...), dim3 grid, dim3 block, si
 // Measured, one instruction against one per counter (cell kernels, one B200): 2D 2048^2 0.325 / 0.335 -> 0.320 /
 // 0.326 ms, 3D 256^3 2.35 / 2.36 -> 2.30 / 2.31 ms, p-T-mu 1024^2 0.359 -> 0.347 ms (no atomics at all: 0.310 / 0.318,
 // 2.28 / 2.29, 0.347; cell blocks of 64 threads 0.338 / 0.390 and 2.47 ms with one per counter, of 32 0.70 and 4.39 ms).
-// Every thread of the block must call it.
+// Every thread of the block must call it; THREADS: the block's size.
+template <int THREADS>
 __device__ __forceinline__ void block_counters(DevStats* st, unsigned int relax, unsigned int iters,
                                                unsigned int fallback, unsigned int seeded, unsigned int rejected,
                                                unsigned int nonfinite, unsigned int ptmu, unsigned int max_iters,
                                                bool hist) {
-  __shared__ unsigned int sc[8][24];  // up to 256 threads
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = (int)(blockDim.x >> 5);
+  static_assert(THREADS % 32 == 0 && THREADS >= 32 && THREADS <= 1024, "whole warps");
+  constexpr int nw = THREADS / 32;
+  __shared__ unsigned int sc[nw][24];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned full = 0xffffffffu;
   const unsigned int nr = __reduce_add_sync(full, relax), ni = __reduce_add_sync(full, iters);
   const unsigned int mx = __reduce_max_sync(full, max_iters);
