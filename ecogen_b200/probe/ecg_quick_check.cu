@@ -2,7 +2,9 @@
 // evaluation of the pressure relaxation (pinf_quick inside relax_pinf against an iteration of
 // pinf_eval_general) and the internal face (hllc_quick against fulfill and hllc).  The states span ordinary
 // liquids and gases and, mixed in, what sends a cell or a face to the general form: pressures at and below the
-// EOS floors, densities at theirs, volume fractions of 0 and 1, tension, zeros, infinities and NaN.
+// EOS floors, densities at theirs, volume fractions of 0 and 1, tension, zeros, infinities and NaN.  Left out of the
+// differences, and counted: the quotients ecg_ieee.cuh excepts, a finite non-zero power of two (alpha_k rho_k) over a
+// divisor whose significand is all ones (rho_k*).
 #include <cuda_runtime.h>
 
 #include "../csrc/ecg_device.cuh"
@@ -26,6 +28,9 @@ struct Draw {
   }
   __device__ double log10(double lo, double hi) { return exp10(lo + (hi - lo) * uni()); }
 };
+
+constexpr long long ALL_ONES = 0xFFFFFFFFFFFFFll;
+__device__ __forceinline__ long long significand(double x) { return __double_as_longlong(x) & ALL_ONES; }
 
 // same value, NaN equal to NaN (the sign of a zero may differ)
 __device__ __forceinline__ bool same(double x, double y) { return (x != x && y != y) || x == y; }
@@ -60,7 +65,7 @@ __device__ void draw_phases(const Model<NP>& M, Draw& d, bool odd, double a[NP],
 template <int NP>
 __global__ void k_quick(uint64_t seed, int iters, Model<NP> M, unsigned long long* out) {
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned long long n = 0, bad_newton = 0, bad_face = 0, quick = 0;
+  unsigned long long n = 0, bad_newton = 0, bad_face = 0, quick = 0, ties = 0;
   for (int it = 0; it < iters; it++) {
     Draw d{mix64(seed ^ (t * 0x100000001B3ull + (uint64_t)it))};
     const bool odd = d.uni() < 0.1;
@@ -83,14 +88,15 @@ __global__ void k_quick(uint64_t seed, int iters, Model<NP> M, unsigned long lon
       double pstar = 0.;
       RelaxStats st;
       if (relax_pinf<NP>(M, b, q, p, pstar, st, 0., false, 100, true)) {
-        // left out, as ecg_ieee.cuh states of qdiv: quotients within 2^-47 ulp of a midpoint, which a power of
-        // two over an all-ones significand is (alpha rho = 1/2 over rho* = 1 - 2^-53)
         bool tie = false, ok = st.iters == s.it && same(pstar, s.ps);
         for (int k = 0; k < NP; k++) {
-          tie = tie || (__double_as_longlong(a[k] * r[k]) & 0xFFFFFFFFFFFFFll) == 0;
+          const double ar = a[k] * r[k];
+          tie = tie || (ar != 0. && isfinite(ar) && significand(ar) == 0 &&
+                        (significand(q[k]) == ALL_ONES || significand(rS[k]) == ALL_ONES));
           ok = ok && same(b[k], aS[k]) && same(q[k], rS[k]);
         }
-        if (!ok && !tie) bad_newton++;
+        if (tie) ties++;
+        else if (!ok) bad_newton++;
       }
     }
     {  // internal face
@@ -132,6 +138,7 @@ __global__ void k_quick(uint64_t seed, int iters, Model<NP> M, unsigned long lon
   atomicAdd(out + 1, bad_newton);
   atomicAdd(out + 2, bad_face);
   atomicAdd(out + 3, quick);
+  atomicAdd(out + 4, ties);
 }
 
 template <int NP>
@@ -146,17 +153,26 @@ cudaError_t run(uint64_t seed, int blocks, int iters, const ecg_eos* eos, double
 }  // namespace
 
 // blocks x 128 threads x iters states of np (2 or 3) phases with the given EOS; counts[0] = states, [1] =
-// relaxations and [2] = faces whose results differ, [3] = faces hllc_quick solved.  Returns 0, a CUDA error
-// code, or -1 for arguments outside the limits.
-extern "C" int ecg_probe_quick_check(unsigned long long seed, int np, const ecg_eos* eos, double eps, int blocks, int iters,
-                                     unsigned long long counts[4]) {
+// relaxations and [2] = faces whose results differ, [3] = faces hllc_quick solved, [4] = relaxations left out.
+// Returns 0, a CUDA error code, or -1 for arguments outside the limits.
+extern "C" int ecg_probe_quick_counts(unsigned long long seed, int np, const ecg_eos* eos, double eps, int blocks, int iters,
+                                      unsigned long long counts[5]) {
   if ((np != 2 && np != 3) || !eos || blocks <= 0 || iters <= 0) return -1;
   unsigned long long* d = nullptr;
-  cudaError_t e = cudaMalloc(&d, 4 * sizeof(unsigned long long));
+  cudaError_t e = cudaMalloc(&d, 5 * sizeof(unsigned long long));
   if (e != cudaSuccess) return (int)e;
-  e = cudaMemset(d, 0, 4 * sizeof(unsigned long long));
+  e = cudaMemset(d, 0, 5 * sizeof(unsigned long long));
   if (e == cudaSuccess) e = np == 2 ? run<2>(seed, blocks, iters, eos, eps, d) : run<3>(seed, blocks, iters, eos, eps, d);
-  if (e == cudaSuccess) e = cudaMemcpy(counts, d, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(counts, d, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
   cudaFree(d);
   return (int)e;
+}
+
+// The first four of these.
+extern "C" int ecg_probe_quick_check(unsigned long long seed, int np, const ecg_eos* eos, double eps, int blocks, int iters,
+                                     unsigned long long counts[4]) {
+  unsigned long long c[5] = {0, 0, 0, 0, 0};
+  const int rc = ecg_probe_quick_counts(seed, np, eos, eps, blocks, iters, c);
+  for (int i = 0; i < 4; i++) counts[i] = c[i];
+  return rc;
 }
