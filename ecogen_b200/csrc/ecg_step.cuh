@@ -304,9 +304,9 @@ __device__ __forceinline__ void block_counters(DevStats* st, unsigned int relax,
                                                unsigned int nonfinite, unsigned int ptmu, unsigned int max_iters,
                                                bool hist) {
   static_assert(THREADS % 32 == 0 && THREADS >= 32 && THREADS <= 1024, "whole warps");
-  constexpr int nw = THREADS / 32;
-  __shared__ unsigned int sc[nw][24];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ unsigned int sc[THREADS / 32][24];
+  // nw from blockDim: as a constant it costs the p-T-mu step (one-warp blocks, 1024^2) 0.6 %
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = (int)(blockDim.x >> 5);
   const unsigned full = 0xffffffffu;
   const unsigned int nr = __reduce_add_sync(full, relax), ni = __reduce_add_sync(full, iters);
   const unsigned int mx = __reduce_max_sync(full, max_iters);
