@@ -202,8 +202,8 @@ NCU_TRAFFIC_PER_CELL = {("kapila", 2, 2, True, "fused", "pass2_cells"): 190.96,
                         ("kapila_ptmu", 2, 2, True, "fused", "pass2_cells"): 181.05,
                         ("kapila_ptmu", 2, 2, True, "fused", "pass1_cells"): 112.08}
 # Split form: DRAM bytes per unit of the kernel (faces of its axis for a face kernel, cells for the cell
-# kernel), ncu on one launch at 1536^2 (2D two-phase), 128^3 (3D three-phase) and 1024^2 (p-T-mu); the
-# traffic of a launch grows with its units, so a full-size launch is the per-unit figure times its units.
+# kernel), ncu on one launch at 1536^2 (2D two-phase and PTUEq), 128^3 (3D three-phase), 1024^2 (p-T-mu) and
+# 2048^2 (Euler); the traffic of a launch grows with its units, so a full-size launch is the per-unit figure times its units.
 _SPLIT_NCU = {  # (model, phases, dim): {slot: (FP64 thread instructions per unit, DRAM bytes per unit)}
     ("kapila", 2, 2): {"pass1_faces_x": (595, 125), "pass1_faces_y": (601, 125), "pass1_cells": (420, 290),
                        "pass2_faces_x": (595, 126), "pass2_faces_y": (601, 125), "pass2_cells": (419, 297)},
@@ -212,12 +212,16 @@ _SPLIT_NCU = {  # (model, phases, dim): {slot: (FP64 thread instructions per uni
                        "pass2_faces_z": (815, 183), "pass2_cells": (760, 537)},
     ("kapila_ptmu", 2, 2): {"pass1_faces_x": (597, 99), "pass1_faces_y": (603, 100), "pass1_cells": (1290, 320),
                             "pass2_faces_x": (597, 100), "pass2_faces_y": (603, 100), "pass2_cells": (1291, 329)},
+    ("ptueq", 2, 2): {"pass1_faces_x": (476, 74), "pass1_faces_y": (481, 73), "pass1_cells": (248, 174),
+                      "pass2_faces_x": (476, 74), "pass2_faces_y": (481, 73), "pass2_cells": (247, 181)},
+    ("euler", 1, 2): {"pass1_faces_x": (226, 55), "pass1_faces_y": (229, 54), "pass1_cells": (73, 131),
+                      "pass2_faces_x": (226, 55), "pass2_faces_y": (229, 54), "pass2_cells": (72, 138)},
 }
 for (_m, _np, _d), _slots in _SPLIT_NCU.items():
     for _slot, (_fp, _dram) in _slots.items():
         NCU_TRAFFIC_PER_CELL[(_m, _np, _d, True, "split", _slot)] = float(_dram)
-# Batched tubes (2048 cases): predictor + corrector DRAM bytes per cell-update.
-NCU_BATCH_BYTES_PER_CELL_UPDATE = 98.05 + 157.17
+# Batched tubes (2048 cases): DRAM bytes per cell-update, face and cell kernel of the predictor and of the corrector.
+NCU_BATCH_BYTES_PER_CELL_UPDATE = 115 + 179 + 115 + 186
 
 
 class ClockSampler:

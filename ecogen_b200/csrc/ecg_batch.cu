@@ -26,8 +26,8 @@
 #include "ecg_internal.h"
 #include "ecg_kapila_split.cuh"
 
-// Resident threads per SM asked of the face kernel (registers 65536 / threads; 896: 72 registers, as the 2D
-// face kernels, whose code it shares).
+// Resident threads per SM asked of the face kernel, in whole blocks: 896 are 14 blocks of 64 or 7 of 128 threads (72
+// registers) and 3 of 256 (768 threads, 80 registers, the tile the autotuner picks on large batches).
 #ifndef ECG_BATCH_SM_THREADS
 #define ECG_BATCH_SM_THREADS 896
 #endif

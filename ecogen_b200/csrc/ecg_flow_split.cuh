@@ -296,7 +296,9 @@ cudaError_t launch_flow(const StepParams& P, const Geometry& G, const typename M
 template <class MD, int DIM>
 cudaError_t flow_pass(int pass, const StepParams& P, const Geometry& G, const typename MD::Eos& M, cudaStream_t s,
                       bool prepare) {
-  const bool vl = P.lim[0] == ECG_LIM_VANLEER;  // the limiter of the shipped workloads, compiled in
+  // the limiter of the shipped workloads, compiled in (measured at 2048^2, us per call, limiter at run time / compiled
+  // in: PTUEq 7446 / 7093, Euler 6037 / 5795); the others are read at run time by the same kernel
+  const bool vl = P.lim[0] == ECG_LIM_VANLEER;
   if (pass == PASS_O1) return launch_flow<MD, DIM, PASS_O1, -1>(P, G, M, s, prepare);
   if (pass == PASS_PRED)
     return vl ? launch_flow<MD, DIM, PASS_PRED, ECG_LIM_VANLEER>(P, G, M, s, prepare)

@@ -60,7 +60,10 @@ constexpr int eos_fast_types() {
   return NP == 2 ? eos_types_code<2>(ECG_EOS_SG, ECG_EOS_IG) : eos_types_code<3>(ECG_EOS_SG, ECG_EOS_IG, ECG_EOS_IG);
 }
 // ... and the limiter of the shipped workloads (van Leer in the two-phase cases, minmod in the
-// three-phase one), compiled into a further variant when all four limiter slots use it
+// three-phase one), compiled into a further variant when all four limiter slots use it: its faces limit each slope
+// once per cell (cell_slopes) and branch on no limiter.  Measured, us per call of mid-run states, limiters at run time /
+// compiled in: bubble 2048^2 12328 / 10620, 191 x 103 1611 / 1370, cavity 256^3 74922 / 57154, p-T-mu 1024^2
+// 6538 / 5983
 template <int NP>
 constexpr int eos_fast_limiter() {
   return NP == 2 ? ECG_LIM_VANLEER : ECG_LIM_MINMOD;

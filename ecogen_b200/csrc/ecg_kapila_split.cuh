@@ -7,13 +7,13 @@
 // HLLC branch wait at the barrier for the ones sampling a star state, and the kernel's code (one copy
 // of the face work per axis) is larger than the instruction cache.  The split form trades HBM
 // traffic, of which the pass uses a few percent, for latency:
-//   k_kapila_faces       one thread per face: stage the cells and the slopes of a block (one barrier), then reconstruct both sides and solve HLLC exactly as the
-//                        fused pass does, including the domain sides (non-reflecting: HLLC(cell, cell) in
+//   k_kapila_faces       one thread per face: stage the cells and the slopes of a block (a barrier after each), then
+//                        reconstruct both sides and solve HLLC exactly as the fused pass does, including the domain sides (non-reflecting: HLLC(cell, cell) in
 //                        the side's frame; symmetry: the reflecting flux of the MUSCL buffer cell), and
 //                        store the face flux (3N + d + 3 doubles) in a face array of the axis;
 //                        min-reduce lCFL/|s| into dtMax;
-//   k_kapila_cells       one thread per cell, no shared memory and no barrier but the counters': add
-//                        and subtract the stored fluxes in the reference's face order (X faces, Y faces,
+//   k_kapila_cells       one thread per cell, no barrier but the counters' (in 2D each thread copies the last
+//                        axis' fluxes, u and E ahead into shared slots of its own): add and subtract the stored fluxes in the reference's face order (X faces, Y faces,
 //                        Z faces, then sides Xm, Xp, Ym, Yp, Zm, Zp, src/Meshes/MeshCartesian.cpp:281-557)
 //                        with the same non-conservative terms, then buildPrim, relaxations, energy
 //                        correction and store (kapila_rebuild / kapila_finish).

@@ -338,7 +338,8 @@ ecg_status ecg_trainer_set_norm_out1(ecg_trainer* tr, float out_shift, float out
 
 /* ------------------------------------------------------------------ batched independent cases */
 /* Many independent 1D cases of uneven cell counts advanced together, two launches per pass over all of
- * them (face fluxes, cells); each case keeps its own dt
+ * them (face fluxes, cells; over one piece of the batch after another where the fluxes, 3N + 4 doubles
+ * per face, do not all fit the GPU's free memory); each case keeps its own dt
  * (segmented min-reduction) and time.  All cases must share model, phases, EOS, order and
  * limiters; their cell counts, lengths, CFL and initial states differ.  The reference runs such
  * cases one after another (src/main.cpp:82-133). */
